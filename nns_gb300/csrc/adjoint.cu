@@ -44,7 +44,7 @@ struct TapeStep {
     int *meta = nullptr, *parent = nullptr, *val = nullptr, *body_node = nullptr;
     float4 *body4 = nullptr;
     int *lists = nullptr, *list_len = nullptr;
-    unsigned *lvl = nullptr;  // BFS level starts (kMaxLevel + 2 entries)
+    unsigned *lvl = nullptr;  // [64] BFS level starts (past the deepest level: the node count)
 };
 
 struct Adj {
@@ -63,6 +63,7 @@ struct Adj {
     // saved context pointers (the tape steps are swapped in for recording)
     float4 *ctx_node4 = nullptr, *ctx_body4 = nullptr;
     int *ctx_meta = nullptr, *ctx_parent = nullptr, *ctx_val = nullptr, *ctx_body_node = nullptr;
+    unsigned *ctx_lvl_start = nullptr;
     float fwd_ms = 0.f, bwd_ms = 0.f;
     bool tail_taped = false;  // the forward recorded the last segment into the tape
     float *mass = nullptr;    // [n] the caller's masses, copied by the forward
@@ -472,15 +473,6 @@ __global__ void k_r64_loss(const double *r64, const float *target, int n, double
     if ((threadIdx.x & 31) == 0) atomicAdd(loss, acc);
 }
 
-__global__ void k_copy_lvl(const unsigned *hist, int ntiles, const unsigned *totals, unsigned *lvl) {
-    const int l = threadIdx.x;
-    if (l <= kMaxLevel + 1) {
-        const unsigned T = totals[1];
-        unsigned v = l >= 64 ? T : hist[(size_t)(l << 2) * ntiles];
-        lvl[l] = v < T ? v : T;
-    }
-}
-
 int grid_for(int n) {
     int g = ceil_div(n, kB);
     return g < 1 ? 1 : (g > 2048 ? 2048 : g);
@@ -494,6 +486,7 @@ void swap_in(Ctx *ctx, Adj *a, int j) {
     ctx->d_val = t.val;
     ctx->d_body_node = t.body_node;
     ctx->d_body4 = t.body4;
+    ctx->d_lvl_start = t.lvl;
 }
 
 // Back to the context's own node arrays.  Its per-build arrays (roots, cell
@@ -506,6 +499,7 @@ void swap_out(Ctx *ctx, Adj *a) {
     ctx->d_val = a->ctx_val;
     ctx->d_body_node = a->ctx_body_node;
     ctx->d_body4 = a->ctx_body4;
+    ctx->d_lvl_start = a->ctx_lvl_start;
 }
 
 template <typename T>
@@ -525,11 +519,7 @@ int amalloc(Ctx *ctx, Adj *a, T **p, size_t count) {
 int recorded_step(Ctx *ctx, Adj *a, const nbx_state *s, int j, cudaStream_t st) {
     swap_in(ctx, a, j);
     int rc = build_tree(ctx, s, st, false, nullptr);
-    if (!rc) {
-        k_copy_lvl<<<1, 64, 0, st>>>(ctx->d_hist, ctx->cap_tiles_node, ctx->d_totals, a->tape[j].lvl);
-        ++ctx->launches;
-        rc = walk2_record(ctx, s, a->tape[j].lists, a->tape[j].list_len, a->lcap, st);
-    }
+    if (!rc) rc = walk2_record(ctx, s, a->tape[j].lists, a->tape[j].list_len, a->lcap, st);
     if (!rc) rc = integrate(ctx, s, ctx->p.dt, ctx->p.dampening, a->n, st);
     swap_out(ctx, a);
     return rc;
@@ -668,7 +658,7 @@ int adjoint_create(Ctx *ctx, int T, int C, int lcap, int tape_steps, Adj **out) 
         rc |= amalloc(ctx, a, &t.body4, ctx->cap_bodies);
         rc |= amalloc(ctx, a, &t.lists, (size_t)a->ngroups * lcap);
         rc |= amalloc(ctx, a, &t.list_len, a->ngroups);
-        rc |= amalloc(ctx, a, &t.lvl, kMaxLevel + 2);
+        rc |= amalloc(ctx, a, &t.lvl, 64);
     }
     a->ctx_node4 = ctx->d_node4;
     a->ctx_meta = ctx->d_meta;
@@ -676,6 +666,7 @@ int adjoint_create(Ctx *ctx, int T, int C, int lcap, int tape_steps, Adj **out) 
     a->ctx_val = ctx->d_val;
     a->ctx_body_node = ctx->d_body_node;
     a->ctx_body4 = ctx->d_body4;
+    a->ctx_lvl_start = ctx->d_lvl_start;
     *out = a;
     return rc;
 }

@@ -106,9 +106,9 @@ void free_all(Ctx *ctx) {
                     ctx->d_bbox_u, ctx->d_bbox, ctx->d_bbox64, ctx->d_depth0, ctx->d_root_first, ctx->d_sys_lvl,
                     ctx->d_root_nch, ctx->d_key, ctx->d_key_alt, ctx->d_key_lo, ctx->d_val, ctx->d_val_alt,
                     ctx->d_body4, ctx->d_delta, ctx->d_bucket, ctx->d_ecount, ctx->d_body_node, ctx->d_gstat,
-                    ctx->d_ent, ctx->d_ent_alt, ctx->d_flags, ctx->d_node4, ctx->d_meta, ctx->d_parent,
-                    ctx->d_sums, ctx->d_count, ctx->d_arrive, ctx->d_lvl8, ctx->d_fcl, ctx->d_cl, ctx->d_hist,
-                    ctx->d_scan_blk, ctx->d_totals, ctx->d_totals64, ctx->d_status, ctx->d_m2, ctx->d_quad4,
+                    ctx->d_ent, ctx->d_lvl_counts, ctx->d_lvl_tot, ctx->d_lvl_start, ctx->d_node4, ctx->d_meta, ctx->d_parent,
+                    ctx->d_sums, ctx->d_count, ctx->d_arrive, ctx->d_lvl8, ctx->d_hist,
+                    ctx->d_scan_blk, ctx->d_totals, ctx->d_totals64, ctx->d_status, ctx->d_m2, ctx->d_com, ctx->d_quad4,
                     ctx->d_quad2, ctx->d_seg_slot, ctx->d_lb_counts, ctx->d_lb_status, ctx->d_lb, ctx->d_tiles_sw,
                     ctx->d_sys_tiles_sw};
     for (void *p : ptrs)
@@ -152,13 +152,16 @@ int alloc_quadrupoles(Ctx *ctx) {
     if (ctx->d_m2) return NBX_OK;
     const size_t nc = (size_t)ctx->cap_nodes;
     int rc = dmalloc(ctx, &ctx->d_m2, 3 * nc);
+    if (rc == 0) rc = dmalloc(ctx, &ctx->d_com, 3 * nc);
     if (rc == 0) rc = dmalloc(ctx, &ctx->d_quad4, nc);
     if (rc == 0) rc = dmalloc(ctx, &ctx->d_quad2, nc);
     if (rc) {
         cudaFree(ctx->d_m2);
+        cudaFree(ctx->d_com);
         cudaFree(ctx->d_quad4);
         cudaFree(ctx->d_quad2);
         ctx->d_m2 = nullptr;
+        ctx->d_com = nullptr;
         ctx->d_quad4 = nullptr;
         ctx->d_quad2 = nullptr;
     }
@@ -279,13 +282,8 @@ int nbx_create(const nbx_params *p, nbx_ctx **out) {
     // no tile is smaller than kTileMin: a small context never needs more tiles than this
     const int64_t most_tiles = (int64_t)B / nbx::kTileMin + Ss + 1;
     if (most_tiles < ctx->cap_tiles_body) ctx->cap_tiles_body = (int)most_tiles;
-    ctx->tile_node = nbx::tile_for(ctx->cap_nodes, ctx->nsm);
-    ctx->cap_tiles_node = nbx::ceil_div(ctx->cap_nodes, ctx->tile_node);
-    const int64_t hist = (1ll << nbx::kMaxRadixBits) * (ctx->cap_tiles_body > ctx->cap_tiles_node ? ctx->cap_tiles_body : ctx->cap_tiles_node);
-    int64_t scan_max = hist;
-    if (ctx->cap_nodes > scan_max) scan_max = ctx->cap_nodes;
-    if (B > scan_max) scan_max = B;
-    ctx->cap_scan_blk = nbx::ceil_div(scan_max, nbx::kScanItems) + 1;
+    const int64_t hist = (1ll << nbx::kMaxRadixBits) * ctx->cap_tiles_body;
+    ctx->cap_scan_blk = nbx::ceil_div(hist, nbx::kScanItems) + 1;
     const int NC = ctx->cap_nodes;
     const int G = B / 32 + Ss + 1;
     int rc = 0;
@@ -316,8 +314,6 @@ int nbx_create(const nbx_params *p, nbx_ctx **out) {
     rc |= nbx::dmalloc(ctx, &ctx->d_body_node, B);
     rc |= nbx::dmalloc(ctx, &ctx->d_gstat, G);
     rc |= nbx::dmalloc(ctx, &ctx->d_ent, NC);
-    rc |= nbx::dmalloc(ctx, &ctx->d_ent_alt, NC);
-    rc |= nbx::dmalloc(ctx, &ctx->d_flags, NC);
     rc |= nbx::dmalloc(ctx, &ctx->d_node4, NC);
     rc |= nbx::dmalloc(ctx, &ctx->d_meta, NC);
     rc |= nbx::dmalloc(ctx, &ctx->d_parent, NC);
@@ -325,8 +321,9 @@ int nbx_create(const nbx_params *p, nbx_ctx **out) {
     rc |= nbx::dmalloc(ctx, &ctx->d_count, NC);
     rc |= nbx::dmalloc(ctx, &ctx->d_arrive, NC);
     rc |= nbx::dmalloc(ctx, &ctx->d_lvl8, NC);
-    rc |= nbx::dmalloc(ctx, &ctx->d_fcl, (size_t)NC + Ss + 2);
-    rc |= nbx::dmalloc(ctx, &ctx->d_cl, (size_t)NC + Ss + 2);
+    rc |= nbx::dmalloc(ctx, &ctx->d_lvl_counts, 64 * (size_t)nbx::ceil_div(B, nbx::kPosBlock));
+    rc |= nbx::dmalloc(ctx, &ctx->d_lvl_tot, 64);
+    rc |= nbx::dmalloc(ctx, &ctx->d_lvl_start, 64);
     rc |= nbx::dmalloc(ctx, &ctx->d_hist, hist + 1);  // + the scanned total
     // one-sweep body sort: a system of several tiles takes at least two, so at most
     // half the tiles (plus one) hold count slots; status words per tile and digit

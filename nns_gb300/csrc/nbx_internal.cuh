@@ -45,6 +45,7 @@ constexpr int kMaxLevel = 43;     // 42 key levels + the body level
 constexpr int kBodyFlag = int(0x80000000u);
 constexpr int kLevelShift = 26;   // build node entry = level << 26 | sorted position
 constexpr int kMaxNodes = 1 << 28; // cells + bodies: meta's first-child field has 28 bits
+constexpr int kPosBlock = 512;    // sorted positions per block of the node kernels (k_delta, k_bucket, k_nodes)
 constexpr int kScanItems = 4096;  // elements per scan block (1024 threads x 4)
 constexpr int kMaxRun = 4096;     // longest run of equal 21-level keys refined
 
@@ -74,8 +75,8 @@ struct Ctx {
     std::string last_error;
 
     // capacity
-    int cap_bodies, cap_sys, cap_nodes, cap_tiles_body, cap_tiles_node;
-    int tile_body = kTile, tile_node = kTile;  // radix tile sizes (tile_for)
+    int cap_bodies, cap_sys, cap_nodes, cap_tiles_body;
+    int tile_body = kTile; // radix tile size (tile_for)
     int nsm = 152;         // multiprocessors of the device
     int smem_optin = 0;    // shared memory per block (opt-in maximum)
     long long launches = 0;  // kernels launched by this context
@@ -113,13 +114,12 @@ struct Ctx {
     float4 *d_body4 = nullptr;   // [B] sorted bodies (x,y,z,m)
     unsigned char *d_delta = nullptr;  // [B]
     unsigned char *d_bucket = nullptr; // [B] leaf buckets: level of the bucket cell of each sorted position
-    unsigned *d_ecount = nullptr;      // [B] entries per position -> exclusive offsets
+    unsigned *d_ecount = nullptr;      // [B] node entries before each position (depth-first pre-order)
     int *d_body_node = nullptr;        // [B] node of sorted position
     int2 *d_gstat = nullptr;           // [G] per walk group: list length, opened cells (last walk)
 
     // per node (entry / BFS order)
-    unsigned *d_ent = nullptr, *d_ent_alt = nullptr;  // [NC] packed level<<26 | position
-    unsigned long long *d_flags = nullptr;            // [NC] cell<<32 | first-child
+    unsigned *d_ent = nullptr;                        // [NC] packed level<<26 | position
     float4 *d_node4 = nullptr;                        // [NC]
     int *d_meta = nullptr;                            // [NC]
     int *d_parent = nullptr;                          // [NC]
@@ -129,10 +129,12 @@ struct Ctx {
     unsigned char *d_lvl8 = nullptr;                  // [NC] tree level of each node (root children: 1)
     double2 *d_m2 = nullptr;       // [3 NC] quadrupole mode: FP64 second moments about the cell's centre of
                                    // mass, (xx, yy) (zz, xy) (xz, yz)
+    double *d_com = nullptr;       // [3 NC] quadrupole mode: FP64 centres of mass of cells
     float4 *d_quad4 = nullptr;     // [NC] quadrupole mode: P = -Q (Q traceless) of cells in FP32, (xx, yy, zz, xy)
     float2 *d_quad2 = nullptr;     // [NC]                                              (xz, yz)
-    int *d_fcl = nullptr;                             // [NC+S+1] first-child list
-    int *d_cl = nullptr;                              // [NC+S] cell list (BFS index)
+    unsigned *d_lvl_counts = nullptr;                 // [position blocks][64] nodes per level
+    unsigned *d_lvl_tot = nullptr;                    // [64] nodes of each level
+    unsigned *d_lvl_start = nullptr;                  // [64] first node of each level (past the deepest: the node count)
 
     // radix + scan scratch
     unsigned *d_hist = nullptr;        // [2^kMaxRadixBits * max(tiles)]
@@ -140,7 +142,7 @@ struct Ctx {
     unsigned long long *d_lb_status = nullptr;  // [tiles][2^kMaxRadixBits] look-back status words
     unsigned *d_lb = nullptr;          // [16] build counter, next tile of each pass
     unsigned long long *d_scan_blk = nullptr;  // block sums
-    unsigned *d_totals = nullptr;      // [8] device-side totals: 0 entries, 1 cells+first..., etc
+    unsigned *d_totals = nullptr;      // [8] 0 nodes of the tree, 1 nodes in use (0 when they exceed the pool)
     unsigned long long *d_totals64 = nullptr;
     int cap_scan_blk = 0;
 
@@ -212,11 +214,8 @@ __device__ __forceinline__ int digit_of(unsigned long long hi, unsigned long lon
 // scan.cu
 int scan_exclusive_u32(Ctx *ctx, const unsigned *in, unsigned *out, int n_cap,
                        const unsigned *n_dev, unsigned *total_out, cudaStream_t st);
-int scan_exclusive_u64(Ctx *ctx, const unsigned long long *in, unsigned long long *out, int n_cap,
-                       const unsigned *n_dev, unsigned long long *total_out, cudaStream_t st);
 // radix.cu
 int radix_sort_bodies(Ctx *ctx, cudaStream_t st);
-int radix_sort_entries(Ctx *ctx, cudaStream_t st);
 int radix_init(Ctx *ctx);
 int radix_selftest_wait(Ctx *ctx, cudaStream_t st);
 // tree.cu

@@ -529,24 +529,6 @@ int radix_sort_bodies(Ctx *ctx, cudaStream_t st) {
     return ctx->radix_bits == 9 ? sort_bodies<9>(ctx, st) : sort_bodies<8>(ctx, st);
 }
 
-// Stable sort of the node entries (level << 26 | position) by level: one pass
-// on bits 24..31, which orders by level and keeps position order within a
-// level.  Input d_ent, output d_ent_alt; the element count is on the device.
-int radix_sort_entries(Ctx *ctx, cudaStream_t st) {
-    const int nt = ctx->cap_tiles_node;
-    TileMap tm{nullptr, nullptr, &ctx->d_totals[1], nt, ctx->tile_node};  // clamped node count (0 on overflow)
-    const int grid = ceil_div(nt, kWarpsPerBlock);
-    const int nh = nt * 256;
-    k_radix_hist<unsigned, false, 8><<<grid, kWarpsPerBlock * 32, 0, st>>>(ctx->d_ent, tm, 24, ctx->d_hist);
-    ++ctx->launches;
-    int rc = scan_exclusive_u32(ctx, ctx->d_hist, ctx->d_hist, nh, nullptr, ctx->d_hist + nh, st);
-    if (rc) return rc;
-    launch_scatter<unsigned, int, false, 8>(ctx, nt, ctx->d_ent, ctx->d_ent_alt, (const int *)nullptr, (int *)nullptr,
-                                         tm, 24, st);
-    NBX_CUDA(cudaGetLastError());
-    return NBX_OK;
-}
-
 // Self-test of the one-sweep pass's bounded wait (nbx_selftest_sort_wait): a
 // system of two 256-key tiles on scratch of its own, whose tile counter starts
 // at 1, so the one block takes the second tile, publishes its counts and waits
@@ -598,8 +580,6 @@ int radix_init(Ctx *ctx) {
     NBX_CUDA(cudaFuncSetAttribute(k_radix_scatter<unsigned long long, int, true, 9>,
                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)stage_bytes<unsigned long long, int, 9>(kTile)));
-    NBX_CUDA(cudaFuncSetAttribute(k_radix_scatter<unsigned, int, false, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)stage_bytes<unsigned, int, 8>(kTile)));
     NBX_CUDA(cudaFuncSetAttribute(k_radix_scatter<unsigned long long, int, true, 8, true>,
                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)stage_bytes<unsigned long long, int, 8, true>(kTile)));

@@ -168,9 +168,4 @@ int scan_exclusive_u32(Ctx *ctx, const unsigned *in, unsigned *out, int n_cap,
     return scan_impl<unsigned>(ctx, in, out, n_cap, n_dev, total_out, st);
 }
 
-int scan_exclusive_u64(Ctx *ctx, const unsigned long long *in, unsigned long long *out, int n_cap,
-                       const unsigned *n_dev, unsigned long long *total_out, cudaStream_t st) {
-    return scan_impl<unsigned long long>(ctx, in, out, n_cap, n_dev, total_out, st);
-}
-
 }  // namespace nbx

@@ -14,13 +14,15 @@
 //           position a iff delta(a-1) < L <= delta(a); the body at position i sits
 //           at level max(delta(i-1), delta(i)) + 1.  Position i therefore owns the
 //           node levels lo..hi = delta(i-1)+1 .. max(delta(i-1),delta(i))+1.
-//  nodes    entries (level, position) generated in position order are the
-//           depth-first pre-order; a stable sort by level gives breadth-first
-//           order, in which the children of every cell are contiguous.
-//  links    a node is the first child of its parent iff the parent starts at the
-//           same position.  The k-th first child in BFS order belongs to the k-th
-//           cell in BFS order (roots first), so two prefix counts give every cell's
-//           child block and every node's parent -- no search, no locks.
+//  nodes    in breadth-first order a node's index is the start of its level plus
+//           the number of that level's nodes at earlier positions, so per-block
+//           counts of the nodes of every level (k_delta) give every index without
+//           materialising and sorting the entries.
+//  links    a cell (level l, position p) has its first child at (l + 1, p); the
+//           topmost node of a position that shares levels with its predecessor
+//           is a later child of the last level-(lo-1) node before it.  Both are
+//           ranks in their levels, so the thread of p links its nodes by itself
+//           (k_nodes) -- no search, no locks, no sort.
 //  moments  bottom-up FP64 sums in child order, deterministic: one BFS level
 //           per launch, deepest first, or for small systems one launch in
 //           which the last child to finish sums its parent.
@@ -35,14 +37,23 @@ constexpr int kBlock = 256;
 #define NBX_MOMENTS_UP_MAX (1 << 21)
 #endif
 constexpr int kMomentsUpMaxBodies = NBX_MOMENTS_UP_MAX;  // one-launch moments up to this many bodies
+constexpr int kUpRounds = 4;    // largest number of 32-node rounds a warp of k_moments_up lists at once
+constexpr int kLvlRow = 64;     // per-block counts of levels 0 .. kMaxLevel, padded to a row
+static_assert(kLvlRow > kMaxLevel, "a row holds every level");
+// k_nodes sums the earlier blocks' counts itself up to this many blocks: every
+// block reads all rows, which beyond costs more than the scan's launch
+constexpr int kDirectBlocks = 256;
 
 __device__ __forceinline__ int grid_stride_start() { return blockIdx.x * blockDim.x + threadIdx.x; }
 __device__ __forceinline__ int grid_stride() { return gridDim.x * blockDim.x; }
 
-__global__ void k_step_reset(unsigned *bbox_u, int nsys, DevStatus *st, int *sys_lvl) {
+__global__ void k_step_reset(unsigned *bbox_u, int nsys, DevStatus *st, int *sys_lvl, int *root_nch) {
     int i = grid_stride_start();
     if (i < 6 * nsys) bbox_u[i] = f2ord(0.0f);  // Kernels.cu:56-62: the box contains the origin
-    if (i < nsys) sys_lvl[i] = 0;
+    if (i < nsys) {
+        sys_lvl[i] = 0;
+        root_nch[i] = 0;  // k_nodes counts the root children up
+    }
     if (i == 0) {
         st->refined_runs = 0;
         st->max_level = 0;
@@ -169,15 +180,18 @@ __device__ __forceinline__ unsigned long long make_key(float px, float py, float
 }
 
 // Also packs the bodies as float4 (x, y, z, m) in their original order, so that
-// the gather into sorted order reads one 16-byte record per body.
+// the gather into sorted order reads one 16-byte record per body, and zeroes the
+// node records' meta words, which k_nodes adds up.
 __global__ void __launch_bounds__(kBlock) k_keys(const float *__restrict__ x, const float *__restrict__ y,
                                                   const float *__restrict__ z, const float *__restrict__ m,
                                                   const int *__restrict__ body_sys,
                                                   const float *__restrict__ bbox, int n,
                                                   unsigned long long *__restrict__ key, int *__restrict__ val,
-                                                  float4 *__restrict__ pos4, DevStatus *st, int order) {
+                                                  float4 *__restrict__ pos4, DevStatus *st, int order,
+                                                  int *__restrict__ meta, int cap_nodes) {
     __shared__ unsigned char ht[96];
     load_hilbert(ht, order);
+    for (int i = grid_stride_start(); i < cap_nodes; i += grid_stride()) meta[i] = 0;
     for (int i = grid_stride_start(); i < n; i += grid_stride()) {
         const float px = x[i], py = y[i], pz = z[i];
         pos4[i] = make_float4(px, py, pz, m[i]);
@@ -254,34 +268,6 @@ __device__ __forceinline__ int delta_of(const unsigned long long *key, const uns
     return d > 41 ? 41 : d;  // equal 42-level keys were reported as NBX_ERR_DEPTH
 }
 
-// Sorted bodies as float4 plus delta and the number of node entries per position.
-__global__ void __launch_bounds__(kBlock) k_delta(const float4 *__restrict__ pos4,
-                                                   const int *__restrict__ body_sys, const int *__restrict__ sys_off,
-                                                   int n, const unsigned long long *__restrict__ key,
-                                                   const unsigned long long *__restrict__ key_lo,
-                                                   const int *__restrict__ val, float4 *__restrict__ body4,
-                                                   unsigned char *__restrict__ delta,
-                                                   unsigned *__restrict__ ecount, DevStatus *st,
-                                                   int *__restrict__ sys_lvl) {
-    int lvl_max = 0;
-    for (int p = grid_stride_start(); p < n; p += grid_stride()) {
-        const int s = body_sys[p];
-        const int beg = sys_off[s], end = sys_off[s + 1];
-        const int di = p + 1 < end ? delta_of(key, key_lo, p) : 0;
-        const int dp = p > beg ? delta_of(key, key_lo, p - 1) : 0;
-        delta[p] = (unsigned char)di;
-        ecount[p] = (unsigned)((di > dp ? di - dp : 0) + 1);
-        body4[p] = pos4[val[p]];
-        const int lv = max(di, dp) + 1;
-        lvl_max = max(lvl_max, lv);
-        // each system's deepest level (the walk's depth-first reserve of its
-        // groups); the L2 read skips the atomic for all but the few new maxima
-        if (lv > __ldcg(&sys_lvl[s])) atomicMax(&sys_lvl[s], lv);
-    }
-    lvl_max = __reduce_max_sync(0xffffffffu, lvl_max);
-    if ((threadIdx.x & 31) == 0 && lvl_max > 0) atomicMax(&st->max_level, lvl_max);
-}
-
 // Node levels owned by sorted position p: the cells starting at p (levels
 // lo..hi-1) and the body (level hi).  With leaf buckets (bucket != nullptr) the
 // body hangs directly below its bucket cell (level bucket[p]): deeper cells
@@ -298,17 +284,73 @@ __device__ __forceinline__ void levels_of(const unsigned char *delta, const unsi
     }
 }
 
+// The nodes of every level among a block's kPosBlock positions, stored
+// [block][level] in rows of kLvlRow.  Lanes without a position pass lo > hi.
+__device__ __forceinline__ void count_levels(int lo, int hi, unsigned *cnt, unsigned *__restrict__ counts) {
+    for (int l = threadIdx.x; l < kLvlRow; l += blockDim.x) cnt[l] = 0u;
+    __syncthreads();
+    const int a = __reduce_min_sync(0xffffffffu, lo <= hi ? lo : kLvlRow);
+    const int b = __reduce_max_sync(0xffffffffu, lo <= hi ? hi : 0);
+    for (int l = a; l <= b; l++) {
+        const unsigned m = __ballot_sync(0xffffffffu, lo <= l && l <= hi);
+        if ((threadIdx.x & 31) == 0 && m) atomicAdd(&cnt[l], (unsigned)__popc(m));
+    }
+    __syncthreads();
+    for (int l = threadIdx.x; l < kLvlRow; l += blockDim.x) counts[(size_t)blockIdx.x * kLvlRow + l] = cnt[l];
+}
+
+// Sorted bodies as float4 plus delta and (without leaf buckets) the block's
+// nodes per level.  One position per thread.
+__global__ void __launch_bounds__(kPosBlock) k_delta(const float4 *__restrict__ pos4,
+                                                      const int *__restrict__ body_sys,
+                                                      const int *__restrict__ sys_off, int n,
+                                                      const unsigned long long *__restrict__ key,
+                                                      const unsigned long long *__restrict__ key_lo,
+                                                      const int *__restrict__ val, float4 *__restrict__ body4,
+                                                      unsigned char *__restrict__ delta,
+                                                      unsigned *__restrict__ counts, DevStatus *st,
+                                                      int *__restrict__ sys_lvl) {
+    __shared__ unsigned cnt[kLvlRow];
+    const int p = blockIdx.x * kPosBlock + threadIdx.x;
+    int lo = 1, hi = 0, s = -1;
+    if (p < n) {
+        s = body_sys[p];
+        const int beg = sys_off[s], end = sys_off[s + 1];
+        body4[p] = pos4[val[p]];
+        const int di = p + 1 < end ? delta_of(key, key_lo, p) : 0;
+        const int dp = p > beg ? delta_of(key, key_lo, p - 1) : 0;
+        delta[p] = (unsigned char)di;
+        lo = dp + 1;
+        hi = max(di, dp) + 1;
+    }
+    // each system's deepest level (the walk's depth-first reserve of its groups):
+    // one atomic per warp where the warp lies in one system, and none where the
+    // L2 copy is no smaller (an atomic per body on one word took 13 us of a
+    // 16384-body k_delta and 29 us of a 65536-body one)
+    const int lvl_max = __reduce_max_sync(0xffffffffu, hi);
+    const bool one = __all_sync(0xffffffffu, s == __shfl_sync(0xffffffffu, s, 0) || s < 0);
+    const int lv = one ? lvl_max : hi;
+    if (s >= 0 && (!one || (threadIdx.x & 31) == 0) && lv > __ldcg(&sys_lvl[s])) atomicMax(&sys_lvl[s], lv);
+    if ((threadIdx.x & 31) == 0 && lvl_max > __ldcg(&st->max_level)) atomicMax(&st->max_level, lvl_max);
+    if (counts) count_levels(lo, hi, cnt, counts);
+}
+
 // Leaf buckets (nbx_params.leaf_size k > 1; not the reference's tree, which has
 // one body per leaf): the bucket of a body is the shallowest cell around it
 // holding at most k bodies.  The cell at level L around p holds more than k
 // bodies exactly when some window of k+1 consecutive positions of the system
 // containing p shares at least L levels, i.e. all k deltas inside the window
 // are >= L; so the bucket level is 1 + the largest inner-delta minimum over
-// those windows.  Rewrites the node entries per position accordingly.
-__global__ void __launch_bounds__(kBlock) k_bucket(const int *__restrict__ body_sys, const int *__restrict__ sys_off,
-                                                    int n, int k, const unsigned char *__restrict__ delta,
-                                                    unsigned char *__restrict__ bucket, unsigned *__restrict__ ecount) {
-    for (int p = grid_stride_start(); p < n; p += grid_stride()) {
+// those windows.  Counts the nodes per level accordingly.
+__global__ void __launch_bounds__(kPosBlock) k_bucket(const int *__restrict__ body_sys,
+                                                       const int *__restrict__ sys_off, int n, int k,
+                                                       const unsigned char *__restrict__ delta,
+                                                       unsigned char *__restrict__ bucket,
+                                                       unsigned *__restrict__ counts) {
+    __shared__ unsigned cnt[kLvlRow];
+    const int p = blockIdx.x * kPosBlock + threadIdx.x;
+    int lo = 1, hi = 0;
+    if (p < n) {
         const int s = body_sys[p];
         const int beg = sys_off[s], end = sys_off[s + 1];
         int best = 0;
@@ -318,143 +360,274 @@ __global__ void __launch_bounds__(kBlock) k_bucket(const int *__restrict__ body_
             best = max(best, mn);
         }
         bucket[p] = (unsigned char)(best + 1);
-        int lo, hi, dp;
+        int dp;
         levels_of(delta, bucket, p, beg, lo, hi, dp);
-        ecount[p] = (unsigned)(hi - lo + 1);
     }
+    count_levels(lo, hi, cnt, counts);
 }
 
-// Node entries (level << 26 | position) in position order = depth-first pre-order.
-__global__ void __launch_bounds__(kBlock) k_entries(const int *__restrict__ body_sys,
-                                                     const int *__restrict__ sys_off, int n,
-                                                     const unsigned char *__restrict__ delta,
-                                                     const unsigned char *__restrict__ bucket,
-                                                     const unsigned *__restrict__ eoff, unsigned *totals,
-                                                     int cap_nodes, unsigned *__restrict__ ent,
-                                                     DevStatus *st) {
-    if (grid_stride_start() == 0) {
-        unsigned T = totals[0];
-        if (T > (unsigned)cap_nodes) {
-            set_status(st, NBX_ERR_CAPACITY, (int)min(T, 0x7fffffffu));
-            T = 0u;  // nothing downstream reads a partial entry list
+// Exclusive scan of every level's counts over the blocks (one block per level),
+// in place; the level's total goes to totals[level].
+__global__ void __launch_bounds__(1024) k_level_scan(unsigned *__restrict__ counts, int nblk,
+                                                      unsigned *__restrict__ totals) {
+    constexpr int kPer = 8;
+    __shared__ unsigned wt[32];
+    const int l = blockIdx.x, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    unsigned carry = 0;
+    for (int b0 = 0; b0 < nblk; b0 += 1024 * kPer) {
+        const int base = b0 + kPer * (int)threadIdx.x;
+        unsigned v[kPer], s = 0;
+#pragma unroll
+        for (int k = 0; k < kPer; k++) {
+            v[k] = base + k < nblk ? counts[(size_t)(base + k) * kLvlRow + l] : 0u;
+            s += v[k];
         }
-        totals[1] = T;  // node count used downstream
+        unsigned incl = s;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned u = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += u;
+        }
+        if (lane == 31) wt[w] = incl;
+        __syncthreads();
+        if (w == 0) {
+            unsigned t = wt[lane];
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const unsigned u = __shfl_up_sync(0xffffffffu, t, o);
+                if (lane >= o) t += u;
+            }
+            wt[lane] = t;
+        }
+        __syncthreads();
+        unsigned run = carry + (w ? wt[w - 1] : 0u) + incl - s;
+#pragma unroll
+        for (int k = 0; k < kPer; k++) {
+            if (base + k < nblk) counts[(size_t)(base + k) * kLvlRow + l] = run;
+            run += v[k];
+        }
+        carry += wt[31];
+        __syncthreads();
     }
-    for (int p = grid_stride_start(); p < n; p += grid_stride()) {
-        const int beg = sys_off[body_sys[p]];
-        int lo, hi, dp;
+    if (threadIdx.x == 0) totals[l] = carry;
+}
+
+// Writes every node of the tree in breadth-first order, one position per
+// thread.  The block's base in every level comes from the scanned counts, or
+// (Direct, up to kDirectBlocks blocks) from a sum over the earlier blocks' raw
+// counts, which saves the scan's launch; ranks inside the block are ballots.
+// A cell's meta (first child, children - 1) is gathered by atomic adds on a
+// zeroed word: its own thread adds the first child, every later child's thread
+// adds one to the count.  Bound by its scattered writes; DRAM at large sizes.
+template <bool Direct>
+__global__ void __launch_bounds__(kPosBlock) k_nodes(const int *__restrict__ body_sys,
+                                                      const int *__restrict__ sys_off, int n,
+                                                      const unsigned char *__restrict__ delta,
+                                                      const unsigned char *__restrict__ bucket,
+                                                      const unsigned *__restrict__ counts, int nblk,
+                                                      const unsigned *__restrict__ lvl_tot, int cap_nodes,
+                                                      const float4 *__restrict__ body4, unsigned *__restrict__ totals,
+                                                      unsigned long long *__restrict__ totals64,
+                                                      unsigned *__restrict__ lvl_start, unsigned *__restrict__ eoff,
+                                                      unsigned *__restrict__ ent, float4 *__restrict__ node4,
+                                                      int *__restrict__ meta, int *__restrict__ parent,
+                                                      int *__restrict__ body_node, int *__restrict__ count,
+                                                      int *__restrict__ arrive, unsigned char *__restrict__ lvl8,
+                                                      int *__restrict__ root_first, int *__restrict__ root_nch,
+                                                      DevStatus *st) {
+    constexpr int kWarps = kPosBlock / 32, kRows = kPosBlock / kLvlRow;
+    __shared__ unsigned part[2][kRows][kLvlRow];  // Direct: partial sums (all blocks, earlier blocks)
+    __shared__ unsigned base[kLvlRow];            // index of the block's first node of each level
+    __shared__ unsigned wcnt[kWarps][kLvlRow];    // nodes per warp and level, then the warps' bases
+    __shared__ unsigned went[kWarps];             // entries per warp
+    __shared__ unsigned s_T, s_ebase;
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const unsigned lt = (1u << lane) - 1u;
+    const int p = blockIdx.x * kPosBlock + threadIdx.x;
+    int lo = 1, hi = 0, dp = 0, s = 0, beg = 0;
+    if (p < n) {
+        s = body_sys[p];
+        beg = sys_off[s];
         levels_of(delta, bucket, p, beg, lo, hi, dp);
-        const unsigned e = eoff[p];
-        if (e + (unsigned)(hi - lo + 1) > (unsigned)cap_nodes) continue;
-        for (int l = lo; l <= hi; l++) ent[e + (l - lo)] = ((unsigned)l << kLevelShift) | (unsigned)p;
     }
-}
-
-__device__ __forceinline__ void node_kind(unsigned u, const int *body_sys, const int *sys_off,
-                                          const unsigned char *delta, const unsigned char *bucket, int &p, int &l,
-                                          bool &is_cell, bool &first) {
-    l = (int)(u >> kLevelShift);
-    p = (int)(u & ((1u << kLevelShift) - 1u));
-    const int beg = sys_off[body_sys[p]];
-    int lo, hi, dp;
-    levels_of(delta, bucket, p, beg, lo, hi, dp);
-    is_cell = l < hi;
-    first = (l == 1) ? (p == beg) : (dp < l - 1);
-}
-
-__global__ void __launch_bounds__(kBlock) k_node_flags(const unsigned *__restrict__ ent_bfs,
-                                                        const unsigned *__restrict__ totals,
-                                                        const int *__restrict__ body_sys,
-                                                        const int *__restrict__ sys_off,
-                                                        const unsigned char *__restrict__ delta,
-                                                     const unsigned char *__restrict__ bucket,
-                                                        unsigned long long *__restrict__ flags) {
-    const int T = (int)totals[1];
-    for (int b = grid_stride_start(); b < T; b += grid_stride()) {
-        int p, l;
-        bool c, f;
-        node_kind(ent_bfs[b], body_sys, sys_off, delta, bucket, p, l, c, f);
-        flags[b] = ((unsigned long long)c << 32) | (unsigned long long)f;
+    // nodes and entries per warp
+    const int wlo = __reduce_min_sync(0xffffffffu, lo <= hi ? lo : kLvlRow);
+    const int whi = __reduce_max_sync(0xffffffffu, hi);
+    wcnt[w][lane] = 0u;
+    wcnt[w][lane + 32] = 0u;
+    __syncwarp();
+    for (int l = wlo; l <= whi; l++) {
+        const unsigned m = __ballot_sync(0xffffffffu, lo <= l && l <= hi);
+        if (lane == 0) wcnt[w][l] = __popc(m);
     }
-}
-
-__global__ void __launch_bounds__(kBlock) k_nodes_a(const unsigned *__restrict__ ent_bfs,
-                                                     const unsigned *__restrict__ totals,
-                                                     const unsigned long long *__restrict__ totals64,
-                                                     const int *__restrict__ body_sys,
-                                                     const int *__restrict__ sys_off,
-                                                     const unsigned char *__restrict__ delta,
-                                                     const unsigned char *__restrict__ bucket,
-                                                     const unsigned long long *__restrict__ flags_ex,
-                                                     const float4 *__restrict__ body4, int nsys,
-                                                     int *__restrict__ fcl, int *__restrict__ cl,
-                                                     float4 *__restrict__ node4, int *__restrict__ meta,
-                                                     int *__restrict__ body_node, int *__restrict__ count,
-                                                     int *__restrict__ arrive, unsigned char *__restrict__ lvl8,
-                                                     DevStatus *st) {
-    const int T = (int)totals[1];
-    if (grid_stride_start() == 0) {
-        const unsigned long long tot = totals64[0];
-        const int ncell = (int)(tot >> 32), nfirst = (int)(tot & 0xffffffffull);
-        if (nfirst != nsys + ncell && st->code == 0) set_status(st, NBX_ERR_STATE, nfirst);
-        fcl[nsys + ncell] = T;
+    const unsigned ne = (unsigned)(hi - lo + 1);
+    unsigned einc = ne;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned u = __shfl_up_sync(0xffffffffu, einc, o);
+        if (lane >= o) einc += u;
     }
-    for (int b = grid_stride_start(); b < T; b += grid_stride()) {
-        int p, l;
-        bool c, f;
-        node_kind(ent_bfs[b], body_sys, sys_off, delta, bucket, p, l, c, f);
-        const unsigned long long ex = flags_ex[b];
-        if (f) fcl[(int)(ex & 0xffffffffull)] = b;
-        arrive[b] = 0;
-        lvl8[b] = (unsigned char)l;
-        if (c) {
-            cl[nsys + (int)(ex >> 32)] = b;
-        } else {
-            node4[b] = body4[p];
-            meta[b] = kBodyFlag | p;
-            body_node[p] = b;
-            count[b] = 1;
+    if (lane == 31) went[w] = einc;
+    // the level totals and the counts of the blocks before
+    if (Direct) {
+        const int l = threadIdx.x & (kLvlRow - 1), r = threadIdx.x / kLvlRow;
+        unsigned all = 0, before = 0;
+#pragma unroll 4
+        for (int b = r; b < nblk; b += kRows) {
+            const unsigned c = counts[(size_t)b * kLvlRow + l];
+            all += c;
+            if (b < (int)blockIdx.x) before += c;
         }
+        part[0][r][l] = all;
+        part[1][r][l] = before;
     }
-}
-
-__global__ void __launch_bounds__(kBlock) k_nodes_b(const unsigned *__restrict__ ent_bfs,
-                                                     const unsigned *__restrict__ totals,
-                                                     const int *__restrict__ body_sys,
-                                                     const int *__restrict__ sys_off,
-                                                     const unsigned char *__restrict__ delta,
-                                                     const unsigned char *__restrict__ bucket,
-                                                     const unsigned long long *__restrict__ flags_ex,
-                                                     int nsys, const int *__restrict__ fcl,
-                                                     const int *__restrict__ cl, int *__restrict__ meta,
-                                                     int *__restrict__ parent, int *__restrict__ root_first,
-                                                     int *__restrict__ root_nch, DevStatus *st) {
-    const int T = (int)totals[1];
-    for (int s = grid_stride_start(); s < nsys; s += grid_stride()) {
-        const bool ok = st->code == 0;  // a failed build leaves empty roots
-        root_first[s] = ok ? fcl[s] : 0;
-        root_nch[s] = ok ? fcl[s + 1] - fcl[s] : 0;
-    }
-    for (int b = grid_stride_start(); b < T; b += grid_stride()) {
-        int p, l;
-        bool c, f;
-        node_kind(ent_bfs[b], body_sys, sys_off, delta, bucket, p, l, c, f);
-        const unsigned long long ex = flags_ex[b];
-        const int fcx = (int)(ex & 0xffffffffull);
-        if (c) {
-            const int k = nsys + (int)(ex >> 32);
-            const int first = fcl[k];
-            const int nch = fcl[k + 1] - first;
-            if (nch < 1 || nch > 8) {
-                set_status(st, NBX_ERR_STATE, b);
-                meta[b] = first;  // keeps the walk in bounds
+    __syncthreads();
+    if (w == 0) {
+        unsigned tot[2], bef[2];
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            const int l = 2 * lane + h;
+            if (Direct) {
+                tot[h] = bef[h] = 0u;
+#pragma unroll
+                for (int r = 0; r < kRows; r++) {
+                    tot[h] += part[0][r][l];
+                    bef[h] += part[1][r][l];
+                }
             } else {
-                meta[b] = first | ((nch - 1) << 28);
+                tot[h] = lvl_tot[l];
+                bef[h] = counts[(size_t)blockIdx.x * kLvlRow + l];
             }
         }
-        const int j = fcx + (f ? 1 : 0) - 1;
-        parent[b] = j < nsys ? (-1 - j) : cl[j];
+        unsigned incl = tot[0] + tot[1];
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned u = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += u;
+        }
+        const unsigned excl = incl - tot[0] - tot[1];
+        base[2 * lane] = excl + bef[0];
+        base[2 * lane + 1] = excl + tot[0] + bef[1];
+        const unsigned eb = __reduce_add_sync(0xffffffffu, bef[0] + bef[1]);
+        const unsigned T = __shfl_sync(0xffffffffu, incl, 31);
+        if (lane == 0) {
+            s_T = T;
+            s_ebase = eb;
+        }
+        if (blockIdx.x == 0) {
+            const bool fits = T <= (unsigned)cap_nodes;
+            lvl_start[2 * lane] = fits ? excl : 0u;
+            lvl_start[2 * lane + 1] = fits ? excl + tot[0] : 0u;
+            if (lane == 0) {
+                if (!fits) set_status(st, NBX_ERR_CAPACITY, (int)min(T, 0x7fffffffu));
+                totals[0] = T;
+                totals[1] = fits ? T : 0u;  // nothing downstream reads a partial tree
+                totals64[0] = fits ? (unsigned long long)(T - (unsigned)n) << 32 : 0ull;
+            }
+        }
     }
+    __syncthreads();
+    // the warps' bases in every level, and this warp's first entry
+    if (threadIdx.x < kLvlRow) {
+        unsigned run = base[threadIdx.x];
+#pragma unroll
+        for (int v = 0; v < kWarps; v++) {
+            const unsigned c = wcnt[v][threadIdx.x];
+            wcnt[v][threadIdx.x] = run;
+            run += c;
+        }
+    }
+    unsigned e = s_ebase + einc - ne;
+    for (int v = 0; v < w; v++) e += went[v];
+    __syncthreads();
+    const bool fits = s_T <= (unsigned)cap_nodes;
+    const bool ok = fits && st->code == 0;  // a failed build leaves empty roots
+    if (p < n) eoff[p] = e;
+    if (!fits) {
+        if (p < n && p == beg) root_first[s] = 0;
+        return;
+    }
+    int b = 0;  // this position's node at the level before l
+    for (int l = wlo - 1; l <= whi; l++) {
+        const unsigned m = __ballot_sync(0xffffffffu, lo <= l && l <= hi);
+        if (l < lo - 1 || l > hi) continue;
+        const int i = (int)(wcnt[w][l] + __popc(m & lt));
+        if (l == lo - 1) {
+            b = i - 1;  // the last level-l node before p: the parent of p's top node
+            continue;
+        }
+        lvl8[i] = (unsigned char)l;
+        ent[i] = ((unsigned)l << kLevelShift) | (unsigned)p;
+        arrive[i] = 0;
+        if (l == 1) {
+            parent[i] = -1 - s;
+            if (p == beg) root_first[s] = ok ? i : 0;
+            if (ok) atomicAdd(&root_nch[s], 1);
+        } else {
+            parent[i] = b;
+            // the first child of the cell at this position, or a later child
+            atomicAdd(&meta[b], l > lo ? i : 1 << 28);
+        }
+        if (l == hi) {
+            node4[i] = body4[p];
+            meta[i] = kBodyFlag | p;
+            body_node[p] = i;
+            count[i] = 1;
+        }
+        b = i;
+    }
+}
+
+// (double)f in integer operations: FP64 instructions and conversions run at a
+// small fraction of the FP32 rate on this part (a warp instruction holds the
+// pipe for tens of cycles), and the moments are bound by them.
+__device__ __forceinline__ double widen(float f) {
+    const unsigned u = __float_as_uint(f);
+    const unsigned e = (u >> 23) & 255u;
+    if (e - 1u >= 254u && (u << 1) != 0u) return (double)f;  // subnormal, infinity, NaN
+    const unsigned hi = (u & 0x80000000u) | ((u << 1) ? ((u >> 3) & 0x0fffffffu) + 0x38000000u : 0u);
+    return __hiloint2double((int)hi, (int)(u << 29));
+}
+
+// Moments of a cell by a group of lanes (4, or 8 with quadrupoles), lane k of
+// the group holding component k & 3 of (m, m x, m y, m z): the children are
+// summed in child order, one FP64 instruction per child for all components
+// (a body's m x is exact in FP64, so the fused product adds it with one
+// rounding), and one division gives the three coordinates of the centre.
+// Lanes of inactive groups pass nch = 0 and store nothing.  The loads of all
+// children are issued together; a child's kind picks the value.
+struct CellSum {
+    double acc;
+    int cnt;
+};
+
+__device__ __forceinline__ CellSum sum_cell(int k, int first, int nch, const int *__restrict__ meta,
+                                            const float4 *node4, const double4 *sums, const int *count) {
+    int mk[8], ck[8];
+    float mb[8], fb[8];
+    double v[8];
+#pragma unroll
+    for (int j = 0; j < 8; j++) {
+        if (j < nch) {
+            const int c = first + j;
+            mk[j] = meta[c];
+            const float *q = reinterpret_cast<const float *>(&node4[c]);
+            mb[j] = q[3];
+            fb[j] = k == 0 ? 1.f : q[k - 1];
+            v[j] = __ldcg(reinterpret_cast<const double *>(&sums[c]) + k);
+            ck[j] = __ldcg(&count[c]);
+        }
+    }
+    CellSum r{0.0, 0};
+#pragma unroll
+    for (int j = 0; j < 8; j++) {
+        if (j < nch) {
+            const bool body = mk[j] < 0;
+            r.acc = __fma_rn(body ? widen(mb[j]) : v[j], body ? widen(fb[j]) : 1.0, r.acc);
+            r.cnt += body ? 1 : ck[j];
+        }
+    }
+    return r;
 }
 
 // Quadrupole mode: the FP64 second moments of a cell about its centre of mass c,
@@ -464,207 +637,208 @@ __global__ void __launch_bounds__(kBlock) k_nodes_b(const unsigned *__restrict__
 // stored negated in FP32 as P = -Q = tr(M2) I - 3 M2 (the walk's form of the
 // term; the FP64 differences are negated before rounding, so P is exactly -Q).
 // Every FP64 operation is rounded explicitly (no contraction), in the order of
-// the oracle's restatement, so both give the same bits.
-__device__ __forceinline__ void m2_add_point(double *a, double mc, double dx, double dy, double dz) {
-    a[0] = __dadd_rn(a[0], __dmul_rn(__dmul_rn(mc, dx), dx));
-    a[1] = __dadd_rn(a[1], __dmul_rn(__dmul_rn(mc, dy), dy));
-    a[2] = __dadd_rn(a[2], __dmul_rn(__dmul_rn(mc, dz), dz));
-    a[3] = __dadd_rn(a[3], __dmul_rn(__dmul_rn(mc, dx), dy));
-    a[4] = __dadd_rn(a[4], __dmul_rn(__dmul_rn(mc, dx), dz));
-    a[5] = __dadd_rn(a[5], __dmul_rn(__dmul_rn(mc, dy), dz));
+// the oracle's restatement, so both give the same bits.  Lane k < 6 of the
+// group holds component k of (xx, yy, zz, xy, xz, yz); com is the centres' FP64
+// array, (x, y, z) per cell.
+__device__ __forceinline__ void quad_cell(int k, int b, int first, int nch, double q0, const int *__restrict__ meta,
+                                          const float4 *node4, const double4 *sums, double *com, double2 *m2,
+                                          float4 *quad4, float2 *quad2) {
+    const int ka = k < 3 ? k : (k == 5 ? 1 : 0);   // first axis of the component
+    const int kb = k < 3 ? k : (k == 3 ? 1 : 2);   // second axis
+    const int g = threadIdx.x & 24;                // first lane of the group
+    // q0: lane 1..3 hold the cell's own centre (x, y, z)
+    const double ca = __shfl_sync(0xffffffffu, q0, g + 1 + min(ka, 2));
+    const double cb = __shfl_sync(0xffffffffu, q0, g + 1 + min(kb, 2));
+    if (k < 3 && nch > 0) com[3 * (size_t)b + k] = ca;
+    double a = 0.0;
+    if (k < 6) {
+#pragma unroll 4
+        for (int j = 0; j < nch; j++) {
+            const int c = first + j;
+            double mc, xa, xb;
+            if (meta[c] < 0) {
+                const float *q = reinterpret_cast<const float *>(&node4[c]);
+                mc = widen(q[3]);
+                xa = widen(q[ka]);
+                xb = widen(q[kb]);
+            } else {
+                mc = __ldcg(reinterpret_cast<const double *>(&sums[c]));
+                xa = __ldcg(&com[3 * (size_t)c + ka]);
+                xb = __ldcg(&com[3 * (size_t)c + kb]);
+                a = __dadd_rn(a, __ldcg(reinterpret_cast<const double *>(&m2[3 * (size_t)c]) + k));
+            }
+            a = __dadd_rn(a, __dmul_rn(__dmul_rn(mc, __dsub_rn(xa, ca)), __dsub_rn(xb, cb)));
+        }
+    }
+    const double axx = __shfl_sync(0xffffffffu, a, g), ayy = __shfl_sync(0xffffffffu, a, g + 1);
+    const double azz = __shfl_sync(0xffffffffu, a, g + 2);
+    const double tr = __dadd_rn(__dadd_rn(axx, ayy), azz);
+    if (k < 6 && nch > 0) {
+        reinterpret_cast<double *>(&m2[3 * (size_t)b])[k] = a;
+        const double t3 = __dmul_rn(k < 3 ? 3.0 : -3.0, a);
+        const float P = (float)(k < 3 ? __dsub_rn(tr, t3) : t3);
+        if (k < 4) reinterpret_cast<float *>(&quad4[b])[k] = P;
+        else reinterpret_cast<float *>(&quad2[b])[k - 4] = P;
+    }
 }
 
-// b: the cell; its children [first, first + nch); (cx, cy, cz) its FP64 centre of mass
-__device__ __forceinline__ void quad_cell(int b, int first, int nch, double cx, double cy, double cz,
-                                          const int *__restrict__ meta, const float4 *node4, const double4 *sums,
-                                          double2 *m2, float4 *quad4, float2 *quad2) {
-    double a[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-    for (int c = first; c < first + nch; c++) {
-        double mc, dx, dy, dz;
-        if (meta[c] < 0) {
-            const float4 q = node4[c];
-            mc = (double)q.w;
-            dx = __dsub_rn((double)q.x, cx);
-            dy = __dsub_rn((double)q.y, cy);
-            dz = __dsub_rn((double)q.z, cz);
-        } else {
-            const double2 *vp = reinterpret_cast<const double2 *>(&sums[c]);
-            const double2 v0 = __ldcg(vp), v1 = __ldcg(vp + 1);
-            mc = v0.x;
-            dx = __dsub_rn(__ddiv_rn(v0.y, mc), cx);
-            dy = __dsub_rn(__ddiv_rn(v1.x, mc), cy);
-            dz = __dsub_rn(__ddiv_rn(v1.y, mc), cz);
-            const double2 w0 = __ldcg(&m2[3 * (size_t)c]), w1 = __ldcg(&m2[3 * (size_t)c + 1]),
-                          w2 = __ldcg(&m2[3 * (size_t)c + 2]);
-            a[0] = __dadd_rn(a[0], w0.x);
-            a[1] = __dadd_rn(a[1], w0.y);
-            a[2] = __dadd_rn(a[2], w1.x);
-            a[3] = __dadd_rn(a[3], w1.y);
-            a[4] = __dadd_rn(a[4], w2.x);
-            a[5] = __dadd_rn(a[5], w2.y);
-        }
-        m2_add_point(a, mc, dx, dy, dz);
-    }
-    m2[3 * (size_t)b] = make_double2(a[0], a[1]);
-    m2[3 * (size_t)b + 1] = make_double2(a[2], a[3]);
-    m2[3 * (size_t)b + 2] = make_double2(a[4], a[5]);
-    const double tr = __dadd_rn(__dadd_rn(a[0], a[1]), a[2]);
-    quad4[b] = make_float4((float)__dsub_rn(tr, __dmul_rn(3.0, a[0])), (float)__dsub_rn(tr, __dmul_rn(3.0, a[1])),
-                           (float)__dsub_rn(tr, __dmul_rn(3.0, a[2])), (float)__dmul_rn(-3.0, a[3]));
-    quad2[b] = make_float2((float)__dmul_rn(-3.0, a[4]), (float)__dmul_rn(-3.0, a[5]));
+// A cell's sums, and (finish) its centre of mass, node record and quadrupole.
+template <bool Quad>
+__device__ __forceinline__ double finish_cell(int k, int b, int first, int nch, double acc, const int *__restrict__ meta,
+                                              float4 *node4, const double4 *sums, double *com, double2 *m2,
+                                              float4 *quad4, float2 *quad2) {
+    constexpr int kLanes = Quad ? 8 : 4;
+    const int kc = k & 3;
+    const double m = __shfl_sync(0xffffffffu, acc, (threadIdx.x & 31) & ~(kLanes - 1));
+    const double q = kc == 0 ? acc : acc / (nch > 0 ? m : 1.0);
+    if (k < 4 && nch > 0) reinterpret_cast<float *>(&node4[b])[kc == 0 ? 3 : kc - 1] = (float)q;
+    if (Quad) quad_cell(k, b, first, nch, q, meta, node4, sums, com, m2, quad4, quad2);
+    return q;
 }
 
 // Bottom-up FP64 moments, one BFS level per launch (deepest first): a cell sums
 // its children -- contiguous, one level below, already final -- in child order,
 // so the result is deterministic.  Level L occupies BFS indices
-// [start(L), start(L+1)); start(L) is the scanned count of level-sort digit 4L.
+// [lvl_start[L], lvl_start[L+1]); each warp lists the cells among 32 nodes and
+// gives each a group of lanes.
 template <bool Quad>
-__global__ void __launch_bounds__(kBlock) k_moments_level(int level, const unsigned *__restrict__ lvl_off,
-                                                           int ntiles, const unsigned *__restrict__ totals,
-                                                           const unsigned long long *__restrict__ totals64,
-                                                           const unsigned long long *__restrict__ flags_ex,
-                                                           const int *__restrict__ cl, int nsys,
+__global__ void __launch_bounds__(kBlock) k_moments_level(int level, const unsigned *__restrict__ lvl_start,
                                                            const int *__restrict__ meta, float4 *node4,
-                                                           double4 *sums, int *count, double2 *m2, float4 *quad4,
-                                                           float2 *quad2, const DevStatus *st) {
+                                                           double4 *sums, int *count, double *com, double2 *m2,
+                                                           float4 *quad4, float2 *quad2, const DevStatus *st) {
+    constexpr int kLanes = Quad ? 8 : 4, kGroups = 32 / kLanes;
     if (st->code != 0) return;  // an inconsistent tree is never summed
-    const unsigned T = totals[1];
-    unsigned beg = lvl_off[(size_t)(level << 2) * ntiles];
-    unsigned end = lvl_off[(size_t)((level + 1) << 2) * ntiles];
-    if (end > T) end = T;
-    if (beg > end) beg = end;
-    // the level's cells are a contiguous range of the BFS-ordered cell list:
-    // their ranks are the scanned cell flags at the level's first and end nodes
-    const unsigned ncell = (unsigned)(totals64[0] >> 32);
-    const unsigned cbeg = beg < T ? (unsigned)(flags_ex[beg] >> 32) : ncell;
-    const unsigned cend = end < T ? (unsigned)(flags_ex[end] >> 32) : ncell;
-    for (unsigned k = cbeg + grid_stride_start(); k < cend; k += grid_stride()) {
-        const int b = cl[nsys + k];
-        const int pm = meta[b];
-        if (pm < 0) continue;  // never: the list holds cells only
-        const int first = pm & 0x0fffffff;
-        const int nch = ((pm >> 28) & 7) + 1;
-        double sm = 0.0, sx = 0.0, sy = 0.0, sz = 0.0;
-        int cnt = 0;
-        for (int c = first; c < first + nch; c++) {
-            if (meta[c] < 0) {
-                const float4 q = node4[c];
-                const double mb = (double)q.w;
-                sm += mb;
-                sx += mb * (double)q.x;
-                sy += mb * (double)q.y;
-                sz += mb * (double)q.z;
-                cnt += 1;
-            } else {
-                const double4 v = sums[c];
-                sm += v.x;
-                sx += v.y;
-                sy += v.z;
-                sz += v.w;
-                cnt += count[c];
+    __shared__ int list[kBlock / 32][32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, k = lane & (kLanes - 1);
+    const unsigned lt = (1u << lane) - 1u;
+    const unsigned beg = lvl_start[level], end = lvl_start[level + 1];
+    for (unsigned c0 = beg + 32u * (blockIdx.x * (kBlock / 32) + w); c0 < end; c0 += 32u * gridDim.x * (kBlock / 32)) {
+        const bool cell = c0 + lane < end && meta[c0 + lane] >= 0;
+        const unsigned m = __ballot_sync(0xffffffffu, cell);
+        __syncwarp();
+        if (cell) list[w][__popc(m & lt)] = (int)c0 + lane;
+        __syncwarp();
+        const int nc = __popc(m);
+        for (int i = lane / kLanes; i - lane / kLanes < nc; i += kGroups) {
+            int b = 0, first = 0, nch = 0;
+            if (i < nc) {
+                b = list[w][i];
+                const int pm = meta[b];
+                first = pm & 0x0fffffff;
+                nch = ((pm >> 28) & 7) + 1;
             }
+            const CellSum r = sum_cell(k & 3, first, nch, meta, node4, sums, count);
+            if (i < nc && k < 4) {
+                reinterpret_cast<double *>(&sums[b])[k] = r.acc;
+                if (k == 0) count[b] = r.cnt;
+            }
+            finish_cell<Quad>(k, b, first, nch, r.acc, meta, node4, sums, com, m2, quad4, quad2);
         }
-        sums[b] = make_double4(sm, sx, sy, sz);
-        count[b] = cnt;
-        node4[b] = make_float4((float)(sx / sm), (float)(sy / sm), (float)(sz / sm), (float)sm);
-        if (Quad) quad_cell(b, first, nch, sx / sm, sy / sm, sz / sm, meta, node4, sums, m2, quad4, quad2);
     }
 }
 
-// Bottom-up FP64 moments in one launch, one thread per cell in BFS order.
-// Every child arrives once at its cell's counter: the cell's own thread adds
-// the number of its body children in one step, and each child cell arrives
-// when it is complete.  The arrival that brings the count to the cell's number
-// of children sums the cell (children in child order: the same additions as
-// k_moments_level) and climbs on to the parent.  Nothing waits: a thread whose
-// arrival is not the last stops.  A cell's arrival is acquire-release: it
-// publishes the thread's sums and, when last, orders the reads of the
-// siblings' sums (through L2) after their arrivals.  Counters are zeroed by
-// k_nodes_a.
 __device__ __forceinline__ int arrive_acq_rel(int *p) {
     int old;
     asm volatile("atom.acq_rel.gpu.global.add.s32 %0, [%1], 1;" : "=r"(old) : "l"(p) : "memory");
     return old;
 }
 
-// A cell's sums from its children in child order.  Every child's body record
-// and cell sums are loaded at once and the child's kind picks one (a body's
-// sums entry is never read for its value), so the loads take one round trip.
+// Bottom-up FP64 moments in one launch.  A warp takes kUpNodes nodes in BFS
+// order and lists the cells whose children are all bodies; every group of lanes
+// sums a listed cell and climbs: every child arrives once at its cell's counter
+// (the body children in one step, by the warp that meets the cell; a child cell
+// when it is complete), and the arrival that brings the count to the cell's
+// number of children sums the cell (children in child order: the same additions
+// as k_moments_level) and climbs on to the parent.  A group whose arrival is
+// not the last takes the warp's next listed cell.  Nothing waits.  A cell's
+// arrival is acquire-release: it publishes the group's sums (ordered before it
+// by the warp barrier) and, when last, orders the reads of the siblings' sums
+// (through L2) after their arrivals.  Counters are zeroed by k_nodes.
+// Bound by the chain of levels, and in a level by the FP64 pipe: one thread per
+// cell issued about 15 FP64 instructions per child and three divisions per
+// level (4.5 us a level); the lanes share them.  The mode without quadrupoles
+// arrives before its division, which then runs while the arrival returns.
 template <bool Quad>
-__device__ __forceinline__ void sum_cell(int b, int first, int nch, const int *__restrict__ meta, float4 *node4,
-                                         double4 *sums, int *count, double2 *m2, float4 *quad4, float2 *quad2) {
-    int mk[8], ck[8];
-    float4 q[8];
-    double2 v0[8], v1[8];
-#pragma unroll
-    for (int j = 0; j < 8; j++) {
-        if (j < nch) {
-            const int c = first + j;
-            mk[j] = meta[c];
-            q[j] = node4[c];
-            const double2 *v = reinterpret_cast<const double2 *>(&sums[c]);
-            v0[j] = __ldcg(v);
-            v1[j] = __ldcg(v + 1);
-            ck[j] = __ldcg(&count[c]);
-        }
-    }
-    double sm = 0.0, sx = 0.0, sy = 0.0, sz = 0.0;
-    int cnt = 0;
-#pragma unroll
-    for (int j = 0; j < 8; j++) {
-        if (j < nch) {
-            if (mk[j] < 0) {
-                const double mb = (double)q[j].w;
-                sm += mb;
-                sx += mb * (double)q[j].x;
-                sy += mb * (double)q[j].y;
-                sz += mb * (double)q[j].z;
-                cnt += 1;
-            } else {
-                sm += v0[j].x;
-                sx += v0[j].y;
-                sy += v1[j].x;
-                sz += v1[j].y;
-                cnt += ck[j];
-            }
-        }
-    }
-    sums[b] = make_double4(sm, sx, sy, sz);
-    count[b] = cnt;
-    node4[b] = make_float4((float)(sx / sm), (float)(sy / sm), (float)(sz / sm), (float)sm);
-    if (Quad) quad_cell(b, first, nch, sx / sm, sy / sm, sz / sm, meta, node4, sums, m2, quad4, quad2);
-}
-
-template <bool Quad>
-__global__ void __launch_bounds__(kBlock) k_moments_up(const unsigned long long *__restrict__ totals64,
-                                                       const int *__restrict__ cl, int nsys,
+__global__ void __launch_bounds__(kBlock) k_moments_up(const unsigned *__restrict__ totals, int rounds,
                                                        const int *__restrict__ parent,
                                                        const int *__restrict__ meta, float4 *node4,
-                                                       double4 *sums, int *count, int *counter, double2 *m2,
-                                                       float4 *quad4, float2 *quad2, const DevStatus *st) {
+                                                       double4 *sums, int *count, int *counter, double *com,
+                                                       double2 *m2, float4 *quad4, float2 *quad2,
+                                                       const DevStatus *st) {
+    constexpr int kLanes = Quad ? 8 : 4;
     if (st->code != 0) return;  // an inconsistent tree is never summed
-    const int ncell = (int)(totals64[0] >> 32);
-    for (int k = grid_stride_start(); k < ncell; k += grid_stride()) {
-        int b = cl[nsys + k];
-        int pm = meta[b];
-        int first = pm & 0x0fffffff, nch = ((pm >> 28) & 7) + 1;
-        int nbody = 0;
-        for (int c = first; c < first + nch; c++) nbody += meta[c] < 0;
-        if (nbody == 0) continue;  // completed by the arrival of its last child cell
-        if (nbody < nch) {  // cell children too: the bodies arrive together (relaxed: nothing to publish)
-            if (atomicAdd(&counter[b], nbody) + nbody != nch) continue;
-            asm volatile("fence.acq_rel.gpu;" ::: "memory");
+    __shared__ int list[kBlock / 32][32 * kUpRounds];
+    const int T = (int)totals[1];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, k = lane & (kLanes - 1);
+    const int lead = lane & ~(kLanes - 1);
+    const unsigned lt = (1u << lane) - 1u;
+    const int nwarps = gridDim.x * (kBlock / 32);
+    for (int c0 = 32 * rounds * (blockIdx.x * (kBlock / 32) + w); c0 < T; c0 += 32 * rounds * nwarps) {
+        int nlist = 0;
+        __syncwarp();
+        for (int r = 0; r < rounds; r++) {
+            const int b = c0 + 32 * r + lane;
+            const int pm = b < T ? meta[b] : -1;
+            bool ready = false;
+            if (pm >= 0) {
+                const int first = pm & 0x0fffffff, nch = ((pm >> 28) & 7) + 1;
+                int nbody = 0;
+#pragma unroll
+                for (int j = 0; j < 8; j++)
+                    if (j < nch) nbody += meta[first + j] < 0;
+                // no body child: completed by the arrival of its last child cell;
+                // both kinds: the bodies arrive together (relaxed: nothing to publish)
+                ready = nbody == nch;
+                if (nbody > 0 && !ready) {
+                    ready = atomicAdd(&counter[b], nbody) + nbody == nch;
+                    if (ready) asm volatile("fence.acq_rel.gpu;" ::: "memory");
+                }
+            }
+            const unsigned m = __ballot_sync(0xffffffffu, ready);
+            if (ready) list[w][nlist + __popc(m & lt)] = b;
+            nlist += __popc(m);
         }
+        __syncwarp();
+        int next = 0, b = -1, pm = 0, up = -1;
         for (;;) {
-            // the parent and its meta load while the sums do
-            const int up = parent[b];
-            sum_cell<Quad>(b, first, nch, meta, node4, sums, count, m2, quad4, quad2);
-            if (up < 0) break;
-            pm = meta[up];
-            if (arrive_acq_rel(&counter[up]) != ((pm >> 28) & 7)) break;  // last of its children?
-            b = up;
-            first = pm & 0x0fffffff;
-            nch = ((pm >> 28) & 7) + 1;
+            // groups without a cell take the next listed ones
+            const unsigned want = __ballot_sync(0xffffffffu, b < 0 && k == 0);
+            if (b < 0) {
+                const int i = next + __popc(want & ((1u << lead) - 1u));
+                if (i < nlist) {
+                    b = list[w][i];
+                    pm = meta[b];
+                    up = parent[b];
+                }
+            }
+            next += __popc(want);
+            const bool on = b >= 0;
+            if (!__any_sync(0xffffffffu, on)) break;
+            const int first = on ? pm & 0x0fffffff : 0, nch = on ? ((pm >> 28) & 7) + 1 : 0;
+            // the parent's record loads with the children; in a small tree (one round
+            // per warp) its parent too, which shortens the chain of a climb but is
+            // one more load for every group that stops
+            int upm = 0, up2 = -1;
+            if (on && up >= 0) {
+                upm = meta[up];
+                if (rounds == 1) up2 = parent[up];
+            }
+            const CellSum r = sum_cell(k & 3, first, nch, meta, node4, sums, count);
+            if (on && k < 4) {
+                reinterpret_cast<double *>(&sums[b])[k] = r.acc;
+                if (k == 0) count[b] = r.cnt;
+            }
+            if (Quad) finish_cell<true>(k, b, first, nch, r.acc, meta, node4, sums, com, m2, quad4, quad2);
+            __syncwarp();  // the group's stores come before its arrival
+            int old = -1;
+            if (on && up >= 0 && k == 0) old = arrive_acq_rel(&counter[up]);
+            if (!Quad) finish_cell<false>(k, b, first, nch, r.acc, meta, node4, sums, com, m2, quad4, quad2);
+            old = __shfl_sync(0xffffffffu, old, lead);
+            __syncwarp();  // the reads of the siblings' sums come after it
+            const bool last = on && up >= 0 && old == ((upm >> 28) & 7);  // of the parent's children
+            b = last ? up : -1;
+            pm = upm;
+            up = last && rounds > 1 ? parent[up] : up2;
         }
     }
 }
@@ -678,7 +852,8 @@ int build_tree(Ctx *ctx, const nbx_state *s, cudaStream_t st, bool external_bbox
     const int S = ctx->nsys;
     if (n <= 0 || S <= 0) return NBX_ERR_STATE;
     const int gb = ceil_div(n, kBlock) < ctx->nsm * 8 ? ceil_div(n, kBlock) : ctx->nsm * 8;
-    k_step_reset<<<ceil_div(6 * S + 1, kBlock), kBlock, 0, st>>>(ctx->d_bbox_u, S, ctx->d_status, ctx->d_sys_lvl);
+    k_step_reset<<<ceil_div(6 * S + 1, kBlock), kBlock, 0, st>>>(ctx->d_bbox_u, S, ctx->d_status, ctx->d_sys_lvl,
+                                                            ctx->d_root_nch);
     ++ctx->launches;
     if (!external_bbox) {
         k_bbox<<<ctx->ntiles_body, kBlock, 0, st>>>(s->x, s->y, s->z, ctx->d_tiles, ctx->ntiles_body,
@@ -699,46 +874,37 @@ int build_tree(Ctx *ctx, const nbx_state *s, cudaStream_t st, bool external_bbox
     const bool alt = radix_passes(ctx->radix_bits) & 1;
     k_keys<<<gb, kBlock, 0, st>>>(s->x, s->y, s->z, s->m, ctx->d_body_sys, ctx->d_bbox, n,
                                   alt ? ctx->d_key_alt : ctx->d_key, alt ? ctx->d_val_alt : ctx->d_val, pos4,
-                                  ctx->d_status, ctx->key_order);
+                                  ctx->d_status, ctx->key_order, ctx->d_meta, ctx->cap_nodes);
     ++ctx->launches;
     int rc = radix_sort_bodies(ctx, st);
     if (rc) return rc;
     k_refine<<<gb, kBlock, 0, st>>>(s->x, s->y, s->z, ctx->d_body_sys, ctx->d_sys_off, ctx->d_bbox, n,
                                     ctx->d_key, ctx->d_key_lo, ctx->d_val, ctx->d_status, ctx->key_order);
     ++ctx->launches;
-    k_delta<<<gb, kBlock, 0, st>>>(pos4, ctx->d_body_sys, ctx->d_sys_off, n, ctx->d_key,
-                                   ctx->d_key_lo, ctx->d_val, ctx->d_body4, ctx->d_delta, ctx->d_ecount,
-                                   ctx->d_status, ctx->d_sys_lvl);
-    ++ctx->launches;
     const unsigned char *bucket = ctx->leaf_size > 1 ? ctx->d_bucket : nullptr;
+    const int nblk = ceil_div(n, kPosBlock);
+    k_delta<<<nblk, kPosBlock, 0, st>>>(pos4, ctx->d_body_sys, ctx->d_sys_off, n, ctx->d_key, ctx->d_key_lo,
+                                        ctx->d_val, ctx->d_body4, ctx->d_delta, bucket ? nullptr : ctx->d_lvl_counts,
+                                        ctx->d_status, ctx->d_sys_lvl);
+    ++ctx->launches;
     if (bucket) {
-        k_bucket<<<gb, kBlock, 0, st>>>(ctx->d_body_sys, ctx->d_sys_off, n, ctx->leaf_size, ctx->d_delta,
-                                        ctx->d_bucket, ctx->d_ecount);
+        k_bucket<<<nblk, kPosBlock, 0, st>>>(ctx->d_body_sys, ctx->d_sys_off, n, ctx->leaf_size, ctx->d_delta,
+                                             ctx->d_bucket, ctx->d_lvl_counts);
         ++ctx->launches;
     }
-    rc = scan_exclusive_u32(ctx, ctx->d_ecount, ctx->d_ecount, n, nullptr, &ctx->d_totals[0], st);
-    if (rc) return rc;
-    k_entries<<<gb, kBlock, 0, st>>>(ctx->d_body_sys, ctx->d_sys_off, n, ctx->d_delta, bucket, ctx->d_ecount,
-                                     ctx->d_totals, ctx->cap_nodes, ctx->d_ent, ctx->d_status);
+    const bool direct = nblk <= kDirectBlocks;
+    if (!direct) {
+        k_level_scan<<<kLvlRow, 1024, 0, st>>>(ctx->d_lvl_counts, nblk, ctx->d_lvl_tot);
+        ++ctx->launches;
+    }
+    auto nodes = direct ? k_nodes<true> : k_nodes<false>;
+    nodes<<<nblk, kPosBlock, 0, st>>>(ctx->d_body_sys, ctx->d_sys_off, n, ctx->d_delta, bucket, ctx->d_lvl_counts, nblk,
+                                      ctx->d_lvl_tot, ctx->cap_nodes, ctx->d_body4, ctx->d_totals, ctx->d_totals64,
+                                      ctx->d_lvl_start, ctx->d_ecount, ctx->d_ent, ctx->d_node4, ctx->d_meta,
+                                      ctx->d_parent, ctx->d_body_node, ctx->d_count, ctx->d_arrive, ctx->d_lvl8,
+                                      ctx->d_root_first, ctx->d_root_nch, ctx->d_status);
     ++ctx->launches;
-    rc = radix_sort_entries(ctx, st);  // d_ent -> d_ent_alt (BFS order)
-    if (rc) return rc;
     const int gn = ceil_div(ctx->cap_nodes, kBlock) < ctx->nsm * 8 ? ceil_div(ctx->cap_nodes, kBlock) : ctx->nsm * 8;
-    k_node_flags<<<gn, kBlock, 0, st>>>(ctx->d_ent_alt, ctx->d_totals, ctx->d_body_sys, ctx->d_sys_off,
-                                        ctx->d_delta, bucket, ctx->d_flags);
-    ++ctx->launches;
-    rc = scan_exclusive_u64(ctx, ctx->d_flags, ctx->d_flags, ctx->cap_nodes, &ctx->d_totals[1],
-                            &ctx->d_totals64[0], st);
-    if (rc) return rc;
-    k_nodes_a<<<gn, kBlock, 0, st>>>(ctx->d_ent_alt, ctx->d_totals, ctx->d_totals64, ctx->d_body_sys,
-                                     ctx->d_sys_off, ctx->d_delta, bucket, ctx->d_flags, ctx->d_body4, S, ctx->d_fcl,
-                                     ctx->d_cl, ctx->d_node4, ctx->d_meta, ctx->d_body_node, ctx->d_count,
-                                     ctx->d_arrive, ctx->d_lvl8, ctx->d_status);
-    ++ctx->launches;
-    k_nodes_b<<<gn, kBlock, 0, st>>>(ctx->d_ent_alt, ctx->d_totals, ctx->d_body_sys, ctx->d_sys_off,
-                                     ctx->d_delta, bucket, ctx->d_flags, S, ctx->d_fcl, ctx->d_cl, ctx->d_meta,
-                                     ctx->d_parent, ctx->d_root_first, ctx->d_root_nch, ctx->d_status);
-    ++ctx->launches;
     // up to 2^21 bodies the 41 per-level launches cost more than the sums: one
     // bottom-up launch (2^16: 0.37 against 0.55 ms per build); above, the
     // per-level launches stream the levels and are faster
@@ -746,19 +912,22 @@ int build_tree(Ctx *ctx, const nbx_state *s, cudaStream_t st, bool external_bbox
     const bool quad = ctx->multipole != 0;
     if (quad && !ctx->d_m2) return NBX_ERR_STATE;
     if (mode == 2 || (mode == 0 && n <= kMomentsUpMaxBodies)) {
+        // one round of 32 nodes per warp until that fills the GPU's warps (a small
+        // tree wants its chains started at once), then up to four (fuller groups)
+        int rounds = (int)(3ll * n / 2 / (32ll * 32 * ctx->nsm));
+        rounds = rounds < 1 ? 1 : (rounds > kUpRounds ? kUpRounds : rounds);
         auto kern = quad ? k_moments_up<true> : k_moments_up<false>;
-        kern<<<gn, kBlock, 0, st>>>(ctx->d_totals64, ctx->d_cl, S, ctx->d_parent, ctx->d_meta, ctx->d_node4,
-                                    ctx->d_sums, ctx->d_count, ctx->d_arrive, ctx->d_m2, ctx->d_quad4, ctx->d_quad2,
+        kern<<<gn, kBlock, 0, st>>>(ctx->d_totals, rounds, ctx->d_parent, ctx->d_meta, ctx->d_node4, ctx->d_sums,
+                                    ctx->d_count, ctx->d_arrive, ctx->d_com, ctx->d_m2, ctx->d_quad4, ctx->d_quad2,
                                     ctx->d_status);
         ++ctx->launches;
     } else {
         // cells exist at levels 1..41 (two bodies share at most 41 levels without error)
         auto kern = quad ? k_moments_level<true> : k_moments_level<false>;
         for (int level = kMaxLevel - 2; level >= 1; level--) {
-            kern<<<ctx->nsm * 4, kBlock, 0, st>>>(level, ctx->d_hist, ctx->cap_tiles_node, ctx->d_totals,
-                                                  ctx->d_totals64, ctx->d_flags, ctx->d_cl, S, ctx->d_meta,
-                                                  ctx->d_node4, ctx->d_sums, ctx->d_count, ctx->d_m2, ctx->d_quad4,
-                                                  ctx->d_quad2, ctx->d_status);
+            kern<<<ctx->nsm * 4, kBlock, 0, st>>>(level, ctx->d_lvl_start, ctx->d_meta, ctx->d_node4, ctx->d_sums,
+                                                  ctx->d_count, ctx->d_com, ctx->d_m2, ctx->d_quad4, ctx->d_quad2,
+                                                  ctx->d_status);
             ++ctx->launches;
         }
     }
@@ -874,7 +1043,7 @@ int export_tree_impl(Ctx *ctx, int sys, int *perm, int *root_child, int *cell_ch
     if (root_child) NBX_CUDA(cudaMemsetAsync(root_child, 0xff, 8 * sizeof(int), st));
     if (cell_child && nc > 0) NBX_CUDA(cudaMemsetAsync(cell_child, 0xff, 8 * sizeof(int) * (size_t)nc, st));
     const int gn = ceil_div(ctx->cap_nodes, kBlock) < ctx->nsm * 8 ? ceil_div(ctx->cap_nodes, kBlock) : ctx->nsm * 8;
-    k_export<<<gn, kBlock, 0, st>>>(ctx->d_ent_alt, ctx->d_totals, ctx->d_body_sys, ctx->d_sys_off,
+    k_export<<<gn, kBlock, 0, st>>>(ctx->d_ent, ctx->d_totals, ctx->d_body_sys, ctx->d_sys_off,
                                     ctx->d_delta, ctx->d_ecount, ctx->d_key, ctx->d_key_lo, ctx->d_val,
                                     ctx->d_parent, ctx->d_node4, ctx->d_sums, ctx->d_count, sys, cells_before,
                                     cap_cells, root_child, cell_child, cell_start, cell_count, cell_level, cx,

@@ -1,0 +1,31 @@
+"""Tree build at the sizes where its kernels change shape: block edges of the node
+kernels (512 positions), the switch between summed and scanned level counts
+(131072 positions), and both centre-of-mass passes.  Bit-exact against the oracle.
+"""
+import numpy as np
+import pytest
+
+from nns_gb300 import ic
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+def _check(b, gt, ot):
+    assert np.array_equal(gt["perm"], ot.perm)
+    assert np.array_equal(gt["root_child"], ot.root_child)
+    assert gt["ncells"] == ot.ncells
+    for k in ("cell_child", "cell_start", "cell_count", "cell_level", "cell_x", "cell_y", "cell_z", "cell_m"):
+        assert np.array_equal(gt[k], getattr(ot, k)), k
+
+
+@pytest.mark.parametrize("n", [511, 512, 513, 1025, 131072, 131073])
+@pytest.mark.parametrize("moments_mode", [1, 2])
+def test_node_blocks(cuda, n, moments_mode):
+    from nns_gb300.barnes_hut import Context, State
+    b = ic.plummer(n, seed=n)
+    ctx = Context(max_bodies=n, moments_mode=moments_mode)
+    ctx.set_systems([0, n])
+    ctx.build(State.from_bodies(b))
+    ctx.sync()
+    _check(b, ctx.export_tree(0), O.build(b.x, b.y, b.z, b.m))
