@@ -110,7 +110,7 @@ void free_all(Ctx *ctx) {
                     ctx->d_sums, ctx->d_count, ctx->d_arrive, ctx->d_lvl8, ctx->d_hist,
                     ctx->d_scan_blk, ctx->d_totals, ctx->d_totals64, ctx->d_status, ctx->d_m2, ctx->d_com, ctx->d_quad4,
                     ctx->d_quad2, ctx->d_seg_slot, ctx->d_lb_counts, ctx->d_lb_status, ctx->d_lb, ctx->d_tiles_sw,
-                    ctx->d_sys_tiles_sw};
+                    ctx->d_sys_tiles_sw, ctx->d_tiles_mg, ctx->d_runs_mg};
     for (void *p : ptrs)
         if (p) cudaFree(p);
     if (ctx->h_status) cudaFreeHost(ctx->h_status);
@@ -294,6 +294,8 @@ int nbx_create(const nbx_params *p, nbx_ctx **out) {
     rc |= nbx::dmalloc(ctx, &ctx->d_seg_slot, Ss);
     rc |= nbx::dmalloc(ctx, &ctx->d_tiles_sw, ctx->cap_tiles_body);
     rc |= nbx::dmalloc(ctx, &ctx->d_sys_tiles_sw, Ss);
+    rc |= nbx::dmalloc(ctx, &ctx->d_tiles_mg, (size_t)B / nbx::kMergeTile + Ss + 1);
+    rc |= nbx::dmalloc(ctx, &ctx->d_runs_mg, (size_t)B / nbx::kMergeRun + Ss + 1);
     rc |= nbx::dmalloc(ctx, &ctx->d_groups, G);
     rc |= nbx::dmalloc(ctx, &ctx->d_bbox_u, 6 * Ss + 6);
     rc |= nbx::dmalloc(ctx, &ctx->d_bbox, 6 * Ss);
@@ -344,6 +346,7 @@ int nbx_create(const nbx_params *p, nbx_ctx **out) {
     if (rc == 0 && ctx->multipole) rc = nbx::alloc_quadrupoles(ctx);
     if (rc == 0) rc = nbx::walk_init(ctx);
     if (rc == 0) rc = nbx::radix_init(ctx);
+    if (rc == 0) rc = nbx::merge_init(ctx);
     if (rc != 0) {
         nbx::free_all(ctx);
         delete ctx;
@@ -468,7 +471,8 @@ int nbx_set_systems(nbx_ctx *c, int nsys, const int64_t *offsets) {
     // between a system's tiles, so its tiles are at least kTileSweep keys
     const int tile_sw = tile > nbx::kTileSweep ? tile : (nbx::kTileSweep < nbx::kTile ? nbx::kTileSweep : nbx::kTile);
     std::vector<int> off(nsys + 1);
-    std::vector<int4> tiles, tiles_sw;
+    std::vector<int4> tiles, tiles_sw, tiles_mg, runs_mg;
+    int max_sys = 0;
     std::vector<int2> st(nsys), st_sw(nsys);
     std::vector<int> slot(nsys);
     std::vector<int> groups;
@@ -492,7 +496,17 @@ int nbx_set_systems(nbx_ctx *c, int nsys, const int64_t *offsets) {
             tiles_sw.push_back(make_int4(a, len, s, t));
         }
         for (int g = beg; g < end; g += 32) groups.push_back(g);
+        max_sys = max_sys > end - beg ? max_sys : end - beg;
     }
+    if (max_sys <= nbx::kMergeMaxBodies)
+        for (int s = 0; s < nsys; s++) {
+            const auto cut = [&](std::vector<int4> &to, int width) {
+                for (int a = off[s], t = 0; a < off[s + 1]; a += width, t++)
+                    to.push_back(make_int4(a, off[s + 1] - a < width ? off[s + 1] - a : width, s, t));
+            };
+            cut(tiles_mg, nbx::kMergeTile);
+            cut(runs_mg, nbx::kMergeRun);
+        }
     if ((int)tiles.size() > ctx->cap_tiles_body || (int)tiles_sw.size() > ctx->cap_tiles_body) return NBX_ERR_ARG;
     NBX_CUDA(cudaMemcpy(ctx->d_sys_off, off.data(), sizeof(int) * (nsys + 1), cudaMemcpyHostToDevice));
     NBX_CUDA(cudaMemcpy(ctx->d_tiles, tiles.data(), sizeof(int4) * tiles.size(), cudaMemcpyHostToDevice));
@@ -500,6 +514,10 @@ int nbx_set_systems(nbx_ctx *c, int nsys, const int64_t *offsets) {
     NBX_CUDA(cudaMemcpy(ctx->d_seg_slot, slot.data(), sizeof(int) * nsys, cudaMemcpyHostToDevice));
     NBX_CUDA(cudaMemcpy(ctx->d_tiles_sw, tiles_sw.data(), sizeof(int4) * tiles_sw.size(), cudaMemcpyHostToDevice));
     NBX_CUDA(cudaMemcpy(ctx->d_sys_tiles_sw, st_sw.data(), sizeof(int2) * nsys, cudaMemcpyHostToDevice));
+    if (!tiles_mg.empty()) {
+        NBX_CUDA(cudaMemcpy(ctx->d_tiles_mg, tiles_mg.data(), sizeof(int4) * tiles_mg.size(), cudaMemcpyHostToDevice));
+        NBX_CUDA(cudaMemcpy(ctx->d_runs_mg, runs_mg.data(), sizeof(int4) * runs_mg.size(), cudaMemcpyHostToDevice));
+    }
     NBX_CUDA(cudaMemcpy(ctx->d_groups, groups.data(), sizeof(int) * groups.size(), cudaMemcpyHostToDevice));
     nbx::k_body_sys<<<nbx::ceil_div(n, 256) < 4096 ? nbx::ceil_div(n, 256) : 4096, 256>>>(ctx->d_sys_off, nsys, n,
                                                                                           ctx->d_body_sys);
@@ -512,6 +530,9 @@ int nbx_set_systems(nbx_ctx *c, int nsys, const int64_t *offsets) {
     ctx->nslots = nslots;
     ctx->ntiles_sw = (int)tiles_sw.size();
     ctx->tile_sw = tile_sw;
+    ctx->ntiles_mg = (int)tiles_mg.size();
+    ctx->nruns_mg = (int)runs_mg.size();
+    ctx->max_sys = max_sys;
     ctx->tile_body = tile;
     ctx->ngroups = (int)groups.size();
     ctx->built = false;

@@ -35,6 +35,14 @@ inline int tile_for(long long n, int nsm) {
     while (t > kTileMin && n < (long long)t * want) t >>= 1;
     return t;
 }
+// body-key sort by merging (merge.cu): systems of up to kMergeMaxBodies bodies
+constexpr int kMergeTile = 256;   // keys of a merging block
+constexpr int kMergeRun = 1024;   // keys of a first run
+constexpr int kMergeFan = 16;     // most runs merged by one launch
+#ifndef NBX_MERGE_MAX
+#define NBX_MERGE_MAX (1 << 19)
+#endif
+constexpr int kMergeMaxBodies = NBX_MERGE_MAX;
 constexpr int kMaxRadixBits = 9;  // body-key digits: 8 or 9 bits (histograms sized for 9)
 // LSD passes over the 63-bit body keys for a digit width
 constexpr int radix_passes(int bits) { return (63 + bits - 1) / bits; }
@@ -96,6 +104,11 @@ struct Ctx {
     int *d_seg_slot = nullptr;      // [S] count slot of a system of several tiles, else -1
     int ntiles_sw = 0, tile_sw = 0;
     int nslots = 0;                 // systems of several tiles (count slots in use)
+    int4 *d_tiles_mg = nullptr;     // [merge tiles] of kMergeTile keys: start, len, sys, local tile index
+    int4 *d_runs_mg = nullptr;      // [first runs] of kMergeRun keys, the same
+    int nruns_mg = 0;
+    int ntiles_mg = 0;              // 0: a system is too large, the keys sort by radix
+    int max_sys = 0;                // bodies of the largest system
     int *d_groups = nullptr;        // [G] first sorted position of each walk group
 
     // per-system tree parameters
@@ -217,6 +230,10 @@ int scan_exclusive_u32(Ctx *ctx, const unsigned *in, unsigned *out, int n_cap,
 // radix.cu
 int radix_sort_bodies(Ctx *ctx, cudaStream_t st);
 int radix_init(Ctx *ctx);
+// merge.cu
+int merge_passes(int max_bodies_of_a_system);
+int merge_runs(Ctx *ctx, cudaStream_t st);
+int merge_init(Ctx *ctx);
 int radix_selftest_wait(Ctx *ctx, cudaStream_t st);
 // tree.cu
 int build_tree(Ctx *ctx, const nbx_state *s, cudaStream_t st, bool external_bbox,

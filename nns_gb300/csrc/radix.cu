@@ -18,11 +18,11 @@
 // Segments are the independent systems of a batch, so one launch sorts every
 // system's keys inside its own range; a single system is one segment.
 //
-// Small and mid-size contexts (fewer than 1.5 x 2^20 bodies, 2^17 in a captured
-// graph) sort their body keys in one launch per pass instead (k_radix_counts
-// once, then the same scatter kernel in its one-sweep form on a tiling of its
-// own, whose tiles find their offsets by decoupled look-back); the permutation
-// is the same.
+// Mid-size contexts (fewer than 1.5 x 2^20 bodies, outside a captured graph) sort
+// their body keys in one launch per pass instead (k_radix_counts once, then the
+// same scatter kernel in its one-sweep form on a tiling of its own, whose tiles
+// find their offsets by decoupled look-back); the permutation is the same.
+// Systems of up to kMergeMaxBodies bodies do not come here: merge.cu sorts them.
 #include <cstring>
 
 #include "nbx_internal.cuh"
@@ -41,19 +41,14 @@ constexpr int kWarpsPerBlock = 8;
 #ifndef NBX_RADIX_SWEEP_MAX
 #define NBX_RADIX_SWEEP_MAX (3 << 19)
 #endif
-#ifndef NBX_RADIX_SWEEP_MAX_GRAPH
-#define NBX_RADIX_SWEEP_MAX_GRAPH (1 << 17)
-#endif
-// One-sweep passes below this many bodies (over all systems).  They save four
-// launches per pass, and with their own tiling of at least kTileSweep keys the
-// look-back chains stay short.  Eager builds: 4096 bodies 0.20 against 0.24 ms,
-// 2^17 0.315 against 0.403, 2^20 0.711 against 0.755; from 2^21 the counts pass
-// and the look-back cost more than the launches (1.196 against 1.114 ms, 2^23
-// 3.14 against 2.97).  In a captured graph a launch costs less and the switch
-// comes earlier: whole graph-replayed steps of 65536 bodies 0.421 against 0.442
-// ms, of 2^17 equal.
+// One-sweep passes below this many bodies (over all systems) in eager builds.
+// They save four launches per pass, and with their own tiling of at least
+// kTileSweep keys the look-back chains stay short: 2^20 bodies 0.711 against
+// 0.755 ms; from 2^21 the counts pass and the look-back cost more than the
+// launches (1.196 against 1.114 ms, 2^23 3.14 against 2.97).  In a captured
+// graph a launch costs less and the passes are equal at 2^17 already, below
+// which the keys are merged (merge.cu).
 constexpr int kSweepMaxBodies = NBX_RADIX_SWEEP_MAX;
-constexpr int kSweepMaxBodiesGraph = NBX_RADIX_SWEEP_MAX_GRAPH;
 
 struct TileMap {
     // segmented mode
@@ -523,8 +518,7 @@ int sort_bodies(Ctx *ctx, cudaStream_t st) {
 int radix_sort_bodies(Ctx *ctx, cudaStream_t st) {
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     NBX_CUDA(cudaStreamIsCapturing(st, &cs));
-    const int lim = cs == cudaStreamCaptureStatusActive ? kSweepMaxBodiesGraph : kSweepMaxBodies;
-    if (NBX_RADIX_SWEEP && ctx->nbodies < lim)
+    if (NBX_RADIX_SWEEP && cs != cudaStreamCaptureStatusActive && ctx->nbodies < kSweepMaxBodies)
         return ctx->radix_bits == 9 ? sort_bodies_sweep<9>(ctx, st) : sort_bodies_sweep<8>(ctx, st);
     return ctx->radix_bits == 9 ? sort_bodies<9>(ctx, st) : sort_bodies<8>(ctx, st);
 }
