@@ -5,6 +5,7 @@
 #include <cstdio>
 #include <cstring>
 #include <new>
+#include <utility>
 #include <vector>
 
 #include "nbx_internal.cuh"
@@ -110,7 +111,7 @@ void free_all(Ctx *ctx) {
                     ctx->d_sums, ctx->d_count, ctx->d_arrive, ctx->d_lvl8, ctx->d_hist,
                     ctx->d_scan_blk, ctx->d_totals, ctx->d_totals64, ctx->d_status, ctx->d_m2, ctx->d_com, ctx->d_quad4,
                     ctx->d_quad2, ctx->d_seg_slot, ctx->d_lb_counts, ctx->d_lb_status, ctx->d_lb, ctx->d_tiles_sw,
-                    ctx->d_sys_tiles_sw, ctx->d_tiles_mg, ctx->d_runs_mg};
+                    ctx->d_sys_tiles_sw, ctx->d_tiles_mg, ctx->d_runs_mg, ctx->d_team, ctx->d_solo};
     for (void *p : ptrs)
         if (p) cudaFree(p);
     if (ctx->h_status) cudaFreeHost(ctx->h_status);
@@ -297,6 +298,8 @@ int nbx_create(const nbx_params *p, nbx_ctx **out) {
     rc |= nbx::dmalloc(ctx, &ctx->d_tiles_mg, (size_t)B / nbx::kMergeTile + Ss + 1);
     rc |= nbx::dmalloc(ctx, &ctx->d_runs_mg, (size_t)B / nbx::kMergeRun + Ss + 1);
     rc |= nbx::dmalloc(ctx, &ctx->d_groups, G);
+    rc |= nbx::dmalloc(ctx, &ctx->d_team, G);
+    rc |= nbx::dmalloc(ctx, &ctx->d_solo, G);
     rc |= nbx::dmalloc(ctx, &ctx->d_bbox_u, 6 * Ss + 6);
     rc |= nbx::dmalloc(ctx, &ctx->d_bbox, 6 * Ss);
     rc |= nbx::dmalloc(ctx, &ctx->d_bbox64, 6 * Ss);
@@ -475,7 +478,7 @@ int nbx_set_systems(nbx_ctx *c, int nsys, const int64_t *offsets) {
     int max_sys = 0;
     std::vector<int2> st(nsys), st_sw(nsys);
     std::vector<int> slot(nsys);
-    std::vector<int> groups;
+    std::vector<int> groups, team, solo;
     int nslots = 0;
     for (int s = 0; s <= nsys; s++) off[s] = (int)offsets[s];
     for (int s = 0; s < nsys; s++) {
@@ -495,7 +498,11 @@ int nbx_set_systems(nbx_ctx *c, int nsys, const int64_t *offsets) {
             const int len = (end - a) < tile_sw ? (end - a) : tile_sw;
             tiles_sw.push_back(make_int4(a, len, s, t));
         }
-        for (int g = beg; g < end; g += 32) groups.push_back(g);
+        std::vector<int> &kind = end - beg <= nbx::kTeamMaxBodies ? team : solo;
+        for (int g = beg; g < end; g += 32) {
+            kind.push_back((int)groups.size());
+            groups.push_back(g);
+        }
         max_sys = max_sys > end - beg ? max_sys : end - beg;
     }
     if (max_sys <= nbx::kMergeMaxBodies)
@@ -518,6 +525,10 @@ int nbx_set_systems(nbx_ctx *c, int nsys, const int64_t *offsets) {
         NBX_CUDA(cudaMemcpy(ctx->d_tiles_mg, tiles_mg.data(), sizeof(int4) * tiles_mg.size(), cudaMemcpyHostToDevice));
         NBX_CUDA(cudaMemcpy(ctx->d_runs_mg, runs_mg.data(), sizeof(int4) * runs_mg.size(), cudaMemcpyHostToDevice));
     }
+    if (!team.empty() && !solo.empty()) {
+        NBX_CUDA(cudaMemcpy(ctx->d_team, team.data(), sizeof(int) * team.size(), cudaMemcpyHostToDevice));
+        NBX_CUDA(cudaMemcpy(ctx->d_solo, solo.data(), sizeof(int) * solo.size(), cudaMemcpyHostToDevice));
+    }
     NBX_CUDA(cudaMemcpy(ctx->d_groups, groups.data(), sizeof(int) * groups.size(), cudaMemcpyHostToDevice));
     nbx::k_body_sys<<<nbx::ceil_div(n, 256) < 4096 ? nbx::ceil_div(n, 256) : 4096, 256>>>(ctx->d_sys_off, nsys, n,
                                                                                           ctx->d_body_sys);
@@ -533,6 +544,8 @@ int nbx_set_systems(nbx_ctx *c, int nsys, const int64_t *offsets) {
     ctx->ntiles_mg = (int)tiles_mg.size();
     ctx->nruns_mg = (int)runs_mg.size();
     ctx->max_sys = max_sys;
+    ctx->h_team = std::move(team);
+    ctx->h_solo = std::move(solo);
     ctx->tile_body = tile;
     ctx->ngroups = (int)groups.size();
     ctx->built = false;

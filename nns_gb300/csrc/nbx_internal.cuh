@@ -5,6 +5,7 @@
 #include <stdint.h>
 
 #include <string>
+#include <vector>
 
 #include "../../include/nbx.h"
 
@@ -43,6 +44,11 @@ constexpr int kMergeFan = 16;     // most runs merged by one launch
 #define NBX_MERGE_MAX (1 << 19)
 #endif
 constexpr int kMergeMaxBodies = NBX_MERGE_MAX;
+// systems of up to this many bodies are walked by teams of warps (walk_team.cu)
+#ifndef NBX_TEAM_MAX
+#define NBX_TEAM_MAX (1 << 17)
+#endif
+constexpr int kTeamMaxBodies = NBX_TEAM_MAX;
 constexpr int kMaxRadixBits = 9;  // body-key digits: 8 or 9 bits (histograms sized for 9)
 // LSD passes over the 63-bit body keys for a digit width
 constexpr int radix_passes(int bits) { return (63 + bits - 1) / bits; }
@@ -110,6 +116,11 @@ struct Ctx {
     int ntiles_mg = 0;              // 0: a system is too large, the keys sort by radix
     int max_sys = 0;                // bodies of the largest system
     int *d_groups = nullptr;        // [G] first sorted position of each walk group
+
+    // walk groups of systems of up to kTeamMaxBodies bodies (walked by teams of
+    // warps) and of larger ones, ascending; the device copies exist in a batch of both
+    std::vector<int> h_team, h_solo;
+    int *d_team = nullptr, *d_solo = nullptr;  // [G]
 
     // per-system tree parameters
     unsigned *d_bbox_u = nullptr;   // [6S] ordered-int encodings during the reduction
@@ -244,6 +255,10 @@ int walk_forces(Ctx *ctx, const nbx_state *s, cudaStream_t st);
 int walk_forces_groups(Ctx *ctx, const nbx_state *s, int first, int count, cudaStream_t st);
 int walk_potential(Ctx *ctx, const nbx_state *s, float *pot, cudaStream_t st);
 int walk_fp64_lists(Ctx *ctx, const int *group_starts, int ngroups, double *a64, cudaStream_t st);
+// walk_team.cu
+int walk_team_init(Ctx *ctx);
+int walk_team(Ctx *ctx, const nbx_state *s, float *pot, int mode, bool quad, cudaStream_t st, const int *list,
+              int first, int count, int *rec_list, int *rec_len, int rec_cap);
 // integrate.cu
 int integrate(Ctx *ctx, const nbx_state *s, float dt, float d, int n, cudaStream_t st);
 

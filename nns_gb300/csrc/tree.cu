@@ -679,6 +679,42 @@ __device__ __forceinline__ double widen(float f) {
     return __hiloint2double((int)hi, (int)(u << 29));
 }
 
+// The float nearest to the double nearest to s / m, with one FP64 instruction
+// instead of a division: an FP32 quotient q, the exact remainder s - q m (one
+// fused product) and its FP32 quotient d give s / m to about 2^-41 of itself;
+// q + d then rounds like s / m unless it lies that close to the middle of two
+// floats (or is a power of two, zero, or out of the plain range): then divide.
+__device__ __forceinline__ float narrow(double v) {  // towards zero, in integer operations
+    const unsigned hi = (unsigned)__double2hiint(v), lo = (unsigned)__double2loint(v);
+    return __uint_as_float((hi & 0x80000000u) | ((((hi & 0x7fffffffu) - 0x38000000u) << 3) | (lo >> 29)));
+}
+__device__ __forceinline__ bool plain_range(double v) {  // 2^-60 <= |v| < 2^61
+    return (((unsigned)__double2hiint(v) & 0x7fffffffu) >> 20) - (1023u - 60u) <= 120u;
+}
+__device__ __forceinline__ float quotient32(double s, double m) {
+    if (plain_range(s) && plain_range(m)) {
+        float ri;
+        const float mf = narrow(m);
+        asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(ri) : "f"(mf));
+        const float q0 = narrow(s) * ri;  // within 2^-21; its exponent is within (-122, 122)
+        const double r = __fma_rn(-widen(q0), m, s);
+        const unsigned re = ((unsigned)__double2hiint(r) & 0x7fffffffu) >> 20;
+        if (re - (1023u - 100u) <= 200u) {  // (a zero or tiny remainder divides)
+            const float d = __fmul_rn(narrow(r), ri);
+            const float q = __fadd_rn(q0, d);
+            const float e = __fsub_rn(d, __fsub_rn(q, q0));  // exact: q + e = q0 + d
+            const unsigned qb = __float_as_uint(q);
+            const unsigned qe = (qb >> 23) & 255u;
+            if (qe - 60u <= 135u && (qb & 0x7fffffu) != 0u) {
+                const float half = __uint_as_float((qe - 24u) << 23);   // half a unit in the last place of q
+                const float tol = __uint_as_float((qe - 38u) << 23);    // 2^-38 of q's binade
+                if (half - fabsf(e) > tol) return q;
+            }
+        }
+    }
+    return (float)(s / m);
+}
+
 // Moments of a cell by a group of lanes (4, or 8 with quadrupoles), lane k of
 // the group holding component k & 3 of (m, m x, m y, m z): the children are
 // summed in child order, one FP64 instruction per child for all components
@@ -774,16 +810,22 @@ __device__ __forceinline__ void quad_cell(int k, int b, int first, int nch, doub
 
 // A cell's sums, and (finish) its centre of mass, node record and quadrupole.
 template <bool Quad>
-__device__ __forceinline__ double finish_cell(int k, int b, int first, int nch, double acc, const int *__restrict__ meta,
+__device__ __forceinline__ void finish_cell(int k, int b, int first, int nch, double acc, const int *__restrict__ meta,
                                               float4 *node4, const double4 *sums, double *com, double2 *m2,
                                               float4 *quad4, float2 *quad2) {
     constexpr int kLanes = Quad ? 8 : 4;
     const int kc = k & 3;
     const double m = __shfl_sync(0xffffffffu, acc, (threadIdx.x & 31) & ~(kLanes - 1));
+    if (!Quad) {
+        if (nch > 0) {
+            const float f = kc == 0 ? (float)acc : quotient32(acc, m);
+            reinterpret_cast<float *>(&node4[b])[kc == 0 ? 3 : kc - 1] = f;
+        }
+        return;
+    }
     const double q = kc == 0 ? acc : acc / (nch > 0 ? m : 1.0);
     if (k < 4 && nch > 0) reinterpret_cast<float *>(&node4[b])[kc == 0 ? 3 : kc - 1] = (float)q;
-    if (Quad) quad_cell(k, b, first, nch, q, meta, node4, sums, com, m2, quad4, quad2);
-    return q;
+    quad_cell(k, b, first, nch, q, meta, node4, sums, com, m2, quad4, quad2);
 }
 
 // Bottom-up FP64 moments, one BFS level per launch (deepest first): a cell sums

@@ -26,8 +26,10 @@
 // Accumulation modes: 0 plain FP32 (two packed partial sums), 1 split
 // compensation (plain FP32 within a round, Kahan across rounds), 2 Kahan on
 // every term.  Optional per-body potential for the energy diagnostics.
-#include "f32x2.cuh"
+#include <algorithm>
+
 #include "nbx_internal.cuh"
+#include "walk_eval.cuh"
 
 namespace nbx {
 
@@ -63,19 +65,6 @@ constexpr int kDfsReserve = 7 * 42 + 8;
 constexpr int kBodyUnroll = NBX_BODY_UNROLL;
 constexpr int kCellUnroll = NBX_CELL_UNROLL;
 
-// depth0 * 4^-k exactly (a power-of-two product is exact unless it underflows)
-__device__ __forceinline__ float scale4(float d0, int k) {
-    return d0 * __int_as_float((127 - 2 * k) << 23);
-}
-
-// Kahan step s += v with compensation c (scalar, explicit rounding).
-__device__ __forceinline__ void kahan(float &s, float &c, float v) {
-    const float y = __fsub_rn(v, c);
-    const float t = __fadd_rn(s, y);
-    c = __fsub_rn(__fsub_rn(t, s), y);
-    s = t;
-}
-
 // Per-warp candidate buffers of CB slots each.
 template <int CB>
 struct WarpBuf {
@@ -92,114 +81,6 @@ struct WarpBuf {
     u64 rz[8];              //                                  (z0,z1)
 };
 
-__device__ __forceinline__ void put4(ulonglong2 *a, ulonglong2 *b, int slot, float4 q) {
-    float *pa = reinterpret_cast<float *>(&a[slot >> 1]);
-    float *pb = reinterpret_cast<float *>(&b[slot >> 1]);
-    const int h = slot & 1;
-    pa[h] = q.x;
-    pa[2 + h] = q.y;
-    pb[h] = q.z;
-    pb[2 + h] = q.w;
-}
-
-// Quadrupole mode: the traceless quadrupoles of the cell buffer's slots, in
-// pairs: (xx, yy), (zz, xy), (xz, yz).
-template <int CB>
-struct QuadBuf {
-    static constexpr int kPairs = CB / 2;
-    ulonglong2 qa[kPairs];
-    ulonglong2 qb[kPairs];
-    ulonglong2 qc[kPairs];
-};
-
-__device__ __forceinline__ void putq(ulonglong2 *qa, ulonglong2 *qb, ulonglong2 *qc, int slot, float4 q4, float2 q2) {
-    float *pa = reinterpret_cast<float *>(&qa[slot >> 1]);
-    float *pb = reinterpret_cast<float *>(&qb[slot >> 1]);
-    float *pc = reinterpret_cast<float *>(&qc[slot >> 1]);
-    const int h = slot & 1;
-    pa[h] = q4.x;
-    pa[2 + h] = q4.y;
-    pb[h] = q4.z;
-    pb[2 + h] = q4.w;
-    pc[h] = q2.x;
-    pc[2 + h] = q2.y;
-}
-
-struct Sums {
-    u64 x = 0ull, y = 0ull, z = 0ull, p = 0ull;  // packed partial sums (+0.0f, +0.0f)
-    float kx = 0.f, ky = 0.f, kz = 0.f, cx = 0.f, cy = 0.f, cz = 0.f;  // Kahan totals
-};
-
-// Accumulate the packed force factor f = m*rsqrt(r)^3 of two candidates.
-template <int Mode, bool Pot>
-__device__ __forceinline__ void accumulate(Sums &a, u64 f, u64 mm, u64 ri, u64 dx, u64 dy, u64 dz) {
-    if (Mode == 2) {
-        float xa, xb, ya, yb, za, zb;
-        upk(mul2(f, dx), xa, xb);
-        upk(mul2(f, dy), ya, yb);
-        upk(mul2(f, dz), za, zb);
-        kahan(a.kx, a.cx, xa);
-        kahan(a.kx, a.cx, xb);
-        kahan(a.ky, a.cy, ya);
-        kahan(a.ky, a.cy, yb);
-        kahan(a.kz, a.cz, za);
-        kahan(a.kz, a.cz, zb);
-    } else {
-        a.x = fma2(f, dx, a.x);
-        a.y = fma2(f, dy, a.y);
-        a.z = fma2(f, dz, a.z);
-    }
-    if (Pot) a.p = fma2(mm, ri, a.p);
-}
-
-// Accumulate r^-2 v for two candidates: the quadrupole mode's contribution.
-template <int Mode>
-__device__ __forceinline__ void accumulate_quad(Sums &a, u64 ri2, u64 vx, u64 vy, u64 vz) {
-    if (Mode == 2) {
-        float xa, xb, ya, yb, za, zb;
-        upk(mul2(ri2, vx), xa, xb);
-        upk(mul2(ri2, vy), ya, yb);
-        upk(mul2(ri2, vz), za, zb);
-        kahan(a.kx, a.cx, xa);
-        kahan(a.kx, a.cx, xb);
-        kahan(a.ky, a.cy, ya);
-        kahan(a.ky, a.cy, yb);
-        kahan(a.kz, a.cz, za);
-        kahan(a.kz, a.cz, zb);
-    } else {
-        a.x = fma2(ri2, vx, a.x);
-        a.y = fma2(ri2, vy, a.y);
-        a.z = fma2(ri2, vz, a.z);
-    }
-}
-
-// One pair of cells of the quadrupole mode, with the cells' negated traceless
-// quadrupoles P = -Q from slot pair q of the buffer (d = cell - body,
-// r^2 = |d|^2 + eps^2, e = d / r):
-//   a += m d r^-3 - Q d r^-5 + 5/2 (d.Q.d) d r^-7
-//      = r^-2 [ (m - 5/2 (e.P.e) r^-2) e + (P e) r^-2 ].
-// In the unit-vector form every intermediate is bounded by |Q| or by the
-// mass and force scales, and the only power of r^-1 is r^-2 <= 1 / eps^2.
-// With d itself, r^-5 and r^-7 overflow FP32 once r is below about 1e-8, and
-// d.Q.d (~ |Q| d^2) underflows for cells of about 1e-12 and less, dropping a
-// term that is 1e-2 of such a pair's force.  A rejected half of a voted pair
-// comes with ri = 0, so its e and r^-2, and its whole term, are 0.
-template <int Mode, int CB>
-__device__ __forceinline__ void quad_term(Sums &acc, const QuadBuf<CB> &qbuf, int q, u64 mm, u64 ri, u64 dx, u64 dy,
-                                          u64 dz) {
-    const ulonglong2 QA = qbuf.qa[q], QB = qbuf.qb[q], QC = qbuf.qc[q];
-    const u64 ri2 = mul2(ri, ri);
-    const u64 ex = mul2(dx, ri), ey = mul2(dy, ri), ez = mul2(dz, ri);
-    // P e: P = (xx, yy, zz, xy | xz, yz) in QA = (xx, yy), QB = (zz, xy), QC = (xz, yz)
-    const u64 px = fma2(QC.x, ez, fma2(QB.y, ey, mul2(QA.x, ex)));
-    const u64 py = fma2(QC.y, ez, fma2(QA.y, ey, mul2(QB.y, ex)));
-    const u64 pz = fma2(QB.x, ez, fma2(QC.y, ey, mul2(QC.x, ex)));
-    const u64 epe = fma2(ez, pz, fma2(ey, py, mul2(ex, px)));
-    const u64 mq = fma2(mul2(epe, ri2), pk(-2.5f, -2.5f), mm);
-    accumulate_quad<Mode>(acc, ri2, fma2(mq, ex, mul2(px, ri2)), fma2(mq, ey, mul2(py, ri2)),
-                          fma2(mq, ez, mul2(pz, ri2)));
-}
-
 // CB = 64 and 96: 64-register budget (two 16-warp or four 8-warp blocks per SM);
 // CB = 128: up to 85 registers for more loads in flight (three 8-warp blocks).
 template <int CB>
@@ -212,7 +93,7 @@ template <int CB, int Mode, bool Pot, bool Rec, bool Quad = false>
 __global__ void __launch_bounds__(WalkBounds<CB>::kThreads, WalkBounds<CB>::kMinBlocks)
     k_walk2(const float4 *__restrict__ node4, const int *__restrict__ meta, const unsigned char *__restrict__ lvl8,
             const float4 *__restrict__ quad4, const float2 *__restrict__ quad2, const float4 *__restrict__ body4,
-            const int *__restrict__ val, const int *__restrict__ groups, int ngroups,
+            const int *__restrict__ val, const int *__restrict__ groups, const int *__restrict__ list, int ngroups,
             const int *__restrict__ body_sys, const int *__restrict__ sys_off, const float *__restrict__ depth0,
             const int *__restrict__ root_first, const int *__restrict__ root_nch, const int *__restrict__ sys_lvl,
             float eps2, int stack_cap,
@@ -238,6 +119,7 @@ __global__ void __launch_bounds__(WalkBounds<CB>::kThreads, WalkBounds<CB>::kMin
         if (lane == 0) g = (int)atomicAdd(&st->walk_next, 1u);
         g = __shfl_sync(0xffffffffu, g, 0);
         if (g >= ngroups) break;
+        if (list) g = list[g];
         const int p0 = groups[g];
         const int s = body_sys[p0];
         const int end = min(sys_off[s + 1], p0 + 32);
@@ -642,10 +524,16 @@ __global__ void __launch_bounds__(WalkBounds<CB>::kThreads, WalkBounds<CB>::kMin
     }
 }
 
+// Which groups one launch walks: `count` from the first, or the entries of a list
+// (device array) from there on.
+struct Share {
+    const int *list;
+    int first, count;
+};
+
 template <int CB, int Mode, bool Pot, bool Rec = false, bool Quad = false>
-int launch(Ctx *ctx, const nbx_state *s, float *pot, int warps, cudaStream_t st, int *rec_list = nullptr,
-           int *rec_len = nullptr, int rec_cap = 0, int g_first = 0, int g_count = -1) {
-    if (g_count < 0) g_count = ctx->ngroups - g_first;
+int launch(Ctx *ctx, const nbx_state *s, float *pot, int warps, cudaStream_t st, Share share,
+           int *rec_list = nullptr, int *rec_len = nullptr, int rec_cap = 0) {
     const int cap = ctx->p.stack_depth;
     const size_t smem = (size_t)warps * (sizeof(WarpBuf<CB>) + (Quad ? sizeof(QuadBuf<CB>) : 0) +
                                          (size_t)cap * sizeof(int));
@@ -653,19 +541,21 @@ int launch(Ctx *ctx, const nbx_state *s, float *pot, int warps, cudaStream_t st,
         ctx->last_error = "walk: stack_depth too large for the launch shape's shared memory";
         return NBX_ERR_ARG;
     }
-    const int blocks_needed = ceil_div(g_count, warps);
+    if (share.count <= 0) return NBX_OK;
+    const int blocks_needed = ceil_div(share.count, warps);
     int per_sm = 1;
     NBX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_walk2<CB, Mode, Pot, Rec, Quad>, warps * 32,
                                                            smem));
     if (per_sm < 1) per_sm = 1;
     const int grid = blocks_needed < ctx->nsm * per_sm ? blocks_needed : ctx->nsm * per_sm;
-    if (grid <= 0) return NBX_OK;
+    // without a list the group arrays start at the first group
+    const int off = share.list ? 0 : share.first;
     NBX_CUDA(cudaMemsetAsync(&ctx->d_status->walk_next, 0, sizeof(unsigned), st));
     k_walk2<CB, Mode, Pot, Rec, Quad><<<grid, warps * 32, smem, st>>>(
         ctx->d_node4, ctx->d_meta, ctx->d_lvl8, ctx->d_quad4, ctx->d_quad2, ctx->d_body4, ctx->d_val,
-        ctx->d_groups + g_first, g_count, ctx->d_body_sys, ctx->d_sys_off, ctx->d_depth0, ctx->d_root_first,
-        ctx->d_root_nch, ctx->d_sys_lvl, ctx->eps2, cap, s->ax, s->ay, s->az, pot, ctx->d_gstat + g_first, ctx->d_status, rec_list,
-        rec_len, rec_cap);
+        ctx->d_groups + off, share.list ? share.list + share.first : nullptr, share.count, ctx->d_body_sys,
+        ctx->d_sys_off, ctx->d_depth0, ctx->d_root_first, ctx->d_root_nch, ctx->d_sys_lvl, ctx->eps2, cap, s->ax,
+        s->ay, s->az, pot, ctx->d_gstat + off, ctx->d_status, rec_list, rec_len, rec_cap);
     ++ctx->launches;
     NBX_CUDA(cudaGetLastError());
     return NBX_OK;
@@ -679,28 +569,38 @@ int set_attr(Ctx *ctx, int smem_max) {
 }
 
 template <int CB>
-int forces_cb(Ctx *ctx, const nbx_state *s, float *pot, int warps, cudaStream_t st, int g0, int gn) {
-    if (pot) return launch<CB, 0, true>(ctx, s, pot, warps, st, nullptr, nullptr, 0, g0, gn);
+int forces_cb(Ctx *ctx, const nbx_state *s, float *pot, int warps, cudaStream_t st, Share share) {
+    if (pot) return launch<CB, 0, true>(ctx, s, pot, warps, st, share);
     if (ctx->multipole) {
-        if (!ctx->d_quad4) return NBX_ERR_STATE;
         switch (ctx->compensated) {
-            case 1: return launch<CB, 1, false, false, true>(ctx, s, nullptr, warps, st, nullptr, nullptr, 0, g0, gn);
-            case 2: return launch<CB, 2, false, false, true>(ctx, s, nullptr, warps, st, nullptr, nullptr, 0, g0, gn);
-            default: return launch<CB, 0, false, false, true>(ctx, s, nullptr, warps, st, nullptr, nullptr, 0, g0, gn);
+            case 1: return launch<CB, 1, false, false, true>(ctx, s, nullptr, warps, st, share);
+            case 2: return launch<CB, 2, false, false, true>(ctx, s, nullptr, warps, st, share);
+            default: return launch<CB, 0, false, false, true>(ctx, s, nullptr, warps, st, share);
         }
     }
     switch (ctx->compensated) {
-        case 1: return launch<CB, 1, false>(ctx, s, nullptr, warps, st, nullptr, nullptr, 0, g0, gn);
-        case 2: return launch<CB, 2, false>(ctx, s, nullptr, warps, st, nullptr, nullptr, 0, g0, gn);
-        default: return launch<CB, 0, false>(ctx, s, nullptr, warps, st, nullptr, nullptr, 0, g0, gn);
+        case 1: return launch<CB, 1, false>(ctx, s, nullptr, warps, st, share);
+        case 2: return launch<CB, 2, false>(ctx, s, nullptr, warps, st, share);
+        default: return launch<CB, 0, false>(ctx, s, nullptr, warps, st, share);
     }
+}
+
+// The groups [g0, g0 + gn) of one kind (walked by teams, or by single warps), as
+// a share: of a context whose groups are all of one kind, the range itself;
+// of a batch of both kinds, a stretch of that kind's ascending list.
+Share share_of(const Ctx *ctx, bool team, int g0, int gn) {
+    const std::vector<int> &mine = team ? ctx->h_team : ctx->h_solo;
+    if ((int)mine.size() == ctx->ngroups) return {nullptr, g0, gn};
+    const int a = (int)(std::lower_bound(mine.begin(), mine.end(), g0) - mine.begin());
+    const int b = (int)(std::lower_bound(mine.begin(), mine.end(), g0 + gn) - mine.begin());
+    return {team ? ctx->d_team : ctx->d_solo, a, b - a};
 }
 
 }  // namespace
 
 int walk2_init(Ctx *ctx) {
     const int smem_optin = ctx->smem_optin;
-    int rc = 0;
+    int rc = walk_team_init(ctx);
     rc |= set_attr<64, 0, false>(ctx, smem_optin);
     rc |= set_attr<64, 1, false>(ctx, smem_optin);
     rc |= set_attr<64, 2, false>(ctx, smem_optin);
@@ -729,21 +629,38 @@ int walk2_init(Ctx *ctx) {
 // Plain walk that also records every group's interaction list (node ids, in
 // evaluation order) into rec_list[g * rec_cap ...], its length into rec_len[g].
 int walk2_record(Ctx *ctx, const nbx_state *s, int *rec_list, int *rec_len, int rec_cap, cudaStream_t st) {
-    return launch<96, 0, false, true>(ctx, s, nullptr, ctx->walk_warps, st, rec_list, rec_len, rec_cap);
+    const int rc = launch<96, 0, false, true>(ctx, s, nullptr, ctx->walk_warps, st,
+                                              share_of(ctx, false, 0, ctx->ngroups), rec_list, rec_len, rec_cap);
+    if (rc) return rc;
+    const Share t = share_of(ctx, true, 0, ctx->ngroups);
+    return walk_team(ctx, s, nullptr, 0, false, st, t.list, t.first, t.count, rec_list, rec_len, rec_cap);
 }
 
 // The same walk without recording: the recording adds stores only, so both
 // give the same forces bit for bit (the adjoint's forward and recompute).
 int walk2_unrecorded(Ctx *ctx, const nbx_state *s, cudaStream_t st) {
-    return launch<96, 0, false, false>(ctx, s, nullptr, ctx->walk_warps, st, nullptr, nullptr, 0);
+    const int rc = launch<96, 0, false, false>(ctx, s, nullptr, ctx->walk_warps, st,
+                                               share_of(ctx, false, 0, ctx->ngroups));
+    if (rc) return rc;
+    const Share t = share_of(ctx, true, 0, ctx->ngroups);
+    return walk_team(ctx, s, nullptr, 0, false, st, t.list, t.first, t.count, nullptr, nullptr, 0);
 }
 
-// variant 0: 64-slot candidate buffers; 1: 128-slot buffers (<= 8 warps); 3: 96-slot buffers.
+// variant 0: 64-slot candidate buffers; 1: 128-slot buffers (<= 8 warps); 3: 96-slot buffers
+// (of the single-warp walk; small systems' groups are walked by teams, whose shape is fixed).
 // Walk groups [g0, g0 + gn) of the last build (gn < 0: all groups from g0).
 int walk2_forces(Ctx *ctx, const nbx_state *s, float *pot, int warps, cudaStream_t st, int g0, int gn) {
-    if (ctx->walk_variant == 1) return forces_cb<128>(ctx, s, pot, warps > 8 ? 8 : warps, st, g0, gn);
-    if (ctx->walk_variant == 3) return forces_cb<96>(ctx, s, pot, warps, st, g0, gn);
-    return forces_cb<64>(ctx, s, pot, warps, st, g0, gn);
+    if (gn < 0) gn = ctx->ngroups - g0;
+    if (!pot && ctx->multipole && !ctx->d_quad4) return NBX_ERR_STATE;
+    const Share r = share_of(ctx, false, g0, gn), t = share_of(ctx, true, g0, gn);
+    // (a launch shape that does not fit is refused whatever the groups' kind)
+    int rc;
+    if (ctx->walk_variant == 1) rc = forces_cb<128>(ctx, s, pot, warps > 8 ? 8 : warps, st, r);
+    else if (ctx->walk_variant == 3) rc = forces_cb<96>(ctx, s, pot, warps, st, r);
+    else rc = forces_cb<64>(ctx, s, pot, warps, st, r);
+    if (rc) return rc;
+    return walk_team(ctx, s, pot, ctx->compensated, ctx->multipole != 0, st, t.list, t.first, t.count, nullptr,
+                     nullptr, 0);
 }
 
 }  // namespace nbx

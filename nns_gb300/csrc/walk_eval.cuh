@@ -1,0 +1,131 @@
+// walk_eval.cuh -- evaluation pieces shared by the force walks (walk2.cu,
+// walk_team.cu): candidate slots, packed force terms, accumulation modes.
+#pragma once
+
+#include "f32x2.cuh"
+#include "nbx_internal.cuh"
+
+namespace nbx {
+
+// depth0 * 4^-k exactly (a power-of-two product is exact unless it underflows)
+__device__ __forceinline__ float scale4(float d0, int k) {
+    return d0 * __int_as_float((127 - 2 * k) << 23);
+}
+
+// Kahan step s += v with compensation c (scalar, explicit rounding).
+__device__ __forceinline__ void kahan(float &s, float &c, float v) {
+    const float y = __fsub_rn(v, c);
+    const float t = __fadd_rn(s, y);
+    c = __fsub_rn(__fsub_rn(t, s), y);
+    s = t;
+}
+
+__device__ __forceinline__ void put4(ulonglong2 *a, ulonglong2 *b, int slot, float4 q) {
+    float *pa = reinterpret_cast<float *>(&a[slot >> 1]);
+    float *pb = reinterpret_cast<float *>(&b[slot >> 1]);
+    const int h = slot & 1;
+    pa[h] = q.x;
+    pa[2 + h] = q.y;
+    pb[h] = q.z;
+    pb[2 + h] = q.w;
+}
+
+// Quadrupole mode: the traceless quadrupoles of the cell buffer's slots, in
+// pairs: (xx, yy), (zz, xy), (xz, yz).
+template <int CB>
+struct QuadBuf {
+    static constexpr int kPairs = CB / 2;
+    ulonglong2 qa[kPairs];
+    ulonglong2 qb[kPairs];
+    ulonglong2 qc[kPairs];
+};
+
+__device__ __forceinline__ void putq(ulonglong2 *qa, ulonglong2 *qb, ulonglong2 *qc, int slot, float4 q4, float2 q2) {
+    float *pa = reinterpret_cast<float *>(&qa[slot >> 1]);
+    float *pb = reinterpret_cast<float *>(&qb[slot >> 1]);
+    float *pc = reinterpret_cast<float *>(&qc[slot >> 1]);
+    const int h = slot & 1;
+    pa[h] = q4.x;
+    pa[2 + h] = q4.y;
+    pb[h] = q4.z;
+    pb[2 + h] = q4.w;
+    pc[h] = q2.x;
+    pc[2 + h] = q2.y;
+}
+
+struct Sums {
+    u64 x = 0ull, y = 0ull, z = 0ull, p = 0ull;  // packed partial sums (+0.0f, +0.0f)
+    float kx = 0.f, ky = 0.f, kz = 0.f, cx = 0.f, cy = 0.f, cz = 0.f;  // Kahan totals
+};
+
+// Accumulate the packed force factor f = m*rsqrt(r)^3 of two candidates.
+template <int Mode, bool Pot>
+__device__ __forceinline__ void accumulate(Sums &a, u64 f, u64 mm, u64 ri, u64 dx, u64 dy, u64 dz) {
+    if (Mode == 2) {
+        float xa, xb, ya, yb, za, zb;
+        upk(mul2(f, dx), xa, xb);
+        upk(mul2(f, dy), ya, yb);
+        upk(mul2(f, dz), za, zb);
+        kahan(a.kx, a.cx, xa);
+        kahan(a.kx, a.cx, xb);
+        kahan(a.ky, a.cy, ya);
+        kahan(a.ky, a.cy, yb);
+        kahan(a.kz, a.cz, za);
+        kahan(a.kz, a.cz, zb);
+    } else {
+        a.x = fma2(f, dx, a.x);
+        a.y = fma2(f, dy, a.y);
+        a.z = fma2(f, dz, a.z);
+    }
+    if (Pot) a.p = fma2(mm, ri, a.p);
+}
+
+// Accumulate r^-2 v for two candidates: the quadrupole mode's contribution.
+template <int Mode>
+__device__ __forceinline__ void accumulate_quad(Sums &a, u64 ri2, u64 vx, u64 vy, u64 vz) {
+    if (Mode == 2) {
+        float xa, xb, ya, yb, za, zb;
+        upk(mul2(ri2, vx), xa, xb);
+        upk(mul2(ri2, vy), ya, yb);
+        upk(mul2(ri2, vz), za, zb);
+        kahan(a.kx, a.cx, xa);
+        kahan(a.kx, a.cx, xb);
+        kahan(a.ky, a.cy, ya);
+        kahan(a.ky, a.cy, yb);
+        kahan(a.kz, a.cz, za);
+        kahan(a.kz, a.cz, zb);
+    } else {
+        a.x = fma2(ri2, vx, a.x);
+        a.y = fma2(ri2, vy, a.y);
+        a.z = fma2(ri2, vz, a.z);
+    }
+}
+
+// One pair of cells of the quadrupole mode, with the cells' negated traceless
+// quadrupoles P = -Q from slot pair q of the buffer (d = cell - body,
+// r^2 = |d|^2 + eps^2, e = d / r):
+//   a += m d r^-3 - Q d r^-5 + 5/2 (d.Q.d) d r^-7
+//      = r^-2 [ (m - 5/2 (e.P.e) r^-2) e + (P e) r^-2 ].
+// In the unit-vector form every intermediate is bounded by |Q| or by the
+// mass and force scales, and the only power of r^-1 is r^-2 <= 1 / eps^2.
+// With d itself, r^-5 and r^-7 overflow FP32 once r is below about 1e-8, and
+// d.Q.d (~ |Q| d^2) underflows for cells of about 1e-12 and less, dropping a
+// term that is 1e-2 of such a pair's force.  A rejected half of a voted pair
+// comes with ri = 0, so its e and r^-2, and its whole term, are 0.
+template <int Mode, int CB>
+__device__ __forceinline__ void quad_term(Sums &acc, const QuadBuf<CB> &qbuf, int q, u64 mm, u64 ri, u64 dx, u64 dy,
+                                          u64 dz) {
+    const ulonglong2 QA = qbuf.qa[q], QB = qbuf.qb[q], QC = qbuf.qc[q];
+    const u64 ri2 = mul2(ri, ri);
+    const u64 ex = mul2(dx, ri), ey = mul2(dy, ri), ez = mul2(dz, ri);
+    // P e: P = (xx, yy, zz, xy | xz, yz) in QA = (xx, yy), QB = (zz, xy), QC = (xz, yz)
+    const u64 px = fma2(QC.x, ez, fma2(QB.y, ey, mul2(QA.x, ex)));
+    const u64 py = fma2(QC.y, ez, fma2(QA.y, ey, mul2(QB.y, ex)));
+    const u64 pz = fma2(QB.x, ez, fma2(QC.y, ey, mul2(QC.x, ex)));
+    const u64 epe = fma2(ez, pz, fma2(ey, py, mul2(ex, px)));
+    const u64 mq = fma2(mul2(epe, ri2), pk(-2.5f, -2.5f), mm);
+    accumulate_quad<Mode>(acc, ri2, fma2(mq, ex, mul2(px, ri2)), fma2(mq, ey, mul2(py, ri2)),
+                          fma2(mq, ez, mul2(pz, ri2)));
+}
+
+}  // namespace nbx

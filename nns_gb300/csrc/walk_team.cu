@@ -1,0 +1,597 @@
+// walk_team.cu -- the force walk of small and mid-size systems: the interaction
+// lists and evaluation of walk2.cu, with a team of warps (one block) per group
+// of 32 bodies.
+//
+// One warp per group leaves most of the GPU idle below about 10^5 bodies, and
+// the longest group's chain of rounds (load a cell, load its children, classify,
+// evaluate up to 96 candidates: about 2.4 us) is the walk's time.  Here every
+// warp holds the same 32 bodies and takes its own share of a round's children:
+//   expand   all warps pop the same top-of-stack cells (the shared stack holds
+//            each cell's record and level, so a pop loads nothing from memory),
+//            list their children in shared memory and classify the list's
+//            32-child chunks in turn, warp w the chunks w, w + W, ...;
+//   evaluate each warp evaluates and votes on its own candidates;
+//   push     after a barrier the warps append their rejected cells to the stack
+//            in warp order.
+// The tests, and so the lists, are those of walk2.cu; the sums are the W warps'
+// partial sums added in warp order, so a group's force bits depend on its own
+// system only.  Which systems are walked by teams depends on the system's size
+// alone (kTeamMaxBodies): a batch gives every system the bits of its single run.
+#include "nbx_internal.cuh"
+#include "walk_eval.cuh"
+
+namespace nbx {
+
+namespace {
+
+constexpr int kW = 4;                      // warps of a team
+constexpr int kChunks = 3;                 // 32-child chunks per warp and round
+constexpr int kPops = 4;                   // cells popped per lane and round, at most
+constexpr int kRound = 32 * kW * kChunks;  // most children of a round
+constexpr int kSlots = 32 * kChunks + 8;   // candidate slots per warp (its children, pads of the pair loops)
+constexpr int kStackMul = 2;               // stack entries of a team per stack_depth
+
+// Node ids of a round's candidates (recording only).
+template <bool Rec>
+struct TeamIds {
+    int cid[kSlots];  // cells to vote on
+    int bid[kSlots];  // the round's interactions
+};
+template <>
+struct TeamIds<false> {};
+
+// Per-warp candidate buffers.  The bodies (and, without quadrupoles, the surely
+// accepted cells) fill the slots upwards, the cells to vote on downwards in
+// pairs; with quadrupoles the cells are in the second arrays, those to vote on
+// upwards, the surely accepted ones downwards.
+template <bool Rec, bool Quad>
+struct TeamBuf {
+    static constexpr int kPairs = kSlots / 2, kCellPairs = Quad ? kPairs : 1;
+    ulonglong2 ba[kPairs], bb[kPairs];          // (x0,x1) (y0,y1); (z0,z1) (m0,m1)
+    ulonglong2 ca[kCellPairs], cb[kCellPairs];  // quadrupole mode: cells
+    float cd[kSlots];                           // cells to vote on: opening thresholds
+    u64 crec[kSlots];                           // their stack entries
+    u64 rej[32 * kChunks];                      // rejected cells' stack entries
+    TeamIds<Rec> ids;
+    // slot of the i-th cell to vote on
+    __device__ static int vote_slot(int i) { return Quad ? i : kSlots - 2 - 2 * (i >> 1) + (i & 1); }
+    __device__ ulonglong2 *cells_a() { return Quad ? ca : ba; }
+    __device__ ulonglong2 *cells_b() { return Quad ? cb : bb; }
+};
+
+// A warp's partial results, written over its buffers after the last round.
+struct TeamPart {
+    float a[6][32];  // sums and their compensations
+    float pot[32];
+};
+static_assert(sizeof(TeamPart) <= sizeof(TeamBuf<false, false>), "the partial results replace the buffers");
+
+struct TeamShared {
+    float4 cls[3];      // group box lo, hi, centre
+    ulonglong2 rxy[8];  // representative bodies, in pairs: (x0,x1) (y0,y1)
+    u64 rz[8];          //                                  (z0,z1)
+    int nrej[kW], nrec[kW];
+    int sum[kW][4];     // list length, opened cells, candidates
+    u64 child[kRound];  // the round's children: node, level of its parent
+};
+
+static_assert(sizeof(TeamShared) % 16 == 0 && sizeof(TeamBuf<false, false>) % 16 == 0 &&
+                  sizeof(TeamBuf<true, false>) % 16 == 0 && sizeof(TeamBuf<false, true>) % 16 == 0,
+              "16-byte slots");
+
+__device__ __forceinline__ u64 entry_of(int cm, int lvl) { return (u64)(unsigned)cm | (u64)(unsigned)lvl << 32; }
+
+template <int Mode, bool Pot, bool Rec, bool Quad>
+__global__ void __launch_bounds__(kW * 32, 32 / kW)
+    k_walk_team(const float4 *__restrict__ node4, const int *__restrict__ meta, const float4 *__restrict__ quad4,
+                const float2 *__restrict__ quad2, const float4 *__restrict__ body4, const int *__restrict__ val,
+                const int *__restrict__ groups, const int *__restrict__ list, int g_first,
+                const int *__restrict__ body_sys, const int *__restrict__ sys_off, const float *__restrict__ depth0,
+                const int *__restrict__ root_first, const int *__restrict__ root_nch, const int *__restrict__ sys_lvl,
+                float eps2, int stack_cap, float *__restrict__ ax, float *__restrict__ ay, float *__restrict__ az,
+                float *__restrict__ pot, int2 *__restrict__ gstat, DevStatus *st, int *__restrict__ rec_list,
+                int *__restrict__ rec_len, int rec_cap) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    if (st->code != 0) return;
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    TeamShared &sh = *reinterpret_cast<TeamShared *>(smem_raw);
+    TeamBuf<Rec, Quad> *bufs = reinterpret_cast<TeamBuf<Rec, Quad> *>(smem_raw + sizeof(TeamShared));
+    TeamBuf<Rec, Quad> &buf = bufs[w];
+    const auto part = [&](int v) -> TeamPart & { return *reinterpret_cast<TeamPart *>(&bufs[v]); };
+    QuadBuf<kSlots> &qbuf =
+        reinterpret_cast<QuadBuf<kSlots> *>(smem_raw + sizeof(TeamShared) + kW * sizeof(TeamBuf<Rec, Quad>))[w];
+    u64 *stack = reinterpret_cast<u64 *>(smem_raw + sizeof(TeamShared) + kW * sizeof(TeamBuf<Rec, Quad>) +
+                                         (Quad ? kW * sizeof(QuadBuf<kSlots>) : 0));
+    const unsigned lt = (1u << lane) - 1u;
+    const u64 eps2x2 = pk(eps2, eps2);
+    const int g = list ? list[g_first + blockIdx.x] : g_first + (int)blockIdx.x;
+    const int p0 = groups[g];
+    const int s = body_sys[p0];
+    const int end = min(sys_off[s + 1], p0 + 32);
+    const int reserve = 7 * min(max(sys_lvl[s], 1), 42) + 8;
+    const int p = p0 + lane;
+    const bool valid = p < end;
+    // lanes past the end of the system take lane 0's body (their votes repeat its)
+    const float4 me = body4[valid ? p : p0];
+    const u64 px = pk(me.x, me.x), py = pk(me.y, me.y), pz = pk(me.z, me.z);
+    const float d0 = depth0[s];
+    {
+        // the group's box and, per octant, its representative pair (walk2.cu): warp w
+        // finds the octants w, w + W
+        float b[6] = {me.x, me.x, me.y, me.y, me.z, me.z};
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+#pragma unroll
+            for (int k = 0; k < 6; k += 2) {
+                b[k] = fminf(b[k], __shfl_xor_sync(0xffffffffu, b[k], o));
+                b[k + 1] = fmaxf(b[k + 1], __shfl_xor_sync(0xffffffffu, b[k + 1], o));
+            }
+        }
+        const float ex = me.x - 0.5f * (b[0] + b[1]), ey = me.y - 0.5f * (b[2] + b[3]);
+        const float ez = me.z - 0.5f * (b[4] + b[5]);
+        const unsigned key = __float_as_uint(ex * ex + ey * ey + ez * ez);
+        const unsigned kmin = __reduce_min_sync(0xffffffffu, key);
+        const int lc = __ffs(__ballot_sync(0xffffffffu, key == kmin)) - 1;
+        if (threadIdx.x == 0) {
+            sh.cls[0] = make_float4(b[0], b[2], b[4], 0.f);
+            sh.cls[1] = make_float4(b[1], b[3], b[5], 0.f);
+            sh.cls[2] = make_float4(0.5f * (b[0] + b[1]), 0.5f * (b[2] + b[3]), 0.5f * (b[4] + b[5]), 0.f);
+        }
+        const float nx = __shfl_sync(0xffffffffu, me.x, lc), ny = __shfl_sync(0xffffffffu, me.y, lc);
+        const float nz = __shfl_sync(0xffffffffu, me.z, lc);
+        for (int k = w; k < 8; k += kW) {
+            const float pj = (k & 1 ? ex : -ex) + (k & 2 ? ey : -ey) + (k & 4 ? ez : -ez);
+            const unsigned key_k = valid ? f2ord(pj) : 0u;
+            const unsigned kmax = __reduce_max_sync(0xffffffffu, key_k);
+            const int lf = __ffs(__ballot_sync(0xffffffffu, key_k == kmax)) - 1;
+            const float xk = __shfl_sync(0xffffffffu, me.x, lf), yk = __shfl_sync(0xffffffffu, me.y, lf);
+            const float zk = __shfl_sync(0xffffffffu, me.z, lf);
+            if (lane == k) {
+                sh.rxy[k] = make_ulonglong2(pk(xk, nx), pk(yk, ny));
+                sh.rz[k] = pk(zk, nz);
+            }
+        }
+    }
+    Sums acc;
+    int top = 0, nb = 0, len = 0, opened = 0, nrec = 0;
+    unsigned rounds = 0, cand = 0;
+    bool overflow = false;
+    int *rec = Rec ? rec_list + (size_t)g * rec_cap : nullptr;
+
+    // root children: cells are opened unconditionally, bodies interact (warp 0)
+    {
+        const int rf = root_first[s], rn = min(root_nch[s], 8);
+        int cm = 0;
+        float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (lane < rn) {
+            cm = meta[rf + lane];
+            q = node4[rf + lane];
+        }
+        const unsigned bodies = __ballot_sync(0xffffffffu, lane < rn && cm < 0);
+        const unsigned cells = __ballot_sync(0xffffffffu, lane < rn && cm >= 0);
+        if (w == 0) {
+            if (lane < rn && cm < 0) {
+                put4(buf.ba, buf.bb, __popc(bodies & lt), q);
+                if constexpr (Rec) buf.ids.bid[__popc(bodies & lt)] = rf + lane;
+            }
+            if (lane < rn && cm >= 0) stack[__popc(cells & lt)] = entry_of(cm, 1);
+            nb = __popc(bodies);
+            opened += __popc(cells);
+        }
+        top = __popc(cells);
+    }
+    __syncthreads();
+
+    for (bool first_round = true; top > 0 || first_round; first_round = false) {
+        // ---- expand: lane j pops the kPops entries from stack[top-1-kPops*j] down (the
+        // same in every warp); P = the most top-of-stack cells whose children fit
+        const int avail = min(top, 32 * kPops);
+        u64 e[kPops];
+        int n[kPops], x[kPops + 1];
+        x[0] = 0;
+#pragma unroll
+        for (int i = 0; i < kPops; i++) {
+            const int at = kPops * lane + i;
+            e[i] = at < avail ? stack[top - 1 - at] : 0ull;
+            n[i] = at < avail ? (((int)(unsigned)e[i] >> 28) & 7) + 1 : 0;
+            x[i + 1] = x[i] + n[i];
+        }
+        int incl = x[kPops];
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int u = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += u;
+        }
+        const int excl = incl - x[kPops];  // children before this lane's cells
+        int np = 0, nt = 0;
+#pragma unroll
+        for (int i = 0; i < kPops; i++)
+            if (n[i] > 0 && excl + x[i + 1] <= kRound) {
+                np = i + 1;
+                nt = excl + x[i + 1];
+            }
+        int P = __reduce_add_sync(0xffffffffu, np);
+        int T = __reduce_max_sync(0xffffffffu, nt);
+        // wide rounds only while the stack keeps the depth-first reserve free (walk2.cu)
+        if (P > 1 && top - P + T > stack_cap - reserve) {
+            P = 1;
+            T = __shfl_sync(0xffffffffu, n[0], 0);
+        }
+        if (P > 0 && top - P + T > stack_cap) P = 0;
+        if (P == 0) T = 0;
+        if (P == 0 && top > 0) {
+            overflow = true;
+            break;
+        }
+        // warp w lists the children of every lane's w-th cells
+#pragma unroll
+        for (int i = 0; i < kPops; i++)
+            if (i % kW == w && kPops * lane + i < P) {
+                const int first = (int)(unsigned)e[i] & 0x0fffffff, at = excl + x[i];
+                const u64 lvl = e[i] & 0xffffffff00000000ull;
+#pragma unroll
+                for (int k = 0; k < 8; k++)
+                    if (k < n[i]) sh.child[at + k] = lvl | (unsigned)(first + k);
+            }
+        __syncthreads();
+        top -= P;
+        int nbody = nb, ncell = 0, nacc = 0, nrej = 0;
+        nb = 0;
+#pragma unroll
+        for (int h = 0; h < kChunks; h++) {
+            const int c0 = h * kW + w;  // this warp's chunk: children [32 c0, 32 c0 + 32)
+            if (32 * c0 >= T) break;
+            const int t = 32 * c0 + lane;
+            const bool ok = t < T;
+            const u64 ch = sh.child[ok ? t : 0];
+            const int c = (int)(unsigned)ch, lvp = (int)(ch >> 32);
+            const float dpc = scale4(d0, lvp);  // the child's opening threshold, depth0 * 4^-level(popped cell)
+            const int lvc = lvp + 1;
+            const int cm = ok ? meta[c] : 0;
+            const float4 q = ok ? node4[c] : make_float4(0.f, 0.f, 0.f, 0.f);
+            const bool isc = ok && cm >= 0;
+            float4 qq4 = make_float4(0.f, 0.f, 0.f, 0.f);
+            float2 qq2 = make_float2(0.f, 0.f);
+            if (Quad && isc) {
+                qq4 = quad4[c];
+                qq2 = quad2[c];
+            }
+            // sure accepts and sure rejects, exactly as walk2.cu classifies
+            bool sacc, srej;
+            {
+                const float4 lo = sh.cls[0], hi = sh.cls[1], cen = sh.cls[2];
+                const float gx = fmaxf(0.f, fmaxf(__fsub_rn(lo.x, q.x), __fsub_rn(q.x, hi.x)));
+                const float gy = fmaxf(0.f, fmaxf(__fsub_rn(lo.y, q.y), __fsub_rn(q.y, hi.y)));
+                const float gz = fmaxf(0.f, fmaxf(__fsub_rn(lo.z, q.z), __fsub_rn(q.z, hi.z)));
+                sacc = dpc <= __fmaf_rn(gz, gz, __fmaf_rn(gy, gy, __fmaf_rn(gx, gx, eps2)));
+                const int oct = (q.x > cen.x ? 1 : 0) | (q.y > cen.y ? 2 : 0) | (q.z > cen.z ? 4 : 0);
+                const ulonglong2 R = sh.rxy[oct];
+                const u64 dx = sub2(pk(q.x, q.x), R.x), dy = sub2(pk(q.y, q.y), R.y);
+                const u64 dz = sub2(pk(q.z, q.z), sh.rz[oct]);
+                float ra, rb;
+                upk(fma2(dz, dz, fma2(dy, dy, fma2(dx, dx, eps2x2))), ra, rb);
+                srej = ra < dpc || rb < dpc;
+            }
+            const bool tob = ok && (cm < 0 || (!Quad && isc && sacc));
+            const bool toc = isc && !sacc && !srej;
+            const bool tos = isc && !sacc && srej;
+            const bool toa = Quad && isc && sacc;
+            const unsigned bm = __ballot_sync(0xffffffffu, tob);
+            const unsigned cmk = __ballot_sync(0xffffffffu, toc);
+            const unsigned smk = __ballot_sync(0xffffffffu, tos);
+            const unsigned amk = Quad ? __ballot_sync(0xffffffffu, toa) : 0u;
+            if (toa) {  // surely accepted cells fill the cell buffer downwards
+                const int slot = kSlots - 1 - (nacc + __popc(amk & lt));
+                put4(buf.ca, buf.cb, slot, q);
+                putq(qbuf.qa, qbuf.qb, qbuf.qc, slot, qq4, qq2);
+            }
+            if (tob) {
+                const int slot = nbody + __popc(bm & lt);
+                put4(buf.ba, buf.bb, slot, q);
+                if constexpr (Rec) buf.ids.bid[slot] = c;
+            }
+            if (toc) {
+                const int slot = ncell + __popc(cmk & lt);
+                put4(buf.cells_a(), buf.cells_b(), buf.vote_slot(slot), q);
+                buf.cd[slot] = dpc;
+                buf.crec[slot] = entry_of(cm, lvc);
+                if constexpr (Rec) buf.ids.cid[slot] = c;
+                if (Quad) putq(qbuf.qa, qbuf.qb, qbuf.qc, slot, qq4, qq2);
+            }
+            if (tos) buf.rej[nrej + __popc(smk & lt)] = entry_of(cm, lvc);
+            nbody += __popc(bm);
+            ncell += __popc(cmk);
+            nrej += __popc(smk);
+            nacc += __popc(amk);
+        }
+        // pads: massless far-away candidates fill the bodies to whole batches of four
+        // pairs, the cells and the accepted region to whole pairs
+        const int nbp = ((nbody + 7) >> 3) << 2;
+        if (nbody + lane < 2 * nbp) put4(buf.ba, buf.bb, nbody + lane, make_float4(1e18f, 1e18f, 1e18f, 0.f));
+        if (lane == 8 && (ncell & 1)) {
+            put4(buf.cells_a(), buf.cells_b(), buf.vote_slot(ncell), make_float4(1e18f, 1e18f, 1e18f, 0.f));
+            buf.cd[ncell] = -INFINITY;
+            if (Quad) putq(qbuf.qa, qbuf.qb, qbuf.qc, ncell, make_float4(0.f, 0.f, 0.f, 0.f), make_float2(0.f, 0.f));
+        }
+        const int abeg = (kSlots - nacc) & ~1;
+        if (Quad && lane == 9 && ((kSlots - nacc) & 1)) {
+            put4(buf.ca, buf.cb, abeg, make_float4(1e18f, 1e18f, 1e18f, 0.f));
+            putq(qbuf.qa, qbuf.qb, qbuf.qc, abeg, make_float4(0.f, 0.f, 0.f, 0.f), make_float2(0.f, 0.f));
+        }
+        __syncwarp();
+
+        // ---- evaluate bodies: no MAC
+        for (int q0 = 0; q0 < nbp; q0 += 4) {
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                const ulonglong2 A = buf.ba[q0 + u];
+                const ulonglong2 B = buf.bb[q0 + u];
+                const u64 dx = sub2(A.x, px);
+                const u64 dy = sub2(A.y, py);
+                const u64 dz = sub2(B.x, pz);
+                u64 r = fma2(dx, dx, eps2x2);
+                r = fma2(dy, dy, r);
+                r = fma2(dz, dz, r);
+                float ra, rb;
+                upk(r, ra, rb);
+                const u64 ri = pk(rsq(ra), rsq(rb));
+                const u64 f = mul2(mul2(B.y, ri), mul2(ri, ri));
+                accumulate<Mode, Pot>(acc, f, B.y, ri, dx, dy, dz);
+            }
+        }
+        if (Quad) {  // surely accepted cells, no vote
+#pragma unroll 2
+            for (int q = abeg >> 1; q < kSlots / 2; q++) {
+                const ulonglong2 A = buf.ca[q];
+                const ulonglong2 B = buf.cb[q];
+                const u64 dx = sub2(A.x, px);
+                const u64 dy = sub2(A.y, py);
+                const u64 dz = sub2(B.x, pz);
+                u64 r = fma2(dx, dx, eps2x2);
+                r = fma2(dy, dy, r);
+                r = fma2(dz, dz, r);
+                float ra, rb;
+                upk(r, ra, rb);
+                const u64 ri = pk(rsq(ra), rsq(rb));
+                quad_term<Mode>(acc, qbuf, q, B.y, ri, dx, dy, dz);
+            }
+        }
+        // ---- evaluate cells: one vote per cell, accept or push
+        const int ncp = (ncell + 1) >> 1;
+        const int nsrej = nrej;
+        int nlist = nbody;
+#pragma unroll 2
+        for (int q = 0; q < ncp; q++) {
+            const int at = buf.vote_slot(2 * q) >> 1;
+            const ulonglong2 A = buf.cells_a()[at];
+            const ulonglong2 B = buf.cells_b()[at];
+            const float2 dp = reinterpret_cast<const float2 *>(buf.cd)[q];
+            const float dpa = dp.x, dpb = dp.y;
+            const u64 dx = sub2(A.x, px);
+            const u64 dy = sub2(A.y, py);
+            const u64 dz = sub2(B.x, pz);
+            u64 r = fma2(dx, dx, eps2x2);
+            r = fma2(dy, dy, r);
+            r = fma2(dz, dz, r);
+            float ra, rb;
+            upk(r, ra, rb);
+            const bool oka = __all_sync(0xffffffffu, dpa <= ra);
+            const bool okb = __all_sync(0xffffffffu, dpb <= rb);
+            if (oka || okb) {  // warp-uniform: a pair of rejected cells adds nothing
+                if (!Quad) {
+                    float ma, mb;
+                    upk(B.y, ma, mb);
+                    const u64 ri = pk(rsq(ra), rsq(rb));
+                    const u64 mm = pk(oka ? ma : 0.f, okb ? mb : 0.f);
+                    const u64 f = mul2(mul2(mul2(mm, ri), ri), ri);
+                    accumulate<Mode, Pot>(acc, f, mm, ri, dx, dy, dz);
+                } else {
+                    const u64 ri = pk(oka ? rsq(ra) : 0.f, okb ? rsq(rb) : 0.f);
+                    quad_term<Mode>(acc, qbuf, q, B.y, ri, dx, dy, dz);
+                }
+            }
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                const int slot = 2 * q + h;
+                if (!(h ? okb : oka)) {  // (a pad is accepted)
+                    if (lane == 0) buf.rej[nrej] = buf.crec[slot];
+                    nrej++;
+                } else if constexpr (Rec) {
+                    if (slot < ncell) {
+                        if (lane == 0) buf.ids.bid[nlist] = buf.ids.cid[slot];
+                        nlist++;
+                    }
+                }
+            }
+        }
+        rounds++;
+        cand += (unsigned)(nbody + ncell + nsrej + nacc);
+        len += nbody + ncell - (nrej - nsrej) + nacc;
+        opened += nrej;
+        if (Mode == 1) {  // fold this round's partial sums into the compensated totals
+            float a0, a1;
+            upk(acc.x, a0, a1);
+            kahan(acc.kx, acc.cx, a0);
+            kahan(acc.kx, acc.cx, a1);
+            upk(acc.y, a0, a1);
+            kahan(acc.ky, acc.cy, a0);
+            kahan(acc.ky, acc.cy, a1);
+            upk(acc.z, a0, a1);
+            kahan(acc.kz, acc.cz, a0);
+            kahan(acc.kz, acc.cz, a1);
+            acc.x = acc.y = acc.z = 0ull;
+        }
+        // ---- push: the warps' rejected cells, in warp order
+        if (lane == 0) {
+            sh.nrej[w] = nrej;
+            if (Rec) sh.nrec[w] = nlist;
+        }
+        __syncthreads();
+        int before = 0, all = 0, rbefore = 0, rall = 0;
+#pragma unroll
+        for (int v = 0; v < kW; v++) {
+            const int k = sh.nrej[v];
+            before += v < w ? k : 0;
+            all += k;
+            if (Rec) {
+                const int m = sh.nrec[v];
+                rbefore += v < w ? m : 0;
+                rall += m;
+            }
+        }
+        for (int i = lane; i < nrej; i += 32) stack[top + before + i] = buf.rej[i];
+        top += all;
+        if constexpr (Rec) {
+            for (int i = lane; i < nlist; i += 32) {
+                const int at = nrec + rbefore + i;
+                if (at < rec_cap) rec[at] = buf.ids.bid[i];
+            }
+            nrec += rall;
+        }
+        __syncthreads();
+    }
+    if (overflow) {  // uniform over the block
+        if (threadIdx.x == 0) set_status(st, NBX_ERR_STACK, g);
+        return;
+    }
+    // ---- the warps' partial sums, added in warp order
+    TeamPart &mine = part(w);
+    if (Mode == 0) {
+        float a0, a1;
+        upk(acc.x, a0, a1);
+        mine.a[0][lane] = a0 + a1;
+        upk(acc.y, a0, a1);
+        mine.a[1][lane] = a0 + a1;
+        upk(acc.z, a0, a1);
+        mine.a[2][lane] = a0 + a1;
+    } else {
+        mine.a[0][lane] = acc.kx;
+        mine.a[1][lane] = acc.ky;
+        mine.a[2][lane] = acc.kz;
+        mine.a[3][lane] = acc.cx;
+        mine.a[4][lane] = acc.cy;
+        mine.a[5][lane] = acc.cz;
+    }
+    if (Pot) {
+        float a0, a1;
+        upk(acc.p, a0, a1);
+        mine.pot[lane] = a0 + a1;
+    }
+    if (lane == 0) {
+        sh.sum[w][0] = len;
+        sh.sum[w][1] = opened;
+        sh.sum[w][2] = (int)cand;
+    }
+    __syncthreads();
+    if (w < 3 && valid) {  // warp w: component w
+        float f = 0.f;
+        if (Mode == 0) {
+            f = part(0).a[w][lane];
+#pragma unroll
+            for (int v = 1; v < kW; v++) f += part(v).a[w][lane];
+        } else {
+            float c = 0.f;
+#pragma unroll
+            for (int v = 0; v < kW; v++) {
+                kahan(f, c, part(v).a[w][lane]);
+                kahan(f, c, -part(v).a[3 + w][lane]);
+            }
+            f -= c;
+        }
+        float *out = w == 0 ? ax : (w == 1 ? ay : az);
+        out[val[p]] = f;
+    }
+    if (Pot && w == 3 && valid) {
+        float a = part(0).pot[lane];
+#pragma unroll
+        for (int v = 1; v < kW; v++) a += part(v).pot[lane];
+        // remove the body's own term m * rsqrt(eps2), then phi = -sum
+        pot[val[p]] = -(a - me.w * rsq(eps2));
+    }
+    if (threadIdx.x == 0) {
+        int l = 0, o = 0, n = 0;
+#pragma unroll
+        for (int v = 0; v < kW; v++) {
+            l += sh.sum[v][0];
+            o += sh.sum[v][1];
+            n += sh.sum[v][2];
+        }
+        gstat[g] = make_int2(l, o);
+        if (Rec) {
+            rec_len[g] = nrec < rec_cap ? nrec : rec_cap;
+            if (nrec > rec_cap) set_status(st, NBX_ERR_CAPACITY, g);
+        }
+        atomicAdd(&st->interactions, (unsigned long long)l * (unsigned long long)(end - p0));
+        atomicAdd(&st->opened, (unsigned long long)o);
+        atomicAdd(&st->rounds, (unsigned long long)rounds);
+        atomicAdd(&st->candidates, (unsigned long long)n);
+    }
+}
+
+template <bool Rec, bool Quad>
+size_t team_smem(int stack_depth) {
+    return sizeof(TeamShared) + kW * (sizeof(TeamBuf<Rec, Quad>) + (Quad ? sizeof(QuadBuf<kSlots>) : 0)) +
+           (size_t)kStackMul * stack_depth * sizeof(u64);
+}
+
+template <int Mode, bool Pot, bool Rec, bool Quad>
+int launch_team(Ctx *ctx, const nbx_state *s, float *pot, cudaStream_t st, const int *list, int first, int count,
+                int *rec_list, int *rec_len, int rec_cap) {
+    const size_t smem = team_smem<Rec, Quad>(ctx->p.stack_depth);
+    if (smem > (size_t)ctx->smem_optin) {
+        ctx->last_error = "walk: stack_depth too large for the launch shape's shared memory";
+        return NBX_ERR_ARG;
+    }
+    k_walk_team<Mode, Pot, Rec, Quad><<<count, kW * 32, smem, st>>>(
+        ctx->d_node4, ctx->d_meta, ctx->d_quad4, ctx->d_quad2, ctx->d_body4, ctx->d_val, ctx->d_groups, list, first,
+        ctx->d_body_sys, ctx->d_sys_off, ctx->d_depth0, ctx->d_root_first, ctx->d_root_nch, ctx->d_sys_lvl, ctx->eps2,
+        kStackMul * ctx->p.stack_depth, s->ax, s->ay, s->az, pot, ctx->d_gstat, ctx->d_status, rec_list, rec_len,
+        rec_cap);
+    ++ctx->launches;
+    NBX_CUDA(cudaGetLastError());
+    return NBX_OK;
+}
+
+template <int Mode, bool Pot, bool Rec, bool Quad>
+cudaError_t team_attr(int smem_max) {
+    return cudaFuncSetAttribute(k_walk_team<Mode, Pot, Rec, Quad>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                smem_max);
+}
+
+}  // namespace
+
+int walk_team_init(Ctx *ctx) {
+    const int m = ctx->smem_optin;
+    NBX_CUDA((team_attr<0, false, false, false>(m)));
+    NBX_CUDA((team_attr<1, false, false, false>(m)));
+    NBX_CUDA((team_attr<2, false, false, false>(m)));
+    NBX_CUDA((team_attr<0, true, false, false>(m)));
+    NBX_CUDA((team_attr<0, false, true, false>(m)));
+    NBX_CUDA((team_attr<0, false, false, true>(m)));
+    NBX_CUDA((team_attr<1, false, false, true>(m)));
+    NBX_CUDA((team_attr<2, false, false, true>(m)));
+    return NBX_OK;
+}
+
+// The walk of `count` groups by teams: groups first, first + 1, ..., or the
+// entries first, ... of `list` (device array) where it is given.  mode: -1
+// potential too, 0..2 the accumulation modes; rec_list: recording (mode 0).
+int walk_team(Ctx *ctx, const nbx_state *s, float *pot, int mode, bool quad, cudaStream_t st, const int *list,
+              int first, int count, int *rec_list, int *rec_len, int rec_cap) {
+    if (count <= 0) return NBX_OK;
+    if (rec_list)
+        return launch_team<0, false, true, false>(ctx, s, nullptr, st, list, first, count, rec_list, rec_len, rec_cap);
+    if (pot) return launch_team<0, true, false, false>(ctx, s, pot, st, list, first, count, nullptr, nullptr, 0);
+    if (quad) switch (mode) {
+            case 1: return launch_team<1, false, false, true>(ctx, s, pot, st, list, first, count, nullptr, nullptr, 0);
+            case 2: return launch_team<2, false, false, true>(ctx, s, pot, st, list, first, count, nullptr, nullptr, 0);
+            default: return launch_team<0, false, false, true>(ctx, s, pot, st, list, first, count, nullptr, nullptr, 0);
+        }
+    switch (mode) {
+        case 1: return launch_team<1, false, false, false>(ctx, s, pot, st, list, first, count, nullptr, nullptr, 0);
+        case 2: return launch_team<2, false, false, false>(ctx, s, pot, st, list, first, count, nullptr, nullptr, 0);
+        default: return launch_team<0, false, false, false>(ctx, s, pot, st, list, first, count, nullptr, nullptr, 0);
+    }
+}
+
+}  // namespace nbx
