@@ -212,11 +212,12 @@ __global__ void __launch_bounds__(kBlock) k_keys(const float *__restrict__ x, co
 
 // The first runs of the merging sort (merge.cu): k_keys and a stable sort of
 // every run of 1024 keys, one cluster of four blocks per run.  Each block sorts
-// a quarter by counting, for every key, the quarter's keys before it (256
-// broadcast comparisons: one microsecond with no chain of passes), then reads
-// the other three sorted quarters through distributed shared memory and
-// searches them.  (One block of 1024 threads per run took 13.5 us at 16384
-// bodies on 16 SMs.)
+// a quarter: parts of 64 by counting, for every key, the part's keys before it
+// (broadcast comparisons, no chain of passes), then the four parts by searching
+// the other three; then it reads the other three sorted quarters through
+// distributed shared memory and searches those.  (One block of 1024 threads per
+// run took 13.5 us at 16384 bodies on 16 SMs; counting over all 256 keys of a
+// quarter 220 us for a batch of 3.2 x 10^6 bodies.)
 __global__ void __cluster_dims__(4, 1, 1) __launch_bounds__(kMergeTile)
     k_sort_tiles(const float *__restrict__ x, const float *__restrict__ y, const float *__restrict__ z,
                  const float *__restrict__ m, const int4 *__restrict__ runs, const float *__restrict__ bbox,
@@ -233,7 +234,7 @@ __global__ void __cluster_dims__(4, 1, 1) __launch_bounds__(kMergeTile)
     const int quarter = (int)cluster.block_rank();
     const int4 t = runs[blockIdx.x >> 2];  // start, len, system, run of the system
     const int tid = (int)threadIdx.x;
-    const int i = t.x + quarter * kQ + tid;
+    int i = t.x + quarter * kQ + tid;
     unsigned long long k = 1ull << 63;  // padding: above every 63-bit key
     if (quarter * kQ + tid < t.y) {
         const float px = x[i], py = y[i], pz = z[i];
@@ -244,28 +245,48 @@ __global__ void __cluster_dims__(4, 1, 1) __launch_bounds__(kMergeTile)
         for (int q = 0; q < 6; q++) bb[q] = bbox[6 * t.z + q];
         k = make_key(px, py, pz, bb, order, ht);
     }
-    sk[tid] = k;
-    __syncthreads();
-    const int w0 = tid & ~31;  // earlier warps' equal keys come first, later ones' after
-    int place = 0;
-    const ulonglong2 *s2 = reinterpret_cast<const ulonglong2 *>(sk);
-#pragma unroll 8
-    for (int j = 0; j < w0 / 2; j++) {
-        const ulonglong2 a = s2[j];
-        place += (a.x <= k) + (a.y <= k);
+    // 64 keys at a time by counting; the two warps of a part order their equal keys
+    // by position
+    const int part = tid & ~63, w0 = tid & ~31;
+    int place = part;
+    {
+        so[0][tid] = k;
+        __syncthreads();
+        const ulonglong2 *mine = reinterpret_cast<const ulonglong2 *>(&so[0][w0]);
+        const ulonglong2 *other = reinterpret_cast<const ulonglong2 *>(&so[0][w0 ^ 32]);
+#pragma unroll
+        for (int j = 0; j < 16; j++) {
+            const ulonglong2 a = mine[j];
+            place += (int)(a.x < k) + ((int)(a.x == k) & (int)(w0 + 2 * j < tid)) + (int)(a.y < k) +
+                     ((int)(a.y == k) & (int)(w0 + 2 * j + 1 < tid));
+        }
+        const unsigned long long kq = k + (w0 & 32 ? 1ull : 0ull);  // an earlier warp's equal key comes first
+#pragma unroll
+        for (int j = 0; j < 16; j++) {
+            const ulonglong2 a = other[j];
+            place += (int)(a.x < kq) + (int)(a.y < kq);
+        }
+        so[1][place] = k;
+        __syncthreads();
+        // and the four parts of 64 by search
+        k = so[1][tid];
+        int pos[3] = {0, 0, 0};
+#pragma unroll
+        for (int step = 64; step > 0; step >>= 1) {
+#pragma unroll
+            for (int a = 0; a < 3; a++) {
+                const int q = a + (64 * a >= part);
+                const int p = min(pos[a] + step, 64);
+                const bool before = so[1][64 * q + p - 1] < k + (64 * q < part ? 1ull : 0ull);
+                pos[a] = (int)(pos[a] + step <= 64) & (int)before ? p : pos[a];
+            }
+        }
+        // the body that stands at `place` of its part moves along
+        reinterpret_cast<int *>(so[2])[place] = i;
+        __syncthreads();
+        i = reinterpret_cast<const int *>(so[2])[tid];
+        place = tid - part + pos[0] + pos[1] + pos[2];
     }
-#pragma unroll 8
-    for (int j = w0 / 2; j < w0 / 2 + 16; j++) {
-        const ulonglong2 a = s2[j];
-        place += (int)(a.x < k) + ((int)(a.x == k) & (int)(2 * j < tid)) + (int)(a.y < k) +
-                 ((int)(a.y == k) & (int)(2 * j + 1 < tid));
-    }
-#pragma unroll 8
-    for (int j = w0 / 2 + 16; j < kQ / 2; j++) {
-        const ulonglong2 a = s2[j];
-        place += (a.x < k) + (a.y < k);
-    }
-    __syncthreads();
     sk[place] = k;
     sv[place] = i;
     cluster.sync();
@@ -413,15 +434,22 @@ __global__ void __launch_bounds__(kPosBlock) k_delta(const float4 *__restrict__ 
         lo = dp + 1;
         hi = max(di, dp) + 1;
     }
-    // each system's deepest level (the walk's depth-first reserve of its groups):
-    // one atomic per warp where the warp lies in one system, and none where the
-    // L2 copy is no smaller (an atomic per body on one word took 13 us of a
-    // 16384-body k_delta and 29 us of a 65536-body one)
+    // each system's deepest level (the walk's depth-first reserve of its groups): one
+    // check per block where the block lies in one system, else one per body, and an
+    // atomic only above the L2 copy.  (An atomic per body took 13 us of a
+    // 16384-body k_delta; a check per warp serialised on the one word: 122 us for a
+    // batch of 3.2 x 10^6 bodies.)
+    __shared__ int s_lvl;
+    if (threadIdx.x == 0) s_lvl = 0;
+    __syncthreads();
     const int lvl_max = __reduce_max_sync(0xffffffffu, hi);
-    const bool one = __all_sync(0xffffffffu, s == __shfl_sync(0xffffffffu, s, 0) || s < 0);
-    const int lv = one ? lvl_max : hi;
-    if (s >= 0 && (!one || (threadIdx.x & 31) == 0) && lv > __ldcg(&sys_lvl[s])) atomicMax(&sys_lvl[s], lv);
-    if ((threadIdx.x & 31) == 0 && lvl_max > __ldcg(&st->max_level)) atomicMax(&st->max_level, lvl_max);
+    if ((threadIdx.x & 31) == 0) atomicMax(&s_lvl, lvl_max);
+    const int last = min(n, (int)(blockIdx.x + 1) * kPosBlock) - 1;
+    const bool one = body_sys[blockIdx.x * kPosBlock] == body_sys[last];
+    __syncthreads();
+    const int lv = one ? s_lvl : hi;
+    if (s >= 0 && (!one || threadIdx.x == 0) && lv > __ldcg(&sys_lvl[s])) atomicMax(&sys_lvl[s], lv);
+    if (threadIdx.x == 0 && s_lvl > __ldcg(&st->max_level)) atomicMax(&st->max_level, s_lvl);
     if (counts) count_levels(lo, hi, cnt, counts);
 }
 
@@ -1049,11 +1077,13 @@ int build_tree(Ctx *ctx, const nbx_state *s, cudaStream_t st, bool external_bbox
     const int gn = ceil_div(ctx->cap_nodes, kBlock) < ctx->nsm * 8 ? ceil_div(ctx->cap_nodes, kBlock) : ctx->nsm * 8;
     // up to 2^21 bodies the 41 per-level launches cost more than the sums: one
     // bottom-up launch (2^16: 0.37 against 0.55 ms per build); above, the
-    // per-level launches stream the levels and are faster
+    // per-level launches stream the levels and are faster (a batch's chains are
+    // shorter: 200 systems, 3.2 x 10^6 bodies, 6.10 against 6.18 ms per step)
     const int mode = ctx->p.moments_mode;
     const bool quad = ctx->multipole != 0;
     if (quad && !ctx->d_m2) return NBX_ERR_STATE;
-    if (mode == 2 || (mode == 0 && n <= kMomentsUpMaxBodies)) {
+    const int up_max = S > 1 ? 4 * kMomentsUpMaxBodies : kMomentsUpMaxBodies;
+    if (mode == 2 || (mode == 0 && n <= up_max)) {
         // one round of 32 nodes per warp until that fills the GPU's warps (a small
         // tree wants its chains started at once), then up to four (fuller groups)
         int rounds = (int)(3ll * n / 2 / (32ll * 32 * ctx->nsm));

@@ -1,6 +1,8 @@
 """Tree build at the sizes where its kernels change shape: block edges of the node
 kernels (512 positions), the switch between summed and scanned level counts
-(131072 positions), and both centre-of-mass passes.  Bit-exact against the oracle.
+(131072 positions) and between the one-block and the cluster form of the top
+cells' sums (65536), with the centre-of-mass passes of every mode.  Bit-exact
+against the oracle.
 """
 import numpy as np
 import pytest
@@ -19,8 +21,8 @@ def _check(b, gt, ot):
         assert np.array_equal(gt[k], getattr(ot, k)), k
 
 
-@pytest.mark.parametrize("n", [511, 512, 513, 1025, 131072, 131073])
-@pytest.mark.parametrize("moments_mode", [1, 2])
+@pytest.mark.parametrize("n", [511, 512, 513, 1025, 65536, 65537, 131072, 131073])
+@pytest.mark.parametrize("moments_mode", [0, 1, 2])
 def test_node_blocks(cuda, n, moments_mode):
     from nns_gb300.barnes_hut import Context, State
     b = ic.plummer(n, seed=n)
