@@ -65,16 +65,16 @@ constexpr int kDfsReserve = 7 * 42 + 8;
 constexpr int kBodyUnroll = NBX_BODY_UNROLL;
 constexpr int kCellUnroll = NBX_CELL_UNROLL;
 
-// Per-warp candidate buffers of CB slots each.
-template <int CB>
+// Per-warp candidate buffers for CB children.  The bodies (and, without
+// quadrupoles, the surely accepted cells) fill the slots upwards and the cells to
+// vote on downwards, so one masked store serves both; with quadrupoles the cells
+// have slots of their own.  (Four slots more: each side pads to a whole pair.)
+template <int CB, bool Quad>
 struct WarpBuf {
-    static constexpr int kPairs = CB / 2;
-    ulonglong2 ba[kPairs];  // bodies: (x0,x1) (y0,y1)
-    ulonglong2 bb[kPairs];  //         (z0,z1) (m0,m1)
-    ulonglong2 ca[kPairs];  // cells:  (x0,x1) (y0,y1)
-    ulonglong2 cb[kPairs];  //         (z0,z1) (m0,m1)
-    u64 cd[kPairs];         //         (dp0,dp1)
-    int cid[CB];            //         node index
+    Slots<CB + 4> b;
+    Slots<Quad ? CB : 4> c; // quadrupole mode: cells
+    float cd[CB];           // cells to vote on: opening thresholds
+    int cid[CB];            //                   node index
     int bid[CB];            // body node ids (interaction-list recording only)
     float4 cls[3];          // group box lo, hi, centre
     ulonglong2 rxy[8];      // representative bodies, in pairs: (x0,x1) (y0,y1)
@@ -105,10 +105,10 @@ __global__ void __launch_bounds__(WalkBounds<CB>::kThreads, WalkBounds<CB>::kMin
     const int warps = blockDim.x >> 5;
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     constexpr int kCB = CB;
-    WarpBuf<CB> &buf = reinterpret_cast<WarpBuf<CB> *>(smem_raw)[w];
+    WarpBuf<CB, Quad> &buf = reinterpret_cast<WarpBuf<CB, Quad> *>(smem_raw)[w];
     constexpr size_t kQuadBytes = Quad ? sizeof(QuadBuf<CB>) : 0;
-    QuadBuf<CB> &qbuf = reinterpret_cast<QuadBuf<CB> *>(smem_raw + sizeof(WarpBuf<CB>) * warps)[w];
-    int *stack = reinterpret_cast<int *>(smem_raw + (sizeof(WarpBuf<CB>) + kQuadBytes) * warps) + w * stack_cap;
+    QuadBuf<CB> &qbuf = reinterpret_cast<QuadBuf<CB> *>(smem_raw + sizeof(WarpBuf<CB, Quad>) * warps)[w];
+    int *stack = reinterpret_cast<int *>(smem_raw + (sizeof(WarpBuf<CB, Quad>) + kQuadBytes) * warps) + w * stack_cap;
     const unsigned lt = (1u << lane) - 1u;
     const u64 eps2x2 = pk(eps2, eps2);
     unsigned long long tot_len = 0ull, tot_open = 0ull, tot_rounds = 0ull, tot_cand = 0ull;
@@ -197,7 +197,7 @@ __global__ void __launch_bounds__(WalkBounds<CB>::kThreads, WalkBounds<CB>::kMin
             const unsigned bodies = __ballot_sync(0xffffffffu, lane < rn && cm < 0);
             const unsigned cells = __ballot_sync(0xffffffffu, lane < rn && cm >= 0);
             if (lane < rn && cm < 0) {
-                put4(buf.ba, buf.bb, __popc(bodies & lt), q);
+                buf.b.put(__popc(bodies & lt), q);
                 if (Rec) buf.bid[__popc(bodies & lt)] = rf + lane;
             }
             if (lane < rn && cm >= 0) stack[__popc(cells & lt)] = rf + lane;
@@ -322,21 +322,25 @@ __global__ void __launch_bounds__(WalkBounds<CB>::kThreads, WalkBounds<CB>::kMin
                     const unsigned amk = __ballot_sync(0xffffffffu, toa);
                     if (toa) {
                         const int slot = kCB - 1 - (nacc + __popc(amk & lt));
-                        put4(buf.ca, buf.cb, slot, q);
+                        buf.c.put(slot, q);
                         putq(qbuf.qa, qbuf.qb, qbuf.qc, slot, qq4, qq2);
                     }
                     nacc += __popc(amk);
                 }
-                if (tob) {
-                    put4(buf.ba, buf.bb, nbody + __popc(bm & lt), q);
-                    if (Rec) buf.bid[nbody + __popc(bm & lt)] = c;
+                const int bslot = nbody + __popc(bm & lt), vslot = ncell + __popc(cmk & lt);
+                if (!Quad) {
+                    if (tob || toc) buf.b.put(toc ? slot_down<CB + 4>(vslot) : bslot, q);
+                } else if (tob) {
+                    buf.b.put(bslot, q);
                 }
+                if (Rec && tob) buf.bid[bslot] = c;
                 if (toc) {
-                    const int slot = ncell + __popc(cmk & lt);
-                    put4(buf.ca, buf.cb, slot, q);
-                    reinterpret_cast<float *>(&buf.cd[slot >> 1])[slot & 1] = dpc;
-                    buf.cid[slot] = c;
-                    if (Quad) putq(qbuf.qa, qbuf.qb, qbuf.qc, slot, qq4, qq2);
+                    if (Quad) {
+                        buf.c.put(vslot, q);
+                        putq(qbuf.qa, qbuf.qb, qbuf.qc, vslot, qq4, qq2);
+                    }
+                    buf.cd[vslot] = dpc;
+                    buf.cid[vslot] = c;
                 }
                 if (tos) stack[top + nsrej + __popc(smk & lt)] = c;
                 nbody += __popc(bm);
@@ -345,10 +349,11 @@ __global__ void __launch_bounds__(WalkBounds<CB>::kThreads, WalkBounds<CB>::kMin
             }
             top += nsrej;
             // pad odd buffers with a massless far-away candidate that is accepted
-            if (lane == 0 && (nbody & 1)) put4(buf.ba, buf.bb, nbody, make_float4(1e18f, 1e18f, 1e18f, 0.f));
+            if (lane == 0 && (nbody & 1)) buf.b.put(nbody, make_float4(1e18f, 1e18f, 1e18f, 0.f));
             if (lane == 1 && (ncell & 1)) {
-                put4(buf.ca, buf.cb, ncell, make_float4(1e18f, 1e18f, 1e18f, 0.f));
-                reinterpret_cast<float *>(&buf.cd[ncell >> 1])[1] = -INFINITY;
+                if (Quad) buf.c.put(ncell, make_float4(1e18f, 1e18f, 1e18f, 0.f));
+                else buf.b.put(slot_down<CB + 4>(ncell), make_float4(1e18f, 1e18f, 1e18f, 0.f));
+                buf.cd[ncell] = -INFINITY;
                 if (Quad)
                     putq(qbuf.qa, qbuf.qb, qbuf.qc, ncell, make_float4(0.f, 0.f, 0.f, 0.f), make_float2(0.f, 0.f));
             }
@@ -357,20 +362,16 @@ __global__ void __launch_bounds__(WalkBounds<CB>::kThreads, WalkBounds<CB>::kMin
             // (ncell + nacc < kCB keeps it clear of the voted region's pad)
             const int abeg = (kCB - nacc) & ~1;
             if (Quad && lane == 2 && ((kCB - nacc) & 1)) {
-                put4(buf.ca, buf.cb, abeg, make_float4(1e18f, 1e18f, 1e18f, 0.f));
+                buf.c.put(abeg, make_float4(1e18f, 1e18f, 1e18f, 0.f));
                 putq(qbuf.qa, qbuf.qb, qbuf.qc, abeg, make_float4(0.f, 0.f, 0.f, 0.f), make_float2(0.f, 0.f));
             }
             __syncwarp();
 
             // ---- evaluate bodies: no MAC
-            const int nbp = (nbody + 1) >> 1;
-#pragma unroll (kBodyUnroll)
-            for (int q = 0; q < nbp; q++) {
-                const ulonglong2 A = buf.ba[q];
-                const ulonglong2 B = buf.bb[q];
-                const u64 dx = sub2(A.x, px);
-                const u64 dy = sub2(A.y, py);
-                const u64 dz = sub2(B.x, pz);
+            for_pairs<kBodyUnroll>(buf.b, 0, (nbody + 1) >> 1, [&](int, u64 x, u64 y, u64 z, u64 m) {
+                const u64 dx = sub2(x, px);
+                const u64 dy = sub2(y, py);
+                const u64 dz = sub2(z, pz);
                 u64 r = fma2(dx, dx, eps2x2);
                 r = fma2(dy, dy, r);
                 r = fma2(dz, dz, r);
@@ -378,9 +379,9 @@ __global__ void __launch_bounds__(WalkBounds<CB>::kThreads, WalkBounds<CB>::kMin
                 upk(r, ra, rb);
                 const u64 ri = pk(rsq(ra), rsq(rb));
                 // no MAC depends on this product: (m ri)(ri ri) shortens its dependency chain
-                const u64 f = mul2(mul2(B.y, ri), mul2(ri, ri));
-                accumulate<Mode, Pot>(acc, f, B.y, ri, dx, dy, dz);
-            }
+                const u64 f = mul2(mul2(m, ri), mul2(ri, ri));
+                accumulate<Mode, Pot>(acc, f, m, ri, dx, dy, dz);
+            });
             if (Rec) {  // every body candidate is an interaction
                 for (int t = lane; t < nbody; t += 32)
                     if (nrec + t < rec_cap) rec[nrec + t] = buf.bid[t];
@@ -390,48 +391,36 @@ __global__ void __launch_bounds__(WalkBounds<CB>::kThreads, WalkBounds<CB>::kMin
             if (Quad) {
 #pragma unroll (kCellUnroll)
                 for (int q = abeg >> 1; q < kCB / 2; q++) {
-                    const ulonglong2 A = buf.ca[q];
-                    const ulonglong2 B = buf.cb[q];
-                    const u64 dx = sub2(A.x, px);
-                    const u64 dy = sub2(A.y, py);
-                    const u64 dz = sub2(B.x, pz);
+                    const u64 dx = sub2(reinterpret_cast<const u64 *>(buf.c.x)[q], px);
+                    const u64 dy = sub2(reinterpret_cast<const u64 *>(buf.c.y)[q], py);
+                    const u64 dz = sub2(reinterpret_cast<const u64 *>(buf.c.z)[q], pz);
                     u64 r = fma2(dx, dx, eps2x2);
                     r = fma2(dy, dy, r);
                     r = fma2(dz, dz, r);
                     float ra, rb;
                     upk(r, ra, rb);
                     const u64 ri = pk(rsq(ra), rsq(rb));
-                    quad_term<Mode>(acc, qbuf, q, B.y, ri, dx, dy, dz);
+                    quad_term<Mode>(acc, qbuf, q, reinterpret_cast<const u64 *>(buf.c.m)[q], ri, dx, dy, dz);
                 }
             }
             // ---- evaluate cells: one vote per cell, accept or push
-            const int ncp = (ncell + 1) >> 1;
             int nrej = 0;
-#pragma unroll (kCellUnroll)
-            for (int q = 0; q < ncp; q++) {
-                const ulonglong2 A = buf.ca[q];
-                const ulonglong2 B = buf.cb[q];
-                float dpa, dpb;
-                upk(buf.cd[q], dpa, dpb);
-                const u64 dx = sub2(A.x, px);
-                const u64 dy = sub2(A.y, py);
-                const u64 dz = sub2(B.x, pz);
+            const auto vote_pair = [&](int q, u64 x, u64 y, u64 z, u64 m) {
+                const float2 dp = reinterpret_cast<const float2 *>(buf.cd)[q];
+                const u64 dx = sub2(x, px);
+                const u64 dy = sub2(y, py);
+                const u64 dz = sub2(z, pz);
                 u64 r = fma2(dx, dx, eps2x2);
                 r = fma2(dy, dy, r);
                 r = fma2(dz, dz, r);
                 float ra, rb;
                 upk(r, ra, rb);
-#ifdef NBX_REDUX_VOTE
-                const unsigned vab = __reduce_and_sync(0xffffffffu, (dpa <= ra ? 1u : 0u) | (dpb <= rb ? 2u : 0u));
-                const bool oka = vab & 1u, okb = (vab >> 1) & 1u;
-#else
-                const bool oka = __all_sync(0xffffffffu, dpa <= ra);
-                const bool okb = __all_sync(0xffffffffu, dpb <= rb);
-#endif
+                const bool oka = __all_sync(0xffffffffu, dp.x <= ra);
+                const bool okb = __all_sync(0xffffffffu, dp.y <= rb);
                 if (oka || okb) {  // warp-uniform: a pair of rejected cells adds nothing
                     if (!Quad) {
                         float ma, mb;
-                        upk(B.y, ma, mb);
+                        upk(m, ma, mb);
                         const u64 ri = pk(rsq(ra), rsq(rb));
                         const u64 mm = pk(oka ? ma : 0.f, okb ? mb : 0.f);
                         const u64 f = mul2(mul2(mul2(mm, ri), ri), ri);
@@ -439,7 +428,7 @@ __global__ void __launch_bounds__(WalkBounds<CB>::kThreads, WalkBounds<CB>::kMin
                     } else {
                         // the rejected half of the pair masked through r^-1 (its term is 0)
                         const u64 ri = pk(oka ? rsq(ra) : 0.f, okb ? rsq(rb) : 0.f);
-                        quad_term<Mode>(acc, qbuf, q, B.y, ri, dx, dy, dz);
+                        quad_term<Mode>(acc, qbuf, q, m, ri, dx, dy, dz);
                     }
                 }
                 if (!oka) {
@@ -456,7 +445,9 @@ __global__ void __launch_bounds__(WalkBounds<CB>::kThreads, WalkBounds<CB>::kMin
                     if (lane == 0 && nrec < rec_cap) rec[nrec] = buf.cid[2 * q + 1];
                     nrec++;
                 }
-            }
+            };
+            if constexpr (Quad) for_pairs<kCellUnroll>(buf.c, 0, (ncell + 1) >> 1, vote_pair);
+            else for_pairs_down<kCellUnroll>(buf.b, (ncell + 1) >> 1, vote_pair);
             top += nrej;
             tot_rounds += 1ull;
             tot_cand += (unsigned long long)(nbody + ncell + nsrej + nacc);
@@ -535,7 +526,7 @@ template <int CB, int Mode, bool Pot, bool Rec = false, bool Quad = false>
 int launch(Ctx *ctx, const nbx_state *s, float *pot, int warps, cudaStream_t st, Share share,
            int *rec_list = nullptr, int *rec_len = nullptr, int rec_cap = 0) {
     const int cap = ctx->p.stack_depth;
-    const size_t smem = (size_t)warps * (sizeof(WarpBuf<CB>) + (Quad ? sizeof(QuadBuf<CB>) : 0) +
+    const size_t smem = (size_t)warps * (sizeof(WarpBuf<CB, Quad>) + (Quad ? sizeof(QuadBuf<CB>) : 0) +
                                          (size_t)cap * sizeof(int));
     if (smem > (size_t)ctx->smem_optin) {
         ctx->last_error = "walk: stack_depth too large for the launch shape's shared memory";

@@ -20,14 +20,62 @@ __device__ __forceinline__ void kahan(float &s, float &c, float v) {
     s = t;
 }
 
-__device__ __forceinline__ void put4(ulonglong2 *a, ulonglong2 *b, int slot, float4 q) {
-    float *pa = reinterpret_cast<float *>(&a[slot >> 1]);
-    float *pb = reinterpret_cast<float *>(&b[slot >> 1]);
-    const int h = slot & 1;
-    pa[h] = q.x;
-    pa[2 + h] = q.y;
-    pb[h] = q.z;
-    pb[2 + h] = q.w;
+// Candidate slots, one array per component: a candidate is stored with four
+// 4-byte stores at one offset (consecutive slots, no bank conflicts), and two
+// pairs are read with four 16-byte loads.
+template <int N>
+struct alignas(16) Slots {
+    float x[N], y[N], z[N], m[N];
+    __device__ __forceinline__ void put(int slot, float4 q) {
+        x[slot] = q.x;
+        y[slot] = q.y;
+        z[slot] = q.z;
+        m[slot] = q.w;
+    }
+};
+
+// Calls f(pair index, x, y, z, m) for the packed pairs [0, n) of the slots from
+// `first` (a multiple of four), two pairs per load.
+template <int Unroll, int N, typename F>
+__device__ __forceinline__ void for_pairs(const Slots<N> &s, int first, int n, F &&f) {
+    const ulonglong2 *x = reinterpret_cast<const ulonglong2 *>(s.x + first);
+    const ulonglong2 *y = reinterpret_cast<const ulonglong2 *>(s.y + first);
+    const ulonglong2 *z = reinterpret_cast<const ulonglong2 *>(s.z + first);
+    const ulonglong2 *m = reinterpret_cast<const ulonglong2 *>(s.m + first);
+#pragma unroll (Unroll / 2)
+    for (int q = 0; q < n >> 1; q++) {
+        const ulonglong2 X = x[q], Y = y[q], Z = z[q], M = m[q];
+        f(2 * q, X.x, Y.x, Z.x, M.x);
+        f(2 * q + 1, X.y, Y.y, Z.y, M.y);
+    }
+    if (n & 1) {
+        const int q = n >> 1;
+        f(n - 1, x[q].x, y[q].x, z[q].x, m[q].x);
+    }
+}
+
+// The same for pairs that fill the slots downwards: pair q in the two slots below
+// N - 2 q, its first candidate in the lower one.
+template <int Unroll, int N, typename F>
+__device__ __forceinline__ void for_pairs_down(const Slots<N> &s, int n, F &&f) {
+    static_assert(N % 4 == 0, "whole double pairs");
+    const ulonglong2 *x = reinterpret_cast<const ulonglong2 *>(s.x), *y = reinterpret_cast<const ulonglong2 *>(s.y);
+    const ulonglong2 *z = reinterpret_cast<const ulonglong2 *>(s.z), *m = reinterpret_cast<const ulonglong2 *>(s.m);
+#pragma unroll (Unroll / 2)
+    for (int q = 0; q < n >> 1; q++) {
+        const int at = N / 4 - 1 - q;
+        const ulonglong2 X = x[at], Y = y[at], Z = z[at], M = m[at];
+        f(2 * q, X.y, Y.y, Z.y, M.y);
+        f(2 * q + 1, X.x, Y.x, Z.x, M.x);
+    }
+    if (n & 1) {
+        const int at = N / 4 - 1 - (n >> 1);
+        f(n - 1, x[at].y, y[at].y, z[at].y, m[at].y);
+    }
+}
+template <int N>
+__device__ __forceinline__ constexpr int slot_down(int i) {
+    return N - 2 - 2 * (i >> 1) + (i & 1);
 }
 
 // Quadrupole mode: the traceless quadrupoles of the cell buffer's slots, in

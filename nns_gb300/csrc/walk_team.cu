@@ -6,10 +6,10 @@
 // the longest group's chain of rounds (load a cell, load its children, classify,
 // evaluate up to 96 candidates: about 2.4 us) is the walk's time.  Here every
 // warp holds the same 32 bodies and takes its own share of a round's children:
-//   expand   all warps pop the same top-of-stack cells (the shared stack holds
-//            each cell's record and level, so a pop loads nothing from memory),
-//            list their children in shared memory and classify the list's
-//            32-child chunks in turn, warp w the chunks w, w + W, ...;
+//   expand   warp 0 pops the top-of-stack cells (the shared stack holds each cell's
+//            record and level, so a pop loads nothing from memory) and lists their
+//            children in shared memory; the warps classify the list's 32-child
+//            chunks in turn, warp w the chunks w, w + W, ...;
 //   evaluate each warp evaluates and votes on its own candidates;
 //   push     after a barrier the warps append their rejected cells to the stack
 //            in warp order.
@@ -17,6 +17,8 @@
 // partial sums added in warp order, so a group's force bits depend on its own
 // system only.  Which systems are walked by teams depends on the system's size
 // alone (kTeamMaxBodies): a batch gives every system the bits of its single run.
+#include <type_traits>
+
 #include "nbx_internal.cuh"
 #include "walk_eval.cuh"
 
@@ -45,18 +47,19 @@ struct TeamIds<false> {};
 // pairs; with quadrupoles the cells are in the second arrays, those to vote on
 // upwards, the surely accepted ones downwards.
 template <bool Rec, bool Quad>
-struct TeamBuf {
-    static constexpr int kPairs = kSlots / 2, kCellPairs = Quad ? kPairs : 1;
-    ulonglong2 ba[kPairs], bb[kPairs];          // (x0,x1) (y0,y1); (z0,z1) (m0,m1)
-    ulonglong2 ca[kCellPairs], cb[kCellPairs];  // quadrupole mode: cells
-    float cd[kSlots];                           // cells to vote on: opening thresholds
-    u64 crec[kSlots];                           // their stack entries
-    u64 rej[32 * kChunks];                      // rejected cells' stack entries
+struct alignas(16) TeamBuf {
+    Slots<kSlots> b;
+    Slots<Quad ? kSlots : 4> c;  // quadrupole mode: cells
+    float cd[kSlots];            // cells to vote on: opening thresholds
+    u64 crec[kSlots];            // their stack entries
+    u64 rej[32 * kChunks];       // rejected cells' stack entries
     TeamIds<Rec> ids;
     // slot of the i-th cell to vote on
-    __device__ static int vote_slot(int i) { return Quad ? i : kSlots - 2 - 2 * (i >> 1) + (i & 1); }
-    __device__ ulonglong2 *cells_a() { return Quad ? ca : ba; }
-    __device__ ulonglong2 *cells_b() { return Quad ? cb : bb; }
+    __device__ static int vote_slot(int i) { return Quad ? i : slot_down<kSlots>(i); }
+    __device__ Slots<kSlots> &cells() {
+        if constexpr (Quad) return c;
+        else return b;
+    }
 };
 
 // A warp's partial results, written over its buffers after the last round.
@@ -66,12 +69,14 @@ struct TeamPart {
 };
 static_assert(sizeof(TeamPart) <= sizeof(TeamBuf<false, false>), "the partial results replace the buffers");
 
-struct TeamShared {
+struct alignas(16) TeamShared {
     float4 cls[3];      // group box lo, hi, centre
     ulonglong2 rxy[8];  // representative bodies, in pairs: (x0,x1) (y0,y1)
     u64 rz[8];          //                                  (z0,z1)
-    int nrej[kW], nrec[kW];
-    int sum[kW][4];     // list length, opened cells, candidates
+    int4 nrej, nrec;    // per warp
+    int sum[kW][2];     // list length, opened cells
+    int P, T;           // the round's popped cells and children
+    int pad[2];
     u64 child[kRound];  // the round's children: node, level of its parent
 };
 
@@ -154,7 +159,7 @@ __global__ void __launch_bounds__(kW * 32, 32 / kW)
     }
     Sums acc;
     int top = 0, nb = 0, len = 0, opened = 0, nrec = 0;
-    unsigned rounds = 0, cand = 0;
+    unsigned rounds = 0;
     bool overflow = false;
     int *rec = Rec ? rec_list + (size_t)g * rec_cap : nullptr;
 
@@ -171,7 +176,7 @@ __global__ void __launch_bounds__(kW * 32, 32 / kW)
         const unsigned cells = __ballot_sync(0xffffffffu, lane < rn && cm >= 0);
         if (w == 0) {
             if (lane < rn && cm < 0) {
-                put4(buf.ba, buf.bb, __popc(bodies & lt), q);
+                buf.b.put(__popc(bodies & lt), q);
                 if constexpr (Rec) buf.ids.bid[__popc(bodies & lt)] = rf + lane;
             }
             if (lane < rn && cm >= 0) stack[__popc(cells & lt)] = entry_of(cm, 1);
@@ -180,60 +185,67 @@ __global__ void __launch_bounds__(kW * 32, 32 / kW)
         }
         top = __popc(cells);
     }
+    const int root_cells = top;
     __syncthreads();
 
     for (bool first_round = true; top > 0 || first_round; first_round = false) {
-        // ---- expand: lane j pops the kPops entries from stack[top-1-kPops*j] down (the
-        // same in every warp); P = the most top-of-stack cells whose children fit
-        const int avail = min(top, 32 * kPops);
-        u64 e[kPops];
-        int n[kPops], x[kPops + 1];
-        x[0] = 0;
+        // ---- expand: lane j of warp 0 pops the kPops entries from stack[top-1-kPops*j]
+        // down and lists their children; P = the most top-of-stack cells that fit
+        if (w == 0) {
+            const int avail = min(top, 32 * kPops);
+            u64 e[kPops];
+            int n[kPops], x[kPops + 1];
+            x[0] = 0;
 #pragma unroll
-        for (int i = 0; i < kPops; i++) {
-            const int at = kPops * lane + i;
-            e[i] = at < avail ? stack[top - 1 - at] : 0ull;
-            n[i] = at < avail ? (((int)(unsigned)e[i] >> 28) & 7) + 1 : 0;
-            x[i + 1] = x[i] + n[i];
-        }
-        int incl = x[kPops];
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int u = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o) incl += u;
-        }
-        const int excl = incl - x[kPops];  // children before this lane's cells
-        int np = 0, nt = 0;
-#pragma unroll
-        for (int i = 0; i < kPops; i++)
-            if (n[i] > 0 && excl + x[i + 1] <= kRound) {
-                np = i + 1;
-                nt = excl + x[i + 1];
+            for (int i = 0; i < kPops; i++) {
+                const int at = kPops * lane + i;
+                e[i] = at < avail ? stack[top - 1 - at] : 0ull;
+                n[i] = at < avail ? (((int)(unsigned)e[i] >> 28) & 7) + 1 : 0;
+                x[i + 1] = x[i] + n[i];
             }
-        int P = __reduce_add_sync(0xffffffffu, np);
-        int T = __reduce_max_sync(0xffffffffu, nt);
-        // wide rounds only while the stack keeps the depth-first reserve free (walk2.cu)
-        if (P > 1 && top - P + T > stack_cap - reserve) {
-            P = 1;
-            T = __shfl_sync(0xffffffffu, n[0], 0);
+            int incl = x[kPops];
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int u = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o) incl += u;
+            }
+            const int excl = incl - x[kPops];  // children before this lane's cells
+            int np = 0, nt = 0;
+#pragma unroll
+            for (int i = 0; i < kPops; i++)
+                if (n[i] > 0 && excl + x[i + 1] <= kRound) {
+                    np = i + 1;
+                    nt = excl + x[i + 1];
+                }
+            int P = __reduce_add_sync(0xffffffffu, np);
+            int T = __reduce_max_sync(0xffffffffu, nt);
+            // wide rounds only while the stack keeps the depth-first reserve free (walk2.cu)
+            if (P > 1 && top - P + T > stack_cap - reserve) {
+                P = 1;
+                T = __shfl_sync(0xffffffffu, n[0], 0);
+            }
+            if (P > 0 && top - P + T > stack_cap) P = 0;
+            if (P == 0) T = 0;
+            if (lane == 0) {
+                sh.P = P;
+                sh.T = T;
+            }
+#pragma unroll
+            for (int i = 0; i < kPops; i++)
+                if (kPops * lane + i < P) {
+                    const int first = (int)(unsigned)e[i] & 0x0fffffff, at = excl + x[i];
+                    const u64 lvl = e[i] & 0xffffffff00000000ull;
+#pragma unroll
+                    for (int k = 0; k < 8; k++)
+                        if (k < n[i]) sh.child[at + k] = lvl | (unsigned)(first + k);
+                }
         }
-        if (P > 0 && top - P + T > stack_cap) P = 0;
-        if (P == 0) T = 0;
+        __syncthreads();
+        const int P = sh.P, T = sh.T;
         if (P == 0 && top > 0) {
             overflow = true;
             break;
         }
-        // warp w lists the children of every lane's w-th cells
-#pragma unroll
-        for (int i = 0; i < kPops; i++)
-            if (i % kW == w && kPops * lane + i < P) {
-                const int first = (int)(unsigned)e[i] & 0x0fffffff, at = excl + x[i];
-                const u64 lvl = e[i] & 0xffffffff00000000ull;
-#pragma unroll
-                for (int k = 0; k < 8; k++)
-                    if (k < n[i]) sh.child[at + k] = lvl | (unsigned)(first + k);
-            }
-        __syncthreads();
         top -= P;
         int nbody = nb, ncell = 0, nacc = 0, nrej = 0;
         nb = 0;
@@ -282,21 +294,26 @@ __global__ void __launch_bounds__(kW * 32, 32 / kW)
             const unsigned amk = Quad ? __ballot_sync(0xffffffffu, toa) : 0u;
             if (toa) {  // surely accepted cells fill the cell buffer downwards
                 const int slot = kSlots - 1 - (nacc + __popc(amk & lt));
-                put4(buf.ca, buf.cb, slot, q);
+                buf.cells().put(slot, q);
                 putq(qbuf.qa, qbuf.qb, qbuf.qc, slot, qq4, qq2);
             }
-            if (tob) {
-                const int slot = nbody + __popc(bm & lt);
-                put4(buf.ba, buf.bb, slot, q);
-                if constexpr (Rec) buf.ids.bid[slot] = c;
+            const int vslot = ncell + __popc(cmk & lt);
+            const int bslot = nbody + __popc(bm & lt);
+            if (!Quad) {
+                if (tob || toc) buf.b.put(toc ? buf.vote_slot(vslot) : bslot, q);
+            } else if (tob) {
+                buf.b.put(bslot, q);
             }
+            if constexpr (Rec)
+                if (tob) buf.ids.bid[bslot] = c;
             if (toc) {
-                const int slot = ncell + __popc(cmk & lt);
-                put4(buf.cells_a(), buf.cells_b(), buf.vote_slot(slot), q);
-                buf.cd[slot] = dpc;
-                buf.crec[slot] = entry_of(cm, lvc);
-                if constexpr (Rec) buf.ids.cid[slot] = c;
-                if (Quad) putq(qbuf.qa, qbuf.qb, qbuf.qc, slot, qq4, qq2);
+                if (Quad) {
+                    buf.cells().put(vslot, q);
+                    putq(qbuf.qa, qbuf.qb, qbuf.qc, vslot, qq4, qq2);
+                }
+                buf.cd[vslot] = dpc;
+                buf.crec[vslot] = entry_of(cm, lvc);
+                if constexpr (Rec) buf.ids.cid[vslot] = c;
             }
             if (tos) buf.rej[nrej + __popc(smk & lt)] = entry_of(cm, lvc);
             nbody += __popc(bm);
@@ -304,72 +321,85 @@ __global__ void __launch_bounds__(kW * 32, 32 / kW)
             nrej += __popc(smk);
             nacc += __popc(amk);
         }
-        // pads: massless far-away candidates fill the bodies to whole batches of four
-        // pairs, the cells and the accepted region to whole pairs
-        const int nbp = ((nbody + 7) >> 3) << 2;
-        if (nbody + lane < 2 * nbp) put4(buf.ba, buf.bb, nbody + lane, make_float4(1e18f, 1e18f, 1e18f, 0.f));
+        // pads: massless far-away candidates fill odd last pairs
+        const int nbp = (nbody + 1) >> 1;
+        if (lane == 0 && (nbody & 1)) buf.b.put(nbody, make_float4(1e18f, 1e18f, 1e18f, 0.f));
         if (lane == 8 && (ncell & 1)) {
-            put4(buf.cells_a(), buf.cells_b(), buf.vote_slot(ncell), make_float4(1e18f, 1e18f, 1e18f, 0.f));
+            buf.cells().put(buf.vote_slot(ncell), make_float4(1e18f, 1e18f, 1e18f, 0.f));
             buf.cd[ncell] = -INFINITY;
             if (Quad) putq(qbuf.qa, qbuf.qb, qbuf.qc, ncell, make_float4(0.f, 0.f, 0.f, 0.f), make_float2(0.f, 0.f));
         }
         const int abeg = (kSlots - nacc) & ~1;
         if (Quad && lane == 9 && ((kSlots - nacc) & 1)) {
-            put4(buf.ca, buf.cb, abeg, make_float4(1e18f, 1e18f, 1e18f, 0.f));
+            buf.cells().put(abeg, make_float4(1e18f, 1e18f, 1e18f, 0.f));
             putq(qbuf.qa, qbuf.qb, qbuf.qc, abeg, make_float4(0.f, 0.f, 0.f, 0.f), make_float2(0.f, 0.f));
         }
         __syncwarp();
 
         // ---- evaluate bodies: no MAC
-        for (int q0 = 0; q0 < nbp; q0 += 4) {
+        const auto body_pair = [&](u64 x, u64 y, u64 z, u64 m) {
+            const u64 dx = sub2(x, px);
+            const u64 dy = sub2(y, py);
+            const u64 dz = sub2(z, pz);
+            u64 r = fma2(dx, dx, eps2x2);
+            r = fma2(dy, dy, r);
+            r = fma2(dz, dz, r);
+            float ra, rb;
+            upk(r, ra, rb);
+            const u64 ri = pk(rsq(ra), rsq(rb));
+            const u64 f = mul2(mul2(m, ri), mul2(ri, ri));
+            accumulate<Mode, Pot>(acc, f, m, ri, dx, dy, dz);
+        };
+        const auto body_pairs = [&](int q, auto count) {  // whole double pairs from q
+            constexpr int kN = decltype(count)::value;
 #pragma unroll
-            for (int u = 0; u < 4; u++) {
-                const ulonglong2 A = buf.ba[q0 + u];
-                const ulonglong2 B = buf.bb[q0 + u];
-                const u64 dx = sub2(A.x, px);
-                const u64 dy = sub2(A.y, py);
-                const u64 dz = sub2(B.x, pz);
-                u64 r = fma2(dx, dx, eps2x2);
-                r = fma2(dy, dy, r);
-                r = fma2(dz, dz, r);
-                float ra, rb;
-                upk(r, ra, rb);
-                const u64 ri = pk(rsq(ra), rsq(rb));
-                const u64 f = mul2(mul2(B.y, ri), mul2(ri, ri));
-                accumulate<Mode, Pot>(acc, f, B.y, ri, dx, dy, dz);
+            for (int u = 0; u < kN; u += 2) {
+                const ulonglong2 X = *reinterpret_cast<const ulonglong2 *>(&buf.b.x[2 * (q + u)]);
+                const ulonglong2 Y = *reinterpret_cast<const ulonglong2 *>(&buf.b.y[2 * (q + u)]);
+                const ulonglong2 Z = *reinterpret_cast<const ulonglong2 *>(&buf.b.z[2 * (q + u)]);
+                const ulonglong2 M = *reinterpret_cast<const ulonglong2 *>(&buf.b.m[2 * (q + u)]);
+                body_pair(X.x, Y.x, Z.x, M.x);
+                body_pair(X.y, Y.y, Z.y, M.y);
             }
+        };
+        int q0 = 0;
+        for (; q0 + 8 <= nbp; q0 += 8) body_pairs(q0, std::integral_constant<int, 8>());
+        if (nbp & 4) {
+            body_pairs(q0, std::integral_constant<int, 4>());
+            q0 += 4;
         }
+        if (nbp & 2) {
+            body_pairs(q0, std::integral_constant<int, 2>());
+            q0 += 2;
+        }
+        if (nbp & 1)
+            body_pair(reinterpret_cast<const u64 *>(buf.b.x)[q0], reinterpret_cast<const u64 *>(buf.b.y)[q0],
+                      reinterpret_cast<const u64 *>(buf.b.z)[q0], reinterpret_cast<const u64 *>(buf.b.m)[q0]);
         if (Quad) {  // surely accepted cells, no vote
 #pragma unroll 2
             for (int q = abeg >> 1; q < kSlots / 2; q++) {
-                const ulonglong2 A = buf.ca[q];
-                const ulonglong2 B = buf.cb[q];
-                const u64 dx = sub2(A.x, px);
-                const u64 dy = sub2(A.y, py);
-                const u64 dz = sub2(B.x, pz);
+                const u64 dx = sub2(reinterpret_cast<const u64 *>(buf.cells().x)[q], px);
+                const u64 dy = sub2(reinterpret_cast<const u64 *>(buf.cells().y)[q], py);
+                const u64 dz = sub2(reinterpret_cast<const u64 *>(buf.cells().z)[q], pz);
                 u64 r = fma2(dx, dx, eps2x2);
                 r = fma2(dy, dy, r);
                 r = fma2(dz, dz, r);
                 float ra, rb;
                 upk(r, ra, rb);
                 const u64 ri = pk(rsq(ra), rsq(rb));
-                quad_term<Mode>(acc, qbuf, q, B.y, ri, dx, dy, dz);
+                quad_term<Mode>(acc, qbuf, q, reinterpret_cast<const u64 *>(buf.cells().m)[q], ri, dx, dy, dz);
             }
         }
         // ---- evaluate cells: one vote per cell, accept or push
         const int ncp = (ncell + 1) >> 1;
         const int nsrej = nrej;
         int nlist = nbody;
-#pragma unroll 2
-        for (int q = 0; q < ncp; q++) {
-            const int at = buf.vote_slot(2 * q) >> 1;
-            const ulonglong2 A = buf.cells_a()[at];
-            const ulonglong2 B = buf.cells_b()[at];
+        const auto vote_pair = [&](int q, u64 x, u64 y, u64 z, u64 m) {
             const float2 dp = reinterpret_cast<const float2 *>(buf.cd)[q];
             const float dpa = dp.x, dpb = dp.y;
-            const u64 dx = sub2(A.x, px);
-            const u64 dy = sub2(A.y, py);
-            const u64 dz = sub2(B.x, pz);
+            const u64 dx = sub2(x, px);
+            const u64 dy = sub2(y, py);
+            const u64 dz = sub2(z, pz);
             u64 r = fma2(dx, dx, eps2x2);
             r = fma2(dy, dy, r);
             r = fma2(dz, dz, r);
@@ -380,14 +410,14 @@ __global__ void __launch_bounds__(kW * 32, 32 / kW)
             if (oka || okb) {  // warp-uniform: a pair of rejected cells adds nothing
                 if (!Quad) {
                     float ma, mb;
-                    upk(B.y, ma, mb);
+                    upk(m, ma, mb);
                     const u64 ri = pk(rsq(ra), rsq(rb));
                     const u64 mm = pk(oka ? ma : 0.f, okb ? mb : 0.f);
                     const u64 f = mul2(mul2(mul2(mm, ri), ri), ri);
                     accumulate<Mode, Pot>(acc, f, mm, ri, dx, dy, dz);
                 } else {
                     const u64 ri = pk(oka ? rsq(ra) : 0.f, okb ? rsq(rb) : 0.f);
-                    quad_term<Mode>(acc, qbuf, q, B.y, ri, dx, dy, dz);
+                    quad_term<Mode>(acc, qbuf, q, m, ri, dx, dy, dz);
                 }
             }
 #pragma unroll
@@ -403,9 +433,10 @@ __global__ void __launch_bounds__(kW * 32, 32 / kW)
                     }
                 }
             }
-        }
+        };
+        if constexpr (Quad) for_pairs<4>(buf.cells(), 0, ncp, vote_pair);
+        else for_pairs_down<4>(buf.b, ncp, vote_pair);
         rounds++;
-        cand += (unsigned)(nbody + ncell + nsrej + nacc);
         len += nbody + ncell - (nrej - nsrej) + nacc;
         opened += nrej;
         if (Mode == 1) {  // fold this round's partial sums into the compensated totals
@@ -423,25 +454,20 @@ __global__ void __launch_bounds__(kW * 32, 32 / kW)
         }
         // ---- push: the warps' rejected cells, in warp order
         if (lane == 0) {
-            sh.nrej[w] = nrej;
-            if (Rec) sh.nrec[w] = nlist;
+            reinterpret_cast<int *>(&sh.nrej)[w] = nrej;
+            if (Rec) reinterpret_cast<int *>(&sh.nrec)[w] = nlist;
         }
         __syncthreads();
-        int before = 0, all = 0, rbefore = 0, rall = 0;
-#pragma unroll
-        for (int v = 0; v < kW; v++) {
-            const int k = sh.nrej[v];
-            before += v < w ? k : 0;
-            all += k;
-            if (Rec) {
-                const int m = sh.nrec[v];
-                rbefore += v < w ? m : 0;
-                rall += m;
-            }
-        }
+        static_assert(kW == 4, "one int4 holds a count per warp");
+        const int4 nr = sh.nrej;
+        const int before = (w > 0 ? nr.x : 0) + (w > 1 ? nr.y : 0) + (w > 2 ? nr.z : 0);
+        const int all = nr.x + nr.y + nr.z + nr.w;
         for (int i = lane; i < nrej; i += 32) stack[top + before + i] = buf.rej[i];
         top += all;
         if constexpr (Rec) {
+            const int4 nl = sh.nrec;
+            const int rbefore = (w > 0 ? nl.x : 0) + (w > 1 ? nl.y : 0) + (w > 2 ? nl.z : 0);
+            const int rall = nl.x + nl.y + nl.z + nl.w;
             for (int i = lane; i < nlist; i += 32) {
                 const int at = nrec + rbefore + i;
                 if (at < rec_cap) rec[at] = buf.ids.bid[i];
@@ -480,7 +506,6 @@ __global__ void __launch_bounds__(kW * 32, 32 / kW)
     if (lane == 0) {
         sh.sum[w][0] = len;
         sh.sum[w][1] = opened;
-        sh.sum[w][2] = (int)cand;
     }
     __syncthreads();
     if (w < 3 && valid) {  // warp w: component w
@@ -509,12 +534,11 @@ __global__ void __launch_bounds__(kW * 32, 32 / kW)
         pot[val[p]] = -(a - me.w * rsq(eps2));
     }
     if (threadIdx.x == 0) {
-        int l = 0, o = 0, n = 0;
+        int l = 0, o = 0;
 #pragma unroll
         for (int v = 0; v < kW; v++) {
             l += sh.sum[v][0];
             o += sh.sum[v][1];
-            n += sh.sum[v][2];
         }
         gstat[g] = make_int2(l, o);
         if (Rec) {
@@ -524,7 +548,8 @@ __global__ void __launch_bounds__(kW * 32, 32 / kW)
         atomicAdd(&st->interactions, (unsigned long long)l * (unsigned long long)(end - p0));
         atomicAdd(&st->opened, (unsigned long long)o);
         atomicAdd(&st->rounds, (unsigned long long)rounds);
-        atomicAdd(&st->candidates, (unsigned long long)n);
+        // every child is a list entry or was opened (the root's cells are no one's children)
+        atomicAdd(&st->candidates, (unsigned long long)(l + o - root_cells));
     }
 }
 
