@@ -111,7 +111,7 @@ void free_all(Ctx *ctx) {
                     ctx->d_sums, ctx->d_count, ctx->d_arrive, ctx->d_lvl8, ctx->d_hist,
                     ctx->d_scan_blk, ctx->d_totals, ctx->d_totals64, ctx->d_status, ctx->d_m2, ctx->d_com, ctx->d_quad4,
                     ctx->d_quad2, ctx->d_seg_slot, ctx->d_lb_counts, ctx->d_lb_status, ctx->d_lb, ctx->d_tiles_sw,
-                    ctx->d_sys_tiles_sw, ctx->d_tiles_mg, ctx->d_runs_mg, ctx->d_team, ctx->d_solo};
+                    ctx->d_sys_tiles_sw, ctx->d_tiles_mg, ctx->d_runs_mg, ctx->d_team, ctx->d_solo, ctx->d_bbox_done};
     for (void *p : ptrs)
         if (p) cudaFree(p);
     if (ctx->h_status) cudaFreeHost(ctx->h_status);
@@ -301,6 +301,7 @@ int nbx_create(const nbx_params *p, nbx_ctx **out) {
     rc |= nbx::dmalloc(ctx, &ctx->d_team, G);
     rc |= nbx::dmalloc(ctx, &ctx->d_solo, G);
     rc |= nbx::dmalloc(ctx, &ctx->d_bbox_u, 6 * Ss + 6);
+    rc |= nbx::dmalloc(ctx, &ctx->d_bbox_done, 1);
     rc |= nbx::dmalloc(ctx, &ctx->d_bbox, 6 * Ss);
     rc |= nbx::dmalloc(ctx, &ctx->d_bbox64, 6 * Ss);
     rc |= nbx::dmalloc(ctx, &ctx->d_depth0, Ss);
@@ -345,6 +346,13 @@ int nbx_create(const nbx_params *p, nbx_ctx **out) {
     // status words start at build 0, which no pass ever uses (its tags are >= 1)
     if (rc == 0 && cudaMemset(ctx->d_lb_status, 0, sizeof(unsigned long long) * ((size_t)ctx->cap_tiles_body << nbx::kMaxRadixBits)) != cudaSuccess)
         rc = NBX_ERR_CUDA;
+    // empty boxes: the ordered encoding of 0.0f is the sign bit (k_bbox keeps them so)
+    if (rc == 0) {
+        const std::vector<unsigned> empty(6 * (size_t)Ss + 6, 0x80000000u);
+        if (cudaMemcpy(ctx->d_bbox_u, empty.data(), sizeof(unsigned) * empty.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
+            cudaMemset(ctx->d_bbox_done, 0, sizeof(unsigned)) != cudaSuccess)
+            rc = NBX_ERR_CUDA;
+    }
     if (rc == 0 && cudaMemset(ctx->d_lb, 0, 16 * sizeof(unsigned)) != cudaSuccess) rc = NBX_ERR_CUDA;
     if (rc == 0 && ctx->multipole) rc = nbx::alloc_quadrupoles(ctx);
     if (rc == 0) rc = nbx::walk_init(ctx);

@@ -29,13 +29,15 @@ __global__ void __launch_bounds__(kBlock) k_update(float *__restrict__ x, float 
 }
 
 // The same update, four bodies per thread with 16-byte loads and stores of
-// each array (every array 16-byte aligned; bodies [0, 4*n4)).  Per element the
-// operations are those of k_update, so the results are identical.
+// each array (every array 16-byte aligned); the first threads take the up to three
+// bodies past the last whole four.  Per element the operations are those of
+// k_update, so the results are identical.
 __global__ void __launch_bounds__(kBlock) k_update4(float4 *__restrict__ x, float4 *__restrict__ y,
                                                      float4 *__restrict__ z, float4 *__restrict__ vx,
                                                      float4 *__restrict__ vy, float4 *__restrict__ vz,
                                                      const float4 *__restrict__ ax, const float4 *__restrict__ ay,
-                                                     const float4 *__restrict__ az, int n4, float dt, float ddt) {
+                                                     const float4 *__restrict__ az, int n, float dt, float ddt) {
+    const int n4 = n >> 2;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n4; i += gridDim.x * blockDim.x) {
         float4 v[3] = {vx[i], vy[i], vz[i]};
         const float4 a[3] = {ax[i], ay[i], az[i]};
@@ -57,6 +59,18 @@ __global__ void __launch_bounds__(kBlock) k_update4(float4 *__restrict__ x, floa
         x[i] = p[0];
         y[i] = p[1];
         z[i] = p[2];
+    }
+    const int i = 4 * n4 + (int)threadIdx.x;
+    if (blockIdx.x == 0 && i < n) {
+        const auto one = [&](float4 *p4, float4 *v4, const float4 *a4) {
+            float *p = reinterpret_cast<float *>(p4), *v = reinterpret_cast<float *>(v4);
+            const float nv = __fmaf_rn(dt, reinterpret_cast<const float *>(a4)[i], v[i]);
+            v[i] = nv;
+            p[i] = __fmaf_rn(ddt, nv, p[i]);
+        };
+        one(x, vx, ax);
+        one(y, vy, ay);
+        one(z, vz, az);
     }
 }
 
@@ -128,12 +142,14 @@ __global__ void __launch_bounds__(kBlock) k_bbox_ref(const float *__restrict__ x
     }
 }
 
-__global__ void k_bbox_ref_store(const unsigned *bu, float *minX, float *maxX, float *minY, float *maxY,
+// (also leaves the scratch box empty, as the build's k_bbox expects it)
+__global__ void k_bbox_ref_store(unsigned *bu, float *minX, float *maxX, float *minY, float *maxY,
                                  float *minZ, float *maxZ) {
     if (threadIdx.x == 0) {
         *minX = ord2f(bu[0]); *maxX = ord2f(bu[1]);
         *minY = ord2f(bu[2]); *maxY = ord2f(bu[3]);
         *minZ = ord2f(bu[4]); *maxZ = ord2f(bu[5]);
+        for (int k = 0; k < 6; k++) bu[k] = f2ord(0.0f);
     }
 }
 
@@ -195,11 +211,29 @@ __global__ void __launch_bounds__(kBlock) k_diag_fp64(const float *__restrict__ 
         a[6] += mi * (px * uy - py * ux);
         a[7] += mi;
     }
+    // FP64 instructions and same-address FP64 atomics are slow on this part: the
+    // warp's eight sums are folded with eight shuffles (half of the lanes keep half
+    // of the sums at each of the first three), and a block adds each sum once
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
 #pragma unroll
-    for (int k = 0; k < 8; k++) {
-        double v = a[k];
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-        if ((threadIdx.x & 31) == 0) atomicAdd(&out[k], v);
+    for (int h = 4; h > 0; h >>= 1) {
+        const bool up = lane & h;
+#pragma unroll
+        for (int k = 0; k < h; k++) {
+            const double keep = up ? a[k + h] : a[k], give = up ? a[k] : a[k + h];
+            a[k] = keep + __shfl_xor_sync(0xffffffffu, give, h);
+        }
+    }
+    double v = a[0];  // sum number lane & 7
+    v += __shfl_xor_sync(0xffffffffu, v, 8);
+    v += __shfl_xor_sync(0xffffffffu, v, 16);
+    __shared__ double part[kBlock / 32][8];
+    if (lane < 8) part[w][lane] = v;
+    __syncthreads();
+    if (threadIdx.x < 8) {
+        double t = 0.0;
+        for (int q = 0; q < kBlock / 32; q++) t += part[q][threadIdx.x];
+        atomicAdd(&out[threadIdx.x], t);
     }
 }
 
@@ -211,27 +245,17 @@ int integrate(Ctx *ctx, const nbx_state *s, float dt, float d, int n, cudaStream
     const float *arr[9] = {s->x, s->y, s->z, s->vx, s->vy, s->vz, s->ax, s->ay, s->az};
     bool aligned = true;
     for (const float *a : arr) aligned &= (reinterpret_cast<uintptr_t>(a) & 15u) == 0;
-    int done = 0;  // bodies [0, done) updated four at a time
-    if (aligned && n >= 4) {
-        const int n4 = n >> 2;
-        int grid = ceil_div(n4, kBlock);
-        if (grid > ctx->nsm * 16) grid = ctx->nsm * 16;
+    int grid = ceil_div(aligned && n >= 4 ? n >> 2 : n, kBlock);
+    if (grid > ctx->nsm * 16) grid = ctx->nsm * 16;
+    if (aligned && n >= 4)
         k_update4<<<grid, kBlock, 0, st>>>(
             reinterpret_cast<float4 *>(s->x), reinterpret_cast<float4 *>(s->y), reinterpret_cast<float4 *>(s->z),
             reinterpret_cast<float4 *>(s->vx), reinterpret_cast<float4 *>(s->vy), reinterpret_cast<float4 *>(s->vz),
             reinterpret_cast<const float4 *>(s->ax), reinterpret_cast<const float4 *>(s->ay),
-            reinterpret_cast<const float4 *>(s->az), n4, dt, ddt);
-        ++ctx->launches;
-        done = n4 << 2;
-    }
-    if (done < n) {
-        const int m = n - done;
-        int grid = ceil_div(m, kBlock);
-        if (grid > ctx->nsm * 16) grid = ctx->nsm * 16;
-        k_update<<<grid, kBlock, 0, st>>>(s->x + done, s->y + done, s->z + done, s->vx + done, s->vy + done,
-                                          s->vz + done, s->ax + done, s->ay + done, s->az + done, m, dt, ddt);
-        ++ctx->launches;
-    }
+            reinterpret_cast<const float4 *>(s->az), n, dt, ddt);
+    else
+        k_update<<<grid, kBlock, 0, st>>>(s->x, s->y, s->z, s->vx, s->vy, s->vz, s->ax, s->ay, s->az, n, dt, ddt);
+    ++ctx->launches;
     NBX_CUDA(cudaGetLastError());
     return NBX_OK;
 }
@@ -280,7 +304,7 @@ int direct_fp64(Ctx *ctx, const float *x, const float *y, const float *z, const 
 int diagnostics_fp64(Ctx *ctx, const nbx_state *s, int n, double *out, cudaStream_t st) {
     NBX_CUDA(cudaMemsetAsync(out, 0, 8 * sizeof(double), st));
     int grid = ceil_div(n, kBlock);
-    if (grid > ctx->nsm * 4) grid = ctx->nsm * 4;
+    if (grid > ctx->nsm * 2) grid = ctx->nsm * 2;
     if (grid > 0) {
         k_diag_fp64<<<grid, kBlock, 0, st>>>(s->x, s->y, s->z, s->vx, s->vy, s->vz, s->m, n, out);
         ++ctx->launches;

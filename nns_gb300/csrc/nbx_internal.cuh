@@ -123,7 +123,8 @@ struct Ctx {
     int *d_team = nullptr, *d_solo = nullptr;  // [G]
 
     // per-system tree parameters
-    unsigned *d_bbox_u = nullptr;   // [6S] ordered-int encodings during the reduction
+    unsigned *d_bbox_u = nullptr;   // [6S] ordered-int encodings during the reduction (between builds: empty boxes)
+    unsigned *d_bbox_done = nullptr;  // [1] finished blocks of k_bbox (between builds: 0)
     float *d_bbox = nullptr;        // [6S]
     double *d_bbox64 = nullptr;     // [6S]
     float *d_depth0 = nullptr;      // [S]

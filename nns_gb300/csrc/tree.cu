@@ -51,16 +51,16 @@ constexpr int kDirectBlocks = 256;
 __device__ __forceinline__ int grid_stride_start() { return blockIdx.x * blockDim.x + threadIdx.x; }
 __device__ __forceinline__ int grid_stride() { return gridDim.x * blockDim.x; }
 
-// Also zeroes the nodes' meta words, which k_nodes adds up.
-__global__ void k_step_reset(unsigned *bbox_u, int nsys, DevStatus *st, int *sys_lvl, int *root_nch,
-                             int4 *__restrict__ meta4, int *__restrict__ meta, int cap_nodes) {
-    int i = grid_stride_start();
+// What a build starts from: the per-build counters of the status and of the
+// systems, and the nodes' meta words, which k_nodes adds up.
+__device__ __forceinline__ void reset_build(int nsys, DevStatus *st, int *sys_lvl, int *root_nch, int4 *meta4,
+                                            int *meta, int cap_nodes) {
+    const int i = grid_stride_start();
     for (int j = i; j < cap_nodes / 4; j += grid_stride()) meta4[j] = make_int4(0, 0, 0, 0);
     if (i < (cap_nodes & 3)) meta[(cap_nodes & ~3) + i] = 0;
-    if (i < 6 * nsys) bbox_u[i] = f2ord(0.0f);  // Kernels.cu:56-62: the box contains the origin
-    if (i < nsys) {
-        sys_lvl[i] = 0;
-        root_nch[i] = 0;  // k_nodes counts the root children up
+    for (int j = i; j < nsys; j += grid_stride()) {
+        sys_lvl[j] = 0;
+        root_nch[j] = 0;  // k_nodes counts the root children up
     }
     if (i == 0) {
         st->refined_runs = 0;
@@ -72,13 +72,29 @@ __global__ void k_step_reset(unsigned *bbox_u, int nsys, DevStatus *st, int *sys
     }
 }
 
-// Per-tile min/max of the bodies of one system, merged with ordered-int atomics.
+__global__ void k_step_reset(int nsys, DevStatus *st, int *sys_lvl, int *root_nch, int4 *__restrict__ meta4,
+                             int *__restrict__ meta, int cap_nodes) {
+    reset_build(nsys, st, sys_lvl, root_nch, meta4, meta, cap_nodes);
+}
+
+__device__ __forceinline__ float depth0_of(float mnx, float mxx, float theta_ref) {
+    float r = __fmul_rn(__fsub_rn(mxx, mnx), 0.5f);  // Kernels.cu:477
+    return __fdiv_rn(__fmul_rn(r, r), theta_ref);    // Kernels.cu:513
+}
+
+// The boxes of all systems, and the build's reset, in one launch: per-tile
+// min/max of the bodies of one system, merged with ordered-int atomics; the last
+// block to finish writes every system's box and its walk threshold and leaves
+// the scratch boxes empty (they contain the origin: Kernels.cu:56-62) and the
+// block counter at zero for the next build.
 __global__ void __launch_bounds__(kBlock) k_bbox(const float *__restrict__ x, const float *__restrict__ y,
                                                   const float *__restrict__ z, const int4 *__restrict__ tiles,
-                                                  int ntiles, unsigned *bbox_u) {
-    const int t = blockIdx.x;
-    if (t >= ntiles) return;
-    const int4 tl = tiles[t];
+                                                  int ntiles, unsigned *bbox_u, int nsys, float theta_ref, float *bbox,
+                                                  double *bbox64, float *depth0, unsigned *done, DevStatus *st,
+                                                  int *sys_lvl, int *root_nch, int4 *__restrict__ meta4,
+                                                  int *__restrict__ meta, int cap_nodes) {
+    reset_build(nsys, st, sys_lvl, root_nch, meta4, meta, cap_nodes);
+    const int4 tl = tiles[blockIdx.x];
     float v[6] = {INFINITY, -INFINITY, INFINITY, -INFINITY, INFINITY, -INFINITY};
     for (int i = threadIdx.x; i < tl.y; i += kBlock) {
         float a = x[tl.x + i], b = y[tl.x + i], c = z[tl.x + i];
@@ -95,6 +111,7 @@ __global__ void __launch_bounds__(kBlock) k_bbox(const float *__restrict__ x, co
         }
     }
     __shared__ float part[kBlock / 32][6];
+    __shared__ bool last;
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (lane == 0)
         for (int k = 0; k < 6; k++) part[w][k] = v[k];
@@ -108,25 +125,26 @@ __global__ void __launch_bounds__(kBlock) k_bbox(const float *__restrict__ x, co
             if (k & 1) atomicMax(dst, f2ord(r));
             else atomicMin(dst, f2ord(r));
         }
+        __threadfence();
     }
-}
-
-__device__ __forceinline__ float depth0_of(float mnx, float mxx, float theta_ref) {
-    float r = __fmul_rn(__fsub_rn(mxx, mnx), 0.5f);  // Kernels.cu:477
-    return __fdiv_rn(__fmul_rn(r, r), theta_ref);    // Kernels.cu:513
-}
-
-__global__ void k_bbox_finalize(const unsigned *bbox_u, int nsys, float theta_ref, float *bbox,
-                                double *bbox64, float *depth0) {
-    int s = grid_stride_start();
-    if (s >= nsys) return;
-    float b[6];
-    for (int k = 0; k < 6; k++) {
-        b[k] = __fadd_rn(ord2f(bbox_u[6 * s + k]), 0.0f);  // -0 -> +0
-        bbox[6 * s + k] = b[k];
-        bbox64[6 * s + k] = (double)b[k];
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        last = atomicAdd(done, 1u) == gridDim.x - 1;
+        __threadfence();
     }
-    depth0[s] = depth0_of(b[0], b[1], theta_ref);
+    __syncthreads();
+    if (!last) return;
+    if (threadIdx.x == 0) *done = 0u;
+    for (int s = threadIdx.x; s < nsys; s += kBlock) {
+        float b[6];
+        for (int k = 0; k < 6; k++) {
+            b[k] = __fadd_rn(ord2f(__ldcg(&bbox_u[6 * s + k])), 0.0f);  // -0 -> +0
+            bbox[6 * s + k] = b[k];
+            bbox64[6 * s + k] = (double)b[k];
+            bbox_u[6 * s + k] = f2ord(0.0f);
+        }
+        depth0[s] = depth0_of(b[0], b[1], theta_ref);
+    }
 }
 
 // Single-system box supplied by the caller (reference-compatible entry points).
@@ -1012,24 +1030,22 @@ int build_tree(Ctx *ctx, const nbx_state *s, cudaStream_t st, bool external_bbox
     const int S = ctx->nsys;
     if (n <= 0 || S <= 0) return NBX_ERR_STATE;
     const int gb = ceil_div(n, kBlock) < ctx->nsm * 8 ? ceil_div(n, kBlock) : ctx->nsm * 8;
-    const int need = 6 * S + 1 > ctx->cap_nodes / 4 ? 6 * S + 1 : ctx->cap_nodes / 4;
-    int gr = ceil_div(need, kBlock);
-    if (gr > ctx->nsm * 8) gr = ceil_div(6 * S + 1, kBlock) > ctx->nsm * 8 ? ceil_div(6 * S + 1, kBlock) : ctx->nsm * 8;
-    k_step_reset<<<gr, kBlock, 0, st>>>(ctx->d_bbox_u, S, ctx->d_status, ctx->d_sys_lvl, ctx->d_root_nch,
-                                        reinterpret_cast<int4 *>(ctx->d_meta), ctx->d_meta, ctx->cap_nodes);
-    ++ctx->launches;
+    int4 *meta4 = reinterpret_cast<int4 *>(ctx->d_meta);
     if (!external_bbox) {
-        k_bbox<<<ctx->ntiles_body, kBlock, 0, st>>>(s->x, s->y, s->z, ctx->d_tiles, ctx->ntiles_body,
-                                                    ctx->d_bbox_u);
-        ++ctx->launches;
-        k_bbox_finalize<<<ceil_div(S, kBlock), kBlock, 0, st>>>(ctx->d_bbox_u, S, ctx->theta_ref,
-                                                                ctx->d_bbox, ctx->d_bbox64, ctx->d_depth0);
+        k_bbox<<<ctx->ntiles_body, kBlock, 0, st>>>(s->x, s->y, s->z, ctx->d_tiles, ctx->ntiles_body, ctx->d_bbox_u, S,
+                                                    ctx->theta_ref, ctx->d_bbox, ctx->d_bbox64, ctx->d_depth0,
+                                                    ctx->d_bbox_done, ctx->d_status, ctx->d_sys_lvl, ctx->d_root_nch,
+                                                    meta4, ctx->d_meta, ctx->cap_nodes);
         ++ctx->launches;
     } else {
+        int gr = ceil_div(ctx->cap_nodes, 4 * kBlock);
+        if (gr > ctx->nsm * 8) gr = ctx->nsm * 8;
+        k_step_reset<<<gr, kBlock, 0, st>>>(S, ctx->d_status, ctx->d_sys_lvl, ctx->d_root_nch, meta4, ctx->d_meta,
+                                            ctx->cap_nodes);
         k_bbox_from_ptrs<<<1, 32, 0, st>>>(bbox_ptrs[0], bbox_ptrs[1], bbox_ptrs[2], bbox_ptrs[3],
                                            bbox_ptrs[4], bbox_ptrs[5], ctx->theta_ref, ctx->d_bbox,
                                            ctx->d_bbox64, ctx->d_depth0, ctx->d_status);
-        ++ctx->launches;
+        ctx->launches += 2;
     }
     // the node array is free until the nodes are written: it holds the packed bodies
     float4 *pos4 = ctx->d_node4;
