@@ -467,8 +467,9 @@ class BarnesHut:
         c0 = torch.cuda.Event(enable_timing=True)
         c1 = torch.cuda.Event(enable_timing=True)
         c0.record()
-        self.h_x, self.h_y, self.h_z = (a[:n].cpu().numpy() for a in (self.d_x, self.d_y, self.d_z))
-        self.h_vx, self.h_vy, self.h_vz = (a[:n].cpu().numpy() for a in (self.d_vx, self.d_vy, self.d_vz))
+        # one copy for the six arrays (rows of a fresh host array: earlier steps' stay as they were)
+        self.h_x, self.h_y, self.h_z, self.h_vx, self.h_vy, self.h_vz = torch.stack(
+            [a[:n] for a in (self.d_x, self.d_y, self.d_z, self.d_vx, self.d_vy, self.d_vz)]).cpu().numpy()
         c1.record()
         stop.record()
         stop.synchronize()

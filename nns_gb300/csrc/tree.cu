@@ -1207,13 +1207,17 @@ int export_tree_impl(Ctx *ctx, int sys, int *perm, int *root_child, int *cell_ch
     // the reference's array format holds the reference's tree: Lebesgue order, one body per leaf
     if (!ctx->built || ctx->key_order != 0 || ctx->leaf_size != 1) return NBX_ERR_STATE;
     if (sys < 0 || sys >= ctx->nsys) return NBX_ERR_ARG;
-    int off[2];
-    NBX_CUDA(cudaMemcpyAsync(off, ctx->d_sys_off + sys, 2 * sizeof(int), cudaMemcpyDeviceToHost, st));
+    // a single system's range is the whole context: only the node count is read back
+    int off[2] = {0, (int)ctx->nbodies};
     unsigned e_beg = 0, e_end = 0, T = 0;
-    NBX_CUDA(cudaMemcpyAsync(&e_beg, ctx->d_ecount + off[0], sizeof(unsigned), cudaMemcpyDeviceToHost, st));
+    if (ctx->nsys > 1) {
+        NBX_CUDA(cudaMemcpyAsync(off, ctx->d_sys_off + sys, 2 * sizeof(int), cudaMemcpyDeviceToHost, st));
+        NBX_CUDA(cudaStreamSynchronize(st));
+        NBX_CUDA(cudaMemcpyAsync(&e_beg, ctx->d_ecount + off[0], sizeof(unsigned), cudaMemcpyDeviceToHost, st));
+        if (off[1] < ctx->nbodies)
+            NBX_CUDA(cudaMemcpyAsync(&e_end, ctx->d_ecount + off[1], sizeof(unsigned), cudaMemcpyDeviceToHost, st));
+    }
     NBX_CUDA(cudaMemcpyAsync(&T, ctx->d_totals + 0, sizeof(unsigned), cudaMemcpyDeviceToHost, st));
-    if (off[1] < ctx->nbodies)
-        NBX_CUDA(cudaMemcpyAsync(&e_end, ctx->d_ecount + off[1], sizeof(unsigned), cudaMemcpyDeviceToHost, st));
     NBX_CUDA(cudaStreamSynchronize(st));
     if (off[1] >= ctx->nbodies) e_end = T;
     const int cells_before = (int)e_beg - off[0];
