@@ -55,7 +55,7 @@ struct Adj {
     double *lam = nullptr;   // [7][n]: lx,ly,lz,lvx,lvy,lvz,lm
     float *gcot = nullptr;   // [3][n]
     float *tdx = nullptr;    // [3][n] target terms
-    double *G = nullptr;     // [4][NC]: Gx,Gy,Gz,Gm
+    double4 *G = nullptr;    // [NC]: Gx,Gy,Gz,Gm (one 32-byte sector per node: its four atomics travel together)
     double *loss = nullptr;  // [1]
     double *r64 = nullptr;   // FP64 replay: [10][n] state + [4][NC] moments
     std::vector<TapeStep> tape;
@@ -168,7 +168,7 @@ __global__ void __launch_bounds__(kAdjWarps * 32)
                 const int *__restrict__ body_node, const int *__restrict__ groups, int ngroups,
                 const int *__restrict__ body_sys, const int *__restrict__ sys_off, const int *__restrict__ lists,
                 const int *__restrict__ list_len, int lcap, const float *__restrict__ gcot, int n, float eps2,
-                double *__restrict__ G, int nc_cap, float *__restrict__ tdx) {
+                double4 *__restrict__ G, int nc_cap, float *__restrict__ tdx) {
     __shared__ __align__(16) float red[kAdjWarps][kChunk * 4][kRedStride];
     __shared__ __align__(16) float4 stage[kAdjWarps][2][kChunk];  // node records of two chunks
     __shared__ float part[kAdjWarps][3][32];
@@ -278,7 +278,8 @@ __global__ void __launch_bounds__(kAdjWarps * 32)
                 float a0, a1, a2, a3;
                 upk(s01, a0, a1);
                 upk(s23, a2, a3);
-                if (crow < nc_cap) atomicAdd(&G[(size_t)(lane & 3) * nc_cap + crow], (double)((a0 + a1) + (a2 + a3)));
+                if (crow < nc_cap)
+                    atomicAdd(reinterpret_cast<double *>(&G[crow]) + (lane & 3), (double)((a0 + a1) + (a2 + a3)));
             }
             __syncwarp();  // the staging slot and the reduction rows are free again
             cmine = cnext;
@@ -315,26 +316,21 @@ __global__ void __launch_bounds__(kAdjWarps * 32)
 // written over the cell's G entries (FP64 divisions are slow on this part: one
 // per cell instead of one per body and ancestor).  Body entries stay as they are.
 __global__ void k_adj_cells(const float4 *__restrict__ node4, const int *__restrict__ meta,
-                            const unsigned *__restrict__ lvl, double *__restrict__ G, int nc_cap) {
+                            const unsigned *__restrict__ lvl, double4 *__restrict__ G) {
     const int T = (int)lvl[kMaxLevel + 1];  // node count
     for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < T; c += gridDim.x * blockDim.x) {
         if (meta[c] < 0) continue;
         const float4 q = node4[c];
         const double M = q.w;
-        const double gxc = G[c], gyc = G[(size_t)nc_cap + c], gzc = G[2 * (size_t)nc_cap + c],
-                     gmc = G[3 * (size_t)nc_cap + c];
-        G[c] = gxc / M;
-        G[(size_t)nc_cap + c] = gyc / M;
-        G[2 * (size_t)nc_cap + c] = gzc / M;
-        G[3 * (size_t)nc_cap + c] = gmc - (gxc * q.x + gyc * q.y + gzc * q.z) / M;
+        const double4 g = G[c];
+        G[c] = make_double4(g.x / M, g.y / M, g.z / M, g.w - (g.x * q.x + g.y * q.y + g.z * q.z) / M);
     }
 }
 
 // Gradients through the centres of mass to every body, and the state update.
 __global__ void k_adj_bodies(const float4 *__restrict__ body4, const int *__restrict__ val,
                              const int *__restrict__ body_node, const int *__restrict__ parent,
-                             const double *__restrict__ G, int nc_cap, const float *__restrict__ tdx, double *lam,
-                             int n) {
+                             const double4 *__restrict__ G, const float *__restrict__ tdx, double *lam, int n) {
     for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < n; p += gridDim.x * blockDim.x) {
         const int i = val[p];
         const int b = body_node[p];
@@ -342,18 +338,19 @@ __global__ void k_adj_bodies(const float4 *__restrict__ body4, const int *__rest
         double sax = 0.0, say = 0.0, saz = 0.0, sb = 0.0;
         int cur = parent[b];
         for (int guard = 0; guard < 64 && cur >= 0; guard++) {
-            sax += G[cur];
-            say += G[(size_t)nc_cap + cur];
-            saz += G[2 * (size_t)nc_cap + cur];
-            sb += G[3 * (size_t)nc_cap + cur];
+            const double4 g = G[cur];
             cur = parent[cur];
+            sax += g.x;
+            say += g.y;
+            saz += g.z;
+            sb += g.w;
         }
         const double m = me.w;
-        lam[i] += tdx[i] + m * sax + G[b];
-        lam[n + i] += tdx[n + i] + m * say + G[(size_t)nc_cap + b];
-        lam[2 * n + i] += tdx[2 * n + i] + m * saz + G[2 * (size_t)nc_cap + b];
-        lam[6 * n + i] += (double)me.x * sax + (double)me.y * say + (double)me.z * saz + sb +
-                          G[3 * (size_t)nc_cap + b];
+        const double4 g = G[b];
+        lam[i] += tdx[i] + m * sax + g.x;
+        lam[n + i] += tdx[n + i] + m * say + g.y;
+        lam[2 * n + i] += tdx[2 * n + i] + m * saz + g.z;
+        lam[6 * n + i] += (double)me.x * sax + (double)me.y * say + (double)me.z * saz + sb + g.w;
     }
 }
 
@@ -601,13 +598,13 @@ int reverse_step(Ctx *ctx, Adj *a, int j, cudaStream_t st) {
     const double dt = ctx->p.dt, ddt = (double)ctx->p.dampening * ctx->p.dt;
     TapeStep &t = a->tape[j];
     k_adj_prep<<<grid_for(n), kB, 0, st>>>(a->lam, a->gcot, n, dt, ddt);
-    NBX_CUDA(cudaMemsetAsync(a->G, 0, sizeof(double) * 4 * (size_t)NC, st));
+    NBX_CUDA(cudaMemsetAsync(a->G, 0, sizeof(double4) * (size_t)NC, st));
     const int blocks = a->ngroups;
     k_adj_force<<<blocks < ctx->nsm * 16 ? blocks : ctx->nsm * 16, kAdjWarps * 32, 0, st>>>(
         t.node4, t.body4, t.val, t.body_node, ctx->d_groups, a->ngroups, ctx->d_body_sys, ctx->d_sys_off, t.lists,
         t.list_len, a->lcap, a->gcot, n, ctx->eps2, a->G, NC, a->tdx);
-    k_adj_cells<<<grid_for(NC), kB, 0, st>>>(t.node4, t.meta, t.lvl, a->G, NC);
-    k_adj_bodies<<<grid_for(n), kB, 0, st>>>(t.body4, t.val, t.body_node, t.parent, a->G, NC, a->tdx, a->lam, n);
+    k_adj_cells<<<grid_for(NC), kB, 0, st>>>(t.node4, t.meta, t.lvl, a->G);
+    k_adj_bodies<<<grid_for(n), kB, 0, st>>>(t.body4, t.val, t.body_node, t.parent, a->G, a->tdx, a->lam, n);
     ctx->launches += 4;
     NBX_CUDA(cudaGetLastError());
     return NBX_OK;
@@ -634,7 +631,7 @@ int adjoint_create(Ctx *ctx, int T, int C, int lcap, int tape_steps, Adj **out) 
     rc |= amalloc(ctx, a, &a->lam, (size_t)7 * n);
     rc |= amalloc(ctx, a, &a->gcot, (size_t)3 * n);
     rc |= amalloc(ctx, a, &a->tdx, (size_t)3 * n);
-    rc |= amalloc(ctx, a, &a->G, (size_t)4 * NC);
+    rc |= amalloc(ctx, a, &a->G, (size_t)NC);
     rc |= amalloc(ctx, a, &a->loss, 2);
     rc |= amalloc(ctx, a, &a->r64, (size_t)10 * n + (size_t)4 * NC);
     rc |= amalloc(ctx, a, &a->mass, (size_t)n);
