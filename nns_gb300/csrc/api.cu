@@ -645,6 +645,7 @@ int nbx_compute_forces(nbx_ctx *c, float *x, float *y, float *z, float *vx, floa
                        float g, void *stream, float *ms) {
     (void)x; (void)y; (void)z; (void)vx; (void)vy; (void)vz; (void)mass; (void)sorted; (void)child; (void)g;
     if (!c || !ax || !ay || !az || !minX || !maxX) return NBX_ERR_ARG;
+    C(c)->chain = false;
     Ctx *ctx = C(c);
     if (!ctx->built || ctx->nbodies != n) return NBX_ERR_STATE;
     nbx::Timer t(ms, S(stream));
@@ -658,6 +659,7 @@ int nbx_compute_forces(nbx_ctx *c, float *x, float *y, float *z, float *vx, floa
 int nbx_update(nbx_ctx *c, float *x, float *y, float *z, float *vx, float *vy, float *vz, float *ax, float *ay,
                float *az, int n, float dt, float d, void *stream, float *ms) {
     if (!c || !x || !vx || !ax || n < 0) return NBX_ERR_ARG;
+    C(c)->chain = false;
     nbx::Timer t(ms, S(stream));
     nbx_state s{x, y, z, vx, vy, vz, ax, ay, az, nullptr};
     return t.finish(nbx::integrate(C(c), &s, dt, d, n, S(stream)));
@@ -681,6 +683,7 @@ int nbx_build(nbx_ctx *c, const nbx_state *s, void *stream) {
 
 int nbx_forces(nbx_ctx *c, const nbx_state *s, void *stream) {
     if (!c || !s || !s->ax || !s->ay || !s->az) return NBX_ERR_ARG;
+    C(c)->chain = false;
     Range r("nbx_forces");
     return nbx::walk_forces(C(c), s, S(stream));
 }
@@ -693,6 +696,7 @@ int nbx_group_count(nbx_ctx *c, int *ngroups) {
 
 int nbx_forces_groups(nbx_ctx *c, const nbx_state *s, int first_group, int ngroups, void *stream) {
     if (!c || !s || !s->ax || !s->ay || !s->az) return NBX_ERR_ARG;
+    C(c)->chain = false;
     Range r("nbx_forces_groups");
     return nbx::walk_forces_groups(C(c), s, first_group, ngroups, S(stream));
 }
@@ -713,6 +717,7 @@ int nbx_export_group_stats(nbx_ctx *c, int *list_len, int *opened, void *stream)
 
 int nbx_integrate(nbx_ctx *c, const nbx_state *s, void *stream) {
     if (!c || !s || !s->vx || !s->ax) return NBX_ERR_ARG;
+    C(c)->chain = false;
     Range r("nbx_integrate");
     Ctx *ctx = C(c);
     return nbx::integrate(ctx, s, ctx->p.dt, ctx->p.dampening, (int)ctx->nbodies, S(stream));
@@ -913,6 +918,7 @@ int nbx_forces_fp64_lists(nbx_ctx *c, const int *group_starts, int ngroups, doub
 
 int nbx_potential(nbx_ctx *c, const nbx_state *s, float *phi, void *stream) {
     if (!c || !s || !phi) return NBX_ERR_ARG;
+    C(c)->chain = false;
     if (!(C(c)->eps2 > 0.f)) return NBX_ERR_ARG;
     return nbx::walk_potential(C(c), s, phi, S(stream));
 }

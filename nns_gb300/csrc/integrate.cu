@@ -15,6 +15,7 @@ __global__ void __launch_bounds__(kBlock) k_update(float *__restrict__ x, float 
                                                     float *__restrict__ vy, float *__restrict__ vz,
                                                     const float *__restrict__ ax, const float *__restrict__ ay,
                                                     const float *__restrict__ az, int n, float dt, float ddt) {
+    grid_dependency();
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const float nvx = __fmaf_rn(dt, ax[i], vx[i]);
         const float nvy = __fmaf_rn(dt, ay[i], vy[i]);
@@ -37,6 +38,7 @@ __global__ void __launch_bounds__(kBlock) k_update4(float4 *__restrict__ x, floa
                                                      float4 *__restrict__ vy, float4 *__restrict__ vz,
                                                      const float4 *__restrict__ ax, const float4 *__restrict__ ay,
                                                      const float4 *__restrict__ az, int n, float dt, float ddt) {
+    grid_dependency();
     const int n4 = n >> 2;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n4; i += gridDim.x * blockDim.x) {
         float4 v[3] = {vx[i], vy[i], vz[i]};
@@ -248,14 +250,14 @@ int integrate(Ctx *ctx, const nbx_state *s, float dt, float d, int n, cudaStream
     int grid = ceil_div(aligned && n >= 4 ? n >> 2 : n, kBlock);
     if (grid > ctx->nsm * 16) grid = ctx->nsm * 16;
     if (aligned && n >= 4)
-        k_update4<<<grid, kBlock, 0, st>>>(
-            reinterpret_cast<float4 *>(s->x), reinterpret_cast<float4 *>(s->y), reinterpret_cast<float4 *>(s->z),
-            reinterpret_cast<float4 *>(s->vx), reinterpret_cast<float4 *>(s->vy), reinterpret_cast<float4 *>(s->vz),
-            reinterpret_cast<const float4 *>(s->ax), reinterpret_cast<const float4 *>(s->ay),
-            reinterpret_cast<const float4 *>(s->az), n, dt, ddt);
+        launch_chained(ctx, st, grid, kBlock, 0, k_update4, reinterpret_cast<float4 *>(s->x),
+                       reinterpret_cast<float4 *>(s->y), reinterpret_cast<float4 *>(s->z),
+                       reinterpret_cast<float4 *>(s->vx), reinterpret_cast<float4 *>(s->vy),
+                       reinterpret_cast<float4 *>(s->vz), reinterpret_cast<const float4 *>(s->ax),
+                       reinterpret_cast<const float4 *>(s->ay), reinterpret_cast<const float4 *>(s->az), n, dt, ddt);
     else
-        k_update<<<grid, kBlock, 0, st>>>(s->x, s->y, s->z, s->vx, s->vy, s->vz, s->ax, s->ay, s->az, n, dt, ddt);
-    ++ctx->launches;
+        launch_chained(ctx, st, grid, kBlock, 0, k_update, s->x, s->y, s->z, s->vx, s->vy, s->vz, s->ax, s->ay, s->az, n,
+                       dt, ddt);
     NBX_CUDA(cudaGetLastError());
     return NBX_OK;
 }

@@ -38,6 +38,7 @@ __global__ void __launch_bounds__(kThreads) k_merge(const int4 *__restrict__ til
                                                     const int *__restrict__ val_in,
                                                     unsigned long long *__restrict__ key_out,
                                                     int *__restrict__ val_out) {
+    grid_dependency();
     extern __shared__ __align__(16) unsigned long long stage[];  // [cap]
     __shared__ int s_lo[kMergeFan], s_len[kMergeFan], s_off[kMergeFan];
     const int4 t = tiles[blockIdx.x];  // start, len, system, tile of the system
@@ -199,9 +200,8 @@ int merge_runs(Ctx *ctx, cudaStream_t st) {
     int R = kMergeRun;
     for (int pass = 0; pass < passes; pass++) {
         const int cap = stage_cap(fan);
-        k_merge<<<ctx->ntiles_mg, kThreads, sizeof(unsigned long long) * cap, st>>>(ctx->d_tiles_mg, ctx->d_sys_off, R,
-                                                                                   fan, cap, k0, v0, k1, v1);
-        ++ctx->launches;
+        launch_chained(ctx, st, ctx->ntiles_mg, kThreads, sizeof(unsigned long long) * cap, k_merge, ctx->d_tiles_mg,
+                       ctx->d_sys_off, R, fan, cap, k0, v0, k1, v1);
         std::swap(k0, k1);
         std::swap(v0, v1);
         R *= fan;

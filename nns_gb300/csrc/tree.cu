@@ -74,6 +74,7 @@ __device__ __forceinline__ void reset_build(int nsys, DevStatus *st, int *sys_lv
 
 __global__ void k_step_reset(int nsys, DevStatus *st, int *sys_lvl, int *root_nch, int4 *__restrict__ meta4,
                              int *__restrict__ meta, int cap_nodes) {
+    grid_dependency();
     reset_build(nsys, st, sys_lvl, root_nch, meta4, meta, cap_nodes);
 }
 
@@ -93,6 +94,7 @@ __global__ void __launch_bounds__(kBlock) k_bbox(const float *__restrict__ x, co
                                                   double *bbox64, float *depth0, unsigned *done, DevStatus *st,
                                                   int *sys_lvl, int *root_nch, int4 *__restrict__ meta4,
                                                   int *__restrict__ meta, int cap_nodes) {
+    grid_dependency();
     reset_build(nsys, st, sys_lvl, root_nch, meta4, meta, cap_nodes);
     const int4 tl = tiles[blockIdx.x];
     float v[6] = {INFINITY, -INFINITY, INFINITY, -INFINITY, INFINITY, -INFINITY};
@@ -152,6 +154,7 @@ __global__ void k_bbox_from_ptrs(const float *mnx, const float *mxx, const float
                                  const float *mxy, const float *mnz, const float *mxz,
                                  float theta_ref, float *bbox, double *bbox64, float *depth0,
                                  DevStatus *st) {
+    grid_dependency();
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
     float b[6] = {*mnx, *mxx, *mny, *mxy, *mnz, *mxz};
     for (int k = 0; k < 6; k++) { bbox[k] = b[k]; bbox64[k] = (double)b[k]; }
@@ -213,6 +216,7 @@ __global__ void __launch_bounds__(kBlock) k_keys(const float *__restrict__ x, co
                                                   const float *__restrict__ bbox, int n,
                                                   unsigned long long *__restrict__ key, int *__restrict__ val,
                                                   float4 *__restrict__ pos4, DevStatus *st, int order) {
+    grid_dependency();
     __shared__ unsigned char ht[96];
     load_hilbert(ht, order);
     for (int i = grid_stride_start(); i < n; i += grid_stride()) {
@@ -241,6 +245,7 @@ __global__ void __cluster_dims__(4, 1, 1) __launch_bounds__(kMergeTile)
                  const float *__restrict__ m, const int4 *__restrict__ runs, const float *__restrict__ bbox,
                  unsigned long long *__restrict__ key, int *__restrict__ val, float4 *__restrict__ pos4, DevStatus *st,
                  int order) {
+    grid_dependency();
     constexpr int kQ = kMergeTile;  // a quarter
     static_assert(kMergeRun == 4 * kQ, "four quarters");
     __shared__ unsigned char ht[96];
@@ -341,6 +346,7 @@ __global__ void k_refine(const float *__restrict__ x, const float *__restrict__ 
                          const unsigned long long *__restrict__ key,
                          unsigned long long *__restrict__ key_lo, int *__restrict__ val,
                          DevStatus *st, int order) {
+    grid_dependency();
     __shared__ unsigned char ht[96];
     load_hilbert(ht, order);
     for (int p = grid_stride_start(); p < n; p += grid_stride()) {
@@ -439,6 +445,7 @@ __global__ void __launch_bounds__(kPosBlock) k_delta(const float4 *__restrict__ 
                                                       unsigned char *__restrict__ delta,
                                                       unsigned *__restrict__ counts, DevStatus *st,
                                                       int *__restrict__ sys_lvl) {
+    grid_dependency();
     __shared__ unsigned cnt[kLvlRow];
     const int p = blockIdx.x * kPosBlock + threadIdx.x;
     int lo = 1, hi = 0, s = -1;
@@ -483,6 +490,7 @@ __global__ void __launch_bounds__(kPosBlock) k_bucket(const int *__restrict__ bo
                                                        const unsigned char *__restrict__ delta,
                                                        unsigned char *__restrict__ bucket,
                                                        unsigned *__restrict__ counts) {
+    grid_dependency();
     __shared__ unsigned cnt[kLvlRow];
     const int p = blockIdx.x * kPosBlock + threadIdx.x;
     int lo = 1, hi = 0;
@@ -506,6 +514,7 @@ __global__ void __launch_bounds__(kPosBlock) k_bucket(const int *__restrict__ bo
 // in place; the level's total goes to totals[level].
 __global__ void __launch_bounds__(1024) k_level_scan(unsigned *__restrict__ counts, int nblk,
                                                       unsigned *__restrict__ totals) {
+    grid_dependency();
     constexpr int kPer = 8;
     __shared__ unsigned wt[32];
     const int l = blockIdx.x, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -571,6 +580,7 @@ __global__ void __launch_bounds__(kPosBlock) k_nodes(const int *__restrict__ bod
                                                       int *__restrict__ arrive, unsigned char *__restrict__ lvl8,
                                                       int *__restrict__ root_first, int *__restrict__ root_nch,
                                                       DevStatus *st) {
+    grid_dependency();
     constexpr int kWarps = kPosBlock / 32, kRows = kPosBlock / kLvlRow;
     __shared__ unsigned part[2][kRows][kLvlRow];  // Direct: partial sums (all blocks, earlier blocks)
     __shared__ unsigned base[kLvlRow];            // index of the block's first node of each level
@@ -884,6 +894,7 @@ __global__ void __launch_bounds__(kBlock) k_moments_level(int level, const unsig
                                                            const int *__restrict__ meta, float4 *node4,
                                                            double4 *sums, int *count, double *com, double2 *m2,
                                                            float4 *quad4, float2 *quad2, const DevStatus *st) {
+    grid_dependency();
     constexpr int kLanes = Quad ? 8 : 4, kGroups = 32 / kLanes;
     if (st->code != 0) return;  // an inconsistent tree is never summed
     __shared__ int list[kBlock / 32][32];
@@ -943,6 +954,7 @@ __global__ void __launch_bounds__(kBlock) k_moments_up(const unsigned *__restric
                                                        double4 *sums, int *count, int *counter, double *com,
                                                        double2 *m2, float4 *quad4, float2 *quad2,
                                                        const DevStatus *st) {
+    grid_dependency();
     constexpr int kLanes = Quad ? 8 : 4;
     if (st->code != 0) return;  // an inconsistent tree is never summed
     __shared__ int list[kBlock / 32][32 * kUpRounds];
@@ -1029,23 +1041,21 @@ int build_tree(Ctx *ctx, const nbx_state *s, cudaStream_t st, bool external_bbox
     const int n = (int)ctx->nbodies;
     const int S = ctx->nsys;
     if (n <= 0 || S <= 0) return NBX_ERR_STATE;
+    ctx->chain = false;
     const int gb = ceil_div(n, kBlock) < ctx->nsm * 8 ? ceil_div(n, kBlock) : ctx->nsm * 8;
     int4 *meta4 = reinterpret_cast<int4 *>(ctx->d_meta);
     if (!external_bbox) {
-        k_bbox<<<ctx->ntiles_body, kBlock, 0, st>>>(s->x, s->y, s->z, ctx->d_tiles, ctx->ntiles_body, ctx->d_bbox_u, S,
-                                                    ctx->theta_ref, ctx->d_bbox, ctx->d_bbox64, ctx->d_depth0,
-                                                    ctx->d_bbox_done, ctx->d_status, ctx->d_sys_lvl, ctx->d_root_nch,
-                                                    meta4, ctx->d_meta, ctx->cap_nodes);
-        ++ctx->launches;
+        launch_chained(ctx, st, ctx->ntiles_body, kBlock, 0, k_bbox, s->x, s->y, s->z, ctx->d_tiles, ctx->ntiles_body,
+                       ctx->d_bbox_u, S, ctx->theta_ref, ctx->d_bbox, ctx->d_bbox64, ctx->d_depth0, ctx->d_bbox_done,
+                       ctx->d_status, ctx->d_sys_lvl, ctx->d_root_nch, meta4, ctx->d_meta, ctx->cap_nodes);
     } else {
         int gr = ceil_div(ctx->cap_nodes, 4 * kBlock);
         if (gr > ctx->nsm * 8) gr = ctx->nsm * 8;
-        k_step_reset<<<gr, kBlock, 0, st>>>(S, ctx->d_status, ctx->d_sys_lvl, ctx->d_root_nch, meta4, ctx->d_meta,
-                                            ctx->cap_nodes);
-        k_bbox_from_ptrs<<<1, 32, 0, st>>>(bbox_ptrs[0], bbox_ptrs[1], bbox_ptrs[2], bbox_ptrs[3],
-                                           bbox_ptrs[4], bbox_ptrs[5], ctx->theta_ref, ctx->d_bbox,
-                                           ctx->d_bbox64, ctx->d_depth0, ctx->d_status);
-        ctx->launches += 2;
+        launch_chained(ctx, st, gr, kBlock, 0, k_step_reset, S, ctx->d_status, ctx->d_sys_lvl, ctx->d_root_nch, meta4,
+                       ctx->d_meta, ctx->cap_nodes);
+        launch_chained(ctx, st, 1, 32, 0, k_bbox_from_ptrs, bbox_ptrs[0], bbox_ptrs[1], bbox_ptrs[2], bbox_ptrs[3],
+                       bbox_ptrs[4], bbox_ptrs[5], ctx->theta_ref, ctx->d_bbox, ctx->d_bbox64, ctx->d_depth0,
+                       ctx->d_status);
     }
     // the node array is free until the nodes are written: it holds the packed bodies
     float4 *pos4 = ctx->d_node4;
@@ -1056,40 +1066,32 @@ int build_tree(Ctx *ctx, const nbx_state *s, cudaStream_t st, bool external_bbox
     unsigned long long *key0 = alt ? ctx->d_key_alt : ctx->d_key;
     int *val0 = alt ? ctx->d_val_alt : ctx->d_val;
     if (merge)
-        k_sort_tiles<<<4 * ctx->nruns_mg, kMergeTile, 0, st>>>(s->x, s->y, s->z, s->m, ctx->d_runs_mg, ctx->d_bbox,
-                                                          key0, val0, pos4, ctx->d_status, ctx->key_order);
+        launch_chained(ctx, st, 4 * ctx->nruns_mg, kMergeTile, 0, k_sort_tiles, s->x, s->y, s->z, s->m, ctx->d_runs_mg,
+                       ctx->d_bbox, key0, val0, pos4, ctx->d_status, ctx->key_order);
     else
-        k_keys<<<gb, kBlock, 0, st>>>(s->x, s->y, s->z, s->m, ctx->d_body_sys, ctx->d_bbox, n, key0, val0, pos4,
-                                      ctx->d_status, ctx->key_order);
-    ++ctx->launches;
+        launch_chained(ctx, st, gb, kBlock, 0, k_keys, s->x, s->y, s->z, s->m, ctx->d_body_sys, ctx->d_bbox, n, key0,
+                       val0, pos4, ctx->d_status, ctx->key_order);
     int rc = merge ? merge_runs(ctx, st) : radix_sort_bodies(ctx, st);
     if (rc) return rc;
-    k_refine<<<gb, kBlock, 0, st>>>(s->x, s->y, s->z, ctx->d_body_sys, ctx->d_sys_off, ctx->d_bbox, n,
-                                    ctx->d_key, ctx->d_key_lo, ctx->d_val, ctx->d_status, ctx->key_order);
-    ++ctx->launches;
+    launch_chained(ctx, st, gb, kBlock, 0, k_refine, s->x, s->y, s->z, ctx->d_body_sys, ctx->d_sys_off, ctx->d_bbox, n,
+                   ctx->d_key, ctx->d_key_lo, ctx->d_val, ctx->d_status, ctx->key_order);
     const unsigned char *bucket = ctx->leaf_size > 1 ? ctx->d_bucket : nullptr;
     const int nblk = ceil_div(n, kPosBlock);
-    k_delta<<<nblk, kPosBlock, 0, st>>>(pos4, ctx->d_body_sys, ctx->d_sys_off, n, ctx->d_key, ctx->d_key_lo,
-                                        ctx->d_val, ctx->d_body4, ctx->d_delta, bucket ? nullptr : ctx->d_lvl_counts,
-                                        ctx->d_status, ctx->d_sys_lvl);
-    ++ctx->launches;
-    if (bucket) {
-        k_bucket<<<nblk, kPosBlock, 0, st>>>(ctx->d_body_sys, ctx->d_sys_off, n, ctx->leaf_size, ctx->d_delta,
-                                             ctx->d_bucket, ctx->d_lvl_counts);
-        ++ctx->launches;
-    }
+    launch_chained(ctx, st, nblk, kPosBlock, 0, k_delta, pos4, ctx->d_body_sys, ctx->d_sys_off, n, ctx->d_key,
+                   ctx->d_key_lo, ctx->d_val, ctx->d_body4, ctx->d_delta, bucket ? nullptr : ctx->d_lvl_counts,
+                   ctx->d_status, ctx->d_sys_lvl);
+    if (bucket)
+        launch_chained(ctx, st, nblk, kPosBlock, 0, k_bucket, ctx->d_body_sys, ctx->d_sys_off, n, ctx->leaf_size,
+                       ctx->d_delta, ctx->d_bucket, ctx->d_lvl_counts);
     const bool direct = nblk <= kDirectBlocks;
-    if (!direct) {
-        k_level_scan<<<kLvlRow, 1024, 0, st>>>(ctx->d_lvl_counts, nblk, ctx->d_lvl_tot);
-        ++ctx->launches;
-    }
+    if (!direct)
+        launch_chained(ctx, st, kLvlRow, 1024, 0, k_level_scan, ctx->d_lvl_counts, nblk, ctx->d_lvl_tot);
     auto nodes = direct ? k_nodes<true> : k_nodes<false>;
-    nodes<<<nblk, kPosBlock, 0, st>>>(ctx->d_body_sys, ctx->d_sys_off, n, ctx->d_delta, bucket, ctx->d_lvl_counts, nblk,
-                                      ctx->d_lvl_tot, ctx->cap_nodes, ctx->d_body4, ctx->d_totals, ctx->d_totals64,
-                                      ctx->d_lvl_start, ctx->d_ecount, ctx->d_ent, ctx->d_node4, ctx->d_meta,
-                                      ctx->d_parent, ctx->d_body_node, ctx->d_count, ctx->d_arrive, ctx->d_lvl8,
-                                      ctx->d_root_first, ctx->d_root_nch, ctx->d_status);
-    ++ctx->launches;
+    launch_chained(ctx, st, nblk, kPosBlock, 0, nodes, ctx->d_body_sys, ctx->d_sys_off, n, ctx->d_delta, bucket,
+                   ctx->d_lvl_counts, nblk, ctx->d_lvl_tot, ctx->cap_nodes, ctx->d_body4, ctx->d_totals,
+                   ctx->d_totals64, ctx->d_lvl_start, ctx->d_ecount, ctx->d_ent, ctx->d_node4, ctx->d_meta,
+                   ctx->d_parent, ctx->d_body_node, ctx->d_count, ctx->d_arrive, ctx->d_lvl8, ctx->d_root_first,
+                   ctx->d_root_nch, ctx->d_status);
     const int gn = ceil_div(ctx->cap_nodes, kBlock) < ctx->nsm * 8 ? ceil_div(ctx->cap_nodes, kBlock) : ctx->nsm * 8;
     // up to 2^21 bodies the 41 per-level launches cost more than the sums: one
     // bottom-up launch (2^16: 0.37 against 0.55 ms per build); above, the
@@ -1105,19 +1107,16 @@ int build_tree(Ctx *ctx, const nbx_state *s, cudaStream_t st, bool external_bbox
         int rounds = (int)(3ll * n / 2 / (32ll * 32 * ctx->nsm));
         rounds = rounds < 1 ? 1 : (rounds > kUpRounds ? kUpRounds : rounds);
         auto kern = quad ? k_moments_up<true> : k_moments_up<false>;
-        kern<<<gn, kBlock, 0, st>>>(ctx->d_totals, rounds, ctx->d_parent, ctx->d_meta, ctx->d_node4, ctx->d_sums,
-                                    ctx->d_count, ctx->d_arrive, ctx->d_com, ctx->d_m2, ctx->d_quad4, ctx->d_quad2,
-                                    ctx->d_status);
-        ++ctx->launches;
+        launch_chained(ctx, st, gn, kBlock, 0, kern, ctx->d_totals, rounds, ctx->d_parent, ctx->d_meta, ctx->d_node4,
+                       ctx->d_sums, ctx->d_count, ctx->d_arrive, ctx->d_com, ctx->d_m2, ctx->d_quad4, ctx->d_quad2,
+                       ctx->d_status);
     } else {
         // cells exist at levels 1..41 (two bodies share at most 41 levels without error)
         auto kern = quad ? k_moments_level<true> : k_moments_level<false>;
-        for (int level = kMaxLevel - 2; level >= 1; level--) {
-            kern<<<ctx->nsm * 4, kBlock, 0, st>>>(level, ctx->d_lvl_start, ctx->d_meta, ctx->d_node4, ctx->d_sums,
-                                                  ctx->d_count, ctx->d_com, ctx->d_m2, ctx->d_quad4, ctx->d_quad2,
-                                                  ctx->d_status);
-            ++ctx->launches;
-        }
+        for (int level = kMaxLevel - 2; level >= 1; level--)
+            launch_chained(ctx, st, ctx->nsm * 4, kBlock, 0, kern, level, ctx->d_lvl_start, ctx->d_meta, ctx->d_node4,
+                           ctx->d_sums, ctx->d_count, ctx->d_com, ctx->d_m2, ctx->d_quad4, ctx->d_quad2,
+                           ctx->d_status);
     }
     NBX_CUDA(cudaGetLastError());
     ctx->built = true;

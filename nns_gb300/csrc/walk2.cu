@@ -100,6 +100,7 @@ __global__ void __launch_bounds__(WalkBounds<CB>::kThreads, WalkBounds<CB>::kMin
             float *__restrict__ ax, float *__restrict__ ay, float *__restrict__ az, float *__restrict__ pot,
             int2 *__restrict__ gstat, DevStatus *st, int *__restrict__ rec_list,
             int *__restrict__ rec_len, int rec_cap) {
+    grid_dependency();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     if (st->code != 0) return;
     const int warps = blockDim.x >> 5;
@@ -542,12 +543,13 @@ int launch(Ctx *ctx, const nbx_state *s, float *pot, int warps, cudaStream_t st,
     // without a list the group arrays start at the first group
     const int off = share.list ? 0 : share.first;
     NBX_CUDA(cudaMemsetAsync(&ctx->d_status->walk_next, 0, sizeof(unsigned), st));
-    k_walk2<CB, Mode, Pot, Rec, Quad><<<grid, warps * 32, smem, st>>>(
+    ctx->chain = false;  // (a memory operation came between)
+    launch_chained(
+        ctx, st, grid, warps * 32, smem, k_walk2<CB, Mode, Pot, Rec, Quad>,
         ctx->d_node4, ctx->d_meta, ctx->d_lvl8, ctx->d_quad4, ctx->d_quad2, ctx->d_body4, ctx->d_val,
         ctx->d_groups + off, share.list ? share.list + share.first : nullptr, share.count, ctx->d_body_sys,
         ctx->d_sys_off, ctx->d_depth0, ctx->d_root_first, ctx->d_root_nch, ctx->d_sys_lvl, ctx->eps2, cap, s->ax,
         s->ay, s->az, pot, ctx->d_gstat + off, ctx->d_status, rec_list, rec_len, rec_cap);
-    ++ctx->launches;
     NBX_CUDA(cudaGetLastError());
     return NBX_OK;
 }

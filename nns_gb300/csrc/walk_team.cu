@@ -96,6 +96,7 @@ __global__ void __launch_bounds__(kW * 32, 32 / kW)
                 float eps2, int stack_cap, float *__restrict__ ax, float *__restrict__ ay, float *__restrict__ az,
                 float *__restrict__ pot, int2 *__restrict__ gstat, DevStatus *st, int *__restrict__ rec_list,
                 int *__restrict__ rec_len, int rec_cap) {
+    grid_dependency();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     if (st->code != 0) return;
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -567,12 +568,11 @@ int launch_team(Ctx *ctx, const nbx_state *s, float *pot, cudaStream_t st, const
         ctx->last_error = "walk: stack_depth too large for the launch shape's shared memory";
         return NBX_ERR_ARG;
     }
-    k_walk_team<Mode, Pot, Rec, Quad><<<count, kW * 32, smem, st>>>(
-        ctx->d_node4, ctx->d_meta, ctx->d_quad4, ctx->d_quad2, ctx->d_body4, ctx->d_val, ctx->d_groups, list, first,
-        ctx->d_body_sys, ctx->d_sys_off, ctx->d_depth0, ctx->d_root_first, ctx->d_root_nch, ctx->d_sys_lvl, ctx->eps2,
-        kStackMul * ctx->p.stack_depth, s->ax, s->ay, s->az, pot, ctx->d_gstat, ctx->d_status, rec_list, rec_len,
-        rec_cap);
-    ++ctx->launches;
+    launch_chained(ctx, st, count, kW * 32, smem, k_walk_team<Mode, Pot, Rec, Quad>, ctx->d_node4, ctx->d_meta,
+                   ctx->d_quad4, ctx->d_quad2, ctx->d_body4, ctx->d_val, ctx->d_groups, list, first, ctx->d_body_sys,
+                   ctx->d_sys_off, ctx->d_depth0, ctx->d_root_first, ctx->d_root_nch, ctx->d_sys_lvl, ctx->eps2,
+                   kStackMul * ctx->p.stack_depth, s->ax, s->ay, s->az, pot, ctx->d_gstat, ctx->d_status, rec_list,
+                   rec_len, rec_cap);
     NBX_CUDA(cudaGetLastError());
     return NBX_OK;
 }
