@@ -44,9 +44,16 @@ constexpr int kMergeFan = 16;     // most runs merged by one launch
 #define NBX_MERGE_MAX (1 << 19)
 #endif
 constexpr int kMergeMaxBodies = NBX_MERGE_MAX;
-// systems of up to this many bodies are walked by teams of warps (walk_team.cu)
+// Systems of up to this many bodies are walked by teams of warps (walk_team.cu).
+// The rule sees a system's own size only, so that a batch gives every system the
+// bits of its single run.  Alone, teams win up to about 2^17 bodies (walk at 2^16:
+// 148 against 193 us, at 2^17 240 against 305); in a batch that fills the GPU they
+// cost 10 % more than single warps (400 systems of 2^11 to 2^16 bodies, walk 11.2
+// against 10.0 ms), which outweighs what the build gained once large systems are
+// in.  At 2^14 a system alone gains most (70 against 212 us) and batches of any
+// sizes stay ahead.
 #ifndef NBX_TEAM_MAX
-#define NBX_TEAM_MAX (1 << 17)
+#define NBX_TEAM_MAX (1 << 14)
 #endif
 constexpr int kTeamMaxBodies = NBX_TEAM_MAX;
 constexpr int kMaxRadixBits = 9;  // body-key digits: 8 or 9 bits (histograms sized for 9)

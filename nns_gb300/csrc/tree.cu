@@ -1096,11 +1096,12 @@ int build_tree(Ctx *ctx, const nbx_state *s, cudaStream_t st, bool external_bbox
     // up to 2^21 bodies the 41 per-level launches cost more than the sums: one
     // bottom-up launch (2^16: 0.37 against 0.55 ms per build); above, the
     // per-level launches stream the levels and are faster (a batch's chains are
-    // shorter: 200 systems, 3.2 x 10^6 bodies, 6.10 against 6.18 ms per step)
+    // shorter: 200 systems, 3.2 x 10^6 bodies, 6.10 against 6.18 ms per step;
+    // with quadrupoles the one launch loses there, 3.04 against 2.86 ms per build)
     const int mode = ctx->p.moments_mode;
     const bool quad = ctx->multipole != 0;
     if (quad && !ctx->d_m2) return NBX_ERR_STATE;
-    const int up_max = S > 1 ? 4 * kMomentsUpMaxBodies : kMomentsUpMaxBodies;
+    const int up_max = S > 1 && !quad ? 4 * kMomentsUpMaxBodies : kMomentsUpMaxBodies;
     if (mode == 2 || (mode == 0 && n <= up_max)) {
         // one round of 32 nodes per warp until that fills the GPU's warps (a small
         // tree wants its chains started at once), then up to four (fuller groups)

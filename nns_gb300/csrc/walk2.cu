@@ -516,6 +516,12 @@ __global__ void __launch_bounds__(WalkBounds<CB>::kThreads, WalkBounds<CB>::kMin
     }
 }
 
+#ifndef NBX_SPREAD_BLOCK
+#define NBX_SPREAD_BLOCK 2
+#endif
+constexpr int kSpreadBlock = NBX_SPREAD_BLOCK;  // warps of a block of a launch that fits the GPU at once
+constexpr int kSpreadWarps = 32;                // such a launch has at most this many groups per SM
+
 // Which groups one launch walks: `count` from the first, or the entries of a list
 // (device array) from there on.
 struct Share {
@@ -526,7 +532,7 @@ struct Share {
 template <int CB, int Mode, bool Pot, bool Rec = false, bool Quad = false>
 int launch(Ctx *ctx, const nbx_state *s, float *pot, int warps, cudaStream_t st, Share share,
            int *rec_list = nullptr, int *rec_len = nullptr, int rec_cap = 0) {
-    const int cap = ctx->p.stack_depth;
+    const int cap = ctx->p.stack_depth, asked = warps;
     const size_t smem = (size_t)warps * (sizeof(WarpBuf<CB, Quad>) + (Quad ? sizeof(QuadBuf<CB>) : 0) +
                                          (size_t)cap * sizeof(int));
     if (smem > (size_t)ctx->smem_optin) {
@@ -534,10 +540,14 @@ int launch(Ctx *ctx, const nbx_state *s, float *pot, int warps, cudaStream_t st,
         return NBX_ERR_ARG;
     }
     if (share.count <= 0) return NBX_OK;
+    // groups that all fit the GPU at once go out in small blocks, which spread
+    // evenly over the SMs (the sums do not depend on the shape)
+    if (share.count <= kSpreadWarps * ctx->nsm && warps > kSpreadBlock) warps = kSpreadBlock;
+    const size_t block_smem = smem / asked * warps;
     const int blocks_needed = ceil_div(share.count, warps);
     int per_sm = 1;
     NBX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_walk2<CB, Mode, Pot, Rec, Quad>, warps * 32,
-                                                           smem));
+                                                           block_smem));
     if (per_sm < 1) per_sm = 1;
     const int grid = blocks_needed < ctx->nsm * per_sm ? blocks_needed : ctx->nsm * per_sm;
     // without a list the group arrays start at the first group
@@ -545,7 +555,7 @@ int launch(Ctx *ctx, const nbx_state *s, float *pot, int warps, cudaStream_t st,
     NBX_CUDA(cudaMemsetAsync(&ctx->d_status->walk_next, 0, sizeof(unsigned), st));
     ctx->chain = false;  // (a memory operation came between)
     launch_chained(
-        ctx, st, grid, warps * 32, smem, k_walk2<CB, Mode, Pot, Rec, Quad>,
+        ctx, st, grid, warps * 32, block_smem, k_walk2<CB, Mode, Pot, Rec, Quad>,
         ctx->d_node4, ctx->d_meta, ctx->d_lvl8, ctx->d_quad4, ctx->d_quad2, ctx->d_body4, ctx->d_val,
         ctx->d_groups + off, share.list ? share.list + share.first : nullptr, share.count, ctx->d_body_sys,
         ctx->d_sys_off, ctx->d_depth0, ctx->d_root_first, ctx->d_root_nch, ctx->d_sys_lvl, ctx->eps2, cap, s->ax,

@@ -1,4 +1,4 @@
-"""The walk by teams of warps (systems of up to 131072 bodies) beside the walk by
+"""The walk by teams of warps (systems of up to 16384 bodies) beside the walk by
 single warps: a batch of both kinds gives every system the bits of its single
 run in every mode, group ranges of it sum to the full walk, and the lists and
 forces of small and odd systems match the oracle.
@@ -29,7 +29,7 @@ def _run(b, off, **kw):
                                 {"multipole": 1, "compensated": 1}, {"leaf_size": 4}],
                          ids=["plain", "split", "kahan", "quad", "quad-split", "buckets"])
 def test_batch_of_both_kinds(cuda, kw):
-    sizes = [333, 131073, 1, 131072, 4097]
+    sizes = [333, 16385, 1, 16384, 4097]
     systems = [ic.plummer(k, seed=21 + j) for j, k in enumerate(sizes)]
     off = np.concatenate([[0], np.cumsum(sizes)])
     b = ic.Bodies(*(np.concatenate([getattr(q, f) for q in systems]) for f in ("x", "y", "z", "vx", "vy", "vz", "m")))
@@ -43,7 +43,7 @@ def test_batch_of_both_kinds(cuda, kw):
         assert np.array_equal(nl[off[j]:off[j + 1]], l1) and np.array_equal(no[off[j]:off[j + 1]], o1), j
     ng = ctx.group_count()
     total = np.zeros_like(acc)
-    for a, e in ((0, 7), (7, 4000), (4000, 4000), (4000, 8300), (8300, ng)):
+    for a, e in ((0, 7), (7, 400), (400, 400), (400, 830), (830, ng)):
         for t in (s.ax, s.ay, s.az):
             t.zero_()
         ctx.forces_groups(s, a, e - a)
