@@ -8,6 +8,11 @@
 // run is its place in its own run plus, for each other run, the number of that
 // run's keys that precede it (equal keys keep the order of the runs: the sort is
 // stable).  All keys do this at once, so a launch is two dependent phases.
+// Bound by the latency of its phases below about 10^5 keys, by shared-memory
+// searches above (about 15 runs x 6 steps per key and launch).  Keys + sort, eight
+// one-sweep passes against this: 1000 bodies 58 -> 6.5 us, 16384 80 -> 17 us,
+// 131071 116 -> 43 us; at 2^20 the merges take 309 us, the passes 275 us, so
+// systems above kMergeMaxBodies sort by radix.
 #include <utility>
 
 #include "nbx_internal.cuh"

@@ -37,6 +37,7 @@ inline int tile_for(long long n, int nsm) {
     return t;
 }
 // body-key sort by merging (merge.cu): systems of up to kMergeMaxBodies bodies
+// (2^19: 135 us against about 170 by radix passes; 2^20: 309 against 275)
 constexpr int kMergeTile = 256;   // keys of a merging block
 constexpr int kMergeRun = 1024;   // keys of a first run
 constexpr int kMergeFan = 16;     // most runs merged by one launch
