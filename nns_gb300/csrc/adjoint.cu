@@ -19,7 +19,7 @@
 //
 // Memory: checkpoints of (x, v) every C steps; a segment of C steps is
 // recomputed with each step's tree and interaction lists recorded on a tape,
-// then reversed.  The forward steps with the recording walk's kernel (96-slot
+// then reversed.  The forward steps with the recording walk's kernel (variant 3
 // buffers, plain FP32) without the recording, so the recompute is bit-identical
 // (every kernel is deterministic).  The forward records the last segment as it
 // goes, so the reverse pass starts without recomputing it.

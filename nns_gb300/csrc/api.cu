@@ -203,7 +203,7 @@ void nbx_params_default(nbx_params *p) {
     p->leaf_size = 1;
     p->radix_bits = 8;
     p->walk_warps = 0;
-    p->walk_variant = 3;  // 96-slot buffers: the fastest at 2^20 and 2^24 bodies
+    p->walk_variant = 3;  // 128-slot buffers at 64 registers
     p->device = 0;
     p->block_size = 256;
     p->grid_size = 1024;

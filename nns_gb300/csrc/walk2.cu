@@ -69,28 +69,34 @@ constexpr int kCellUnroll = NBX_CELL_UNROLL;
 // quadrupoles, the surely accepted cells) fill the slots upwards and the cells to
 // vote on downwards, so one masked store serves both; with quadrupoles the cells
 // have slots of their own.  (Four slots more: each side pads to a whole pair.)
-template <int CB, bool Quad>
+template <int CB, bool Rec, bool Quad>
 struct WarpBuf {
     Slots<CB + 4> b;
     Slots<Quad ? CB : 4> c; // quadrupole mode: cells
     float cd[CB];           // cells to vote on: opening thresholds
     int cid[CB];            //                   node index
-    int bid[CB];            // body node ids (interaction-list recording only)
+    int bid[Rec ? CB : 4];  // body node ids (interaction-list recording only)
     float4 cls[3];          // group box lo, hi, centre
     ulonglong2 rxy[8];      // representative bodies, in pairs: (x0,x1) (y0,y1)
     u64 rz[8];              //                                  (z0,z1)
 };
 
-// CB = 64 and 96: 64-register budget (two 16-warp or four 8-warp blocks per SM);
-// CB = 128: up to 85 registers for more loads in flight (three 8-warp blocks).
-template <int CB>
-struct WalkBounds {
-    static constexpr int kThreads = CB <= 96 ? NBX_WALK64_THREADS : NBX_WALK128_THREADS;
-    static constexpr int kMinBlocks = CB <= 96 ? NBX_WALK64_MINB : NBX_WALK128_MINB;
+// The buffer variants: children per round and register budget.  0: 64 children;
+// 3: 128 (96 with quadrupoles, whose slots take more shared memory), both at 64
+// registers (two 16-warp or four 8-warp blocks per SM); 1: 128 at up to 85
+// registers, for more loads in flight (three 8-warp blocks).  Rounds of 128 pay
+// their fixed instructions less often than rounds of 96: 131071 bodies 1.69 ->
+// 1.63 ms for four steps, 2^24 155.4 -> 153.7 ms; with quadrupoles they cost an
+// eighth of the warps (700001 bodies 8.21 against 7.19 ms).
+template <int V, bool Quad>
+struct WalkShape {
+    static constexpr int kSlots = V == 0 ? 64 : (V == 3 && Quad ? 96 : 128);
+    static constexpr int kThreads = V != 1 ? NBX_WALK64_THREADS : NBX_WALK128_THREADS;
+    static constexpr int kMinBlocks = V != 1 ? NBX_WALK64_MINB : NBX_WALK128_MINB;
 };
 
-template <int CB, int Mode, bool Pot, bool Rec, bool Quad = false>
-__global__ void __launch_bounds__(WalkBounds<CB>::kThreads, WalkBounds<CB>::kMinBlocks)
+template <int V, int Mode, bool Pot, bool Rec, bool Quad = false>
+__global__ void __launch_bounds__(WalkShape<V, Quad>::kThreads, WalkShape<V, Quad>::kMinBlocks)
     k_walk2(const float4 *__restrict__ node4, const int *__restrict__ meta, const unsigned char *__restrict__ lvl8,
             const float4 *__restrict__ quad4, const float2 *__restrict__ quad2, const float4 *__restrict__ body4,
             const int *__restrict__ val, const int *__restrict__ groups, const int *__restrict__ list, int ngroups,
@@ -105,11 +111,12 @@ __global__ void __launch_bounds__(WalkBounds<CB>::kThreads, WalkBounds<CB>::kMin
     if (st->code != 0) return;
     const int warps = blockDim.x >> 5;
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    constexpr int kCB = CB;
-    WarpBuf<CB, Quad> &buf = reinterpret_cast<WarpBuf<CB, Quad> *>(smem_raw)[w];
+    constexpr int CB = WalkShape<V, Quad>::kSlots, kCB = CB;
+    using Buf = WarpBuf<CB, Rec, Quad>;
+    Buf &buf = reinterpret_cast<Buf *>(smem_raw)[w];
     constexpr size_t kQuadBytes = Quad ? sizeof(QuadBuf<CB>) : 0;
-    QuadBuf<CB> &qbuf = reinterpret_cast<QuadBuf<CB> *>(smem_raw + sizeof(WarpBuf<CB, Quad>) * warps)[w];
-    int *stack = reinterpret_cast<int *>(smem_raw + (sizeof(WarpBuf<CB, Quad>) + kQuadBytes) * warps) + w * stack_cap;
+    QuadBuf<CB> &qbuf = reinterpret_cast<QuadBuf<CB> *>(smem_raw + sizeof(Buf) * warps)[w];
+    int *stack = reinterpret_cast<int *>(smem_raw + (sizeof(Buf) + kQuadBytes) * warps) + w * stack_cap;
     const unsigned lt = (1u << lane) - 1u;
     const u64 eps2x2 = pk(eps2, eps2);
     unsigned long long tot_len = 0ull, tot_open = 0ull, tot_rounds = 0ull, tot_cand = 0ull;
@@ -529,11 +536,12 @@ struct Share {
     int first, count;
 };
 
-template <int CB, int Mode, bool Pot, bool Rec = false, bool Quad = false>
+template <int V, int Mode, bool Pot, bool Rec = false, bool Quad = false>
 int launch(Ctx *ctx, const nbx_state *s, float *pot, int warps, cudaStream_t st, Share share,
            int *rec_list = nullptr, int *rec_len = nullptr, int rec_cap = 0) {
+    constexpr int kCB = WalkShape<V, Quad>::kSlots;
     const int cap = ctx->p.stack_depth, asked = warps;
-    const size_t smem = (size_t)warps * (sizeof(WarpBuf<CB, Quad>) + (Quad ? sizeof(QuadBuf<CB>) : 0) +
+    const size_t smem = (size_t)warps * (sizeof(WarpBuf<kCB, Rec, Quad>) + (Quad ? sizeof(QuadBuf<kCB>) : 0) +
                                          (size_t)cap * sizeof(int));
     if (smem > (size_t)ctx->smem_optin) {
         ctx->last_error = "walk: stack_depth too large for the launch shape's shared memory";
@@ -546,7 +554,7 @@ int launch(Ctx *ctx, const nbx_state *s, float *pot, int warps, cudaStream_t st,
     const size_t block_smem = smem / asked * warps;
     const int blocks_needed = ceil_div(share.count, warps);
     int per_sm = 1;
-    NBX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_walk2<CB, Mode, Pot, Rec, Quad>, warps * 32,
+    NBX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_walk2<V, Mode, Pot, Rec, Quad>, warps * 32,
                                                            block_smem));
     if (per_sm < 1) per_sm = 1;
     const int grid = blocks_needed < ctx->nsm * per_sm ? blocks_needed : ctx->nsm * per_sm;
@@ -555,7 +563,7 @@ int launch(Ctx *ctx, const nbx_state *s, float *pot, int warps, cudaStream_t st,
     NBX_CUDA(cudaMemsetAsync(&ctx->d_status->walk_next, 0, sizeof(unsigned), st));
     ctx->chain = false;  // (a memory operation came between)
     launch_chained(
-        ctx, st, grid, warps * 32, block_smem, k_walk2<CB, Mode, Pot, Rec, Quad>,
+        ctx, st, grid, warps * 32, block_smem, k_walk2<V, Mode, Pot, Rec, Quad>,
         ctx->d_node4, ctx->d_meta, ctx->d_lvl8, ctx->d_quad4, ctx->d_quad2, ctx->d_body4, ctx->d_val,
         ctx->d_groups + off, share.list ? share.list + share.first : nullptr, share.count, ctx->d_body_sys,
         ctx->d_sys_off, ctx->d_depth0, ctx->d_root_first, ctx->d_root_nch, ctx->d_sys_lvl, ctx->eps2, cap, s->ax,
@@ -564,27 +572,27 @@ int launch(Ctx *ctx, const nbx_state *s, float *pot, int warps, cudaStream_t st,
     return NBX_OK;
 }
 
-template <int CB, int Mode, bool Pot, bool Rec = false, bool Quad = false>
+template <int V, int Mode, bool Pot, bool Rec = false, bool Quad = false>
 int set_attr(Ctx *ctx, int smem_max) {
-    NBX_CUDA(cudaFuncSetAttribute(k_walk2<CB, Mode, Pot, Rec, Quad>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    NBX_CUDA(cudaFuncSetAttribute(k_walk2<V, Mode, Pot, Rec, Quad>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   smem_max));
     return NBX_OK;
 }
 
-template <int CB>
+template <int V>
 int forces_cb(Ctx *ctx, const nbx_state *s, float *pot, int warps, cudaStream_t st, Share share) {
-    if (pot) return launch<CB, 0, true>(ctx, s, pot, warps, st, share);
+    if (pot) return launch<V, 0, true>(ctx, s, pot, warps, st, share);
     if (ctx->multipole) {
         switch (ctx->compensated) {
-            case 1: return launch<CB, 1, false, false, true>(ctx, s, nullptr, warps, st, share);
-            case 2: return launch<CB, 2, false, false, true>(ctx, s, nullptr, warps, st, share);
-            default: return launch<CB, 0, false, false, true>(ctx, s, nullptr, warps, st, share);
+            case 1: return launch<V, 1, false, false, true>(ctx, s, nullptr, warps, st, share);
+            case 2: return launch<V, 2, false, false, true>(ctx, s, nullptr, warps, st, share);
+            default: return launch<V, 0, false, false, true>(ctx, s, nullptr, warps, st, share);
         }
     }
     switch (ctx->compensated) {
-        case 1: return launch<CB, 1, false>(ctx, s, nullptr, warps, st, share);
-        case 2: return launch<CB, 2, false>(ctx, s, nullptr, warps, st, share);
-        default: return launch<CB, 0, false>(ctx, s, nullptr, warps, st, share);
+        case 1: return launch<V, 1, false>(ctx, s, nullptr, warps, st, share);
+        case 2: return launch<V, 2, false>(ctx, s, nullptr, warps, st, share);
+        default: return launch<V, 0, false>(ctx, s, nullptr, warps, st, share);
     }
 }
 
@@ -604,35 +612,35 @@ Share share_of(const Ctx *ctx, bool team, int g0, int gn) {
 int walk2_init(Ctx *ctx) {
     const int smem_optin = ctx->smem_optin;
     int rc = walk_team_init(ctx);
-    rc |= set_attr<64, 0, false>(ctx, smem_optin);
-    rc |= set_attr<64, 1, false>(ctx, smem_optin);
-    rc |= set_attr<64, 2, false>(ctx, smem_optin);
-    rc |= set_attr<64, 0, true>(ctx, smem_optin);
-    rc |= set_attr<128, 0, false>(ctx, smem_optin);
-    rc |= set_attr<128, 1, false>(ctx, smem_optin);
-    rc |= set_attr<128, 2, false>(ctx, smem_optin);
-    rc |= set_attr<128, 0, true>(ctx, smem_optin);
-    rc |= set_attr<96, 0, false>(ctx, smem_optin);
-    rc |= set_attr<96, 1, false>(ctx, smem_optin);
-    rc |= set_attr<96, 2, false>(ctx, smem_optin);
-    rc |= set_attr<96, 0, true>(ctx, smem_optin);
-    rc |= set_attr<96, 0, false, true>(ctx, smem_optin);
-    rc |= set_attr<64, 0, false, false, true>(ctx, smem_optin);
-    rc |= set_attr<64, 1, false, false, true>(ctx, smem_optin);
-    rc |= set_attr<64, 2, false, false, true>(ctx, smem_optin);
-    rc |= set_attr<128, 0, false, false, true>(ctx, smem_optin);
-    rc |= set_attr<128, 1, false, false, true>(ctx, smem_optin);
-    rc |= set_attr<128, 2, false, false, true>(ctx, smem_optin);
-    rc |= set_attr<96, 0, false, false, true>(ctx, smem_optin);
-    rc |= set_attr<96, 1, false, false, true>(ctx, smem_optin);
-    rc |= set_attr<96, 2, false, false, true>(ctx, smem_optin);
+    rc |= set_attr<0, 0, false>(ctx, smem_optin);
+    rc |= set_attr<0, 1, false>(ctx, smem_optin);
+    rc |= set_attr<0, 2, false>(ctx, smem_optin);
+    rc |= set_attr<0, 0, true>(ctx, smem_optin);
+    rc |= set_attr<1, 0, false>(ctx, smem_optin);
+    rc |= set_attr<1, 1, false>(ctx, smem_optin);
+    rc |= set_attr<1, 2, false>(ctx, smem_optin);
+    rc |= set_attr<1, 0, true>(ctx, smem_optin);
+    rc |= set_attr<3, 0, false>(ctx, smem_optin);
+    rc |= set_attr<3, 1, false>(ctx, smem_optin);
+    rc |= set_attr<3, 2, false>(ctx, smem_optin);
+    rc |= set_attr<3, 0, true>(ctx, smem_optin);
+    rc |= set_attr<3, 0, false, true>(ctx, smem_optin);
+    rc |= set_attr<0, 0, false, false, true>(ctx, smem_optin);
+    rc |= set_attr<0, 1, false, false, true>(ctx, smem_optin);
+    rc |= set_attr<0, 2, false, false, true>(ctx, smem_optin);
+    rc |= set_attr<1, 0, false, false, true>(ctx, smem_optin);
+    rc |= set_attr<1, 1, false, false, true>(ctx, smem_optin);
+    rc |= set_attr<1, 2, false, false, true>(ctx, smem_optin);
+    rc |= set_attr<3, 0, false, false, true>(ctx, smem_optin);
+    rc |= set_attr<3, 1, false, false, true>(ctx, smem_optin);
+    rc |= set_attr<3, 2, false, false, true>(ctx, smem_optin);
     return rc;
 }
 
 // Plain walk that also records every group's interaction list (node ids, in
 // evaluation order) into rec_list[g * rec_cap ...], its length into rec_len[g].
 int walk2_record(Ctx *ctx, const nbx_state *s, int *rec_list, int *rec_len, int rec_cap, cudaStream_t st) {
-    const int rc = launch<96, 0, false, true>(ctx, s, nullptr, ctx->walk_warps, st,
+    const int rc = launch<3, 0, false, true>(ctx, s, nullptr, ctx->walk_warps, st,
                                               share_of(ctx, false, 0, ctx->ngroups), rec_list, rec_len, rec_cap);
     if (rc) return rc;
     const Share t = share_of(ctx, true, 0, ctx->ngroups);
@@ -642,14 +650,14 @@ int walk2_record(Ctx *ctx, const nbx_state *s, int *rec_list, int *rec_len, int 
 // The same walk without recording: the recording adds stores only, so both
 // give the same forces bit for bit (the adjoint's forward and recompute).
 int walk2_unrecorded(Ctx *ctx, const nbx_state *s, cudaStream_t st) {
-    const int rc = launch<96, 0, false, false>(ctx, s, nullptr, ctx->walk_warps, st,
+    const int rc = launch<3, 0, false, false>(ctx, s, nullptr, ctx->walk_warps, st,
                                                share_of(ctx, false, 0, ctx->ngroups));
     if (rc) return rc;
     const Share t = share_of(ctx, true, 0, ctx->ngroups);
     return walk_team(ctx, s, nullptr, 0, false, st, t.list, t.first, t.count, nullptr, nullptr, 0);
 }
 
-// variant 0: 64-slot candidate buffers; 1: 128-slot buffers (<= 8 warps); 3: 96-slot buffers
+// variants 0, 1 (<= 8 warps) and 3: WalkShape
 // (of the single-warp walk; small systems' groups are walked by teams, whose shape is fixed).
 // Walk groups [g0, g0 + gn) of the last build (gn < 0: all groups from g0).
 int walk2_forces(Ctx *ctx, const nbx_state *s, float *pot, int warps, cudaStream_t st, int g0, int gn) {
@@ -658,9 +666,9 @@ int walk2_forces(Ctx *ctx, const nbx_state *s, float *pot, int warps, cudaStream
     const Share r = share_of(ctx, false, g0, gn), t = share_of(ctx, true, g0, gn);
     // (a launch shape that does not fit is refused whatever the groups' kind)
     int rc;
-    if (ctx->walk_variant == 1) rc = forces_cb<128>(ctx, s, pot, warps > 8 ? 8 : warps, st, r);
-    else if (ctx->walk_variant == 3) rc = forces_cb<96>(ctx, s, pot, warps, st, r);
-    else rc = forces_cb<64>(ctx, s, pot, warps, st, r);
+    if (ctx->walk_variant == 1) rc = forces_cb<1>(ctx, s, pot, warps > 8 ? 8 : warps, st, r);
+    else if (ctx->walk_variant == 3) rc = forces_cb<3>(ctx, s, pot, warps, st, r);
+    else rc = forces_cb<0>(ctx, s, pot, warps, st, r);
     if (rc) return rc;
     return walk_team(ctx, s, pot, ctx->compensated, ctx->multipole != 0, st, t.list, t.first, t.count, nullptr,
                      nullptr, 0);
