@@ -107,11 +107,11 @@ void free_all(Ctx *ctx) {
                     ctx->d_bbox_u, ctx->d_bbox, ctx->d_bbox64, ctx->d_depth0, ctx->d_root_first, ctx->d_sys_lvl,
                     ctx->d_root_nch, ctx->d_key, ctx->d_key_alt, ctx->d_key_lo, ctx->d_val, ctx->d_val_alt,
                     ctx->d_body4, ctx->d_delta, ctx->d_bucket, ctx->d_ecount, ctx->d_body_node, ctx->d_gstat,
-                    ctx->d_ent, ctx->d_lvl_counts, ctx->d_lvl_tot, ctx->d_lvl_start, ctx->d_node4, ctx->d_meta, ctx->d_parent,
+                    ctx->d_ent, ctx->d_lvl_counts, ctx->d_lvl_tot, ctx->d_node4, ctx->d_meta, ctx->d_parent,
                     ctx->d_sums, ctx->d_count, ctx->d_arrive, ctx->d_lvl8, ctx->d_hist,
                     ctx->d_scan_blk, ctx->d_totals, ctx->d_totals64, ctx->d_status, ctx->d_m2, ctx->d_com, ctx->d_quad4,
                     ctx->d_quad2, ctx->d_seg_slot, ctx->d_lb_counts, ctx->d_lb_status, ctx->d_lb, ctx->d_tiles_sw,
-                    ctx->d_sys_tiles_sw, ctx->d_tiles_mg, ctx->d_runs_mg, ctx->d_team, ctx->d_solo, ctx->d_bbox_done};
+                    ctx->d_sys_tiles_sw, ctx->d_tiles_mg, ctx->d_team};
     for (void *p : ptrs)
         if (p) cudaFree(p);
     if (ctx->h_status) cudaFreeHost(ctx->h_status);
@@ -295,13 +295,11 @@ int nbx_create(const nbx_params *p, nbx_ctx **out) {
     rc |= nbx::dmalloc(ctx, &ctx->d_seg_slot, Ss);
     rc |= nbx::dmalloc(ctx, &ctx->d_tiles_sw, ctx->cap_tiles_body);
     rc |= nbx::dmalloc(ctx, &ctx->d_sys_tiles_sw, Ss);
-    rc |= nbx::dmalloc(ctx, &ctx->d_tiles_mg, (size_t)B / nbx::kMergeTile + Ss + 1);
-    rc |= nbx::dmalloc(ctx, &ctx->d_runs_mg, (size_t)B / nbx::kMergeRun + Ss + 1);
+    // merging sort: the tiles, and behind them the first runs (nbx_set_systems)
+    rc |= nbx::dmalloc(ctx, &ctx->d_tiles_mg, (size_t)B / nbx::kMergeTile + (size_t)B / nbx::kMergeRun + 2 * (size_t)Ss + 2);
     rc |= nbx::dmalloc(ctx, &ctx->d_groups, G);
-    rc |= nbx::dmalloc(ctx, &ctx->d_team, G);
-    rc |= nbx::dmalloc(ctx, &ctx->d_solo, G);
+    if (Ss > 1) rc |= nbx::dmalloc(ctx, &ctx->d_team, G);  // both lists of a mixed batch
     rc |= nbx::dmalloc(ctx, &ctx->d_bbox_u, 6 * Ss + 6);
-    rc |= nbx::dmalloc(ctx, &ctx->d_bbox_done, 1);
     rc |= nbx::dmalloc(ctx, &ctx->d_bbox, 6 * Ss);
     rc |= nbx::dmalloc(ctx, &ctx->d_bbox64, 6 * Ss);
     rc |= nbx::dmalloc(ctx, &ctx->d_depth0, Ss);
@@ -328,8 +326,11 @@ int nbx_create(const nbx_params *p, nbx_ctx **out) {
     rc |= nbx::dmalloc(ctx, &ctx->d_arrive, NC);
     rc |= nbx::dmalloc(ctx, &ctx->d_lvl8, NC);
     rc |= nbx::dmalloc(ctx, &ctx->d_lvl_counts, 64 * (size_t)nbx::ceil_div(B, nbx::kPosBlock));
-    rc |= nbx::dmalloc(ctx, &ctx->d_lvl_tot, 64);
-    rc |= nbx::dmalloc(ctx, &ctx->d_lvl_start, 64);
+    rc |= nbx::dmalloc(ctx, &ctx->d_lvl_tot, 3 * 64);
+    if (rc == 0) {
+        ctx->d_lvl_start = ctx->d_lvl_tot + 64;
+        ctx->d_bbox_done = ctx->d_lvl_tot + 128;
+    }
     rc |= nbx::dmalloc(ctx, &ctx->d_hist, hist + 1);  // + the scanned total
     // one-sweep body sort: a system of several tiles takes at least two, so at most
     // half the tiles (plus one) hold count slots; status words per tile and digit
@@ -357,7 +358,6 @@ int nbx_create(const nbx_params *p, nbx_ctx **out) {
     if (rc == 0 && ctx->multipole) rc = nbx::alloc_quadrupoles(ctx);
     if (rc == 0) rc = nbx::walk_init(ctx);
     if (rc == 0) rc = nbx::radix_init(ctx);
-    if (rc == 0) rc = nbx::merge_init(ctx);
     if (rc != 0) {
         nbx::free_all(ctx);
         delete ctx;
@@ -529,11 +529,14 @@ int nbx_set_systems(nbx_ctx *c, int nsys, const int64_t *offsets) {
     NBX_CUDA(cudaMemcpy(ctx->d_seg_slot, slot.data(), sizeof(int) * nsys, cudaMemcpyHostToDevice));
     NBX_CUDA(cudaMemcpy(ctx->d_tiles_sw, tiles_sw.data(), sizeof(int4) * tiles_sw.size(), cudaMemcpyHostToDevice));
     NBX_CUDA(cudaMemcpy(ctx->d_sys_tiles_sw, st_sw.data(), sizeof(int2) * nsys, cudaMemcpyHostToDevice));
-    if (!tiles_mg.empty()) {
+    const size_t ntiles_mg = tiles_mg.size();
+    if (ntiles_mg) {
+        tiles_mg.insert(tiles_mg.end(), runs_mg.begin(), runs_mg.end());
         NBX_CUDA(cudaMemcpy(ctx->d_tiles_mg, tiles_mg.data(), sizeof(int4) * tiles_mg.size(), cudaMemcpyHostToDevice));
-        NBX_CUDA(cudaMemcpy(ctx->d_runs_mg, runs_mg.data(), sizeof(int4) * runs_mg.size(), cudaMemcpyHostToDevice));
     }
-    if (!team.empty() && !solo.empty()) {
+    ctx->d_runs_mg = ctx->d_tiles_mg + ntiles_mg;
+    if (!team.empty() && !solo.empty()) {  // (several systems: the lists are there)
+        ctx->d_solo = ctx->d_team + team.size();
         NBX_CUDA(cudaMemcpy(ctx->d_team, team.data(), sizeof(int) * team.size(), cudaMemcpyHostToDevice));
         NBX_CUDA(cudaMemcpy(ctx->d_solo, solo.data(), sizeof(int) * solo.size(), cudaMemcpyHostToDevice));
     }
@@ -549,7 +552,7 @@ int nbx_set_systems(nbx_ctx *c, int nsys, const int64_t *offsets) {
     ctx->nslots = nslots;
     ctx->ntiles_sw = (int)tiles_sw.size();
     ctx->tile_sw = tile_sw;
-    ctx->ntiles_mg = (int)tiles_mg.size();
+    ctx->ntiles_mg = (int)ntiles_mg;
     ctx->nruns_mg = (int)runs_mg.size();
     ctx->max_sys = max_sys;
     ctx->h_team = std::move(team);

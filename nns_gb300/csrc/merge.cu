@@ -175,7 +175,8 @@ __global__ void __launch_bounds__(kThreads) k_merge(const int4 *__restrict__ til
 
 // staged keys of a block: the expected stretches (its own width per run) and a
 // quarter more
-int stage_cap(int fan) { return fan * (kMergeTile + kMergeTile / 4); }
+constexpr int stage_cap(int fan) { return fan * (kMergeTile + kMergeTile / 4); }
+static_assert(stage_cap(kMergeFan) * sizeof(unsigned long long) <= 46 * 1024, "within every kernel's shared memory");
 
 }  // namespace
 
@@ -212,12 +213,6 @@ int merge_runs(Ctx *ctx, cudaStream_t st) {
         R *= fan;
     }
     NBX_CUDA(cudaGetLastError());
-    return NBX_OK;
-}
-
-int merge_init(Ctx *ctx) {
-    NBX_CUDA(cudaFuncSetAttribute(k_merge, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)sizeof(unsigned long long) * stage_cap(kMergeFan)));
     return NBX_OK;
 }
 

@@ -120,7 +120,7 @@ struct Ctx {
     int ntiles_sw = 0, tile_sw = 0;
     int nslots = 0;                 // systems of several tiles (count slots in use)
     int4 *d_tiles_mg = nullptr;     // [merge tiles] of kMergeTile keys: start, len, sys, local tile index
-    int4 *d_runs_mg = nullptr;      // [first runs] of kMergeRun keys, the same
+    int4 *d_runs_mg = nullptr;      // [first runs] of kMergeRun keys, the same (behind the tiles)
     int nruns_mg = 0;
     int ntiles_mg = 0;              // 0: a system is too large, the keys sort by radix
     int max_sys = 0;                // bodies of the largest system
@@ -129,7 +129,7 @@ struct Ctx {
     // walk groups of systems of up to kTeamMaxBodies bodies (walked by teams of
     // warps) and of larger ones, ascending; the device copies exist in a batch of both
     std::vector<int> h_team, h_solo;
-    int *d_team = nullptr, *d_solo = nullptr;  // [G]
+    int *d_team = nullptr, *d_solo = nullptr;  // [G] together
 
     // per-system tree parameters
     unsigned *d_bbox_u = nullptr;   // [6S] ordered-int encodings during the reduction (between builds: empty boxes)
@@ -167,7 +167,7 @@ struct Ctx {
     float4 *d_quad4 = nullptr;     // [NC] quadrupole mode: P = -Q (Q traceless) of cells in FP32, (xx, yy, zz, xy)
     float2 *d_quad2 = nullptr;     // [NC]                                              (xz, yz)
     unsigned *d_lvl_counts = nullptr;                 // [position blocks][64] nodes per level
-    unsigned *d_lvl_tot = nullptr;                    // [64] nodes of each level
+    unsigned *d_lvl_tot = nullptr;                    // [64] nodes of each level (lvl_start, bbox_done: behind it)
     unsigned *d_lvl_start = nullptr;                  // [64] first node of each level (past the deepest: the node count)
 
     // radix + scan scratch
@@ -288,7 +288,6 @@ int radix_init(Ctx *ctx);
 // merge.cu
 int merge_passes(int max_bodies_of_a_system);
 int merge_runs(Ctx *ctx, cudaStream_t st);
-int merge_init(Ctx *ctx);
 int radix_selftest_wait(Ctx *ctx, cudaStream_t st);
 // tree.cu
 int build_tree(Ctx *ctx, const nbx_state *s, cudaStream_t st, bool external_bbox,
@@ -300,7 +299,6 @@ int walk_forces_groups(Ctx *ctx, const nbx_state *s, int first, int count, cudaS
 int walk_potential(Ctx *ctx, const nbx_state *s, float *pot, cudaStream_t st);
 int walk_fp64_lists(Ctx *ctx, const int *group_starts, int ngroups, double *a64, cudaStream_t st);
 // walk_team.cu
-int walk_team_init(Ctx *ctx);
 int walk_team(Ctx *ctx, const nbx_state *s, float *pot, int mode, bool quad, cudaStream_t st, const int *list,
               int first, int count, int *rec_list, int *rec_len, int rec_cap);
 // integrate.cu

@@ -611,7 +611,7 @@ Share share_of(const Ctx *ctx, bool team, int g0, int gn) {
 
 int walk2_init(Ctx *ctx) {
     const int smem_optin = ctx->smem_optin;
-    int rc = walk_team_init(ctx);
+    int rc = 0;
     rc |= set_attr<0, 0, false>(ctx, smem_optin);
     rc |= set_attr<0, 1, false>(ctx, smem_optin);
     rc |= set_attr<0, 2, false>(ctx, smem_optin);

@@ -574,6 +574,10 @@ int launch_team(Ctx *ctx, const nbx_state *s, float *pot, cudaStream_t st, const
         ctx->last_error = "walk: stack_depth too large for the launch shape's shared memory";
         return NBX_ERR_ARG;
     }
+    // (only deep stacks and the quadrupoles' slots need more than the default limit)
+    if (smem > 48 * 1024)
+        NBX_CUDA(cudaFuncSetAttribute(k_walk_team<Mode, Pot, Rec, Quad>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      ctx->smem_optin));
     launch_chained(ctx, st, count, kW * 32, smem, k_walk_team<Mode, Pot, Rec, Quad>, ctx->d_node4, ctx->d_meta,
                    ctx->d_quad4, ctx->d_quad2, ctx->d_body4, ctx->d_val, ctx->d_groups, list, first, ctx->d_body_sys,
                    ctx->d_sys_off, ctx->d_depth0, ctx->d_root_first, ctx->d_root_nch, ctx->d_sys_lvl, ctx->eps2,
@@ -583,26 +587,7 @@ int launch_team(Ctx *ctx, const nbx_state *s, float *pot, cudaStream_t st, const
     return NBX_OK;
 }
 
-template <int Mode, bool Pot, bool Rec, bool Quad>
-cudaError_t team_attr(int smem_max) {
-    return cudaFuncSetAttribute(k_walk_team<Mode, Pot, Rec, Quad>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                smem_max);
-}
-
 }  // namespace
-
-int walk_team_init(Ctx *ctx) {
-    const int m = ctx->smem_optin;
-    NBX_CUDA((team_attr<0, false, false, false>(m)));
-    NBX_CUDA((team_attr<1, false, false, false>(m)));
-    NBX_CUDA((team_attr<2, false, false, false>(m)));
-    NBX_CUDA((team_attr<0, true, false, false>(m)));
-    NBX_CUDA((team_attr<0, false, true, false>(m)));
-    NBX_CUDA((team_attr<0, false, false, true>(m)));
-    NBX_CUDA((team_attr<1, false, false, true>(m)));
-    NBX_CUDA((team_attr<2, false, false, true>(m)));
-    return NBX_OK;
-}
 
 // The walk of `count` groups by teams: groups first, first + 1, ..., or the
 // entries first, ... of `list` (device array) where it is given.  mode: -1
