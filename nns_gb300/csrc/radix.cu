@@ -51,36 +51,24 @@ constexpr int kWarpsPerBlock = 8;
 constexpr int kSweepMaxBodies = NBX_RADIX_SWEEP_MAX;
 
 struct TileMap {
-    // segmented mode
     const int4 *tiles;      // start, len, seg, local tile
     const int2 *seg_tiles;  // tile base, ntiles of the segment
-    // uniform mode
-    const unsigned *count;  // device-side element count
     int ntiles;             // tiles in the launch
     int tile;               // keys per tile (<= kTile)
 };
 
-template <bool Seg, int Bins>
+template <int Bins>
 __device__ __forceinline__ void tile_info(const TileMap &tm, int t, int &start, int &len,
                                           int64_t &hbase, int &hstride) {
-    if (Seg) {
-        int4 d = tm.tiles[t];
-        int2 s = tm.seg_tiles[d.z];
-        start = d.x;
-        len = d.y;
-        hbase = (int64_t)s.x * Bins + d.w;
-        hstride = s.y;
-    } else {
-        int64_t st = (int64_t)t * tm.tile;
-        int64_t n = (int64_t)*tm.count;
-        start = (int)st;
-        len = (int)(n > st ? (n - st < tm.tile ? n - st : tm.tile) : 0);
-        hbase = t;
-        hstride = tm.ntiles;
-    }
+    const int4 d = tm.tiles[t];
+    const int2 s = tm.seg_tiles[d.z];
+    start = d.x;
+    len = d.y;
+    hbase = (int64_t)s.x * Bins + d.w;
+    hstride = s.y;
 }
 
-template <typename K, bool Seg, int Bits>
+template <typename K, int Bits>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32)
     k_radix_hist(const K *__restrict__ key, TileMap tm, int shift, unsigned *__restrict__ hist) {
     constexpr int kBins = 1 << Bits;
@@ -93,7 +81,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32)
     __syncwarp();
     int start, len, hstride;
     int64_t hbase;
-    tile_info<Seg, kBins>(tm, t, start, len, hbase, hstride);
+    tile_info<kBins>(tm, t, start, len, hbase, hstride);
     constexpr int kBatch = 8;  // loads in flight together (the atomics would serialise them)
     for (int i0 = 0; i0 < len; i0 += 32 * kBatch) {
         unsigned d[kBatch];
@@ -220,12 +208,11 @@ __global__ void __launch_bounds__(256) k_radix_counts(const unsigned long long *
 
 // (six blocks of 4 warps per SM: 80 registers, as the tile's keys and values
 // live in registers)
-template <typename K, typename V, bool Seg, int Bits, bool Sweep = false>
+template <typename K, typename V, int Bits, bool Sweep = false>
 __global__ void __launch_bounds__(kScatterWarps * 32, 6)
     k_radix_scatter(const K *__restrict__ key_in, K *__restrict__ key_out,
                     const V *__restrict__ val_in, V *__restrict__ val_out, TileMap tm, int shift,
                     const unsigned *__restrict__ offs, SweepArgs sw) {
-    static_assert(!Sweep || Seg, "the one-sweep pass runs on the systems' tiles");
     constexpr int kBins = 1 << Bits;
     constexpr unsigned kMask = kBins - 1;
     constexpr int kW = kScatterWarps;
@@ -243,7 +230,7 @@ __global__ void __launch_bounds__(kScatterWarps * 32, 6)
     if (t >= tm.ntiles) return;  // uniform over the block
     int start, len, hstride;
     int64_t hbase;
-    tile_info<Seg, kBins>(tm, t, start, len, hbase, hstride);
+    tile_info<kBins>(tm, t, start, len, hbase, hstride);
     if (!Sweep && len <= 0) return;  // (a sweep tile always publishes its counts)
     unsigned *gbase = reinterpret_cast<unsigned *>(smem_raw);
     unsigned *lstart = gbase + kBins;
@@ -434,11 +421,11 @@ __global__ void __launch_bounds__(kScatterWarps * 32, 6)
     }
 }
 
-template <typename K, typename V, bool Seg, int Bits>
+template <typename K, typename V, int Bits>
 int launch_scatter(Ctx *ctx, int nt, const K *kin, K *kout, const V *vin, V *vout, const TileMap &tm, int shift,
                    cudaStream_t st) {
     const size_t smem = stage_bytes<K, V, Bits>(tm.tile);
-    k_radix_scatter<K, V, Seg, Bits><<<nt, kScatterWarps * 32, smem, st>>>(kin, kout, vin, vout, tm, shift,
+    k_radix_scatter<K, V, Bits><<<nt, kScatterWarps * 32, smem, st>>>(kin, kout, vin, vout, tm, shift,
                                                                            ctx->d_hist, SweepArgs{});
     ++ctx->launches;
     return NBX_OK;
@@ -448,7 +435,7 @@ int launch_scatter(Ctx *ctx, int nt, const K *kin, K *kout, const V *vin, V *vou
 // per pass.
 template <int Bits>
 int sort_bodies_sweep(Ctx *ctx, cudaStream_t st) {
-    TileMap tm{ctx->d_tiles_sw, ctx->d_sys_tiles_sw, nullptr, ctx->ntiles_sw, ctx->tile_sw};
+    TileMap tm{ctx->d_tiles_sw, ctx->d_sys_tiles_sw, ctx->ntiles_sw, ctx->tile_sw};
     const int nt = ctx->ntiles_sw;
     if (nt == 0) return NBX_OK;
     constexpr int kBins = 1 << Bits, kPasses = radix_passes(Bits);
@@ -469,7 +456,7 @@ int sort_bodies_sweep(Ctx *ctx, cudaStream_t st) {
     for (int pass = 0; pass < kPasses; pass++) {
         SweepArgs sw{ctx->d_seg_slot, ctx->d_lb_counts, ctx->d_lb_status, ctx->d_lb, ctx->d_lb, ctx->d_status, pass,
                      ctx->nbodies};
-        k_radix_scatter<unsigned long long, int, true, Bits, true>
+        k_radix_scatter<unsigned long long, int, Bits, true>
             <<<nt, kScatterWarps * 32, smem, st>>>(k0, k1, v0, v1, tm, Bits * pass, nullptr, sw);
         ++ctx->launches;
         std::swap(k0, k1);
@@ -481,7 +468,7 @@ int sort_bodies_sweep(Ctx *ctx, cudaStream_t st) {
 
 template <int Bits>
 int sort_bodies(Ctx *ctx, cudaStream_t st) {
-    TileMap tm{ctx->d_tiles, ctx->d_sys_tiles, nullptr, ctx->ntiles_body, ctx->tile_body};
+    TileMap tm{ctx->d_tiles, ctx->d_sys_tiles, ctx->ntiles_body, ctx->tile_body};
     const int nt = ctx->ntiles_body;
     if (nt == 0) return NBX_OK;
     const int grid = ceil_div(nt, kWarpsPerBlock);
@@ -496,12 +483,12 @@ int sort_bodies(Ctx *ctx, cudaStream_t st) {
     }
     for (int pass = 0; pass < passes; pass++) {
         const int shift = Bits * pass;
-        k_radix_hist<unsigned long long, true, Bits>
+        k_radix_hist<unsigned long long, Bits>
             <<<grid, kWarpsPerBlock * 32, 0, st>>>(k0, tm, shift, ctx->d_hist);
         ++ctx->launches;
         int rc = scan_exclusive_u32(ctx, ctx->d_hist, ctx->d_hist, nh, nullptr, ctx->d_hist + nh, st);
         if (rc) return rc;
-        launch_scatter<unsigned long long, int, true, Bits>(ctx, nt, k0, k1, v0, v1, tm, shift, st);
+        launch_scatter<unsigned long long, int, Bits>(ctx, nt, k0, k1, v0, v1, tm, shift, st);
         std::swap(k0, k1);
         std::swap(v0, v1);
     }
@@ -553,9 +540,9 @@ int radix_selftest_wait(Ctx *ctx, cudaStream_t st) {
     int rc = NBX_OK;
     if (cudaMemcpyAsync(d, &h, sizeof(Scratch), cudaMemcpyHostToDevice, st) != cudaSuccess) rc = NBX_ERR_CUDA;
     if (rc == NBX_OK) {
-        TileMap tm{d->tiles, d->seg_tiles, nullptr, 2, kT};
+        TileMap tm{d->tiles, d->seg_tiles, 2, kT};
         SweepArgs sw{d->seg_slot, d->counts, d->status, d->lb, d->lb, ctx->d_status, 0, kN};
-        k_radix_scatter<unsigned long long, int, true, 8, true>
+        k_radix_scatter<unsigned long long, int, 8, true>
             <<<1, kScatterWarps * 32, stage_bytes<unsigned long long, int, 8, true>(kT), st>>>(
                 d->key_in, d->key_out, d->val_in, d->val_out, tm, 0, nullptr, sw);
         ++ctx->launches;
@@ -568,16 +555,16 @@ int radix_selftest_wait(Ctx *ctx, cudaStream_t st) {
 }
 
 int radix_init(Ctx *ctx) {
-    NBX_CUDA(cudaFuncSetAttribute(k_radix_scatter<unsigned long long, int, true, 8>,
+    NBX_CUDA(cudaFuncSetAttribute(k_radix_scatter<unsigned long long, int, 8>,
                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)stage_bytes<unsigned long long, int, 8>(kTile)));
-    NBX_CUDA(cudaFuncSetAttribute(k_radix_scatter<unsigned long long, int, true, 9>,
+    NBX_CUDA(cudaFuncSetAttribute(k_radix_scatter<unsigned long long, int, 9>,
                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)stage_bytes<unsigned long long, int, 9>(kTile)));
-    NBX_CUDA(cudaFuncSetAttribute(k_radix_scatter<unsigned long long, int, true, 8, true>,
+    NBX_CUDA(cudaFuncSetAttribute(k_radix_scatter<unsigned long long, int, 8, true>,
                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)stage_bytes<unsigned long long, int, 8, true>(kTile)));
-    NBX_CUDA(cudaFuncSetAttribute(k_radix_scatter<unsigned long long, int, true, 9, true>,
+    NBX_CUDA(cudaFuncSetAttribute(k_radix_scatter<unsigned long long, int, 9, true>,
                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)stage_bytes<unsigned long long, int, 9, true>(kTile)));
     return NBX_OK;
