@@ -104,7 +104,10 @@ __global__ void __launch_bounds__(kW * 32, 32 / kW)
                 int *__restrict__ rec_len, int rec_cap) {
     grid_dependency();
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    if (st->code != 0) return;
+    // decided by the whole block: another block of this launch may report an error
+    // (a full recording list) while these warps read the status, and a team that
+    // lost some of its warps would run on with shared words nobody wrote
+    if (__syncthreads_or(st->code != 0)) return;
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     TeamShared &sh = *reinterpret_cast<TeamShared *>(smem_raw);
     TeamBuf<Rec, Quad> *bufs = reinterpret_cast<TeamBuf<Rec, Quad> *>(smem_raw + sizeof(TeamShared));
