@@ -656,6 +656,18 @@ int adjoint_create(Ctx *ctx, int T, int C, int lcap, int tape_steps, Adj **out) 
         rc |= amalloc(ctx, a, &t.lists, (size_t)a->ngroups * lcap);
         rc |= amalloc(ctx, a, &t.list_len, a->ngroups);
         rc |= amalloc(ctx, a, &t.lvl, 64);
+        // a walk or build that an error status stops leaves its part of the tape as it
+        // was, and a reverse or replay pass over it still indexes by what is there:
+        // empty lists and node 0 until a tree is recorded
+        if (rc == 0 && (cudaMemset(t.meta, 0, sizeof(int) * (size_t)NC) != cudaSuccess ||
+                        cudaMemset(t.parent, 0, sizeof(int) * (size_t)NC) != cudaSuccess ||
+                        cudaMemset(t.val, 0, sizeof(int) * (size_t)ctx->cap_bodies) != cudaSuccess ||
+                        cudaMemset(t.body_node, 0, sizeof(int) * (size_t)ctx->cap_bodies) != cudaSuccess ||
+                        cudaMemset(t.list_len, 0, sizeof(int) * (size_t)a->ngroups) != cudaSuccess ||
+                        cudaMemset(t.lvl, 0, sizeof(unsigned) * 64) != cudaSuccess)) {
+            ctx->last_error = "adjoint: clearing the tape failed";
+            rc = NBX_ERR_CUDA;
+        }
     }
     a->ctx_node4 = ctx->d_node4;
     a->ctx_meta = ctx->d_meta;

@@ -1,8 +1,9 @@
 """Recording lists that overflow (nbx_adjoint_create's list_capacity): the adjoint
 of a batch of small systems, whose walk groups outnumber the blocks that the GPU
 holds at once, so that blocks of one launch start after others have reported the
-full list.  The forward reports NBX_ERR_CAPACITY and nothing else, and the context
-goes on as a fresh one does.
+full list.  The forward reports NBX_ERR_CAPACITY and nothing else, the context goes on
+as a fresh one does, and passes over a tape whose recording was stopped stay
+within it.
 """
 import numpy as np
 import pytest
@@ -49,5 +50,34 @@ def test_full_lists_are_reported(cuda):
         with pytest.raises(NbxError) as e:
             adj.forward(State.from_bodies(b), target)
         assert e.value.code == NBX_ERR_CAPACITY
+    for got, want in zip(_stepped(ctx, b), _stepped(_context(off), b)):
+        assert np.array_equal(got, want)
+
+
+def test_passes_over_a_stopped_recording(cuda):
+    """The first recorded step overflows, so the later steps' trees are built empty
+    and their lists never written: the reverse pass and the FP64 replay over that
+    tape have nothing to index by but what the adjoint's creation left there."""
+    import torch
+    from nns_gb300._lib import NbxError
+    from nns_gb300.adjoint import Adjoint
+    from nns_gb300.barnes_hut import State
+    b, off = _batch([4000] * 4)
+    n = int(off[-1])
+    ctx = _context(off)
+    target = torch.zeros(3, n, device="cuda")
+    adj = Adjoint(ctx, 4, 4, 64)
+    s = State.from_bodies(b)
+    with pytest.raises(NbxError) as e:
+        adj.forward(s, target)
+    assert e.value.code == NBX_ERR_CAPACITY
+    g = adj.backward(s)
+    torch.cuda.synchronize()
+    assert [t.shape[-1] for t in g] == [n] * 3
+    with pytest.raises(NbxError) as e:
+        adj.record(s)
+    assert e.value.code == NBX_ERR_CAPACITY
+    adj.replay_fp64(torch.zeros(7, n, dtype=torch.float64, device="cuda"))
+    torch.cuda.synchronize()
     for got, want in zip(_stepped(ctx, b), _stepped(_context(off), b)):
         assert np.array_equal(got, want)
