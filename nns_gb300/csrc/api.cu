@@ -344,14 +344,17 @@ int nbx_create(const nbx_params *p, nbx_ctx **out) {
     if (rc == 0 && cudaMallocHost((void **)&ctx->h_status, sizeof(nbx::DevStatus)) != cudaSuccess) rc = NBX_ERR_NOMEM;
     if (rc == 0 && cudaMemset(ctx->d_status, 0, sizeof(nbx::DevStatus)) != cudaSuccess) rc = NBX_ERR_CUDA;
     if (rc == 0 && cudaMemset(ctx->d_totals, 0, 8 * sizeof(unsigned)) != cudaSuccess) rc = NBX_ERR_CUDA;
+    // no tree yet: every build clears the meta words of the tree before it (tree.cu)
+    if (rc == 0 && (cudaMemset(ctx->d_meta, 0, sizeof(int) * (size_t)NC) != cudaSuccess ||
+                    cudaMemset(ctx->d_lvl_tot, 0, 3 * 64 * sizeof(unsigned)) != cudaSuccess))
+        rc = NBX_ERR_CUDA;
     // status words start at build 0, which no pass ever uses (its tags are >= 1)
     if (rc == 0 && cudaMemset(ctx->d_lb_status, 0, sizeof(unsigned long long) * ((size_t)ctx->cap_tiles_body << nbx::kMaxRadixBits)) != cudaSuccess)
         rc = NBX_ERR_CUDA;
     // empty boxes: the ordered encoding of 0.0f is the sign bit (k_bbox keeps them so)
     if (rc == 0) {
         const std::vector<unsigned> empty(6 * (size_t)Ss + 6, 0x80000000u);
-        if (cudaMemcpy(ctx->d_bbox_u, empty.data(), sizeof(unsigned) * empty.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
-            cudaMemset(ctx->d_bbox_done, 0, sizeof(unsigned)) != cudaSuccess)
+        if (cudaMemcpy(ctx->d_bbox_u, empty.data(), sizeof(unsigned) * empty.size(), cudaMemcpyHostToDevice) != cudaSuccess)
             rc = NBX_ERR_CUDA;
     }
     if (rc == 0 && cudaMemset(ctx->d_lb, 0, 16 * sizeof(unsigned)) != cudaSuccess) rc = NBX_ERR_CUDA;
@@ -523,6 +526,14 @@ int nbx_set_systems(nbx_ctx *c, int nsys, const int64_t *offsets) {
             cut(runs_mg, nbx::kMergeRun);
         }
     if ((int)tiles.size() > ctx->cap_tiles_body || (int)tiles_sw.size() > ctx->cap_tiles_body) return NBX_ERR_ARG;
+    // the meta words of a much larger tree are cleared here by the whole GPU; the
+    // next build has blocks for its own bodies only
+    if (ctx->nbodies > 16ll * n) {
+        ctx->built = false;
+        NBX_CUDA(cudaDeviceSynchronize());
+        NBX_CUDA(cudaMemset(ctx->d_meta, 0, sizeof(int) * (size_t)ctx->cap_nodes));
+        NBX_CUDA(cudaMemset(ctx->d_lvl_start, 0, 64 * sizeof(unsigned)));
+    }
     NBX_CUDA(cudaMemcpy(ctx->d_sys_off, off.data(), sizeof(int) * (nsys + 1), cudaMemcpyHostToDevice));
     NBX_CUDA(cudaMemcpy(ctx->d_tiles, tiles.data(), sizeof(int4) * tiles.size(), cudaMemcpyHostToDevice));
     NBX_CUDA(cudaMemcpy(ctx->d_sys_tiles, st.data(), sizeof(int2) * nsys, cudaMemcpyHostToDevice));

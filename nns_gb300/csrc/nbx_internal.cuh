@@ -168,7 +168,8 @@ struct Ctx {
     float2 *d_quad2 = nullptr;     // [NC]                                              (xz, yz)
     unsigned *d_lvl_counts = nullptr;                 // [position blocks][64] nodes per level
     unsigned *d_lvl_tot = nullptr;                    // [64] nodes of each level (lvl_start, bbox_done: behind it)
-    unsigned *d_lvl_start = nullptr;                  // [64] first node of each level (past the deepest: the node count)
+    unsigned *d_lvl_start = nullptr;                  // [64] first node of each level (past the deepest: the node count
+                                                      // of the tree in d_meta, by which the next build clears it)
 
     // radix + scan scratch
     unsigned *d_hist = nullptr;        // [2^kMaxRadixBits * max(tiles)]

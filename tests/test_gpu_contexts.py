@@ -1,0 +1,108 @@
+"""Contexts that are larger than their systems, or used for one system after another:
+every build starts from what the trees before it left behind.  Trees against the
+oracle (bit-exact) after larger and smaller systems, batches and failed builds; and
+a small system's step costs in a large context what it costs in one of its size.
+"""
+import numpy as np
+import pytest
+
+from nns_gb300 import ic
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+def _joined(systems):
+    off = np.concatenate([[0], np.cumsum([len(q.x) for q in systems])])
+    b = ic.Bodies(*(np.concatenate([getattr(q, f) for q in systems]) for f in ("x", "y", "z", "vx", "vy", "vz", "m")))
+    return b, off
+
+
+def _build(ctx, systems):
+    from nns_gb300.barnes_hut import State
+    b, off = _joined(systems)
+    ctx.set_systems(off)
+    s = State.from_bodies(b)
+    ctx.build(s)
+    return s
+
+
+def _check(ctx, systems):
+    for j, q in enumerate(systems):
+        gt, ot = ctx.export_tree(j), O.build(q.x, q.y, q.z, q.m)
+        assert gt["ncells"] == ot.ncells
+        for k in ("perm", "root_child", "cell_child", "cell_start", "cell_count", "cell_level", "cell_x", "cell_y",
+                  "cell_z", "cell_m"):
+            assert np.array_equal(gt[k], getattr(ot, k)), (j, k)
+
+
+def _failing(n):
+    b = ic.plummer(n, seed=n)
+    x, y, z = b.x.copy(), b.y.copy(), b.z.copy()
+    x[7], y[7], z[7] = x[8], y[8], z[8]  # the same place: NBX_ERR_DEPTH
+    return ic.Bodies(x, y, z, b.vx, b.vy, b.vz, b.m)
+
+
+def test_one_system_after_another(cuda):
+    from nns_gb300._lib import NbxError
+    from nns_gb300.barnes_hut import Context
+    ctx = Context(max_bodies=70000, max_systems=40)
+    runs = [[65536], [1000], [3], [70000], [20000], [1, 300, 5000, 2, 257], [66000], [100] * 40, [4097], [1]]
+    for j, sizes in enumerate(runs):
+        systems = [ic.plummer(k, seed=100 * j + i) for i, k in enumerate(sizes)]
+        _build(ctx, systems)
+        ctx.sync()
+        _check(ctx, systems)
+        if j % 3 == 0:
+            _build(ctx, [_failing(30000)])
+            with pytest.raises(NbxError) as e:
+                ctx.sync()
+            assert e.value.code == 3  # NBX_ERR_DEPTH
+
+
+def test_after_a_tree_that_did_not_fit(cuda):
+    from nns_gb300._lib import NbxError
+    from nns_gb300.barnes_hut import Context
+    ctx = Context(max_bodies=5000, node_capacity=5001)
+    small = [ic.plummer(2000, seed=5)]
+    for _ in range(2):
+        _build(ctx, small)
+        ctx.sync()
+        _check(ctx, small)
+        _build(ctx, [ic.plummer(5000, seed=6)])
+        with pytest.raises(NbxError) as e:
+            ctx.sync()
+        assert e.value.code == 4  # NBX_ERR_CAPACITY
+
+
+def _best_us(fn, reps=30):
+    import torch
+    best = 1e30
+    for _ in range(reps):
+        a, b = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+        a.record()
+        fn()
+        b.record()
+        b.synchronize()
+        best = min(best, a.elapsed_time(b) * 1e3)
+    return best
+
+
+@pytest.mark.parametrize("before", [0, 1 << 22])
+def test_a_small_system_in_a_large_context(cuda, before):
+    """A step of 1000 bodies in a context of 2^24, also after a large system, within
+    half as much again of one in a context of 1000 (clearing the whole node pool
+    took eight times as long)."""
+    from nns_gb300.barnes_hut import Context, State
+    b = ic.star_disk(1000)
+    us = []
+    for cap in (1000, 1 << 24):
+        ctx = Context(max_bodies=cap, theta=0.5, eps=0.01, dt=1e-6)
+        if before and cap > before:
+            _build(ctx, [ic.plummer(before, seed=1)])
+            ctx.sync()
+        ctx.set_systems([0, 1000])
+        s = State.from_bodies(b)
+        us.append(_best_us(lambda: ctx.step(s, 1)))
+        ctx.sync()
+    assert us[1] < 1.5 * us[0], us
