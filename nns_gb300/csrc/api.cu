@@ -47,7 +47,8 @@ void adjoint_times(const Adj *a, float *fwd_ms, float *bwd_ms);
 
 namespace {
 
-__global__ void k_body_sys(const int *sys_off, int nsys, int n, int *body_sys) {
+// Each body's system; and every system's scratch box starts empty (k_bbox keeps it so).
+__global__ void k_body_sys(const int *sys_off, int nsys, int n, int *body_sys, unsigned *bbox_u, unsigned *bbox_done) {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         int lo = 0, hi = nsys - 1;
         while (lo < hi) {
@@ -56,6 +57,10 @@ __global__ void k_body_sys(const int *sys_off, int nsys, int n, int *body_sys) {
             else hi = mid - 1;
         }
         body_sys[i] = lo;
+        if (i < nsys) {  // (no system is empty: nsys <= n)
+            for (int k = 0; k < 6; k++) bbox_u[6 * i + k] = f2ord(0.0f);
+            bbox_done[i] = 0u;
+        }
     }
 }
 
@@ -299,7 +304,8 @@ int nbx_create(const nbx_params *p, nbx_ctx **out) {
     rc |= nbx::dmalloc(ctx, &ctx->d_tiles_mg, (size_t)B / nbx::kMergeTile + (size_t)B / nbx::kMergeRun + 2 * (size_t)Ss + 2);
     rc |= nbx::dmalloc(ctx, &ctx->d_groups, G);
     if (Ss > 1) rc |= nbx::dmalloc(ctx, &ctx->d_team, G);  // both lists of a mixed batch
-    rc |= nbx::dmalloc(ctx, &ctx->d_bbox_u, 6 * Ss + 6);
+    rc |= nbx::dmalloc(ctx, &ctx->d_bbox_u, 7 * (size_t)Ss);
+    if (rc == 0) ctx->d_bbox_done = ctx->d_bbox_u + 6 * (size_t)Ss;
     rc |= nbx::dmalloc(ctx, &ctx->d_bbox, 6 * Ss);
     rc |= nbx::dmalloc(ctx, &ctx->d_bbox64, 6 * Ss);
     rc |= nbx::dmalloc(ctx, &ctx->d_depth0, Ss);
@@ -326,11 +332,8 @@ int nbx_create(const nbx_params *p, nbx_ctx **out) {
     rc |= nbx::dmalloc(ctx, &ctx->d_arrive, NC);
     rc |= nbx::dmalloc(ctx, &ctx->d_lvl8, NC);
     rc |= nbx::dmalloc(ctx, &ctx->d_lvl_counts, 64 * (size_t)nbx::ceil_div(B, nbx::kPosBlock));
-    rc |= nbx::dmalloc(ctx, &ctx->d_lvl_tot, 3 * 64);
-    if (rc == 0) {
-        ctx->d_lvl_start = ctx->d_lvl_tot + 64;
-        ctx->d_bbox_done = ctx->d_lvl_tot + 128;
-    }
+    rc |= nbx::dmalloc(ctx, &ctx->d_lvl_tot, 2 * 64);
+    if (rc == 0) ctx->d_lvl_start = ctx->d_lvl_tot + 64;
     rc |= nbx::dmalloc(ctx, &ctx->d_hist, hist + 1);  // + the scanned total
     // one-sweep body sort: a system of several tiles takes at least two, so at most
     // half the tiles (plus one) hold count slots; status words per tile and digit
@@ -346,17 +349,11 @@ int nbx_create(const nbx_params *p, nbx_ctx **out) {
     if (rc == 0 && cudaMemset(ctx->d_totals, 0, 8 * sizeof(unsigned)) != cudaSuccess) rc = NBX_ERR_CUDA;
     // no tree yet: every build clears the meta words of the tree before it (tree.cu)
     if (rc == 0 && (cudaMemset(ctx->d_meta, 0, sizeof(int) * (size_t)NC) != cudaSuccess ||
-                    cudaMemset(ctx->d_lvl_tot, 0, 3 * 64 * sizeof(unsigned)) != cudaSuccess))
+                    cudaMemset(ctx->d_lvl_tot, 0, 2 * 64 * sizeof(unsigned)) != cudaSuccess))
         rc = NBX_ERR_CUDA;
     // status words start at build 0, which no pass ever uses (its tags are >= 1)
     if (rc == 0 && cudaMemset(ctx->d_lb_status, 0, sizeof(unsigned long long) * ((size_t)ctx->cap_tiles_body << nbx::kMaxRadixBits)) != cudaSuccess)
         rc = NBX_ERR_CUDA;
-    // empty boxes: the ordered encoding of 0.0f is the sign bit (k_bbox keeps them so)
-    if (rc == 0) {
-        const std::vector<unsigned> empty(6 * (size_t)Ss + 6, 0x80000000u);
-        if (cudaMemcpy(ctx->d_bbox_u, empty.data(), sizeof(unsigned) * empty.size(), cudaMemcpyHostToDevice) != cudaSuccess)
-            rc = NBX_ERR_CUDA;
-    }
     if (rc == 0 && cudaMemset(ctx->d_lb, 0, 16 * sizeof(unsigned)) != cudaSuccess) rc = NBX_ERR_CUDA;
     if (rc == 0 && ctx->multipole) rc = nbx::alloc_quadrupoles(ctx);
     if (rc == 0) rc = nbx::walk_init(ctx);
@@ -552,8 +549,8 @@ int nbx_set_systems(nbx_ctx *c, int nsys, const int64_t *offsets) {
         NBX_CUDA(cudaMemcpy(ctx->d_solo, solo.data(), sizeof(int) * solo.size(), cudaMemcpyHostToDevice));
     }
     NBX_CUDA(cudaMemcpy(ctx->d_groups, groups.data(), sizeof(int) * groups.size(), cudaMemcpyHostToDevice));
-    nbx::k_body_sys<<<nbx::ceil_div(n, 256) < 4096 ? nbx::ceil_div(n, 256) : 4096, 256>>>(ctx->d_sys_off, nsys, n,
-                                                                                          ctx->d_body_sys);
+    nbx::k_body_sys<<<nbx::ceil_div(n, 256) < 4096 ? nbx::ceil_div(n, 256) : 4096, 256>>>(
+        ctx->d_sys_off, nsys, n, ctx->d_body_sys, ctx->d_bbox_u, ctx->d_bbox_done);
     ++ctx->launches;
     NBX_CUDA(cudaGetLastError());
     NBX_CUDA(cudaDeviceSynchronize());

@@ -133,7 +133,7 @@ struct Ctx {
 
     // per-system tree parameters
     unsigned *d_bbox_u = nullptr;   // [6S] ordered-int encodings during the reduction (between builds: empty boxes)
-    unsigned *d_bbox_done = nullptr;  // [1] finished blocks of k_bbox (between builds: 0)
+    unsigned *d_bbox_done = nullptr;  // [S] finished blocks of each system's box (between builds: 0)
     float *d_bbox = nullptr;        // [6S]
     double *d_bbox64 = nullptr;     // [6S]
     float *d_depth0 = nullptr;      // [S]
@@ -167,7 +167,7 @@ struct Ctx {
     float4 *d_quad4 = nullptr;     // [NC] quadrupole mode: P = -Q (Q traceless) of cells in FP32, (xx, yy, zz, xy)
     float2 *d_quad2 = nullptr;     // [NC]                                              (xz, yz)
     unsigned *d_lvl_counts = nullptr;                 // [position blocks][64] nodes per level
-    unsigned *d_lvl_tot = nullptr;                    // [64] nodes of each level (lvl_start, bbox_done: behind it)
+    unsigned *d_lvl_tot = nullptr;                    // [64] nodes of each level (lvl_start: behind it)
     unsigned *d_lvl_start = nullptr;                  // [64] first node of each level (past the deepest: the node count
                                                       // of the tree in d_meta, by which the next build clears it)
 

@@ -87,19 +87,23 @@ __device__ __forceinline__ float depth0_of(float mnx, float mxx, float theta_ref
 }
 
 // The boxes of all systems, and the build's reset, in one launch: per-tile
-// min/max of the bodies of one system, merged with ordered-int atomics; the last
-// block to finish writes every system's box and its walk threshold and leaves
-// the scratch boxes empty (they contain the origin: Kernels.cu:56-62) and the
-// block counter at zero for the next build.
+// min/max of the bodies of one system.  A system of one tile has its box at once;
+// of several, they are merged with ordered-int atomics, and the system's last block
+// to finish writes its box and walk threshold and leaves the scratch box empty
+// (boxes contain the origin: Kernels.cu:56-62) and the system's block counter at
+// zero for the next build.  (One last block for the boxes of all systems took as
+// long as the rest of the build for 10^5 systems.)
 __global__ void __launch_bounds__(kBlock) k_bbox(const float *__restrict__ x, const float *__restrict__ y,
                                                   const float *__restrict__ z, const int4 *__restrict__ tiles,
-                                                  int ntiles, unsigned *bbox_u, int nsys, float theta_ref, float *bbox,
-                                                  double *bbox64, float *depth0, unsigned *done, DevStatus *st,
-                                                  int *sys_lvl, int *root_nch, int4 *__restrict__ meta4,
-                                                  int *__restrict__ meta, const unsigned *__restrict__ lvl_start) {
+                                                  const int2 *__restrict__ sys_tiles, unsigned *bbox_u, int nsys,
+                                                  float theta_ref, float *bbox, double *bbox64, float *depth0,
+                                                  unsigned *done, DevStatus *st, int *sys_lvl, int *root_nch,
+                                                  int4 *__restrict__ meta4, int *__restrict__ meta,
+                                                  const unsigned *__restrict__ lvl_start) {
     grid_dependency();
     reset_build(nsys, st, sys_lvl, root_nch, meta4, meta, lvl_start);
     const int4 tl = tiles[blockIdx.x];
+    const int s = tl.z, ntiles = sys_tiles[s].y;
     float v[6] = {INFINITY, -INFINITY, INFINITY, -INFINITY, INFINITY, -INFINITY};
     for (int i = threadIdx.x; i < tl.y; i += kBlock) {
         float a = x[tl.x + i], b = y[tl.x + i], c = z[tl.x + i];
@@ -115,40 +119,47 @@ __global__ void __launch_bounds__(kBlock) k_bbox(const float *__restrict__ x, co
             v[k + 1] = fmaxf(v[k + 1], __shfl_xor_sync(0xffffffffu, v[k + 1], o));
         }
     }
-    __shared__ float part[kBlock / 32][6];
+    __shared__ float part[kBlock / 32][6], box[6];
     __shared__ bool last;
-    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, k = threadIdx.x;
     if (lane == 0)
-        for (int k = 0; k < 6; k++) part[w][k] = v[k];
+        for (int q = 0; q < 6; q++) part[w][q] = v[q];
     __syncthreads();
-    if (threadIdx.x < 6) {
-        const int k = threadIdx.x;
+    if (k < 6) {
         float r = part[0][k];
         for (int q = 1; q < kBlock / 32; q++) r = (k & 1) ? fmaxf(r, part[q][k]) : fminf(r, part[q][k]);
-        if (!isnan(r) && !isinf(r)) {
-            unsigned *dst = &bbox_u[6 * tl.z + k];
-            if (k & 1) atomicMax(dst, f2ord(r));
-            else atomicMin(dst, f2ord(r));
+        const bool finite = !isnan(r) && !isinf(r);
+        if (ntiles == 1) {
+            box[k] = !finite ? 0.0f : ((k & 1) ? fmaxf(r, 0.0f) : fminf(r, 0.0f));
+        } else {
+            if (finite) {
+                unsigned *dst = &bbox_u[6 * s + k];
+                if (k & 1) atomicMax(dst, f2ord(r));
+                else atomicMin(dst, f2ord(r));
+            }
+            __threadfence();
         }
-        __threadfence();
     }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        last = atomicAdd(done, 1u) == gridDim.x - 1;
-        __threadfence();
-    }
-    __syncthreads();
-    if (!last) return;
-    if (threadIdx.x == 0) *done = 0u;
-    for (int s = threadIdx.x; s < nsys; s += kBlock) {
-        float b[6];
-        for (int k = 0; k < 6; k++) {
-            b[k] = __fadd_rn(ord2f(__ldcg(&bbox_u[6 * s + k])), 0.0f);  // -0 -> +0
-            bbox[6 * s + k] = b[k];
-            bbox64[6 * s + k] = (double)b[k];
+    if (ntiles > 1) {  // uniform over the block
+        __syncthreads();
+        if (k == 0) {
+            last = atomicAdd(&done[s], 1u) == (unsigned)ntiles - 1u;
+            __threadfence();
+        }
+        __syncthreads();
+        if (!last) return;
+        if (k == 0) done[s] = 0u;
+        if (k < 6) {
+            box[k] = ord2f(__ldcg(&bbox_u[6 * s + k]));
             bbox_u[6 * s + k] = f2ord(0.0f);
         }
-        depth0[s] = depth0_of(b[0], b[1], theta_ref);
+    }
+    __syncthreads();
+    if (k < 6) {
+        const float b = __fadd_rn(box[k], 0.0f);  // -0 -> +0
+        bbox[6 * s + k] = b;
+        bbox64[6 * s + k] = (double)b;
+        if (k == 0) depth0[s] = depth0_of(b, __fadd_rn(box[1], 0.0f), theta_ref);
     }
 }
 
@@ -1048,7 +1059,7 @@ int build_tree(Ctx *ctx, const nbx_state *s, cudaStream_t st, bool external_bbox
     const int gb = ceil_div(n, kBlock) < ctx->nsm * 8 ? ceil_div(n, kBlock) : ctx->nsm * 8;
     int4 *meta4 = reinterpret_cast<int4 *>(ctx->d_meta);
     if (!external_bbox) {
-        launch_chained(ctx, st, ctx->ntiles_body, kBlock, 0, k_bbox, s->x, s->y, s->z, ctx->d_tiles, ctx->ntiles_body,
+        launch_chained(ctx, st, ctx->ntiles_body, kBlock, 0, k_bbox, s->x, s->y, s->z, ctx->d_tiles, ctx->d_sys_tiles,
                        ctx->d_bbox_u, S, ctx->theta_ref, ctx->d_bbox, ctx->d_bbox64, ctx->d_depth0, ctx->d_bbox_done,
                        ctx->d_status, ctx->d_sys_lvl, ctx->d_root_nch, meta4, ctx->d_meta, ctx->d_lvl_start);
     } else {

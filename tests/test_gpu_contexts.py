@@ -2,6 +2,7 @@
 every build starts from what the trees before it left behind.  Trees against the
 oracle (bit-exact) after larger and smaller systems, batches and failed builds; and
 a small system's step costs in a large context what it costs in one of its size.
+Also the boxes of systems of one block and of several in one batch.
 """
 import numpy as np
 import pytest
@@ -106,3 +107,30 @@ def test_a_small_system_in_a_large_context(cuda, before):
         us.append(_best_us(lambda: ctx.step(s, 1)))
         ctx.sync()
     assert us[1] < 1.5 * us[0], us
+
+
+def test_boxes_of_a_batch(cuda):
+    """Systems of one box block and of many, off centre (the boxes contain the
+    origin), with signed zeros: the keys of every system are those of its own box,
+    in every build."""
+    from nns_gb300.barnes_hut import Context
+    systems = []
+    for j, k in enumerate([1, 2, 255, 256, 257, 40000, 3, 511, 513, 100000, 1, 8, 20000]):
+        b = ic.plummer(k, seed=50 + j)
+        sh = [np.float32(3.0 * ((j + a) % 3 - 1)) for a in range(3)]
+        x, y, z = b.x + sh[0], b.y + sh[1], b.z + sh[2]
+        if j % 2:
+            x[0], y[0], z[0] = np.float32(-0.0), np.float32(0.0), np.float32(-0.0)
+        systems.append(ic.Bodies(x, y, z, b.vx, b.vy, b.vz, b.m))
+    _, off = _joined(systems)
+    ctx = Context(max_bodies=int(off[-1]), max_systems=len(systems))
+    s = _build(ctx, systems)
+    for _ in range(2):
+        ctx.build(s)
+        ctx.sync()
+        keys, perm = ctx.export_keys()
+        for j, q in enumerate(systems):
+            hi, lo = O.keys(q.x, q.y, q.z, O.bbox(q.x, q.y, q.z), 42)
+            o = np.lexsort((lo, hi))
+            assert np.array_equal(perm[off[j]:off[j + 1]] - off[j], o), j
+            assert np.array_equal(keys[off[j]:off[j + 1]], hi[o]), j
