@@ -483,7 +483,7 @@ int nbx_set_systems(nbx_ctx *c, int nsys, const int64_t *offsets) {
     const int tile_sw = tile > nbx::kTileSweep ? tile : (nbx::kTileSweep < nbx::kTile ? nbx::kTileSweep : nbx::kTile);
     std::vector<int> off(nsys + 1);
     std::vector<int4> tiles, tiles_sw, tiles_mg, runs_mg;
-    int max_sys = 0;
+    int max_sys = 0, nsmall_mg = 0;
     std::vector<int2> st(nsys), st_sw(nsys);
     std::vector<int> slot(nsys);
     std::vector<int> groups, team, solo;
@@ -513,15 +513,27 @@ int nbx_set_systems(nbx_ctx *c, int nsys, const int64_t *offsets) {
         }
         max_sys = max_sys > end - beg ? max_sys : end - beg;
     }
-    if (max_sys <= nbx::kMergeMaxBodies)
+    if (max_sys <= nbx::kMergeMaxBodies) {
+        const auto cut = [&](std::vector<int4> &to, int s, int width) {
+            for (int a = off[s], t = 0; a < off[s + 1]; a += width, t++)
+                to.push_back(make_int4(a, off[s + 1] - a < width ? off[s + 1] - a : width, s, t));
+        };
+        // systems of one block's keys have a launch of their own, where they are more
+        // than a few among larger ones (a launch is a few us)
+        const auto one_block = [&](int s) { return off[s + 1] - off[s] <= nbx::kMergeTile; };
+        int small = 0;
+        for (int s = 0; s < nsys; s++) small += one_block(s);
+        const bool apart = small == nsys || small >= 64;
         for (int s = 0; s < nsys; s++) {
-            const auto cut = [&](std::vector<int4> &to, int width) {
-                for (int a = off[s], t = 0; a < off[s + 1]; a += width, t++)
-                    to.push_back(make_int4(a, off[s + 1] - a < width ? off[s + 1] - a : width, s, t));
-            };
-            cut(tiles_mg, nbx::kMergeTile);
-            cut(runs_mg, nbx::kMergeRun);
+            cut(tiles_mg, s, nbx::kMergeTile);
+            if (!apart || !one_block(s)) cut(runs_mg, s, nbx::kMergeRun);
         }
+        if (apart) {
+            nsmall_mg = small;
+            for (int s = 0; s < nsys; s++)
+                if (one_block(s)) cut(runs_mg, s, nbx::kMergeTile);
+        }
+    }
     if ((int)tiles.size() > ctx->cap_tiles_body || (int)tiles_sw.size() > ctx->cap_tiles_body) return NBX_ERR_ARG;
     // the meta words of a much larger tree are cleared here by the whole GPU; the
     // next build has blocks for its own bodies only
@@ -561,7 +573,8 @@ int nbx_set_systems(nbx_ctx *c, int nsys, const int64_t *offsets) {
     ctx->ntiles_sw = (int)tiles_sw.size();
     ctx->tile_sw = tile_sw;
     ctx->ntiles_mg = (int)ntiles_mg;
-    ctx->nruns_mg = (int)runs_mg.size();
+    ctx->nruns_mg = (int)runs_mg.size() - nsmall_mg;
+    ctx->nsmall_mg = nsmall_mg;
     ctx->max_sys = max_sys;
     ctx->h_team = std::move(team);
     ctx->h_solo = std::move(solo);

@@ -120,8 +120,9 @@ struct Ctx {
     int ntiles_sw = 0, tile_sw = 0;
     int nslots = 0;                 // systems of several tiles (count slots in use)
     int4 *d_tiles_mg = nullptr;     // [merge tiles] of kMergeTile keys: start, len, sys, local tile index
-    int4 *d_runs_mg = nullptr;      // [first runs] of kMergeRun keys, the same (behind the tiles)
-    int nruns_mg = 0;
+    int4 *d_runs_mg = nullptr;      // [first runs] of kMergeRun keys, the same (behind the tiles): nruns_mg
+                                    // sorted by clusters, then nsmall_mg whole systems sorted by one block
+    int nruns_mg = 0, nsmall_mg = 0;
     int ntiles_mg = 0;              // 0: a system is too large, the keys sort by radix
     int max_sys = 0;                // bodies of the largest system
     int *d_groups = nullptr;        // [G] first sorted position of each walk group

@@ -246,34 +246,22 @@ __global__ void __launch_bounds__(kBlock) k_keys(const float *__restrict__ x, co
     }
 }
 
-// The first runs of the merging sort (merge.cu): k_keys and a stable sort of
-// every run of 1024 keys, one cluster of four blocks per run.  Each block sorts
-// a quarter: parts of 64 by counting, for every key, the part's keys before it
-// (broadcast comparisons, no chain of passes), then the four parts by searching
-// the other three; then it reads the other three sorted quarters through
-// distributed shared memory and searches those.  (One block of 1024 threads per
-// run took 13.5 us at 16384 bodies on 16 SMs; counting over all 256 keys of a
-// quarter 220 us for a batch of 3.2 x 10^6 bodies.)
-__global__ void __cluster_dims__(4, 1, 1) __launch_bounds__(kMergeTile)
-    k_sort_tiles(const float *__restrict__ x, const float *__restrict__ y, const float *__restrict__ z,
-                 const float *__restrict__ m, const int4 *__restrict__ runs, const float *__restrict__ bbox,
-                 unsigned long long *__restrict__ key, int *__restrict__ val, float4 *__restrict__ pos4, DevStatus *st,
-                 int order) {
-    grid_dependency();
-    constexpr int kQ = kMergeTile;  // a quarter
-    static_assert(kMergeRun == 4 * kQ, "four quarters");
-    __shared__ unsigned char ht[96];
-    __shared__ __align__(16) unsigned long long sk[kQ];     // the quarter's keys, then sorted
-    __shared__ __align__(16) unsigned long long so[3][kQ];  // the other quarters
-    __shared__ int sv[kQ];
-    load_hilbert(ht, order);
-    const cg::cluster_group cluster = cg::this_cluster();
-    const int quarter = (int)cluster.block_rank();
-    const int4 t = runs[blockIdx.x >> 2];  // start, len, system, run of the system
+// The first runs of the merging sort (merge.cu): k_keys and a stable sort.
+//
+// A block's 256 keys: parts of 64 by counting, for every key, the part's keys
+// before it (broadcast comparisons, no chain of passes), then the four parts by
+// searching the other three.  Leaves the sorted keys and their bodies in sk, sv.
+// `first` is this block's first key of the run t.  (Counting over all 256 keys
+// took 220 us for a batch of 3.2 x 10^6 bodies, this 171.)
+__device__ __forceinline__ void sort_block(const float *__restrict__ x, const float *__restrict__ y,
+                                           const float *__restrict__ z, const float *__restrict__ m, int4 t, int first,
+                                           const float *__restrict__ bbox, float4 *__restrict__ pos4, DevStatus *st,
+                                           int order, const unsigned char *ht, unsigned long long *sk, int *sv,
+                                           unsigned long long (*so)[kMergeTile]) {
     const int tid = (int)threadIdx.x;
-    int i = t.x + quarter * kQ + tid;
+    int i = t.x + first + tid;
     unsigned long long k = 1ull << 63;  // padding: above every 63-bit key
-    if (quarter * kQ + tid < t.y) {
+    if (first + tid < t.y) {
         const float px = x[i], py = y[i], pz = z[i];
         pos4[i] = make_float4(px, py, pz, m[i]);
         if (!isfinite(px) || !isfinite(py) || !isfinite(pz)) set_status(st, NBX_ERR_NONFINITE, i);
@@ -286,53 +274,75 @@ __global__ void __cluster_dims__(4, 1, 1) __launch_bounds__(kMergeTile)
     // by position
     const int part = tid & ~63, w0 = tid & ~31;
     int place = part;
-    {
-        so[0][tid] = k;
-        __syncthreads();
-        const ulonglong2 *mine = reinterpret_cast<const ulonglong2 *>(&so[0][w0]);
-        const ulonglong2 *other = reinterpret_cast<const ulonglong2 *>(&so[0][w0 ^ 32]);
+    so[0][tid] = k;
+    __syncthreads();
+    const ulonglong2 *mine = reinterpret_cast<const ulonglong2 *>(&so[0][w0]);
+    const ulonglong2 *other = reinterpret_cast<const ulonglong2 *>(&so[0][w0 ^ 32]);
 #pragma unroll
-        for (int j = 0; j < 16; j++) {
-            const ulonglong2 a = mine[j];
-            place += (int)(a.x < k) + ((int)(a.x == k) & (int)(w0 + 2 * j < tid)) + (int)(a.y < k) +
-                     ((int)(a.y == k) & (int)(w0 + 2 * j + 1 < tid));
-        }
-        const unsigned long long kq = k + (w0 & 32 ? 1ull : 0ull);  // an earlier warp's equal key comes first
-#pragma unroll
-        for (int j = 0; j < 16; j++) {
-            const ulonglong2 a = other[j];
-            place += (int)(a.x < kq) + (int)(a.y < kq);
-        }
-        so[1][place] = k;
-        __syncthreads();
-        // and the four parts of 64 by search
-        k = so[1][tid];
-        int pos[3] = {0, 0, 0};
-#pragma unroll
-        for (int step = 64; step > 0; step >>= 1) {
-#pragma unroll
-            for (int a = 0; a < 3; a++) {
-                const int q = a + (64 * a >= part);
-                const int p = min(pos[a] + step, 64);
-                const bool before = so[1][64 * q + p - 1] < k + (64 * q < part ? 1ull : 0ull);
-                pos[a] = (int)(pos[a] + step <= 64) & (int)before ? p : pos[a];
-            }
-        }
-        // the body that stands at `place` of its part moves along
-        reinterpret_cast<int *>(so[2])[place] = i;
-        __syncthreads();
-        i = reinterpret_cast<const int *>(so[2])[tid];
-        place = tid - part + pos[0] + pos[1] + pos[2];
+    for (int j = 0; j < 16; j++) {
+        const ulonglong2 a = mine[j];
+        place += (int)(a.x < k) + ((int)(a.x == k) & (int)(w0 + 2 * j < tid)) + (int)(a.y < k) +
+                 ((int)(a.y == k) & (int)(w0 + 2 * j + 1 < tid));
     }
+    const unsigned long long kq = k + (w0 & 32 ? 1ull : 0ull);  // an earlier warp's equal key comes first
+#pragma unroll
+    for (int j = 0; j < 16; j++) {
+        const ulonglong2 a = other[j];
+        place += (int)(a.x < kq) + (int)(a.y < kq);
+    }
+    so[1][place] = k;
+    __syncthreads();
+    // and the four parts of 64 by search
+    k = so[1][tid];
+    int pos[3] = {0, 0, 0};
+#pragma unroll
+    for (int step = 64; step > 0; step >>= 1) {
+#pragma unroll
+        for (int a = 0; a < 3; a++) {
+            const int q = a + (64 * a >= part);
+            const int p = min(pos[a] + step, 64);
+            const bool before = so[1][64 * q + p - 1] < k + (64 * q < part ? 1ull : 0ull);
+            pos[a] = (int)(pos[a] + step <= 64) & (int)before ? p : pos[a];
+        }
+    }
+    // the body that stands at `place` of its part moves along
+    reinterpret_cast<int *>(so[2])[place] = i;
+    __syncthreads();
+    i = reinterpret_cast<const int *>(so[2])[tid];
+    place = tid - part + pos[0] + pos[1] + pos[2];
     sk[place] = k;
     sv[place] = i;
+}
+
+// Every run of 1024 keys, one cluster of four blocks per run: each sorts a
+// quarter, reads the other three sorted quarters through distributed shared
+// memory and searches those.  (One block of 1024 threads per run took 13.5 us at
+// 16384 bodies on 16 SMs.)
+__global__ void __cluster_dims__(4, 1, 1) __launch_bounds__(kMergeTile)
+    k_sort_tiles(const float *__restrict__ x, const float *__restrict__ y, const float *__restrict__ z,
+                 const float *__restrict__ m, const int4 *__restrict__ runs, const float *__restrict__ bbox,
+                 unsigned long long *__restrict__ key, int *__restrict__ val, float4 *__restrict__ pos4, DevStatus *st,
+                 int order) {
+    grid_dependency();
+    constexpr int kQ = kMergeTile;  // a quarter
+    static_assert(kMergeRun == 4 * kQ, "four quarters");
+    __shared__ unsigned char ht[96];
+    __shared__ __align__(16) unsigned long long sk[kQ];     // the quarter's keys, sorted
+    __shared__ __align__(16) unsigned long long so[3][kQ];  // the other quarters
+    __shared__ int sv[kQ];
+    load_hilbert(ht, order);
+    const cg::cluster_group cluster = cg::this_cluster();
+    const int quarter = (int)cluster.block_rank();
+    const int4 t = runs[blockIdx.x >> 2];  // start, len, system, run of the system
+    const int tid = (int)threadIdx.x;
+    sort_block(x, y, z, m, t, quarter * kQ, bbox, pos4, st, order, ht, sk, sv, so);
     cluster.sync();
 #pragma unroll
     for (int a = 0; a < 3; a++) so[a][tid] = cluster.map_shared_rank(sk, a + (a >= quarter))[tid];
     __syncthreads();
     // this thread's key is now the sorted quarter's tid-th; the keys of earlier
     // quarters precede an equal one
-    k = sk[tid];
+    const unsigned long long k = sk[tid];
     const int v = sv[tid];
     int pos[3] = {0, 0, 0};
 #pragma unroll
@@ -344,13 +354,36 @@ __global__ void __cluster_dims__(4, 1, 1) __launch_bounds__(kMergeTile)
             pos[a] = (int)(pos[a] + step <= kQ) & (int)before ? p : pos[a];
         }
     }
-    place = tid + pos[0] + pos[1] + pos[2];
+    const int place = tid + pos[0] + pos[1] + pos[2];
     // (padding keys stay behind the valid ones: place < len marks a valid key)
     if (place < t.y) {
         key[t.x + place] = k;
         val[t.x + place] = v;
     }
     cluster.sync();  // the other blocks have read this block's quarter
+}
+
+// Runs of at most 256 keys (systems of at most so many bodies), one block each.
+// (With clusters, whose other three blocks have nothing to sort, the build of 500000
+// systems of four bodies took 23 ms, so 4.1; of 100000 systems of ten 4.8, so 0.94.)
+__global__ void __launch_bounds__(kMergeTile)
+    k_sort_small(const float *__restrict__ x, const float *__restrict__ y, const float *__restrict__ z,
+                 const float *__restrict__ m, const int4 *__restrict__ runs, const float *__restrict__ bbox,
+                 unsigned long long *__restrict__ key, int *__restrict__ val, float4 *__restrict__ pos4, DevStatus *st,
+                 int order) {
+    grid_dependency();
+    __shared__ unsigned char ht[96];
+    __shared__ __align__(16) unsigned long long sk[kMergeTile];
+    __shared__ __align__(16) unsigned long long so[3][kMergeTile];
+    __shared__ int sv[kMergeTile];
+    load_hilbert(ht, order);
+    const int4 t = runs[blockIdx.x];
+    sort_block(x, y, z, m, t, 0, bbox, pos4, st, order, ht, sk, sv, so);
+    __syncthreads();
+    if ((int)threadIdx.x < t.y) {
+        key[t.x + threadIdx.x] = sk[threadIdx.x];
+        val[t.x + threadIdx.x] = sv[threadIdx.x];
+    }
 }
 
 // Runs of equal 21-level keys: compute levels 22..42 and order the run by them.
@@ -1077,10 +1110,14 @@ int build_tree(Ctx *ctx, const nbx_state *s, cudaStream_t st, bool external_bbox
     const bool alt = (merge ? merge_passes(ctx->max_sys) : radix_passes(ctx->radix_bits)) & 1;
     unsigned long long *key0 = alt ? ctx->d_key_alt : ctx->d_key;
     int *val0 = alt ? ctx->d_val_alt : ctx->d_val;
-    if (merge)
-        launch_chained(ctx, st, 4 * ctx->nruns_mg, kMergeTile, 0, k_sort_tiles, s->x, s->y, s->z, s->m, ctx->d_runs_mg,
-                       ctx->d_bbox, key0, val0, pos4, ctx->d_status, ctx->key_order);
-    else
+    if (merge) {
+        if (ctx->nruns_mg)
+            launch_chained(ctx, st, 4 * ctx->nruns_mg, kMergeTile, 0, k_sort_tiles, s->x, s->y, s->z, s->m,
+                           ctx->d_runs_mg, ctx->d_bbox, key0, val0, pos4, ctx->d_status, ctx->key_order);
+        if (ctx->nsmall_mg)
+            launch_chained(ctx, st, ctx->nsmall_mg, kMergeTile, 0, k_sort_small, s->x, s->y, s->z, s->m,
+                           ctx->d_runs_mg + ctx->nruns_mg, ctx->d_bbox, key0, val0, pos4, ctx->d_status, ctx->key_order);
+    } else
         launch_chained(ctx, st, gb, kBlock, 0, k_keys, s->x, s->y, s->z, s->m, ctx->d_body_sys, ctx->d_bbox, n, key0,
                        val0, pos4, ctx->d_status, ctx->key_order);
     int rc = merge ? merge_runs(ctx, st) : radix_sort_bodies(ctx, st);
