@@ -513,7 +513,7 @@ int nbx_set_systems(nbx_ctx *c, int nsys, const int64_t *offsets) {
         }
         max_sys = max_sys > end - beg ? max_sys : end - beg;
     }
-    if (max_sys <= nbx::kMergeMaxBodies) {
+    if (nbx::sorts_by_merging(max_sys, n)) {
         const auto cut = [&](std::vector<int4> &to, int s, int width) {
             for (int a = off[s], t = 0; a < off[s + 1]; a += width, t++)
                 to.push_back(make_int4(a, off[s + 1] - a < width ? off[s + 1] - a : width, s, t));

@@ -12,7 +12,8 @@
 // searches above (about 15 runs x 6 steps per key and launch).  Keys + sort, eight
 // one-sweep passes against this: 1000 bodies 58 -> 6.5 us, 16384 80 -> 17 us,
 // 131071 116 -> 43 us; at 2^20 the merges take 309 us, the passes 275 us, so
-// systems above kMergeMaxBodies sort by radix.
+// systems above kMergeMaxBodies sort by radix (sorts_by_merging, with the rule for
+// batches).
 #include <utility>
 
 #include "nbx_internal.cuh"

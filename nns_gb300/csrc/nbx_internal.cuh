@@ -45,6 +45,18 @@ constexpr int kMergeFan = 16;     // most runs merged by one launch
 #define NBX_MERGE_MAX (1 << 19)
 #endif
 constexpr int kMergeMaxBodies = NBX_MERGE_MAX;
+// Whether the keys of n bodies in systems of up to max_sys sort by merging.  That
+// figure is of one system, whose merges wait on latency; in a batch that fills the
+// GPU they are bound by their searches (about four bits of the run's length per
+// launch), the radix passes by memory.  Builds, merging against radix: 128
+// systems of 16384 0.77 / 0.85 ms, 256 of them 1.52 / 1.44; 16 systems of 65536
+// 0.41 / 0.48 ms, 64 of them 1.50 / 1.48; 4 of 262144 0.50 / 0.49, 8 of them 0.95 /
+// 0.88; 32 systems of 2^19 6.25 / 4.92 ms; one merge of up to four runs stays
+// ahead at every size (4194 systems of 4000 4.92 / 5.10 ms).
+inline bool sorts_by_merging(int max_sys, int n) {
+    if (max_sys > kMergeMaxBodies) return false;
+    return max_sys <= 4 * kMergeRun || n < (max_sys <= kMergeFan * kMergeRun ? 3 << 20 : 2 << 20);
+}
 // Systems of up to this many bodies are walked by teams of warps (walk_team.cu).
 // The rule sees a system's own size only, so that a batch gives every system the
 // bits of its single run.  Alone, teams win up to about 2^17 bodies (walk at 2^16:

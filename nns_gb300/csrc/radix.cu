@@ -22,7 +22,7 @@
 // their body keys in one launch per pass instead (k_radix_counts once, then the
 // same scatter kernel in its one-sweep form on a tiling of its own, whose tiles
 // find their offsets by decoupled look-back); the permutation is the same.
-// Systems of up to kMergeMaxBodies bodies do not come here: merge.cu sorts them.
+// What sorts_by_merging() accepts does not come here: merge.cu sorts it.
 #include <cstring>
 
 #include "nbx_internal.cuh"

@@ -1104,7 +1104,7 @@ int build_tree(Ctx *ctx, const nbx_state *s, cudaStream_t st, bool external_bbox
     }
     // the node array is free until the nodes are written: it holds the packed bodies
     float4 *pos4 = ctx->d_node4;
-    // systems of up to kMergeMaxBodies bodies sort by merging, larger ones by radix;
+    // keys sort by merging or by radix (sorts_by_merging);
     // the last pass writes d_key / d_val: an odd pass count starts from the alternates
     const bool merge = ctx->ntiles_mg > 0;
     const bool alt = (merge ? merge_passes(ctx->max_sys) : radix_passes(ctx->radix_bits)) & 1;

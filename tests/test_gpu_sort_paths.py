@@ -1,6 +1,7 @@
 """Every way the body keys are sorted, against NumPy's stable sort of the 42-level
 keys: batches with many systems of one block's keys (a launch of their own) beside
-larger ones.
+larger ones; the batches on both sides of the rule that picks merges or radix passes;
+and the radix passes of batches, one-sweep and scanned, with both digit widths.
 """
 import numpy as np
 import pytest
@@ -105,3 +106,50 @@ def test_a_build_of_many_tiny_systems(cuda):
         ctx.sync()
         best.append(min(t))
     assert best[1] <= 6 * best[0], best
+
+
+# merging up to 2^19 bodies a system, and in batches by their sum (2^21; 3 x 2^20 where
+# one launch merges; any where it merges four runs); else radix: one-sweep passes below
+# 1.5 x 2^20 bodies outside a captured graph, else scanned ones.  Systems of one radix
+# tile and of several, in one batch.
+SORTS = {
+    "merge-top": [524288],
+    "sweep": [524289],
+    "sweep-batch": [1, 300, 524289, 5000, 2],
+    "scan-batch": [1, 300, 524289, 5000, 1100000, 31],
+    "merge-two": [16385] * 127,
+    "scan-two": [16385] * 129,
+    "merge-one": [16384] * 191,
+    "scan-one": [16384] * 193,
+    "merge-four": [4096] * 800,
+    "scan-five": [4097] * 768 + [1],
+}
+
+
+@pytest.mark.parametrize("name", list(SORTS))
+def test_both_sides_of_the_sort_rule(cuda, name):
+    from nns_gb300.barnes_hut import Context, State
+    sizes = SORTS[name]
+    n = sum(sizes)
+    whole = ic.plummer(n, seed=17)  # any stretch of it is a system of its own box
+    off = np.concatenate([[0], np.cumsum(sizes)])
+    want_k, want_p = np.empty(n, np.uint64), np.empty(n, np.int32)
+    for a, e in zip(off[:-1], off[1:]):
+        x, y, z = (np.ascontiguousarray(v[a:e]) for v in (whole.x, whole.y, whole.z))
+        hi, lo = O.keys(x, y, z, O.bbox(x, y, z), 42)
+        o = np.lexsort((lo, hi))
+        want_k[a:e], want_p[a:e] = hi[o], o + a
+    ctx = Context(max_bodies=n, max_systems=len(sizes), theta=1.0, eps=0.1)
+    ctx.set_systems(off)
+    for bits in (8, 9):
+        for captured in (False, True):
+            ctx.set_tuning(bits, 512)
+            s = State.from_bodies(whole)
+            if captured:
+                ctx.graph_step(s, 1)
+            else:
+                ctx.build(s)
+            ctx.sync()
+            keys, perm = ctx.export_keys()
+            assert np.array_equal(perm, want_p), (bits, captured)
+            assert np.array_equal(keys, want_k), (bits, captured)
