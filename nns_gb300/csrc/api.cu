@@ -481,60 +481,67 @@ int nbx_set_systems(nbx_ctx *c, int nsys, const int64_t *offsets) {
     // the one-sweep sort's tiling: its passes are bound by the look-back chains
     // between a system's tiles, so its tiles are at least kTileSweep keys
     const int tile_sw = tile > nbx::kTileSweep ? tile : (nbx::kTileSweep < nbx::kTile ? nbx::kTileSweep : nbx::kTile);
-    std::vector<int> off(nsys + 1);
-    std::vector<int4> tiles, tiles_sw, tiles_mg, runs_mg;
-    int max_sys = 0, nsmall_mg = 0;
-    std::vector<int2> st(nsys), st_sw(nsys);
-    std::vector<int> slot(nsys);
-    std::vector<int> groups, team, solo;
-    int nslots = 0;
-    for (int s = 0; s <= nsys; s++) off[s] = (int)offsets[s];
+    int max_sys = 0, nteam = 0, ngroups = 0;
+    const auto bodies = [&](int s) { return (int)(offsets[s + 1] - offsets[s]); };
+    const auto by_team = [&](int s) { return bodies(s) <= nbx::kTeamMaxBodies; };
     for (int s = 0; s < nsys; s++) {
-        const int beg = off[s], end = off[s + 1];
-        const int nt = nbx::ceil_div(end - beg, tile);
-        st[s] = make_int2((int)tiles.size(), nt);
-        for (int t = 0; t < nt; t++) {
-            const int a = beg + t * tile;
-            const int len = (end - a) < tile ? (end - a) : tile;
-            tiles.push_back(make_int4(a, len, s, t));
+        max_sys = max_sys > bodies(s) ? max_sys : bodies(s);
+        const int g = nbx::ceil_div(bodies(s), 32);
+        ngroups += g;
+        if (by_team(s)) nteam += g;
+    }
+    // only the lists that this batch's sort and walks read are made
+    const bool merge = nbx::sorts_by_merging(max_sys, n), sweep = !merge && n < nbx::kSweepMaxBodies;
+    const bool mixed = nteam > 0 && nteam < ngroups;
+    std::vector<int> off(offsets, offsets + nsys + 1), groups, team, solo, slot;
+    std::vector<int4> tiles, tiles_sw, tiles_mg, runs_mg;
+    std::vector<int2> st(nsys), st_sw;
+    int nslots = 0, nsmall_mg = 0;
+    const auto cut = [&](std::vector<int4> &to, int s, int width) {
+        for (int a = off[s], t = 0; a < off[s + 1]; a += width, t++)
+            to.push_back(make_int4(a, off[s + 1] - a < width ? off[s + 1] - a : width, s, t));
+    };
+    tiles.reserve((size_t)n / tile + nsys);
+    for (int s = 0; s < nsys; s++) {
+        st[s] = make_int2((int)tiles.size(), nbx::ceil_div(bodies(s), tile));
+        cut(tiles, s, tile);
+    }
+    if ((int)tiles.size() > ctx->cap_tiles_body) return NBX_ERR_ARG;
+    if (sweep) {  // (no more tiles than those: they are no smaller)
+        st_sw.resize(nsys);
+        slot.resize(nsys);
+        for (int s = 0; s < nsys; s++) {
+            st_sw[s] = make_int2((int)tiles_sw.size(), nbx::ceil_div(bodies(s), tile_sw));
+            slot[s] = st_sw[s].y > 1 ? nslots++ : -1;
+            cut(tiles_sw, s, tile_sw);
         }
-        const int nts = nbx::ceil_div(end - beg, tile_sw);
-        st_sw[s] = make_int2((int)tiles_sw.size(), nts);
-        slot[s] = nts > 1 ? nslots++ : -1;
-        for (int t = 0; t < nts; t++) {
-            const int a = beg + t * tile_sw;
-            const int len = (end - a) < tile_sw ? (end - a) : tile_sw;
-            tiles_sw.push_back(make_int4(a, len, s, t));
-        }
-        std::vector<int> &kind = end - beg <= nbx::kTeamMaxBodies ? team : solo;
-        for (int g = beg; g < end; g += 32) {
-            kind.push_back((int)groups.size());
+    }
+    groups.reserve(ngroups);
+    for (int s = 0; s < nsys; s++)
+        for (int g = off[s]; g < off[s + 1]; g += 32) {
+            if (mixed) (by_team(s) ? team : solo).push_back((int)groups.size());
             groups.push_back(g);
         }
-        max_sys = max_sys > end - beg ? max_sys : end - beg;
-    }
-    if (nbx::sorts_by_merging(max_sys, n)) {
-        const auto cut = [&](std::vector<int4> &to, int s, int width) {
-            for (int a = off[s], t = 0; a < off[s + 1]; a += width, t++)
-                to.push_back(make_int4(a, off[s + 1] - a < width ? off[s + 1] - a : width, s, t));
-        };
+    if (merge) {
         // systems of one block's keys have a launch of their own, where they are more
         // than a few among larger ones (a launch is a few us)
-        const auto one_block = [&](int s) { return off[s + 1] - off[s] <= nbx::kMergeTile; };
+        const auto one_block = [&](int s) { return bodies(s) <= nbx::kMergeTile; };
         int small = 0;
         for (int s = 0; s < nsys; s++) small += one_block(s);
         const bool apart = small == nsys || small >= 64;
-        for (int s = 0; s < nsys; s++) {
-            cut(tiles_mg, s, nbx::kMergeTile);
-            if (!apart || !one_block(s)) cut(runs_mg, s, nbx::kMergeRun);
+        runs_mg.reserve((size_t)n / nbx::kMergeRun + nsys);
+        if (nbx::merge_passes(max_sys) > 0) {
+            tiles_mg.reserve((size_t)n / nbx::kMergeTile + (size_t)n / nbx::kMergeRun + 2 * (size_t)nsys);
+            for (int s = 0; s < nsys; s++) cut(tiles_mg, s, nbx::kMergeTile);
         }
+        for (int s = 0; s < nsys; s++)
+            if (!apart || !one_block(s)) cut(runs_mg, s, nbx::kMergeRun);
         if (apart) {
             nsmall_mg = small;
             for (int s = 0; s < nsys; s++)
                 if (one_block(s)) cut(runs_mg, s, nbx::kMergeTile);
         }
     }
-    if ((int)tiles.size() > ctx->cap_tiles_body || (int)tiles_sw.size() > ctx->cap_tiles_body) return NBX_ERR_ARG;
     // the meta words of a much larger tree are cleared here by the whole GPU; the
     // next build has blocks for its own bodies only
     if (ctx->nbodies > 16ll * n) {
@@ -543,24 +550,27 @@ int nbx_set_systems(nbx_ctx *c, int nsys, const int64_t *offsets) {
         NBX_CUDA(cudaMemset(ctx->d_meta, 0, sizeof(int) * (size_t)ctx->cap_nodes));
         NBX_CUDA(cudaMemset(ctx->d_lvl_start, 0, 64 * sizeof(unsigned)));
     }
-    NBX_CUDA(cudaMemcpy(ctx->d_sys_off, off.data(), sizeof(int) * (nsys + 1), cudaMemcpyHostToDevice));
-    NBX_CUDA(cudaMemcpy(ctx->d_tiles, tiles.data(), sizeof(int4) * tiles.size(), cudaMemcpyHostToDevice));
-    NBX_CUDA(cudaMemcpy(ctx->d_sys_tiles, st.data(), sizeof(int2) * nsys, cudaMemcpyHostToDevice));
-    NBX_CUDA(cudaMemcpy(ctx->d_seg_slot, slot.data(), sizeof(int) * nsys, cudaMemcpyHostToDevice));
-    NBX_CUDA(cudaMemcpy(ctx->d_tiles_sw, tiles_sw.data(), sizeof(int4) * tiles_sw.size(), cudaMemcpyHostToDevice));
-    NBX_CUDA(cudaMemcpy(ctx->d_sys_tiles_sw, st_sw.data(), sizeof(int2) * nsys, cudaMemcpyHostToDevice));
     const size_t ntiles_mg = tiles_mg.size();
-    if (ntiles_mg) {
-        tiles_mg.insert(tiles_mg.end(), runs_mg.begin(), runs_mg.end());
-        NBX_CUDA(cudaMemcpy(ctx->d_tiles_mg, tiles_mg.data(), sizeof(int4) * tiles_mg.size(), cudaMemcpyHostToDevice));
-    }
+    tiles_mg.insert(tiles_mg.end(), runs_mg.begin(), runs_mg.end());
+    const auto upload = [](auto *to, const auto &from) {
+        return from.empty() ? cudaSuccess
+                            : cudaMemcpy(to, from.data(), sizeof(from[0]) * from.size(), cudaMemcpyHostToDevice);
+    };
+    NBX_CUDA(upload(ctx->d_sys_off, off));
+    NBX_CUDA(upload(ctx->d_tiles, tiles));
+    NBX_CUDA(upload(ctx->d_sys_tiles, st));
+    NBX_CUDA(upload(ctx->d_seg_slot, slot));
+    NBX_CUDA(upload(ctx->d_tiles_sw, tiles_sw));
+    NBX_CUDA(upload(ctx->d_sys_tiles_sw, st_sw));
+    NBX_CUDA(upload(ctx->d_tiles_mg, tiles_mg));
     ctx->d_runs_mg = ctx->d_tiles_mg + ntiles_mg;
-    if (!team.empty() && !solo.empty()) {  // (several systems: the lists are there)
+    if (mixed) {  // (several systems: the lists are there)
+        std::vector<int> both(team);
+        both.insert(both.end(), solo.begin(), solo.end());
         ctx->d_solo = ctx->d_team + team.size();
-        NBX_CUDA(cudaMemcpy(ctx->d_team, team.data(), sizeof(int) * team.size(), cudaMemcpyHostToDevice));
-        NBX_CUDA(cudaMemcpy(ctx->d_solo, solo.data(), sizeof(int) * solo.size(), cudaMemcpyHostToDevice));
+        NBX_CUDA(upload(ctx->d_team, both));
     }
-    NBX_CUDA(cudaMemcpy(ctx->d_groups, groups.data(), sizeof(int) * groups.size(), cudaMemcpyHostToDevice));
+    NBX_CUDA(upload(ctx->d_groups, groups));
     nbx::k_body_sys<<<nbx::ceil_div(n, 256) < 4096 ? nbx::ceil_div(n, 256) : 4096, 256>>>(
         ctx->d_sys_off, nsys, n, ctx->d_body_sys, ctx->d_bbox_u, ctx->d_bbox_done);
     ++ctx->launches;
@@ -572,10 +582,12 @@ int nbx_set_systems(nbx_ctx *c, int nsys, const int64_t *offsets) {
     ctx->nslots = nslots;
     ctx->ntiles_sw = (int)tiles_sw.size();
     ctx->tile_sw = tile_sw;
+    ctx->merge = merge;
     ctx->ntiles_mg = (int)ntiles_mg;
     ctx->nruns_mg = (int)runs_mg.size() - nsmall_mg;
     ctx->nsmall_mg = nsmall_mg;
     ctx->max_sys = max_sys;
+    ctx->nteam = nteam;
     ctx->h_team = std::move(team);
     ctx->h_solo = std::move(solo);
     ctx->tile_body = tile;

@@ -57,6 +57,17 @@ inline bool sorts_by_merging(int max_sys, int n) {
     if (max_sys > kMergeMaxBodies) return false;
     return max_sys <= 4 * kMergeRun || n < (max_sys <= kMergeFan * kMergeRun ? 3 << 20 : 2 << 20);
 }
+// One-sweep radix passes below this many bodies (over all systems) in eager builds.
+// They save four launches per pass, and with their own tiling of at least
+// kTileSweep keys the look-back chains stay short: 2^20 bodies 0.711 against
+// 0.755 ms; from 2^21 the counts pass and the look-back cost more than the
+// launches (1.196 against 1.114 ms, 2^23 3.14 against 2.97).  In a captured
+// graph a launch costs less and the passes are equal at 2^17 already, below
+// which the keys are merged (merge.cu).
+#ifndef NBX_RADIX_SWEEP_MAX
+#define NBX_RADIX_SWEEP_MAX (3 << 19)
+#endif
+constexpr int kSweepMaxBodies = NBX_RADIX_SWEEP_MAX;
 // Systems of up to this many bodies are walked by teams of warps (walk_team.cu).
 // The rule sees a system's own size only, so that a batch gives every system the
 // bits of its single run.  Alone, teams win up to about 2^17 bodies (walk at 2^16:
@@ -135,12 +146,14 @@ struct Ctx {
     int4 *d_runs_mg = nullptr;      // [first runs] of kMergeRun keys, the same (behind the tiles): nruns_mg
                                     // sorted by clusters, then nsmall_mg whole systems sorted by one block
     int nruns_mg = 0, nsmall_mg = 0;
-    int ntiles_mg = 0;              // 0: a system is too large, the keys sort by radix
+    int ntiles_mg = 0;              // (none where every system is one run)
+    bool merge = false;             // the keys sort by merging (sorts_by_merging), else by radix
     int max_sys = 0;                // bodies of the largest system
     int *d_groups = nullptr;        // [G] first sorted position of each walk group
 
     // walk groups of systems of up to kTeamMaxBodies bodies (walked by teams of
-    // warps) and of larger ones, ascending; the device copies exist in a batch of both
+    // warps): their number, and in a batch of both kinds the groups of each, ascending
+    int nteam = 0;
     std::vector<int> h_team, h_solo;
     int *d_team = nullptr, *d_solo = nullptr;  // [G] together
 

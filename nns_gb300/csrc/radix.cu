@@ -38,17 +38,6 @@ constexpr int kWarpsPerBlock = 8;
 #ifndef NBX_RADIX_SWEEP
 #define NBX_RADIX_SWEEP 1  // body keys: 1 one-sweep passes below the size switch, 0 always histogram + scan + scatter
 #endif
-#ifndef NBX_RADIX_SWEEP_MAX
-#define NBX_RADIX_SWEEP_MAX (3 << 19)
-#endif
-// One-sweep passes below this many bodies (over all systems) in eager builds.
-// They save four launches per pass, and with their own tiling of at least
-// kTileSweep keys the look-back chains stay short: 2^20 bodies 0.711 against
-// 0.755 ms; from 2^21 the counts pass and the look-back cost more than the
-// launches (1.196 against 1.114 ms, 2^23 3.14 against 2.97).  In a captured
-// graph a launch costs less and the passes are equal at 2^17 already, below
-// which the keys are merged (merge.cu).
-constexpr int kSweepMaxBodies = NBX_RADIX_SWEEP_MAX;
 
 struct TileMap {
     const int4 *tiles;      // start, len, seg, local tile

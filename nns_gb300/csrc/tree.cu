@@ -1106,7 +1106,7 @@ int build_tree(Ctx *ctx, const nbx_state *s, cudaStream_t st, bool external_bbox
     float4 *pos4 = ctx->d_node4;
     // keys sort by merging or by radix (sorts_by_merging);
     // the last pass writes d_key / d_val: an odd pass count starts from the alternates
-    const bool merge = ctx->ntiles_mg > 0;
+    const bool merge = ctx->merge;
     const bool alt = (merge ? merge_passes(ctx->max_sys) : radix_passes(ctx->radix_bits)) & 1;
     unsigned long long *key0 = alt ? ctx->d_key_alt : ctx->d_key;
     int *val0 = alt ? ctx->d_val_alt : ctx->d_val;

@@ -600,8 +600,10 @@ int forces_cb(Ctx *ctx, const nbx_state *s, float *pot, int warps, cudaStream_t 
 // a share: of a context whose groups are all of one kind, the range itself;
 // of a batch of both kinds, a stretch of that kind's ascending list.
 Share share_of(const Ctx *ctx, bool team, int g0, int gn) {
+    const int all = team ? ctx->nteam : ctx->ngroups - ctx->nteam;
+    if (all == 0) return {nullptr, 0, 0};
+    if (all == ctx->ngroups) return {nullptr, g0, gn};
     const std::vector<int> &mine = team ? ctx->h_team : ctx->h_solo;
-    if ((int)mine.size() == ctx->ngroups) return {nullptr, g0, gn};
     const int a = (int)(std::lower_bound(mine.begin(), mine.end(), g0) - mine.begin());
     const int b = (int)(std::lower_bound(mine.begin(), mine.end(), g0 + gn) - mine.begin());
     return {team ? ctx->d_team : ctx->d_solo, a, b - a};

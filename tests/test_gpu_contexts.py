@@ -134,3 +134,27 @@ def test_boxes_of_a_batch(cuda):
             o = np.lexsort((lo, hi))
             assert np.array_equal(perm[off[j]:off[j + 1]] - off[j], o), j
             assert np.array_equal(keys[off[j]:off[j + 1]], hi[o]), j
+
+
+def test_one_kind_of_sort_after_another(cuda):
+    """A context holds the lists of its present sort and walks only: systems set one
+    after another for every kind (one block's keys, merges, one-sweep and scanned
+    radix passes, both walks) sort and walk as in a context of their own."""
+    from nns_gb300.barnes_hut import Context
+    runs = [[524289], [200], [1000, 40000], [1, 300, 524289, 5000], [30] * 64 + [20000], [1600000], [16384] * 3,
+            [600000, 900000, 100], [16385], [3, 5]]
+    whole = ic.plummer(1600000, seed=23)
+    one = Context(max_bodies=1600000, max_systems=65, theta=1.0, eps=0.1)
+    for sizes in runs:
+        off = np.concatenate([[0], np.cumsum(sizes)])
+        systems = [ic.Bodies(*(np.ascontiguousarray(getattr(whole, f)[a:e])
+                               for f in ("x", "y", "z", "vx", "vy", "vz", "m"))) for a, e in zip(off[:-1], off[1:])]
+        own = Context(max_bodies=int(off[-1]), max_systems=len(sizes), theta=1.0, eps=0.1)
+        got = []
+        for ctx in (one, own):
+            s = _build(ctx, systems)
+            ctx.forces(s)
+            ctx.sync()
+            got.append(ctx.export_keys() + (s.acc(),))
+        for u, v in zip(*got):
+            assert np.array_equal(u, v), sizes
