@@ -1144,13 +1144,16 @@ int build_tree(Ctx *ctx, const nbx_state *s, cudaStream_t st, bool external_bbox
     const int gn = ceil_div(ctx->cap_nodes, kBlock) < ctx->nsm * 8 ? ceil_div(ctx->cap_nodes, kBlock) : ctx->nsm * 8;
     // up to 2^21 bodies the 41 per-level launches cost more than the sums: one
     // bottom-up launch (2^16: 0.37 against 0.55 ms per build); above, the
-    // per-level launches stream the levels and are faster (a batch's chains are
-    // shorter: 200 systems, 3.2 x 10^6 bodies, 6.10 against 6.18 ms per step;
-    // with quadrupoles the one launch loses there, 3.04 against 2.86 ms per build)
+    // per-level launches stream the levels.  Batches of systems, whose chains are
+    // shorter and side by side, keep the one launch up to 2^22 bodies, and to 2^23
+    // where no system has more than 2^16: 4 systems of 10^6 1.40 against 1.42 ms,
+    // 800 of 4096 0.99 / 1.03, 250 of 32768 2.52 / 2.56, but 2 of 4 x 10^6 2.54 /
+    // 2.51 and 60 of 131072 2.53 / 2.48.  With quadrupoles it loses there (8 of 2^19
+    // 4.05 against 3.97 ms)
     const int mode = ctx->p.moments_mode;
     const bool quad = ctx->multipole != 0;
     if (quad && !ctx->d_m2) return NBX_ERR_STATE;
-    const int up_max = S > 1 && !quad ? 4 * kMomentsUpMaxBodies : kMomentsUpMaxBodies;
+    const int up_max = S == 1 || quad ? kMomentsUpMaxBodies : (ctx->max_sys <= 1 << 16 ? 4 : 2) * kMomentsUpMaxBodies;
     if (mode == 2 || (mode == 0 && n <= up_max)) {
         // one round of 32 nodes per warp until that fills the GPU's warps (a small
         // tree wants its chains started at once), then up to four (fuller groups)
