@@ -82,21 +82,23 @@ struct WarpBuf {
 };
 
 // The buffer variants: children per round and register budget.  0: 64 children;
-// 3: 128 (96 with quadrupoles, whose slots take more shared memory), both at 64
-// registers (two 16-warp or four 8-warp blocks per SM); 1: 128 at up to 85
-// registers, for more loads in flight (three 8-warp blocks).  Rounds of 128 pay
-// their fixed instructions less often than rounds of 96: 131071 bodies 1.69 ->
-// 1.63 ms for four steps, 2^24 155.4 -> 153.7 ms; with quadrupoles they cost an
-// eighth of the warps (700001 bodies 8.21 against 7.19 ms).
-template <int V, bool Quad>
+// 3: 128 (96 with quadrupoles and with split compensation), both at 64 registers
+// (two 16-warp or four 8-warp blocks per SM); 1: 128 at up to 85 registers, for
+// more loads in flight (three 8-warp blocks).  Rounds of 128 pay their fixed
+// instructions less often than rounds of 96: 131071 bodies 1.69 -> 1.63 ms for
+// four steps, 2^24 155.4 -> 153.7 ms.  With quadrupoles, whose slots take more
+// shared memory, they cost an eighth of the warps (700001 bodies 8.21 against 7.19
+// ms); split compensation (mode 1) sums plainly within a round, so a longer round
+// is a longer uncompensated sum.
+template <int V, int Mode, bool Quad>
 struct WalkShape {
-    static constexpr int kSlots = V == 0 ? 64 : (V == 3 && Quad ? 96 : 128);
+    static constexpr int kSlots = V == 0 ? 64 : (V == 3 && (Quad || Mode == 1) ? 96 : 128);
     static constexpr int kThreads = V != 1 ? NBX_WALK64_THREADS : NBX_WALK128_THREADS;
     static constexpr int kMinBlocks = V != 1 ? NBX_WALK64_MINB : NBX_WALK128_MINB;
 };
 
 template <int V, int Mode, bool Pot, bool Rec, bool Quad = false>
-__global__ void __launch_bounds__(WalkShape<V, Quad>::kThreads, WalkShape<V, Quad>::kMinBlocks)
+__global__ void __launch_bounds__(WalkShape<V, Mode, Quad>::kThreads, WalkShape<V, Mode, Quad>::kMinBlocks)
     k_walk2(const float4 *__restrict__ node4, const int *__restrict__ meta, const unsigned char *__restrict__ lvl8,
             const float4 *__restrict__ quad4, const float2 *__restrict__ quad2, const float4 *__restrict__ body4,
             const int *__restrict__ val, const int *__restrict__ groups, const int *__restrict__ list, int ngroups,
@@ -111,7 +113,7 @@ __global__ void __launch_bounds__(WalkShape<V, Quad>::kThreads, WalkShape<V, Qua
     if (st->code != 0) return;
     const int warps = blockDim.x >> 5;
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    constexpr int CB = WalkShape<V, Quad>::kSlots, kCB = CB;
+    constexpr int CB = WalkShape<V, Mode, Quad>::kSlots, kCB = CB;
     using Buf = WarpBuf<CB, Rec, Quad>;
     Buf &buf = reinterpret_cast<Buf *>(smem_raw)[w];
     constexpr size_t kQuadBytes = Quad ? sizeof(QuadBuf<CB>) : 0;
@@ -539,7 +541,7 @@ struct Share {
 template <int V, int Mode, bool Pot, bool Rec = false, bool Quad = false>
 int launch(Ctx *ctx, const nbx_state *s, float *pot, int warps, cudaStream_t st, Share share,
            int *rec_list = nullptr, int *rec_len = nullptr, int rec_cap = 0) {
-    constexpr int kCB = WalkShape<V, Quad>::kSlots;
+    constexpr int kCB = WalkShape<V, Mode, Quad>::kSlots;
     const int cap = ctx->p.stack_depth, asked = warps;
     const size_t smem = (size_t)warps * (sizeof(WarpBuf<kCB, Rec, Quad>) + (Quad ? sizeof(QuadBuf<kCB>) : 0) +
                                          (size_t)cap * sizeof(int));
