@@ -483,12 +483,11 @@ int nbx_set_systems(nbx_ctx *c, int nsys, const int64_t *offsets) {
     const int tile_sw = tile > nbx::kTileSweep ? tile : (nbx::kTileSweep < nbx::kTile ? nbx::kTileSweep : nbx::kTile);
     int max_sys = 0, nteam = 0, ngroups = 0;
     const auto bodies = [&](int s) { return (int)(offsets[s + 1] - offsets[s]); };
-    const auto by_team = [&](int s) { return bodies(s) <= nbx::kTeamMaxBodies; };
     for (int s = 0; s < nsys; s++) {
         max_sys = max_sys > bodies(s) ? max_sys : bodies(s);
         const int g = nbx::ceil_div(bodies(s), 32);
         ngroups += g;
-        if (by_team(s)) nteam += g;
+        if (nbx::by_team(bodies(s))) nteam += g;
     }
     // only the lists that this batch's sort and walks read are made
     const bool merge = nbx::sorts_by_merging(max_sys, n), sweep = !merge && n < nbx::kSweepMaxBodies;
@@ -519,7 +518,7 @@ int nbx_set_systems(nbx_ctx *c, int nsys, const int64_t *offsets) {
     groups.reserve(ngroups);
     for (int s = 0; s < nsys; s++)
         for (int g = off[s]; g < off[s + 1]; g += 32) {
-            if (mixed) (by_team(s) ? team : solo).push_back((int)groups.size());
+            if (mixed) (nbx::by_team(bodies(s)) ? team : solo).push_back((int)groups.size());
             groups.push_back(g);
         }
     if (merge) {
@@ -868,6 +867,7 @@ int nbx_sync_status(nbx_ctx *c, void *stream) {
         ctx->last_error = buf;
         int zero[2] = {0, 0};
         NBX_CUDA(cudaMemcpy(ctx->d_status, zero, sizeof(zero), cudaMemcpyHostToDevice));
+        NBX_CUDA(cudaMemcpy(&ctx->d_status->walk_next, zero, sizeof(unsigned), cudaMemcpyHostToDevice));
         // the tree of a step that reported an error may be inconsistent: it is
         // never walked again, the next walk needs a new build
         ctx->built = false;

@@ -68,18 +68,24 @@ inline bool sorts_by_merging(int max_sys, int n) {
 #define NBX_RADIX_SWEEP_MAX (3 << 19)
 #endif
 constexpr int kSweepMaxBodies = NBX_RADIX_SWEEP_MAX;
-// Systems of up to this many bodies are walked by teams of warps (walk_team.cu).
-// The rule sees a system's own size only, so that a batch gives every system the
-// bits of its single run.  Alone, teams win up to about 2^17 bodies (walk at 2^16:
-// 148 against 193 us, at 2^17 240 against 305); in a batch that fills the GPU they
-// cost 10 % more than single warps (400 systems of 2^11 to 2^16 bodies, walk 11.2
-// against 10.0 ms), which outweighs what the build gained once large systems are
-// in.  At 2^14 a system alone gains most (70 against 212 us) and batches of any
-// sizes stay ahead.
+// Systems of these sizes are walked by teams of warps (walk_team.cu), others by
+// single warps (walk2.cu).  The rule sees a system's own size only, so that a batch
+// gives every system the bits of its single run.  Alone, teams win up to about 2^17
+// bodies (walk at 2^16: 148 against 193 us, at 2^17 240 against 305); in a batch
+// that fills the GPU they cost more than single warps (400 systems of 2^11 to 2^16
+// bodies, walk 11.2 against 10.0 ms), which outweighs what the build gained once
+// large systems are in.  At 2^14 a system alone gains most (70 against 212 us).
+// Systems of up to 256 bodies have a few rounds of a few cells: alone they take
+// about as long either way (a step of 256 bodies 58 us by single warps, 54 by
+// teams), and a full batch takes a fraction (65536 systems of 128 bodies, walk 1.04
+// against 2.51 ms; 32768 of 256 1.55 against 2.95).
 #ifndef NBX_TEAM_MAX
 #define NBX_TEAM_MAX (1 << 14)
 #endif
-constexpr int kTeamMaxBodies = NBX_TEAM_MAX;
+#ifndef NBX_TEAM_MIN
+#define NBX_TEAM_MIN 257
+#endif
+inline bool by_team(int bodies) { return bodies >= NBX_TEAM_MIN && bodies <= NBX_TEAM_MAX; }
 constexpr int kMaxRadixBits = 9;  // body-key digits: 8 or 9 bits (histograms sized for 9)
 // LSD passes over the 63-bit body keys for a digit width
 constexpr int radix_passes(int bits) { return (63 + bits - 1) / bits; }
@@ -104,7 +110,8 @@ struct DevStatus {
     unsigned long long opened;
     unsigned long long rounds;      // walk expand/evaluate rounds (production walk)
     unsigned long long candidates;  // candidates evaluated by the production walk
-    unsigned walk_next;             // next group of the production walk (cleared per launch)
+    unsigned walk_next;             // next group of the single-warp walk (zero between launches; cleared
+                                    // with an error, which may have stopped some of its warps)
 };
 
 struct Ctx {
@@ -151,8 +158,8 @@ struct Ctx {
     int max_sys = 0;                // bodies of the largest system
     int *d_groups = nullptr;        // [G] first sorted position of each walk group
 
-    // walk groups of systems of up to kTeamMaxBodies bodies (walked by teams of
-    // warps): their number, and in a batch of both kinds the groups of each, ascending
+    // walk groups that are walked by teams (by_team): their number, and in a batch of
+    // both kinds the groups of each, ascending
     int nteam = 0;
     std::vector<int> h_team, h_solo;
     int *d_team = nullptr, *d_solo = nullptr;  // [G] together

@@ -123,12 +123,16 @@ __global__ void __launch_bounds__(WalkShape<V, Mode, Quad>::kThreads, WalkShape<
     const u64 eps2x2 = pk(eps2, eps2);
     unsigned long long tot_len = 0ull, tot_open = 0ull, tot_rounds = 0ull, tot_cand = 0ull;
 
-    // groups are handed out dynamically (costs vary widely between groups)
+    // groups are handed out dynamically (costs vary widely between groups); the last
+    // warp to find none left leaves the counter at zero for the next launch
     for (;;) {
         int g = 0;
         if (lane == 0) g = (int)atomicAdd(&st->walk_next, 1u);
         g = __shfl_sync(0xffffffffu, g, 0);
-        if (g >= ngroups) break;
+        if (g >= ngroups) {
+            if (lane == 0 && g - ngroups == (int)gridDim.x * warps - 1) st->walk_next = 0u;
+            break;
+        }
         if (list) g = list[g];
         const int p0 = groups[g];
         const int s = body_sys[p0];
@@ -562,8 +566,10 @@ int launch(Ctx *ctx, const nbx_state *s, float *pot, int warps, cudaStream_t st,
     const int grid = blocks_needed < ctx->nsm * per_sm ? blocks_needed : ctx->nsm * per_sm;
     // without a list the group arrays start at the first group
     const int off = share.list ? 0 : share.first;
-    NBX_CUDA(cudaMemsetAsync(&ctx->d_status->walk_next, 0, sizeof(unsigned), st));
-    ctx->chain = false;  // (a memory operation came between)
+    // in plain stream order: blocks that are placed while the build's last kernel still
+    // holds some of the SMs fill the others, and the walk lasts as long as the fullest
+    // (an eager step of 65536 bodies 396 against 287 us)
+    ctx->chain = false;
     launch_chained(
         ctx, st, grid, warps * 32, block_smem, k_walk2<V, Mode, Pot, Rec, Quad>,
         ctx->d_node4, ctx->d_meta, ctx->d_lvl8, ctx->d_quad4, ctx->d_quad2, ctx->d_body4, ctx->d_val,

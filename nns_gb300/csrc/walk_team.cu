@@ -16,7 +16,7 @@
 // The tests, and so the lists, are those of walk2.cu; the sums are the W warps'
 // partial sums added in warp order, so a group's force bits depend on its own
 // system only.  Which systems are walked by teams depends on the system's size
-// alone (kTeamMaxBodies): a batch gives every system the bits of its single run.
+// alone (by_team): a batch gives every system the bits of its single run.
 //
 // Bound by latency where the GPU is not full (16384 bodies: 2.9 warps and 0.35
 // instructions per scheduler and cycle), else by issue like walk2.cu, at 9 % more

@@ -37,12 +37,13 @@ def _stepped(ctx, b):
     return s.host() + (s.acc(),)
 
 
-def test_full_lists_are_reported(cuda):
+@pytest.mark.parametrize("sizes", [[4000] * 24, [20000] * 12], ids=["teams", "single-warps"])
+def test_full_lists_are_reported(cuda, sizes):
     import torch
     from nns_gb300._lib import NbxError
     from nns_gb300.adjoint import Adjoint
     from nns_gb300.barnes_hut import State
-    b, off = _batch([4000] * 24)  # 3000 groups
+    b, off = _batch(sizes)  # 3000 and 7500 groups
     ctx = _context(off)
     target = torch.zeros(3, int(off[-1]), device="cuda")
     adj = Adjoint(ctx, 3, 1, 64)
