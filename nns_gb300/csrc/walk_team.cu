@@ -90,6 +90,18 @@ static_assert(sizeof(TeamShared) % 16 == 0 && sizeof(TeamBuf<false, false>) % 16
                   sizeof(TeamBuf<true, false>) % 16 == 0 && sizeof(TeamBuf<false, true>) % 16 == 0,
               "16-byte slots");
 
+// Minimum and maximum over a warp of finite values (one instruction each).
+__device__ __forceinline__ float warp_min(float v) {
+    float r;
+    asm volatile("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+    return r;
+}
+__device__ __forceinline__ float warp_max(float v) {
+    float r;
+    asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+    return r;
+}
+
 __device__ __forceinline__ u64 entry_of(int cm, int lvl) { return (u64)(unsigned)cm | (u64)(unsigned)lvl << 32; }
 
 template <int Mode, bool Pot, bool Rec, bool Quad>
@@ -133,15 +145,8 @@ __global__ void __launch_bounds__(kW * 32, 32 / kW)
     {
         // the group's box and, per octant, its representative pair (walk2.cu): warp w
         // finds the octants w, w + W
-        float b[6] = {me.x, me.x, me.y, me.y, me.z, me.z};
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-#pragma unroll
-            for (int k = 0; k < 6; k += 2) {
-                b[k] = fminf(b[k], __shfl_xor_sync(0xffffffffu, b[k], o));
-                b[k + 1] = fmaxf(b[k + 1], __shfl_xor_sync(0xffffffffu, b[k + 1], o));
-            }
-        }
+        const float b[6] = {warp_min(me.x), warp_max(me.x), warp_min(me.y),
+                            warp_max(me.y), warp_min(me.z), warp_max(me.z)};
         const float ex = me.x - 0.5f * (b[0] + b[1]), ey = me.y - 0.5f * (b[2] + b[3]);
         const float ez = me.z - 0.5f * (b[4] + b[5]);
         const unsigned key = __float_as_uint(ex * ex + ey * ey + ez * ez);
@@ -199,56 +204,65 @@ __global__ void __launch_bounds__(kW * 32, 32 / kW)
     __syncthreads();
 
     for (bool first_round = true; top > 0 || first_round; first_round = false) {
-        // ---- expand: lane j of warp 0 pops the kPops entries from stack[top-1-kPops*j]
-        // down and lists their children; P = the most top-of-stack cells that fit
+        // ---- expand: warp 0 pops and lists the children; P = the most top-of-stack
+        // cells that fit.  Lane j takes the K entries from stack[top-1-K*j] down: one
+        // where that is all of the stack, else four (the list is the same; four always
+        // are three times the instructions: 16384 systems of 512 bodies 3.78 -> 3.62
+        // ms, 8388 of 1000 4.63 -> 4.46; a third form for two gained nothing and cost
+        // 512 systems of 16384 5 %: 10.76 -> 11.34 ms)
         if (w == 0) {
             const int avail = min(top, 32 * kPops);
-            u64 e[kPops];
-            int n[kPops], x[kPops + 1];
-            x[0] = 0;
+            const auto pop = [&](auto entries) {
+                constexpr int K = decltype(entries)::value;
+                u64 e[K];
+                int n[K], x[K + 1];
+                x[0] = 0;
 #pragma unroll
-            for (int i = 0; i < kPops; i++) {
-                const int at = kPops * lane + i;
-                e[i] = at < avail ? stack[top - 1 - at] : 0ull;
-                n[i] = at < avail ? (((int)(unsigned)e[i] >> 28) & 7) + 1 : 0;
-                x[i + 1] = x[i] + n[i];
-            }
-            int incl = x[kPops];
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int u = __shfl_up_sync(0xffffffffu, incl, o);
-                if (lane >= o) incl += u;
-            }
-            const int excl = incl - x[kPops];  // children before this lane's cells
-            int np = 0, nt = 0;
-#pragma unroll
-            for (int i = 0; i < kPops; i++)
-                if (n[i] > 0 && excl + x[i + 1] <= kRound) {
-                    np = i + 1;
-                    nt = excl + x[i + 1];
+                for (int i = 0; i < K; i++) {
+                    const int at = K * lane + i;
+                    e[i] = at < avail ? stack[top - 1 - at] : 0ull;
+                    n[i] = at < avail ? (((int)(unsigned)e[i] >> 28) & 7) + 1 : 0;
+                    x[i + 1] = x[i] + n[i];
                 }
-            int P = __reduce_add_sync(0xffffffffu, np);
-            int T = __reduce_max_sync(0xffffffffu, nt);
-            // wide rounds only while the stack keeps the depth-first reserve free (walk2.cu)
-            if (P > 1 && top - P + T > stack_cap - reserve) {
-                P = 1;
-                T = __shfl_sync(0xffffffffu, n[0], 0);
-            }
-            if (P > 0 && top - P + T > stack_cap) P = 0;
-            if (P == 0) T = 0;
-            if (lane == 0) {
-                sh.P = P;
-                sh.T = T;
-            }
+                int incl = x[K];
 #pragma unroll
-            for (int i = 0; i < kPops; i++)
-                if (kPops * lane + i < P) {
-                    const int first = (int)(unsigned)e[i] & 0x0fffffff, at = excl + x[i];
-                    const u64 lvl = e[i] & 0xffffffff00000000ull;
-#pragma unroll
-                    for (int k = 0; k < 8; k++)
-                        if (k < n[i]) sh.child[at + k] = lvl | (unsigned)(first + k);
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int u = __shfl_up_sync(0xffffffffu, incl, o);
+                    if (lane >= o) incl += u;
                 }
+                const int excl = incl - x[K];  // children before this lane's cells
+                int np = 0, nt = 0;
+#pragma unroll
+                for (int i = 0; i < K; i++)
+                    if (n[i] > 0 && excl + x[i + 1] <= kRound) {
+                        np = i + 1;
+                        nt = excl + x[i + 1];
+                    }
+                int P = __reduce_add_sync(0xffffffffu, np);
+                int T = __reduce_max_sync(0xffffffffu, nt);
+                // wide rounds only while the stack keeps the depth-first reserve free (walk2.cu)
+                if (P > 1 && top - P + T > stack_cap - reserve) {
+                    P = 1;
+                    T = __shfl_sync(0xffffffffu, n[0], 0);
+                }
+                if (P > 0 && top - P + T > stack_cap) P = 0;
+                if (P == 0) T = 0;
+                if (lane == 0) {
+                    sh.P = P;
+                    sh.T = T;
+                }
+#pragma unroll
+                for (int i = 0; i < K; i++)
+                    if (K * lane + i < P) {
+                        const int first = (int)(unsigned)e[i] & 0x0fffffff, at = excl + x[i];
+                        const u64 lvl = e[i] & 0xffffffff00000000ull;
+#pragma unroll
+                        for (int k = 0; k < 8; k++)
+                            if (k < n[i]) sh.child[at + k] = lvl | (unsigned)(first + k);
+                    }
+            };
+            if (avail <= 32) pop(std::integral_constant<int, 1>());
+            else pop(std::integral_constant<int, kPops>());
         }
         __syncthreads();
         const int P = sh.P, T = sh.T;
