@@ -323,7 +323,10 @@ int nbx_diagnostics_fp64(nbx_ctx *ctx, const nbx_state *s, int n, double *out, v
  * it into a context (capacity permitting) sets the systems, constants, walk
  * configuration, multipole order and leaf size and copies the bodies into the
  * caller's device state, so that the run continues bit for bit.  The sort's
- * digit width changes no result and is not recorded. */
+ * digit width changes no result and is not recorded.  A checkpoint also holds the
+ * revision of the walk's order of summation: one written by a library with another
+ * is restored all the same, and nbx_last_error then says that the run does not
+ * continue bit for bit (it is empty after any other restore). */
 int64_t nbx_checkpoint_bytes(int64_t nbodies, int nsystems);
 /* Synchronises `stream`; *written receives the bytes used. */
 int nbx_checkpoint_save(nbx_ctx *ctx, const nbx_state *s, void *host, int64_t capacity, int64_t *written,

@@ -15,6 +15,7 @@ Device memory is held in torch tensors; every computation runs in libnbx.so.
 from __future__ import annotations
 
 import ctypes as C
+import warnings
 from dataclasses import dataclass
 
 import numpy as np
@@ -270,10 +271,15 @@ class Context:
         return buf[: written.value]
 
     def restore(self, s: "State", buf, stream=None) -> None:
-        """Restores a checkpoint into this context (systems, constants) and s (bodies)."""
+        """Restores a checkpoint into this context (systems, constants) and s (bodies).
+        Warns where it was written by a library whose walk sums in another order: the
+        run then does not continue bit for bit."""
         b = np.ascontiguousarray(np.frombuffer(buf, np.uint8) if not isinstance(buf, np.ndarray) else buf, np.uint8)
         check(lib().nbx_checkpoint_restore(self.h, C.byref(s.c), b.ctypes.data_as(C.c_void_p), b.size,
                                            _stream_ptr(stream)), "nbx_checkpoint_restore", self.h)
+        note = lib().nbx_last_error(self.h)
+        if note:
+            warnings.warn(note.decode(), RuntimeWarning, stacklevel=2)
         nsys = int(np.frombuffer(b[12:16].tobytes(), np.int32)[0])
         self.offsets = [int(v) for v in np.frombuffer(b[80:80 + 8 * (nsys + 1)].tobytes(), np.int64)]
 

@@ -6,7 +6,8 @@
 //            the walk's launch shape, buffer variant and stack depth (the
 //            buffer width and the stack depth set how the walk's rounds group
 //            the candidates, i.e. the order of the force sums, so a bit-exact
-//            resume needs them), the multipole order and the leaf bucket size,
+//            resume needs them), the multipole order and the leaf bucket size, the
+//            revision of the walks' order of summation (kWalkRevision),
 //            FNV-1a 64 of the header bytes before it and of the offsets
 //   int64    offsets[nsys + 1]
 //   float    x, y, z, vx, vy, vz, m   [nbodies] each
@@ -34,7 +35,7 @@ struct CkptHeader {
     int32_t compensated, key_order;
     int32_t walk_warps, walk_variant;
     int32_t multipole, leaf_size;
-    int32_t stack_depth, reserved;
+    int32_t stack_depth, walk_revision;  // (0 in files from before the revisions were stored)
     uint64_t header_hash;  // of the bytes above and of the offsets
 };
 static_assert(sizeof(CkptHeader) == 80, "checkpoint header layout");
@@ -120,6 +121,7 @@ extern "C" int nbx_checkpoint_save(nbx_ctx *c, const nbx_state *s, void *host, i
     h.multipole = ctx->multipole;
     h.leaf_size = ctx->leaf_size;
     h.stack_depth = ctx->p.stack_depth;
+    h.walk_revision = nbx::kWalkRevision;
     h.header_hash = nbx::header_hash(h, offs, nsys);
     std::memcpy(out, &h, sizeof(h));
     const uint64_t sum = nbx::payload_sum(payload, (size_t)nbx::kArrays * n);
@@ -181,6 +183,10 @@ extern "C" int nbx_checkpoint_restore(nbx_ctx *c, nbx_state *s, const void *host
     if (rc) return rc;
     ctx->p.dt = h.dt;
     ctx->p.dampening = h.dampening;
+    ctx->last_error.clear();
+    if (h.walk_revision != nbx::kWalkRevision)
+        ctx->last_error = "checkpoint: written by a library whose walk sums the forces in another order; "
+                          "the run continues from the same state, but not bit for bit";
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     for (int k = 0; k < nbx::kArrays; k++)
         NBX_CUDA(cudaMemcpyAsync(arr[k], payload + (size_t)k * n, sizeof(float) * n, cudaMemcpyHostToDevice, st));

@@ -86,6 +86,10 @@ constexpr int kSweepMaxBodies = NBX_RADIX_SWEEP_MAX;
 #define NBX_TEAM_MIN 257
 #endif
 inline bool by_team(int bodies) { return bodies >= NBX_TEAM_MIN && bodies <= NBX_TEAM_MAX; }
+// Revision of the walks' order of summation, which checkpoints store: raised by every
+// change after which the same bodies and settings give other force bits.  (1: teams,
+// rounds of 128 children in the default single-warp walk.)
+constexpr int kWalkRevision = 1;
 constexpr int kMaxRadixBits = 9;  // body-key digits: 8 or 9 bits (histograms sized for 9)
 // LSD passes over the 63-bit body keys for a digit width
 constexpr int radix_passes(int bits) { return (63 + bits - 1) / bits; }
