@@ -70,12 +70,19 @@ typedef struct nbx_params {
                           holds more is a leaf with its bodies as children (fewer cells, longer
                           lists; trees and lists differ from the reference's, nbx_export_tree
                           refuses them).  Not available with the adjoint */
-    int radix_bits;    /* radix digit width of the key sort: 8 (8 passes) or 9 (7 passes) */
-    int walk_warps;    /* warps per block of the walk kernel (0 = autotuned default) */
+    int radix_bits;    /* radix digit width of the key sort: 8 (8 passes) or 9 (7 passes); acts
+                          where a system has more than 2^19 bodies, and in batches of 2^21
+                          and more of systems above 4096 (others sort by merging) */
+    int walk_warps;    /* warps per block of the walk kernel (0: 8), for systems of more than
+                          2^14 bodies (and up to 256) whose groups are more than 32 per SM;
+                          fewer go out in blocks of two warps */
     int device;        /* CUDA device ordinal */
     int block_size;    /* reference launch-shape hints (main.cu:30-31); informational */
     int grid_size;
-    int walk_variant;  /* 0 production walk, 64-slot candidate buffers; 1 the same with
+    int walk_variant;  /* the walk by single warps, of systems of more than 2^14 bodies (and
+                          up to 256); those between are walked by teams of four warps in
+                          every variant but 2:
+                          0 production walk, 64-slot candidate buffers; 1 the same with
                           128-slot buffers; 2 one-cell-at-a-time walk (comparison);
                           3 production walk, 128-slot buffers (96 with quadrupoles
                           or split compensation) at a smaller register budget */
@@ -84,10 +91,11 @@ typedef struct nbx_params {
                           are compact but the interaction lists differ from the reference */
     int node_capacity; /* node pool (cells + bodies); 0: 2*max_bodies + 65536.  A tree that
                           needs more nodes reports NBX_ERR_CAPACITY */
-    int moments_mode;  /* centre-of-mass pass: 0 by size (one launch up to 2^21 bodies,
-                          in batches up to 2^22 or 2^23; per level above); 1 one launch per tree level; 2 one launch in
-                          which the last child to finish sums its parent.  The sums are
-                          the same FP64 additions in the same order in every mode */
+    int moments_mode;  /* centre-of-mass pass: 0 by size (one launch up to 2^21 bodies, in
+                          batches up to 2^22 or 2^23; per level above); 1 one launch per
+                          tree level; 2 one launch in which the last child to finish sums
+                          its parent.  The sums are the same FP64 additions in the same
+                          order in every mode */
     int multipole;     /* 0: monopoles, the reference's force (Kernels.cu:538-551; the parity
                           mode); 1: monopoles plus the traceless quadrupole of every accepted
                           cell (FP64 second moments, FP32 terms).  The interaction lists are
@@ -129,11 +137,12 @@ const char *nbx_last_error(nbx_ctx *ctx);
  * eps2 >= FLT_MIN (NBX_ERR_ARG otherwise). */
 int nbx_get_constants(nbx_ctx *ctx, float *theta_ref, float *eps2);
 int nbx_set_constants(nbx_ctx *ctx, float theta_ref, float eps2, int compensated);
-/* Launch shape of the walk: warps per block (4, 8 or 16) and variant; used by
- * the autotuner (nns_gb300/autotune.py). */
+/* Launch shape of the walk: warps per block (4, 8 or 16) and variant (see
+ * nbx_params.walk_warps and walk_variant for the systems on which they act); used
+ * by the autotuner (nns_gb300/autotune.py). */
 int nbx_set_walk_config(nbx_ctx *ctx, int warps_per_block, int variant);
-/* Sort digit width (8: 8 passes, 9: 7 passes over the 63-bit keys; both give the
- * same stable order) and walk stack entries per warp (360..4096; a launch whose
+/* Sort digit width (8: 8 passes, 9: 7 passes over the 63-bit keys, where the keys
+ * sort by radix: nbx_params.radix_bits; both give the same stable order) and walk stack entries per warp (360..4096; a launch whose
  * stacks and buffers exceed the device's shared memory per block fails with
  * NBX_ERR_ARG).  The stack depth never changes the interaction lists, but it
  * sets how the walk groups candidates into rounds near the depth-first reserve,

@@ -17,8 +17,14 @@ lists (and the error), so the default offers only one body per leaf.
 Candidates are timed with CUDA events on the caller's workload after one
 build, in that order, each stage with the winners of the stages before it
 (leaf sizes first, over whole build + walk steps); the winner is applied to
-the context and cached per (device, n, systems, modes) in
+the context and cached per (device, n, systems, modes, kernels) in
 ``~/.cache/nbx_autotune.json`` (override with NBX_AUTOTUNE_CACHE).
+
+Not every knob acts on every workload: systems of 257 to 2^14 bodies are walked
+by teams of fixed shape, launches of up to 32 groups per SM take blocks of two
+warps, and systems of up to 2^19 bodies sort by merging (include/nbx.h).  Where
+one does nothing its candidates differ by noise, so a candidate takes the place
+of its stage's first, the default, only when it is faster by MARGIN.
 """
 from __future__ import annotations
 
@@ -32,6 +38,8 @@ from ._lib import NbxError
 CANDIDATES = ((8, 3), (16, 3), (4, 3), (8, 0), (16, 0), (8, 1), (4, 1))
 STACK_DEPTHS = (512, 384, 768)
 RADIX_BITS = (8, 9)
+MARGIN = 0.02
+KERNELS = 1  # raised when the kernels that the knobs shape change: older results are not reused
 
 
 def _cache_path():
@@ -42,8 +50,8 @@ def _cache_path():
 def _key(ctx, n):
     name = torch.cuda.get_device_name(ctx.device)
     nsys = 1 if ctx.offsets is None else len(ctx.offsets) - 1
-    return "%s|n=%d|sys=%d|comp=%d|order=%d|moments=%d|multipole=%d" % (
-        name, n, nsys, int(ctx.params.compensated), int(ctx.params.key_order), int(ctx.params.moments_mode),
+    return "%s|kernels=%d|n=%d|sys=%d|comp=%d|order=%d|moments=%d|multipole=%d" % (
+        name, KERNELS, n, nsys, int(ctx.params.compensated), int(ctx.params.key_order), int(ctx.params.moments_mode),
         int(getattr(ctx.params, "multipole", 0)))
 
 
@@ -60,9 +68,15 @@ def _time(fn, reps):
     return ev0.elapsed_time(ev1) / reps
 
 
+def _fastest(times):
+    """The key of the fastest entry; the first one's unless beaten by MARGIN."""
+    first, best = next(iter(times)), min(times, key=times.get)
+    return best if times[best] < (1.0 - MARGIN) * times[first] else first
+
+
 def tune_walk(ctx, state, reps: int = 2, candidates=CANDIDATES, use_cache: bool = True,
               stack_depths=STACK_DEPTHS, radix_bits=RADIX_BITS, timer=None, leaf_sizes=None) -> dict:
-    """Times the candidate configurations and applies the fastest.  ``timer(fn,
+    """Times the candidate configurations and applies the fastest (_fastest).  ``timer(fn,
     reps)`` returns milliseconds per call (CUDA events by default).
     ``leaf_sizes`` (None: keep the context's) are leaf bucket sizes to try."""
     timer = timer or _time
@@ -97,7 +111,7 @@ def tune_walk(ctx, state, reps: int = 2, candidates=CANDIDATES, use_cache: bool 
                 ctx.forces(state)
             ltimes[str(int(k))] = timer(step, reps)
         ctx.sync()
-        ctx.set_leaf_size(int(min(ltimes, key=ltimes.get)))
+        ctx.set_leaf_size(int(_fastest(ltimes)))
     ctx.build(state)
     ctx.sync()
     # 1. walk launch shape
@@ -106,7 +120,7 @@ def tune_walk(ctx, state, reps: int = 2, candidates=CANDIDATES, use_cache: bool 
         ctx.set_walk(warps, variant)
         times["%d/%d" % (warps, variant)] = timer(lambda: ctx.forces(state), reps)
     ctx.sync()
-    wbest = min(times, key=times.get)
+    wbest = _fastest(times)
     warps, variant = (int(v) for v in wbest.split("/"))
     ctx.set_walk(warps, variant)
     # 2. stack depth with that shape (a depth whose stacks do not fit the
@@ -119,14 +133,14 @@ def tune_walk(ctx, state, reps: int = 2, candidates=CANDIDATES, use_cache: bool 
         except NbxError:
             continue
     ctx.sync()
-    depth = int(min(stimes, key=stimes.get)) if stimes else depth0
+    depth = int(_fastest(stimes)) if stimes else depth0
     # 3. sort digit width, timed over whole builds
     btimes = {}
     for bits in radix_bits:
         ctx.set_tuning(bits, depth)
         btimes[str(bits)] = timer(lambda: ctx.build(state), reps)
     ctx.sync()
-    bits = int(min(btimes, key=btimes.get))
+    bits = int(_fastest(btimes))
     ctx.set_tuning(bits, depth)
     ctx.build(state)
     best = {"warps": warps, "variant": variant, "stack_depth": depth, "radix_bits": bits,
