@@ -62,3 +62,138 @@ def test_batches_where_the_walks_change(cuda, n):
         rel = np.linalg.norm(s1.acc() - f.a, axis=1) / np.maximum(np.linalg.norm(f.a, axis=1), 1e-30)
         if sizes[j] > 1:
             assert np.median(rel) <= MED_TOL and rel.max() <= MAX_TOL, j
+
+
+def _rel(a, b):
+    a, b = np.asarray(a, np.float64), np.asarray(b, np.float64)
+    return np.linalg.norm(a - b, axis=1) / np.maximum(np.linalg.norm(b, axis=1), 1e-30)
+
+
+def _walk(b, variant=3, warps=8, eps=0.01, **kw):
+    from nns_gb300.barnes_hut import Context, State
+    n = len(b.x)
+    ctx = Context(max_bodies=n, theta=0.5, eps=eps, **kw)
+    ctx.set_walk(warps, variant)
+    ctx.set_systems([0, n])
+    s = State.from_bodies(b)
+    ctx.build(s)
+    ctx.forces(s)
+    ctx.sync()
+    return ctx, s
+
+
+BODIES = {"disk20011": lambda: ic.star_disk(20011), "plummer16385": lambda: ic.plummer(16385),
+          "binary160033": lambda: ic.binary_disk(160033)}  # the last: more than 32 groups per SM
+_cache = {}
+
+
+def _want(name, leaf, multipole, eps=0.01):
+    key = (name, leaf, multipole)
+    if key not in _cache:
+        b = BODIES[name]()
+        t = O.build(b.x, b.y, b.z, b.m)
+        q = O.quadrupoles(b.x, b.y, b.z, b.m, t) if multipole else None
+        e = np.float32(eps)
+        _cache[key] = b, O.forces(b.x, b.y, b.z, b.m, O.bucket_tree(t, leaf) if leaf > 1 else t, 0.25, float(e * e),
+                                  quad=q)
+    return _cache[key]
+
+
+@pytest.mark.parametrize("name,leaf,multipole", [("disk20011", 1, 0), ("disk20011", 1, 1), ("disk20011", 4, 0),
+                                                 ("disk20011", 4, 1), ("plummer16385", 1, 0), ("plummer16385", 1, 1),
+                                                 ("binary160033", 1, 0), ("binary160033", 1, 1)])
+@pytest.mark.parametrize("variant", [0, 1, 2, 3])
+def test_every_form_matches_oracle(cuda, name, leaf, multipole, variant):
+    """The accumulation modes of every variant (the one-cell walk has no quadrupoles)
+    on the oracle's lists, within the walk tests' bounds of its FP64 sums."""
+    if variant == 2 and multipole:
+        pytest.skip("the one-cell walk has monopoles only")
+    b, f = _want(name, leaf, multipole)
+    for comp in (0, 1, 2):
+        ctx, s = _walk(b, variant, leaf_size=leaf, multipole=multipole, compensated=comp)
+        nl, no = ctx.walk_stats()
+        assert np.array_equal(nl, f.nlist) and np.array_equal(no, f.nopen), comp
+        rel = _rel(s.acc(), f.a64)
+        assert np.median(rel) <= MED_TOL and rel.max() <= MAX_TOL, (comp, np.median(rel), rel.max())
+
+
+@pytest.mark.parametrize("n", [20011, 160033])
+@pytest.mark.parametrize("variant", [0, 1, 3])
+@pytest.mark.parametrize("multipole", [0, 1])
+def test_launch_shapes_agree(cuda, n, variant, multipole):
+    """Blocks of two warps (a launch that fits the GPU at once) and of the asked 4, 8
+    and 16: the same bits."""
+    b = ic.plummer(n)
+    out = [_walk(b, variant, warps, multipole=multipole)[1].acc() for warps in (4, 8, 16)]
+    assert np.array_equal(out[0], out[1]) and np.array_equal(out[0], out[2])
+
+
+def test_potential(cuda):
+    b = ic.plummer(20011)
+    ctx, s = _walk(b)
+    phi = ctx.potential(s)
+    e = np.float32(0.01)
+    tg = np.arange(0, 20011, 7)
+    want = O.direct_potential_fp64(b.x, b.y, b.z, b.m, float(e * e), tg)
+    rel = np.abs(phi[tg] - want) / np.abs(want)
+    assert np.median(rel) < 1e-3 and rel.max() < 2e-2  # the monopole potential's bounds of the parity tests
+
+
+@pytest.mark.parametrize("name", ["collinear", "coplanar", "signed_zeros", "cluster", "deep"])
+@pytest.mark.parametrize("variant", [0, 1, 3])
+@pytest.mark.parametrize("multipole", [0, 1])
+def test_adversarial_geometry(cuda, name, variant, multipole):
+    """The adversarial sets with enough bodies for the walk by single warps: lists
+    bit-exact, each body's error bounded relative to its own force plus the set's
+    median force (pulls that nearly cancel on a line or in a plane)."""
+    from adversarial import CASES, EPS
+    key = (name, multipole)
+    eps = EPS.get(name, 0.01)
+    if key not in _cache:
+        b = CASES[name](24000)
+        assert len(b.x) > 1 << 14
+        t = O.build(b.x, b.y, b.z, b.m)
+        q = O.quadrupoles(b.x, b.y, b.z, b.m, t) if multipole else None
+        e = np.float32(eps)
+        _cache[key] = b, O.forces(b.x, b.y, b.z, b.m, t, 0.25, float(e * e), quad=q)
+    b, f = _cache[key]
+    ctx, s = _walk(b, variant, eps=eps, multipole=multipole)
+    nl, no = ctx.walk_stats()
+    assert np.array_equal(nl, f.nlist) and np.array_equal(no, f.nopen)
+    a = s.acc().astype(np.float64)
+    err, mag = np.linalg.norm(a - f.a64, axis=1), np.linalg.norm(f.a64, axis=1)
+    assert np.median(_rel(a, f.a64)) <= MED_TOL
+    assert (err <= MAX_TOL * (mag + np.median(mag))).all(), (err / (mag + np.median(mag))).max()
+
+
+def test_the_adjoint_records_this_walk(cuda):
+    """The trajectory gradients of a system above the teams' size: the forward ends bit
+    for bit where ordinary steps end, and the gradients agree with FP64 central
+    finite differences of the FP64 replay (bound of the adjoint tests)."""
+    import torch
+    from nns_gb300.adjoint import Adjoint, random_directions
+    from nns_gb300.barnes_hut import Context, State
+    n, T = 20011, 5
+    b = ic.plummer(n, seed=ic.SEED0 + 3)
+    ctx = Context(max_bodies=n, theta=0.5, eps=0.01, dt=1e-3)
+    ctx.set_systems([0, n])
+    s = State.from_bodies(b)
+    ctx.step(s, T)
+    ctx.sync()
+    end = s.host()
+    noise = 0.01 * np.random.default_rng(3).standard_normal((3, n))
+    target = torch.as_tensor((np.stack(end[:3]) + noise).astype(np.float32), device="cuda")
+    adj = Adjoint(ctx, T, 2, 8192, T)
+    r = State.from_bodies(b)
+    loss32 = adj.forward(r, target)
+    for got, want in zip(r.host(), end):
+        assert np.array_equal(got, want)
+    g = np.concatenate([t.cpu().numpy().reshape(-1, n) for t in adj.backward(r)]).astype(np.float64)
+    adj.record(State.from_bodies(b))
+    base = np.stack([b.x, b.y, b.z, b.vx, b.vy, b.vz, b.m]).astype(np.float64)
+    dev = lambda a: torch.as_tensor(a, device="cuda")  # noqa: E731
+    assert abs(adj.replay_fp64(dev(base)) - loss32) / loss32 < 1e-4
+    h, gnorm = 1e-6, np.linalg.norm(g)
+    for u in random_directions(n, 4):
+        fd = (adj.replay_fp64(dev(base + h * u)) - adj.replay_fp64(dev(base - h * u))) / (2 * h)
+        assert abs(fd - float((g * u).sum())) <= 1e-4 * gnorm
