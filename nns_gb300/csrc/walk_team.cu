@@ -7,7 +7,7 @@
 // evaluate up to 96 candidates: about 2.4 us) is the walk's time.  Here every
 // warp holds the same 32 bodies and takes its own share of a round's children:
 //   expand   warp 0 pops the top-of-stack cells (the shared stack holds each cell's
-//            record and level, so a pop loads nothing from memory) and lists their
+//            meta word, so a pop loads nothing from memory) and lists their
 //            children in shared memory; the warps classify the list's 32-child
 //            chunks in turn, warp w the chunks w, w + W, ...;
 //   evaluate each warp evaluates and votes on its own candidates;
@@ -19,10 +19,17 @@
 // alone (by_team): a batch gives every system the bits of its single run.
 //
 // Bound by latency where the GPU is not full (16384 bodies: 2.9 warps and 0.35
-// instructions per scheduler and cycle), else by issue like walk2.cu, at 9 % more
-// instructions.  Walk at 1000 / 16384 bodies: 38 / 212 us by single warps, 19 / 67
-// us by teams.  Four warps, three chunks: two chunks of rounds with 32 pops took
-// 106 us at 16384, 64 pops 81 us, a child list with 128 pops and three chunks 70.
+// instructions per scheduler and cycle).  Where batches fill it, by issue and the
+// rounds' barriers: every warp pays a round's fixed instructions, and a group takes
+// a block's slots, so that full batches cost more than by single warps: walks of
+// 32768 systems of 256 bodies 2.95 against 1.55 ms (those go by single warps,
+// by_team), 8388 of 1000 4.44 / 3.05, 2097 of 4000 6.75 / 5.43, 512 of 16384 10.5 /
+// 9.1.  Walk at 1000 / 16384 bodies: 38 / 212 us by single warps, 19 / 67 us by
+// teams.  Four warps, three chunks: two chunks of rounds with 32 pops took 106 us
+// at 16384, 64 pops 81 us, a child list with 128 pops and three chunks 70.  Two
+// warps that take two shares each, for full batches, gained 7 % at 512 bodies and
+// lost 8 % from 2000; the kernel is near what the instruction cache holds (votes
+// unrolled by eight: 11.8 ms for 512 systems of 16384).
 #include <type_traits>
 
 #include "nbx_internal.cuh"
@@ -57,8 +64,8 @@ struct alignas(16) TeamBuf {
     Slots<kSlots> b;
     Slots<Quad ? kSlots : 4> c;  // quadrupole mode: cells
     float cd[kSlots];            // cells to vote on: opening thresholds
-    u64 crec[kSlots];            // their stack entries
-    u64 rej[32 * kChunks];       // rejected cells' stack entries
+    int crec[kSlots];            // their stack entries
+    int rej[32 * kChunks];       // rejected cells' stack entries
     TeamIds<Rec> ids;
     // slot of the i-th cell to vote on
     __device__ static int vote_slot(int i) { return Quad ? i : slot_down<kSlots>(i); }
@@ -83,7 +90,7 @@ struct alignas(16) TeamShared {
     int sum[kW][2];     // list length, opened cells
     int P, T;           // the round's popped cells and children
     int pad[2];
-    u64 child[kRound];  // the round's children: node, level of its parent
+    int child[kRound];  // the round's children
 };
 
 static_assert(sizeof(TeamShared) % 16 == 0 && sizeof(TeamBuf<false, false>) % 16 == 0 &&
@@ -102,13 +109,11 @@ __device__ __forceinline__ float warp_max(float v) {
     return r;
 }
 
-__device__ __forceinline__ u64 entry_of(int cm, int lvl) { return (u64)(unsigned)cm | (u64)(unsigned)lvl << 32; }
-
 template <int Mode, bool Pot, bool Rec, bool Quad>
 __global__ void __launch_bounds__(kW * 32, 32 / kW)
-    k_walk_team(const float4 *__restrict__ node4, const int *__restrict__ meta, const float4 *__restrict__ quad4,
-                const float2 *__restrict__ quad2, const float4 *__restrict__ body4, const int *__restrict__ val,
-                const int *__restrict__ groups, const int *__restrict__ list, int g_first,
+    k_walk_team(const float4 *__restrict__ node4, const int *__restrict__ meta, const unsigned char *__restrict__ lvl8,
+                const float4 *__restrict__ quad4, const float2 *__restrict__ quad2, const float4 *__restrict__ body4,
+                const int *__restrict__ val, const int *__restrict__ groups, const int *__restrict__ list, int g_first,
                 const int *__restrict__ body_sys, const int *__restrict__ sys_off, const float *__restrict__ depth0,
                 const int *__restrict__ root_first, const int *__restrict__ root_nch, const int *__restrict__ sys_lvl,
                 float eps2, int stack_cap, float *__restrict__ ax, float *__restrict__ ay, float *__restrict__ az,
@@ -127,7 +132,8 @@ __global__ void __launch_bounds__(kW * 32, 32 / kW)
     const auto part = [&](int v) -> TeamPart & { return *reinterpret_cast<TeamPart *>(&bufs[v]); };
     QuadBuf<kSlots> &qbuf =
         reinterpret_cast<QuadBuf<kSlots> *>(smem_raw + sizeof(TeamShared) + kW * sizeof(TeamBuf<Rec, Quad>))[w];
-    u64 *stack = reinterpret_cast<u64 *>(smem_raw + sizeof(TeamShared) + kW * sizeof(TeamBuf<Rec, Quad>) +
+    // the cells' meta words (first child, children - 1): a pop loads nothing from memory
+    int *stack = reinterpret_cast<int *>(smem_raw + sizeof(TeamShared) + kW * sizeof(TeamBuf<Rec, Quad>) +
                                          (Quad ? kW * sizeof(QuadBuf<kSlots>) : 0));
     const unsigned lt = (1u << lane) - 1u;
     const u64 eps2x2 = pk(eps2, eps2);
@@ -194,7 +200,7 @@ __global__ void __launch_bounds__(kW * 32, 32 / kW)
                 buf.b.put(__popc(bodies & lt), q);
                 if constexpr (Rec) buf.ids.bid[__popc(bodies & lt)] = rf + lane;
             }
-            if (lane < rn && cm >= 0) stack[__popc(cells & lt)] = entry_of(cm, 1);
+            if (lane < rn && cm >= 0) stack[__popc(cells & lt)] = cm;
             nb = __popc(bodies);
             opened += __popc(cells);
         }
@@ -214,14 +220,14 @@ __global__ void __launch_bounds__(kW * 32, 32 / kW)
             const int avail = min(top, 32 * kPops);
             const auto pop = [&](auto entries) {
                 constexpr int K = decltype(entries)::value;
-                u64 e[K];
+                int e[K];
                 int n[K], x[K + 1];
                 x[0] = 0;
 #pragma unroll
                 for (int i = 0; i < K; i++) {
                     const int at = K * lane + i;
-                    e[i] = at < avail ? stack[top - 1 - at] : 0ull;
-                    n[i] = at < avail ? (((int)(unsigned)e[i] >> 28) & 7) + 1 : 0;
+                    e[i] = at < avail ? stack[top - 1 - at] : 0;
+                    n[i] = at < avail ? ((e[i] >> 28) & 7) + 1 : 0;
                     x[i + 1] = x[i] + n[i];
                 }
                 int incl = x[K];
@@ -254,11 +260,10 @@ __global__ void __launch_bounds__(kW * 32, 32 / kW)
 #pragma unroll
                 for (int i = 0; i < K; i++)
                     if (K * lane + i < P) {
-                        const int first = (int)(unsigned)e[i] & 0x0fffffff, at = excl + x[i];
-                        const u64 lvl = e[i] & 0xffffffff00000000ull;
+                        const int first = e[i] & 0x0fffffff, at = excl + x[i];
 #pragma unroll
                         for (int k = 0; k < 8; k++)
-                            if (k < n[i]) sh.child[at + k] = lvl | (unsigned)(first + k);
+                            if (k < n[i]) sh.child[at + k] = first + k;
                     }
             };
             if (avail <= 32) pop(std::integral_constant<int, 1>());
@@ -279,10 +284,8 @@ __global__ void __launch_bounds__(kW * 32, 32 / kW)
             if (32 * c0 >= T) break;
             const int t = 32 * c0 + lane;
             const bool ok = t < T;
-            const u64 ch = sh.child[ok ? t : 0];
-            const int c = (int)(unsigned)ch, lvp = (int)(ch >> 32);
-            const float dpc = scale4(d0, lvp);  // the child's opening threshold, depth0 * 4^-level(popped cell)
-            const int lvc = lvp + 1;
+            const int c = sh.child[ok ? t : 0];
+            const float dpc = scale4(d0, (int)lvl8[c] - 1);  // its opening threshold, depth0 * 4^-level(popped cell)
             const int cm = ok ? meta[c] : 0;
             const float4 q = ok ? node4[c] : make_float4(0.f, 0.f, 0.f, 0.f);
             const bool isc = ok && cm >= 0;
@@ -336,10 +339,10 @@ __global__ void __launch_bounds__(kW * 32, 32 / kW)
                     putq(qbuf.qa, qbuf.qb, qbuf.qc, vslot, qq4, qq2);
                 }
                 buf.cd[vslot] = dpc;
-                buf.crec[vslot] = entry_of(cm, lvc);
+                buf.crec[vslot] = cm;
                 if constexpr (Rec) buf.ids.cid[vslot] = c;
             }
-            if (tos) buf.rej[nrej + __popc(smk & lt)] = entry_of(cm, lvc);
+            if (tos) buf.rej[nrej + __popc(smk & lt)] = cm;
             nbody += __popc(bm);
             ncell += __popc(cmk);
             nrej += __popc(smk);
@@ -580,7 +583,7 @@ __global__ void __launch_bounds__(kW * 32, 32 / kW)
 template <bool Rec, bool Quad>
 size_t team_smem(int stack_depth) {
     return sizeof(TeamShared) + kW * (sizeof(TeamBuf<Rec, Quad>) + (Quad ? sizeof(QuadBuf<kSlots>) : 0)) +
-           (size_t)kStackMul * stack_depth * sizeof(u64);
+           (size_t)kStackMul * stack_depth * sizeof(int);
 }
 
 template <int Mode, bool Pot, bool Rec, bool Quad>
@@ -596,7 +599,7 @@ int launch_team(Ctx *ctx, const nbx_state *s, float *pot, cudaStream_t st, const
         NBX_CUDA(cudaFuncSetAttribute(k_walk_team<Mode, Pot, Rec, Quad>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       ctx->smem_optin));
     launch_chained(ctx, st, count, kW * 32, smem, k_walk_team<Mode, Pot, Rec, Quad>, ctx->d_node4, ctx->d_meta,
-                   ctx->d_quad4, ctx->d_quad2, ctx->d_body4, ctx->d_val, ctx->d_groups, list, first, ctx->d_body_sys,
+                   ctx->d_lvl8, ctx->d_quad4, ctx->d_quad2, ctx->d_body4, ctx->d_val, ctx->d_groups, list, first, ctx->d_body_sys,
                    ctx->d_sys_off, ctx->d_depth0, ctx->d_root_first, ctx->d_root_nch, ctx->d_sys_lvl, ctx->eps2,
                    kStackMul * ctx->p.stack_depth, s->ax, s->ay, s->az, pot, ctx->d_gstat, ctx->d_status, rec_list,
                    rec_len, rec_cap);
