@@ -18,10 +18,13 @@
 //            buffer pairs go straight to the accumulation; each cell of the cell
 //            buffer takes one warp vote (dp <= r on every lane) and is
 //            accumulated or pushed.
-// Wide rounds run while the stack keeps a depth-first reserve free (7 entries
-// per level of the group's system's deepest level); beyond that the walk pops
-// one cell per round, which can never outgrow the reserve, so a stack of at
-// least kDfsReserve + 7*8 entries cannot overflow (NBX_ERR_STACK otherwise).
+// A round pops as many cells as leave a depth-first reserve free on the stack (7
+// entries per level of the group's system's deepest level), and one where none do:
+// that can never outgrow the reserve, so a stack of at least kDfsReserve + 7*8
+// entries cannot overflow (NBX_ERR_STACK otherwise).  (Rounds near the reserve
+// popped one cell each before, whatever room was left, which opening angles below
+// 0.25 ran into all the time: 2^20 bodies at 0.1375 37.8 -> 33.3 ms, 131071 with a
+// stack of 384 9.6 -> 4.3.)
 //
 // Accumulation modes: 0 plain FP32 (two packed partial sums), 1 split
 // compensation (plain FP32 within a round, Kahan across rounds), 2 Kahan on
@@ -223,9 +226,10 @@ __global__ void __launch_bounds__(WalkShape<V, Mode, Quad>::kThreads, WalkShape<
 
         while (top > 0 || nb > 0) {
             // ---- expand: lane j pops stack[top-1-j] and copies its children
-            // wide rounds while the stack keeps the depth-first reserve free,
-            // else one cell per round (depth-first), which cannot outgrow it
-            // P = the most top-of-stack cells whose children fit the buffers
+            // P = the most top-of-stack cells whose children fit the buffers and, if
+            // all were pushed, would leave the depth-first reserve free (P cells grow
+            // the stack by at most T - P, which grows with P); where not even one
+            // does, one cell per round (depth-first), which cannot outgrow the reserve
             const int avail = min(top, 32);
             int first = 0, nch = 0;
             float dpp = 0.f;  // the children's opening threshold, depth0 * 4^-level(popped cell)
@@ -246,14 +250,10 @@ __global__ void __launch_bounds__(WalkShape<V, Mode, Quad>::kThreads, WalkShape<
             const int cbase = first - excl;  // child t of this lane's cell is node cbase + t
             // (the quadrupole mode keeps one slot free: its two cell regions are
             // padded to whole pairs independently)
-            int P = __popc(__ballot_sync(0xffffffffu, lane < avail && incl <= kCB - nb - (Quad ? 1 : 0)));
+            int P = __popc(__ballot_sync(0xffffffffu, lane < avail && incl <= kCB - nb - (Quad ? 1 : 0) &&
+                                                          top + incl - lane - 1 <= stack_cap - reserve));
+            if (P == 0 && avail > 0) P = 1;
             int T = __shfl_sync(0xffffffffu, incl, (P + 31) & 31);
-            // the stack grows by at most T - P: wide rounds only while that keeps
-            // the depth-first reserve free, else one cell
-            if (P > 1 && top - P + T > stack_cap - reserve) {
-                P = 1;
-                T = __shfl_sync(0xffffffffu, incl, 0);
-            }
             if (P > 0 && top - P + T > stack_cap) P = 0;
             if (P == 0) T = 0;
             if (P == 0 && nb == 0) {

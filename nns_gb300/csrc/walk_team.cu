@@ -246,10 +246,19 @@ __global__ void __launch_bounds__(kW * 32, 32 / kW)
                     }
                 int P = __reduce_add_sync(0xffffffffu, np);
                 int T = __reduce_max_sync(0xffffffffu, nt);
-                // wide rounds only while the stack keeps the depth-first reserve free (walk2.cu)
+                // only cells that leave the depth-first reserve free, else one (walk2.cu)
                 if (P > 1 && top - P + T > stack_cap - reserve) {
-                    P = 1;
-                    T = __shfl_sync(0xffffffffu, n[0], 0);
+                    np = nt = 0;
+#pragma unroll
+                    for (int i = 0; i < K; i++) {
+                        const int t = excl + x[i + 1], popped = K * lane + i + 1;
+                        if (popped <= P && top - popped + t <= stack_cap - reserve) {
+                            np = i + 1;
+                            nt = t;
+                        }
+                    }
+                    P = max(__reduce_add_sync(0xffffffffu, np), 1);
+                    T = max(__reduce_max_sync(0xffffffffu, nt), __shfl_sync(0xffffffffu, n[0], 0));
                 }
                 if (P > 0 && top - P + T > stack_cap) P = 0;
                 if (P == 0) T = 0;

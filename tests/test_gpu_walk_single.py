@@ -197,3 +197,37 @@ def test_the_adjoint_records_this_walk(cuda):
     for u in random_directions(n, 4):
         fd = (adj.replay_fp64(dev(base + h * u)) - adj.replay_fp64(dev(base - h * u))) / (2 * h)
         assert abs(fd - float((g * u).sum())) <= 1e-4 * gnorm
+
+
+@pytest.mark.parametrize("n", [4000, 20011, 60000])
+@pytest.mark.parametrize("stack_depth", [360, 384, 512])
+@pytest.mark.parametrize("kw", [{}, {"compensated": 1}, {"multipole": 1}], ids=["plain", "split", "quad"])
+def test_small_opening_angles_fill_the_stack(cuda, n, stack_depth, kw):
+    """theta = 0.1375 opens most cells, so the stack fills to its depth-first reserve and
+    rounds pop what room is left: the oracle's lists with any stack, and never more
+    than two and a half times the rounds of a stack that always has room (one cell a
+    round near the reserve took ten times as many)."""
+    from nns_gb300.barnes_hut import Context, State
+    key = ("theta", n, kw.get("multipole", 0))
+    e = np.float32(0.005)
+    if key not in _cache:
+        b = ic.plummer(n)
+        t = O.build(b.x, b.y, b.z, b.m)
+        q = O.quadrupoles(b.x, b.y, b.z, b.m, t) if key[2] else None
+        th = np.float32(0.1375)
+        _cache[key] = b, O.forces(b.x, b.y, b.z, b.m, t, float(th * th), float(e * e), quad=q)
+    b, f = _cache[key]
+    rounds = []
+    for depth in (stack_depth, 2048):
+        ctx = Context(max_bodies=n, theta=0.1375, eps=0.005, stack_depth=depth, **kw)
+        ctx.set_systems([0, n])
+        s = State.from_bodies(b)
+        ctx.build(s)
+        ctx.forces(s)
+        ctx.sync()
+        nl, no = ctx.walk_stats()
+        assert np.array_equal(nl, f.nlist) and np.array_equal(no, f.nopen)
+        rel = _rel(s.acc(), f.a64)
+        assert np.median(rel) <= MED_TOL and rel.max() <= MAX_TOL, depth
+        rounds.append(ctx.tree_info()["rounds"])
+    assert rounds[0] <= 2.5 * rounds[1], rounds
