@@ -88,7 +88,7 @@ constexpr int kSweepMaxBodies = NBX_RADIX_SWEEP_MAX;
 inline bool by_team(int bodies) { return bodies >= NBX_TEAM_MIN && bodies <= NBX_TEAM_MAX; }
 // Revision of the walks' order of summation, which checkpoints store: raised by every
 // change after which the same bodies and settings give other force bits.  (1: teams,
-// rounds of 128 children in the default single-warp walk.)
+// rounds of 128 children in the default single-warp walk, sums folded per round.)
 constexpr int kWalkRevision = 1;
 constexpr int kMaxRadixBits = 9;  // body-key digits: 8 or 9 bits (histograms sized for 9)
 // LSD passes over the 63-bit body keys for a digit width

@@ -26,9 +26,10 @@
 // 0.25 ran into all the time: 2^20 bodies at 0.1375 37.8 -> 33.3 ms, 131071 with a
 // stack of 384 9.6 -> 4.3.)
 //
-// Accumulation modes: 0 plain FP32 (two packed partial sums), 1 split
-// compensation (plain FP32 within a round, Kahan across rounds), 2 Kahan on
-// every term.  Optional per-body potential for the energy diagnostics.
+// Accumulation modes: 0 plain FP32 (two packed partial sums per round, added to two
+// packed totals), 1 split compensation (plain FP32 within a round, Kahan across
+// rounds), 2 Kahan on every term.  Optional per-body potential for the energy
+// diagnostics.
 #include <algorithm>
 
 #include "nbx_internal.cuh"
@@ -72,7 +73,7 @@ constexpr int kCellUnroll = NBX_CELL_UNROLL;
 // quadrupoles, the surely accepted cells) fill the slots upwards and the cells to
 // vote on downwards, so one masked store serves both; with quadrupoles the cells
 // have slots of their own.  (Four slots more: each side pads to a whole pair.)
-template <int CB, bool Rec, bool Quad>
+template <int CB, int Mode, bool Pot, bool Rec, bool Quad>
 struct WarpBuf {
     Slots<CB + 4> b;
     Slots<Quad ? CB : 4> c; // quadrupole mode: cells
@@ -82,6 +83,7 @@ struct WarpBuf {
     float4 cls[3];          // group box lo, hi, centre
     ulonglong2 rxy[8];      // representative bodies, in pairs: (x0,x1) (y0,y1)
     u64 rz[8];              //                                  (z0,z1)
+    Totals<Mode, Pot> tot;
 };
 
 // The buffer variants: children per round and register budget.  0: 64 children;
@@ -117,7 +119,7 @@ __global__ void __launch_bounds__(WalkShape<V, Mode, Quad>::kThreads, WalkShape<
     const int warps = blockDim.x >> 5;
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     constexpr int CB = WalkShape<V, Mode, Quad>::kSlots, kCB = CB;
-    using Buf = WarpBuf<CB, Rec, Quad>;
+    using Buf = WarpBuf<CB, Mode, Pot, Rec, Quad>;
     Buf &buf = reinterpret_cast<Buf *>(smem_raw)[w];
     constexpr size_t kQuadBytes = Quad ? sizeof(QuadBuf<CB>) : 0;
     QuadBuf<CB> &qbuf = reinterpret_cast<QuadBuf<CB> *>(smem_raw + sizeof(Buf) * warps)[w];
@@ -198,6 +200,7 @@ __global__ void __launch_bounds__(WalkShape<V, Mode, Quad>::kThreads, WalkShape<
             __syncwarp();
         }
         Sums acc;
+        clear_totals(buf.tot, lane);
         int top = 0, nb = 0, len = 0, opened = 0, nrec = 0;
         bool overflow = false;
         int *rec = Rec ? rec_list + (size_t)g * rec_cap : nullptr;
@@ -468,19 +471,7 @@ __global__ void __launch_bounds__(WalkShape<V, Mode, Quad>::kThreads, WalkShape<
             len += nbody + ncell - nrej + nacc;
             opened += nrej + nsrej;
             nb = 0;
-            if (Mode == 1) {  // fold this round's partial sums into the compensated totals
-                float a0, a1;
-                upk(acc.x, a0, a1);
-                kahan(acc.kx, acc.cx, a0);
-                kahan(acc.kx, acc.cx, a1);
-                upk(acc.y, a0, a1);
-                kahan(acc.ky, acc.cy, a0);
-                kahan(acc.ky, acc.cy, a1);
-                upk(acc.z, a0, a1);
-                kahan(acc.kz, acc.cz, a0);
-                kahan(acc.kz, acc.cz, a1);
-                acc.x = acc.y = acc.z = 0ull;
-            }
+            fold_round(acc, buf.tot, lane);
             __syncwarp();
         }
         if (overflow) {
@@ -493,13 +484,13 @@ __global__ void __launch_bounds__(WalkShape<V, Mode, Quad>::kThreads, WalkShape<
         }
         if (valid) {
             float fx, fy, fz;
-            if (Mode == 0) {
+            if constexpr (Mode == 0) {
                 float a0, a1;
-                upk(acc.x, a0, a1);
+                upk(buf.tot.x[lane], a0, a1);
                 fx = a0 + a1;
-                upk(acc.y, a0, a1);
+                upk(buf.tot.y[lane], a0, a1);
                 fy = a0 + a1;
-                upk(acc.z, a0, a1);
+                upk(buf.tot.z[lane], a0, a1);
                 fz = a0 + a1;
             } else {
                 fx = acc.kx - acc.cx;
@@ -510,9 +501,9 @@ __global__ void __launch_bounds__(WalkShape<V, Mode, Quad>::kThreads, WalkShape<
             ax[ob] = fx;
             ay[ob] = fy;
             az[ob] = fz;
-            if (Pot) {
+            if constexpr (Pot) {
                 float a0, a1;
-                upk(acc.p, a0, a1);
+                upk(buf.tot.p[lane], a0, a1);
                 // remove the body's own term m * rsqrt(eps2), then phi = -sum
                 pot[ob] = -((a0 + a1) - me.w * rsq(eps2));
             }
@@ -546,10 +537,12 @@ template <int V, int Mode, bool Pot, bool Rec = false, bool Quad = false>
 int launch(Ctx *ctx, const nbx_state *s, float *pot, int warps, cudaStream_t st, Share share,
            int *rec_list = nullptr, int *rec_len = nullptr, int rec_cap = 0) {
     constexpr int kCB = WalkShape<V, Mode, Quad>::kSlots;
-    const int cap = ctx->p.stack_depth, asked = warps;
-    const size_t smem = (size_t)warps * (sizeof(WarpBuf<kCB, Rec, Quad>) + (Quad ? sizeof(QuadBuf<kCB>) : 0) +
-                                         (size_t)cap * sizeof(int));
-    if (smem > (size_t)ctx->smem_optin) {
+    const int cap = ctx->p.stack_depth;
+    const size_t per_warp = sizeof(WarpBuf<kCB, Mode, Pot, Rec, Quad>) + (Quad ? sizeof(QuadBuf<kCB>) : 0) +
+                            (size_t)cap * sizeof(int);
+    // (the rounds' totals came later: a shape that fits without them goes out in
+    // blocks that do, below)
+    if ((size_t)warps * (per_warp - sizeof(Totals<Mode, Pot>)) > (size_t)ctx->smem_optin) {
         ctx->last_error = "walk: stack_depth too large for the launch shape's shared memory";
         return NBX_ERR_ARG;
     }
@@ -557,7 +550,8 @@ int launch(Ctx *ctx, const nbx_state *s, float *pot, int warps, cudaStream_t st,
     // groups that all fit the GPU at once go out in small blocks, which spread
     // evenly over the SMs (the sums do not depend on the shape)
     if (share.count <= kSpreadWarps * ctx->nsm && warps > kSpreadBlock) warps = kSpreadBlock;
-    const size_t block_smem = smem / asked * warps;
+    while (warps > 1 && warps * per_warp > (size_t)ctx->smem_optin) warps >>= 1;
+    const size_t block_smem = warps * per_warp;
     const int blocks_needed = ceil_div(share.count, warps);
     int per_sm = 1;
     NBX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_walk2<V, Mode, Pot, Rec, Quad>, warps * 32,

@@ -59,7 +59,7 @@ struct TeamIds<false> {};
 // accepted cells) fill the slots upwards, the cells to vote on downwards in
 // pairs; with quadrupoles the cells are in the second arrays, those to vote on
 // upwards, the surely accepted ones downwards.
-template <bool Rec, bool Quad>
+template <int Mode, bool Pot, bool Rec, bool Quad>
 struct alignas(16) TeamBuf {
     Slots<kSlots> b;
     Slots<Quad ? kSlots : 4> c;  // quadrupole mode: cells
@@ -67,6 +67,7 @@ struct alignas(16) TeamBuf {
     int crec[kSlots];            // their stack entries
     int rej[32 * kChunks];       // rejected cells' stack entries
     TeamIds<Rec> ids;
+    Totals<Mode, Pot> tot;
     // slot of the i-th cell to vote on
     __device__ static int vote_slot(int i) { return Quad ? i : slot_down<kSlots>(i); }
     __device__ Slots<kSlots> &cells() {
@@ -80,7 +81,7 @@ struct TeamPart {
     float a[6][32];  // sums and their compensations
     float pot[32];
 };
-static_assert(sizeof(TeamPart) <= sizeof(TeamBuf<false, false>), "the partial results replace the buffers");
+static_assert(sizeof(TeamPart) <= sizeof(TeamBuf<1, false, false, false>), "the partial results replace the buffers");
 
 struct alignas(16) TeamShared {
     float4 cls[3];      // group box lo, hi, centre
@@ -93,8 +94,8 @@ struct alignas(16) TeamShared {
     int child[kRound];  // the round's children
 };
 
-static_assert(sizeof(TeamShared) % 16 == 0 && sizeof(TeamBuf<false, false>) % 16 == 0 &&
-                  sizeof(TeamBuf<true, false>) % 16 == 0 && sizeof(TeamBuf<false, true>) % 16 == 0,
+static_assert(sizeof(TeamShared) % 16 == 0 && sizeof(TeamBuf<1, false, false, false>) % 16 == 0 &&
+                  sizeof(TeamBuf<0, false, true, false>) % 16 == 0 && sizeof(TeamBuf<0, false, false, true>) % 16 == 0,
               "16-byte slots");
 
 // Minimum and maximum over a warp of finite values (one instruction each).
@@ -127,13 +128,13 @@ __global__ void __launch_bounds__(kW * 32, 32 / kW)
     if (__syncthreads_or(st->code != 0)) return;
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     TeamShared &sh = *reinterpret_cast<TeamShared *>(smem_raw);
-    TeamBuf<Rec, Quad> *bufs = reinterpret_cast<TeamBuf<Rec, Quad> *>(smem_raw + sizeof(TeamShared));
-    TeamBuf<Rec, Quad> &buf = bufs[w];
+    TeamBuf<Mode, Pot, Rec, Quad> *bufs = reinterpret_cast<TeamBuf<Mode, Pot, Rec, Quad> *>(smem_raw + sizeof(TeamShared));
+    TeamBuf<Mode, Pot, Rec, Quad> &buf = bufs[w];
     const auto part = [&](int v) -> TeamPart & { return *reinterpret_cast<TeamPart *>(&bufs[v]); };
     QuadBuf<kSlots> &qbuf =
-        reinterpret_cast<QuadBuf<kSlots> *>(smem_raw + sizeof(TeamShared) + kW * sizeof(TeamBuf<Rec, Quad>))[w];
+        reinterpret_cast<QuadBuf<kSlots> *>(smem_raw + sizeof(TeamShared) + kW * sizeof(TeamBuf<Mode, Pot, Rec, Quad>))[w];
     // the cells' meta words (first child, children - 1): a pop loads nothing from memory
-    int *stack = reinterpret_cast<int *>(smem_raw + sizeof(TeamShared) + kW * sizeof(TeamBuf<Rec, Quad>) +
+    int *stack = reinterpret_cast<int *>(smem_raw + sizeof(TeamShared) + kW * sizeof(TeamBuf<Mode, Pot, Rec, Quad>) +
                                          (Quad ? kW * sizeof(QuadBuf<kSlots>) : 0));
     const unsigned lt = (1u << lane) - 1u;
     const u64 eps2x2 = pk(eps2, eps2);
@@ -179,6 +180,7 @@ __global__ void __launch_bounds__(kW * 32, 32 / kW)
         }
     }
     Sums acc;
+    clear_totals(buf.tot, lane);
     int top = 0, nb = 0, len = 0, opened = 0, nrec = 0;
     unsigned rounds = 0;
     bool overflow = false;
@@ -475,19 +477,7 @@ __global__ void __launch_bounds__(kW * 32, 32 / kW)
         rounds++;
         len += nbody + ncell - (nrej - nsrej) + nacc;
         opened += nrej;
-        if (Mode == 1) {  // fold this round's partial sums into the compensated totals
-            float a0, a1;
-            upk(acc.x, a0, a1);
-            kahan(acc.kx, acc.cx, a0);
-            kahan(acc.kx, acc.cx, a1);
-            upk(acc.y, a0, a1);
-            kahan(acc.ky, acc.cy, a0);
-            kahan(acc.ky, acc.cy, a1);
-            upk(acc.z, a0, a1);
-            kahan(acc.kz, acc.cz, a0);
-            kahan(acc.kz, acc.cz, a1);
-            acc.x = acc.y = acc.z = 0ull;
-        }
+        fold_round(acc, buf.tot, lane);
         // ---- push: the warps' rejected cells, in warp order
         if (lane == 0) {
             reinterpret_cast<int *>(&sh.nrej)[w] = nrej;
@@ -516,29 +506,27 @@ __global__ void __launch_bounds__(kW * 32, 32 / kW)
         if (threadIdx.x == 0) set_status(st, NBX_ERR_STACK, g);
         return;
     }
-    // ---- the warps' partial sums, added in warp order
+    // ---- the warps' partial sums, added in warp order (this warp's totals leave its
+    // buffers before its results overwrite them)
+    float res[6] = {acc.kx, acc.ky, acc.kz, acc.cx, acc.cy, acc.cz}, res_p = 0.f;
+    if constexpr (Mode == 0) {
+        float a0, a1;
+        upk(buf.tot.x[lane], a0, a1);
+        res[0] = a0 + a1;
+        upk(buf.tot.y[lane], a0, a1);
+        res[1] = a0 + a1;
+        upk(buf.tot.z[lane], a0, a1);
+        res[2] = a0 + a1;
+        if constexpr (Pot) {
+            upk(buf.tot.p[lane], a0, a1);
+            res_p = a0 + a1;
+        }
+    }
+    __syncwarp();
     TeamPart &mine = part(w);
-    if (Mode == 0) {
-        float a0, a1;
-        upk(acc.x, a0, a1);
-        mine.a[0][lane] = a0 + a1;
-        upk(acc.y, a0, a1);
-        mine.a[1][lane] = a0 + a1;
-        upk(acc.z, a0, a1);
-        mine.a[2][lane] = a0 + a1;
-    } else {
-        mine.a[0][lane] = acc.kx;
-        mine.a[1][lane] = acc.ky;
-        mine.a[2][lane] = acc.kz;
-        mine.a[3][lane] = acc.cx;
-        mine.a[4][lane] = acc.cy;
-        mine.a[5][lane] = acc.cz;
-    }
-    if (Pot) {
-        float a0, a1;
-        upk(acc.p, a0, a1);
-        mine.pot[lane] = a0 + a1;
-    }
+#pragma unroll
+    for (int k = 0; k < (Mode == 0 ? 3 : 6); k++) mine.a[k][lane] = res[k];
+    if (Pot) mine.pot[lane] = res_p;
     if (lane == 0) {
         sh.sum[w][0] = len;
         sh.sum[w][1] = opened;
@@ -589,16 +577,16 @@ __global__ void __launch_bounds__(kW * 32, 32 / kW)
     }
 }
 
-template <bool Rec, bool Quad>
+template <int Mode, bool Pot, bool Rec, bool Quad>
 size_t team_smem(int stack_depth) {
-    return sizeof(TeamShared) + kW * (sizeof(TeamBuf<Rec, Quad>) + (Quad ? sizeof(QuadBuf<kSlots>) : 0)) +
+    return sizeof(TeamShared) + kW * (sizeof(TeamBuf<Mode, Pot, Rec, Quad>) + (Quad ? sizeof(QuadBuf<kSlots>) : 0)) +
            (size_t)kStackMul * stack_depth * sizeof(int);
 }
 
 template <int Mode, bool Pot, bool Rec, bool Quad>
 int launch_team(Ctx *ctx, const nbx_state *s, float *pot, cudaStream_t st, const int *list, int first, int count,
                 int *rec_list, int *rec_len, int rec_cap) {
-    const size_t smem = team_smem<Rec, Quad>(ctx->p.stack_depth);
+    const size_t smem = team_smem<Mode, Pot, Rec, Quad>(ctx->p.stack_depth);
     if (smem > (size_t)ctx->smem_optin) {
         ctx->last_error = "walk: stack_depth too large for the launch shape's shared memory";
         return NBX_ERR_ARG;

@@ -231,3 +231,40 @@ def test_small_opening_angles_fill_the_stack(cuda, n, stack_depth, kw):
         assert np.median(rel) <= MED_TOL and rel.max() <= MAX_TOL, depth
         rounds.append(ctx.tree_info()["rounds"])
     assert rounds[0] <= 2.5 * rounds[1], rounds
+
+
+@pytest.mark.parametrize("name", ["star_disk", "binary_disk", "plummer"])
+@pytest.mark.parametrize("n,bound", [(5003, 2.5e-7), (16384, 2.5e-7), (131071, 3.5e-7)])
+def test_plain_sums_keep_their_precision(cuda, name, n, bound):
+    """The plain FP32 sums against FP64 sums of the same lists.  Every body's rounding
+    is that of its own round's terms and one sum per round: with about 20 rounds of
+    64 adds in two halves, r.m.s. below 2^-24 sqrt(20 + 32) = 4.3e-7, as the largest
+    term is rarely most of the force below 3.5e-7, by teams (four sums, 10 rounds of
+    up to 48) below 2.5e-7.  (One running sum had 0.7e-6 to 2.2e-6 on the disks.)"""
+    from nns_gb300.barnes_hut import Context, State
+    b = getattr(ic, name)(n)
+    ctx, s = _walk(b)
+    tg = np.arange(0, n, max(1, n // 8000))
+    a, w = s.acc()[tg].astype(np.float64), ctx.forces_fp64_lists(tg)
+    e = _rel(a, w)
+    assert np.sqrt(np.mean(e * e)) <= bound
+
+
+@pytest.mark.parametrize("warps", [4, 8, 16])
+@pytest.mark.parametrize("stack_depth", [1824, 1940, 2016])
+def test_deep_stacks_fit_as_before(cuda, warps, stack_depth):
+    """Stacks that just fitted a launch shape before the rounds' totals took shared
+    memory of their own go out in smaller blocks, with the same bits."""
+    from nns_gb300.barnes_hut import Context, State
+    b = ic.plummer(160033)
+    acc = []
+    for w in (warps, 4):
+        ctx = Context(max_bodies=len(b.x), theta=0.5, eps=0.01, multipole=1, stack_depth=stack_depth)
+        ctx.set_walk(w, 3)
+        ctx.set_systems([0, len(b.x)])
+        s = State.from_bodies(b)
+        ctx.build(s)
+        ctx.forces(s)
+        ctx.sync()
+        acc.append(s.acc())
+    assert np.array_equal(acc[0], acc[1])
