@@ -481,13 +481,16 @@ int nbx_set_systems(nbx_ctx *c, int nsys, const int64_t *offsets) {
     // the one-sweep sort's tiling: its passes are bound by the look-back chains
     // between a system's tiles, so its tiles are at least kTileSweep keys
     const int tile_sw = tile > nbx::kTileSweep ? tile : (nbx::kTileSweep < nbx::kTile ? nbx::kTileSweep : nbx::kTile);
-    int max_sys = 0, nteam = 0, ngroups = 0;
+    int max_sys = 0, nteam = 0, nteam_sys = 0, ngroups = 0;
     const auto bodies = [&](int s) { return (int)(offsets[s + 1] - offsets[s]); };
     for (int s = 0; s < nsys; s++) {
         max_sys = max_sys > bodies(s) ? max_sys : bodies(s);
         const int g = nbx::ceil_div(bodies(s), 32);
         ngroups += g;
-        if (nbx::by_team(bodies(s))) nteam += g;
+        if (nbx::by_team(bodies(s))) {
+            nteam += g;
+            nteam_sys++;
+        }
     }
     // only the lists that this batch's sort and walks read are made
     const bool merge = nbx::sorts_by_merging(max_sys, n), sweep = !merge && n < nbx::kSweepMaxBodies;
@@ -587,6 +590,7 @@ int nbx_set_systems(nbx_ctx *c, int nsys, const int64_t *offsets) {
     ctx->nsmall_mg = nsmall_mg;
     ctx->max_sys = max_sys;
     ctx->nteam = nteam;
+    ctx->nteam_sys = nteam_sys;
     ctx->h_team = std::move(team);
     ctx->h_solo = std::move(solo);
     ctx->tile_body = tile;

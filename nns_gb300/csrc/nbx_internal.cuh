@@ -164,7 +164,7 @@ struct Ctx {
 
     // walk groups that are walked by teams (by_team): their number, and in a batch of
     // both kinds the groups of each, ascending
-    int nteam = 0;
+    int nteam = 0, nteam_sys = 0;  // (and their systems)
     std::vector<int> h_team, h_solo;
     int *d_team = nullptr, *d_solo = nullptr;  // [G] together
 
