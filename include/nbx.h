@@ -286,7 +286,8 @@ int nbx_direct_fp64(nbx_ctx *ctx, const float *x, const float *y, const float *z
 int nbx_forces_fp64_lists(nbx_ctx *ctx, const int *group_starts, int ngroups, double *acc,
                           void *stream);
 /* Per-body potential phi_i = -sum_j m_j / sqrt(|d|^2+eps2) over the walk's
- * interaction lists (self term removed), original index order; needs eps2 > 0. */
+ * interaction lists (self term removed), original index order; needs eps2 > 0.
+ * The walk stores the accelerations too (s->ax, s->ay, s->az). */
 int nbx_potential(nbx_ctx *ctx, const nbx_state *s, float *phi, void *stream);
 /* ---- differentiation (no counterpart in the reference) -------------------
  * Gradients of L = sum_i |x_i(T) - x*_i|^2 after T kick-drift steps with

@@ -73,8 +73,9 @@ constexpr int kSweepMaxBodies = NBX_RADIX_SWEEP_MAX;
 // gives every system the bits of its single run.  Alone, teams win up to about 2^17
 // bodies (walk at 2^16: 148 against 193 us, at 2^17 240 against 305); in a batch
 // that fills the GPU they cost more than single warps (400 systems of 2^11 to 2^16
-// bodies, walk 11.2 against 10.0 ms), which outweighs what the build gained once
-// large systems are in.  At 2^14 a system alone gains most (70 against 212 us).
+// bodies, walk 11.2 against 10.0 ms; by one warp in a team's stead, walk_team.cu,
+// less), which outweighs what the build gained once large systems are in.  At 2^14 a
+// system alone gains most (70 against 212 us).
 // Systems of up to 256 bodies have a few rounds of a few cells: alone they take
 // about as long either way (a step of 256 bodies 58 us by single warps, 54 by
 // teams), and a full batch takes a fraction (65536 systems of 128 bodies, walk 1.04
