@@ -150,7 +150,7 @@ __device__ __forceinline__ void team_sync() {
 
 // kN warps walk a group: kW, one for each share of a round, or one that takes the
 // shares in turn (the same sums: the same bits).
-// With quadrupoles four warps' slots leave seven blocks an SM: 72 registers, no spills
+// With quadrupoles four warps' slots leave seven blocks an SM: 72 registers, hardly a spill
 // (walk of 6000 / 12000 / 16384 bodies 54.3 / 83.2 / 91.1 us with 64, 51.4 / 78.0 / 85.7).
 template <int kN, int Mode, bool Pot, bool Rec, bool Quad>
 __global__ void __launch_bounds__(kN * 32, (Quad && kN > 1 ? 28 : 32) / kN)
@@ -660,6 +660,11 @@ int launch_warps(Ctx *ctx, const nbx_state *s, float *pot, cudaStream_t st, cons
     if (smem > 48 * 1024)
         NBX_CUDA(cudaFuncSetAttribute(k_walk_team<kN, Mode, Pot, Rec, Quad>,
                                       cudaFuncAttributeMaxDynamicSharedMemorySize, ctx->smem_optin));
+    // in plain stream order, as the walk by single warps: blocks placed while the build's
+    // last kernel holds some of the SMs fill the others (eager steps of 1000 / 6000 /
+    // 16000 bodies 66 / 110 / 149 us chained, 61 / 100 / 129 not; with quadrupoles 99 /
+    // 168 / 215 and 94 / 154 / 192)
+    ctx->chain = false;
     launch_chained(ctx, st, count, kN * 32, smem, k_walk_team<kN, Mode, Pot, Rec, Quad>, ctx->d_node4, ctx->d_meta,
                    ctx->d_lvl8, ctx->d_quad4, ctx->d_quad2, ctx->d_body4, ctx->d_val, ctx->d_groups, list, first,
                    ctx->d_body_sys, ctx->d_sys_off, ctx->d_depth0, ctx->d_root_first, ctx->d_root_nch, ctx->d_sys_lvl,
