@@ -245,7 +245,7 @@ struct Ctx {
         }                                                                   \
     } while (0)
 
-// Kernels of one chain (a build, its walk and its update) are launched so that a
+// Kernels of one chain (a build; a walk, which starts in plain order, and its update) are launched so that a
 // kernel's blocks are set up while its predecessor runs: it waits for the
 // predecessor's completion in grid_dependency(), its first statement.  A launch
 // follows this way only when the stream's last operation is a kernel of the same
